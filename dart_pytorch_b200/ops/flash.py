@@ -164,9 +164,109 @@ class SeparateAttentionFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None, None, None, None, None, None
 
 
+# ------------------------------------------------------------------------------------------------------------ fp32
+class F32View(ctypes.Structure):
+    _fields_ = [("p", c_void_p), ("sb", c_ll), ("ss", c_ll), ("sh", c_ll)]
+
+
+class AttnF32Args(ctypes.Structure):
+    _fields_ = [(n, F32View) for n in ("q", "k", "v", "o", "do", "dq", "dk", "dv")] + \
+        [("lse", c_void_p), ("delta", c_void_p)] + \
+        [(n, c_int) for n in ("B", "Sq", "Sk", "Hq", "Hkv", "hd", "causal", "q_offset")] + \
+        [("scale", c_float), ("backward", c_int)]
+
+
+def _f32_covers(B, Sq, Sk, H, Hkv, hd, q_offset=0) -> bool:
+    """What ``csrc/attention_f32.cu`` takes; the composed path takes the rest."""
+    return 0 < hd <= 128 and B > 0 and Sq > 0 and Sk > 0 and Hkv > 0 and H % Hkv == 0 and q_offset >= 0 and \
+        max(B, H) <= 65535
+
+
+def _f32_rows(t):
+    return t if t.stride(-1) == 1 or t.shape[-1] == 1 else t.contiguous()
+
+
+def attn_f32(q4, k4, v4, o4, causal, q_offset, lse=None, grads=None):
+    """Kernel call on ``[B, S, H, hd]`` views with a contiguous last axis.  Without ``grads`` it writes ``o4`` (and ``lse
+    [B, H, Sq]`` if given); with ``grads = (do, dq, dk, dv)``, views like the operands, it writes the last three."""
+    B, Sq, H, hd = q4.shape
+    a = AttnF32Args()
+    views = (q4, k4, v4, o4) + (grads or ())
+    for name, t in zip(("q", "k", "v", "o", "do", "dq", "dk", "dv"), views):
+        sb, ss, sh, _ = t.stride()
+        setattr(a, name, F32View(t.data_ptr(), sb, ss, sh))
+    delta = torch.empty_like(lse) if grads else None
+    a.lse, a.delta = N.ptr(lse), N.ptr(delta)
+    a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.hd = B, Sq, k4.shape[1], H, k4.shape[2], hd
+    a.causal, a.q_offset, a.scale, a.backward = int(causal), int(q_offset), 1.0 / math.sqrt(hd), int(grads is not None)
+    N.check(N.load().dptb_attn_f32(ctypes.byref(a), N.stream_ptr()), "attn_f32")
+
+
+def _f32_packed_views(x, cfg):
+    B, S, H, Hkv, hd = cfg
+    x4 = x.view(B, S, H + 2 * Hkv, hd)
+    return x4[:, :, :H], x4[:, :, H:H + Hkv], x4[:, :, H + Hkv:]
+
+
+class PackedAttentionF32Fn(torch.autograd.Function):
+    """fp32 ``PackedAttentionFn``."""
+
+    @staticmethod
+    def forward(ctx, qkv, B, S, H, Hkv, hd, causal):
+        qkv = qkv.contiguous()
+        o = torch.empty(B * S, H * hd, dtype=qkv.dtype, device=qkv.device)
+        lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
+        cfg = (B, S, H, Hkv, hd)
+        attn_f32(*_f32_packed_views(qkv, cfg), o.view(B, S, H, hd), causal, 0, lse=lse)
+        ctx.save_for_backward(qkv, o, lse)
+        ctx.cfg, ctx.causal = cfg, causal
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, o, lse = ctx.saved_tensors
+        B, S, H, Hkv, hd = ctx.cfg
+        dqkv = torch.empty_like(qkv)
+        attn_f32(*_f32_packed_views(qkv, ctx.cfg), o.view(B, S, H, hd), ctx.causal, 0, lse=lse,
+                 grads=(do.contiguous().view(B, S, H, hd), *_f32_packed_views(dqkv, ctx.cfg)))
+        return dqkv, None, None, None, None, None, None
+
+
+class AttentionF32Fn(torch.autograd.Function):
+    """fp32 attention of ``[B, S, H, hd]`` views; the output is contiguous in that order."""
+
+    @staticmethod
+    def forward(ctx, q4, k4, v4, causal, q_offset):
+        q4, k4, v4 = _f32_rows(q4), _f32_rows(k4), _f32_rows(v4)
+        B, Sq, H, hd = q4.shape
+        o = torch.empty(B, Sq, H, hd, dtype=q4.dtype, device=q4.device)
+        lse = torch.empty(B, H, Sq, dtype=torch.float32, device=q4.device)
+        attn_f32(q4, k4, v4, o, causal, q_offset, lse=lse)
+        ctx.save_for_backward(q4, k4, v4, o, lse)
+        ctx.cfg = (causal, q_offset)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q4, k4, v4, o, lse = ctx.saved_tensors
+        grads = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q4, k4, v4)]
+        attn_f32(q4, k4, v4, o, *ctx.cfg, lse=lse, grads=(_f32_rows(do), *grads))
+        return (*grads, None, None)
+
+
+def _attention_f32(q4, k4, v4, causal, q_offset):
+    if _wants_grad(q4, k4, v4):
+        return AttentionF32Fn.apply(q4, k4, v4, causal, q_offset)
+    o = torch.empty(q4.shape, dtype=q4.dtype, device=q4.device)
+    attn_f32(_f32_rows(q4), _f32_rows(k4), _f32_rows(v4), o, causal, q_offset)
+    return o
+
+
 def attention_packed(qkv, batch, seq, heads, kv_heads, head_dim, causal=True):
     """Attention over a fused projection output ``[B*S, (H + 2 Hkv) hd]`` -> ``[B*S, H hd]``."""
     d_q, d_kv = heads * head_dim, kv_heads * head_dim
+    if qkv.dtype == torch.float32 and _wants_grad(qkv) and _f32_covers(batch, seq, seq, heads, kv_heads, head_dim):
+        return PackedAttentionF32Fn.apply(qkv, batch, seq, heads, kv_heads, head_dim, causal)
     hd_k = kernel_head_dim(head_dim, backward=_wants_grad(qkv)) if qkv.dtype == torch.bfloat16 else None
     if hd_k == head_dim:
         return PackedAttentionFn.apply(qkv, batch, seq, heads, kv_heads, head_dim, causal)
@@ -179,6 +279,10 @@ def attention_tokens(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causa
     views) -> ``[B*Sq, H hd]``.  bf16 heads of 64 / 128 features run the tensor-core kernels as they are, other sizes
     zero-padded to the next of the two; what the kernels do not cover (see ``kernel_head_dim``) runs the composed path."""
     hd_k = kernel_head_dim(head_dim, backward=_wants_grad(q2, k2, v2)) if q2.dtype == torch.bfloat16 else None
+    if q2.dtype == torch.float32:
+        o = attention_bhsd(_to_bhsd(q2, batch, sq, heads, head_dim), _to_bhsd(k2, batch, sk, kv_heads, head_dim),
+                           _to_bhsd(v2, batch, sk, kv_heads, head_dim), causal, None, q_offset)
+        return o.transpose(1, 2).reshape(batch * sq, heads * head_dim)
     if hd_k is None:
         o = _attention_composed(_to_bhsd(q2, batch, sq, heads, head_dim), _to_bhsd(k2, batch, sk, kv_heads, head_dim),
                                 _to_bhsd(v2, batch, sk, kv_heads, head_dim), causal, None, q_offset)
@@ -193,10 +297,14 @@ def attention_tokens(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causa
 
 def attention_bhsd(q, k, v, causal=False, mask=None, q_offset=0):
     """``[B, H, S, hd]`` operands.  bf16 with a supported head size runs the tensor-core kernel (after a
-    token-major relayout); anything else (fp32, odd head sizes, an additive mask) runs the composed
-    device path: score GEMMs on the SIMT kernel, row softmax kernel."""
+    token-major relayout), fp32 without a mask the fp32 kernels on the operands as they are; anything else (odd head
+    sizes, an additive mask) runs the composed device path: score GEMMs, row softmax kernel."""
     B, H, Sq, hd = q.shape
     Hkv, Sk = k.shape[1], k.shape[2]
+    if q.dtype == torch.float32 and mask is None:
+        if _f32_covers(B, Sq, Sk, H, Hkv, hd, q_offset):
+            q4, k4, v4 = (t.to(q.dtype).transpose(1, 2) for t in (q, k, v))
+            return _attention_f32(q4, k4, v4, causal, q_offset).transpose(1, 2)
     if q.dtype == torch.bfloat16 and mask is None and supported_head_dim(hd, backward=_wants_grad(q, k, v)):
         q2 = q.transpose(1, 2).reshape(B * Sq, H * hd)
         k2 = k.transpose(1, 2).reshape(B * Sk, Hkv * hd)

@@ -1,0 +1,81 @@
+"""fp32 attention kernels against the same formula in fp64: output and gradients, over the edges of their tiles (32 query rows,
+64 keys, 8 rows of a kv head for the split form), grouped queries, offsets, odd head sizes and strides."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from dart_pytorch_b200.ops import flash as A
+
+
+def _exact(q, k, v, causal, off):
+    g = q.shape[1] // k.shape[1]
+    k, v = k.repeat_interleave(g, 1), v.repeat_interleave(g, 1)
+    s = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+    if causal:
+        i = torch.arange(q.shape[2], device=q.device)[:, None] + off
+        s = s.masked_fill(torch.arange(k.shape[2], device=q.device)[None] > i, float("-inf"))
+    return s.softmax(-1) @ v
+
+
+# B, H, Hkv, Sq, Sk, hd, causal, offset.  Bound: a product of hd terms and a softmax-weighted sum, each within a few units of
+# 2^-24 times the root of its length (1.5e-6 at 64 x 1000); gradients pass two of them.
+CASES = [(1, 1, 1, 1, 1, 64, True, 0), (2, 3, 3, 33, 33, 64, True, 0), (1, 2, 2, 32, 64, 32, False, 0), (2, 4, 2, 65, 129, 16, False, 0),
+         (1, 12, 12, 1, 510, 64, True, 509), (2, 8, 1, 1, 1000, 128, True, 999), (1, 4, 2, 4, 65, 64, True, 61),
+         (1, 4, 2, 5, 70, 64, True, 65), (1, 2, 1, 100, 300, 128, True, 200), (2, 2, 2, 40, 40, 10, True, 0), (1, 2, 2, 31, 63, 7, False, 0),
+         (1, 1, 1, 127, 127, 100, True, 0)]
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,hd,causal,off", CASES)
+@pytest.mark.parametrize("layout", ["bhsd", "token", "odd"])
+def test_attention_f32(B, H, Hkv, Sq, Sk, hd, causal, off, layout):
+    g = torch.Generator(device="cuda").manual_seed(Sq * 7 + hd)
+
+    def make(h, s):
+        t = torch.randn(B, s, h, hd, device="cuda", generator=g)
+        if layout == "bhsd":
+            return t.transpose(1, 2).contiguous()
+        if layout == "odd":       # rows start at addresses that are no multiple of 16 bytes
+            wide = torch.zeros(B, s, h, hd + 3, device="cuda")
+            wide[..., 1:hd + 1] = t
+            return wide[..., 1:hd + 1].transpose(1, 2)
+        return t.transpose(1, 2)
+    q, k, v = (make(H, Sq).requires_grad_(True), make(Hkv, Sk).requires_grad_(True), make(Hkv, Sk).requires_grad_(True))
+    o = A.attention_bhsd(q, k, v, causal, None, off)
+    do = torch.randn(o.shape, device="cuda", generator=g)
+    got = torch.autograd.grad(o, (q, k, v), do)
+    with torch.no_grad():
+        assert torch.equal(A.attention_bhsd(q, k, v, causal, None, off), o)
+    d = [t.detach().double().requires_grad_(True) for t in (q, k, v)]
+    ref = _exact(*d, causal, off)
+    want = torch.autograd.grad(ref, d, do.double())
+    for a, b in zip((o.detach(), *got), (ref.detach(), *want)):
+        assert float((a.double() - b).norm() / (b.norm() + 1e-30)) < 3e-6 or float(b.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,hd", [(2, 96, 4, 2, 32), (1, 33, 3, 3, 20)])
+def test_packed_f32_is_one_launch_and_matches_separate_operands(B, S, H, Hkv, hd):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(B * S, (H + 2 * Hkv) * hd, device="cuda", generator=g).requires_grad_(True)
+    do = torch.randn(B * S, H * hd, device="cuda", generator=g)
+    o = A.attention_packed(x, B, S, H, Hkv, hd, True)
+    (dx,) = torch.autograd.grad(o, x, do)
+    dq, dkv = H * hd, Hkv * hd
+    o2 = A.attention_tokens(x[:, :dq], x[:, dq:dq + dkv], x[:, dq + dkv:], B, S, S, H, Hkv, hd, True)
+    (dx2,) = torch.autograd.grad(o2, x, do)
+    assert torch.equal(o, o2) and torch.equal(dx, dx2)
+    with torch.no_grad():
+        assert torch.equal(A.attention_packed(x, B, S, H, Hkv, hd, True), o)
+
+
+def test_non_finite_scores_behave_as_softmax_does():
+    q = torch.ones(1, 1, 40, 16, device="cuda")
+    k, v = torch.randn(1, 1, 40, 16, device="cuda"), torch.randn(1, 1, 40, 16, device="cuda")
+    k[0, 0, 3] = float("-inf")
+    k[0, 0, 20] = float("nan")
+    o = A.attention_bhsd(q, k, v, True, None, 0)
+    ref = _exact(q, k, v, True, 0)
+    assert torch.equal(o.isnan(), ref.isnan())
+    assert torch.allclose(o[~ref.isnan()], ref[~ref.isnan()], rtol=1e-5, atol=1e-6)
