@@ -27,6 +27,7 @@ struct DptbGemmArgs {
   long long ws_bytes;
   int* counters; // zero-initialised per-tile arrival counters (they return to zero after every launch)
   int num_counters;
+  int epi_f32;   // residual, aux_out and aux_in are fp32 (all-fp32 products only)
 };
 
 // Peer-memory description of the all-reduce epilogue (see TpAr).  `partial_elems` / `max_tiles` are capacities that

@@ -70,6 +70,8 @@ gemm_simt_kernel(const TA* __restrict__ A, long long sam, long long sak, const T
 
 using namespace dptb;
 
+int gemm_f32(const DptbGemmArgs* a, void* stream);   // gemm_f32.cu
+
 // Peer-memory description of the all-gather prologue (see TpAg): every rank's shard of A, [rows_per_rank, lda] each.
 struct DptbTpAgArgs {
   int world, rank;
@@ -124,6 +126,10 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
     if (ar->mode == 1 && (a->M % (ar->world * kBM))) return kErrBadShape;   // whole row tiles per shard
   }
   if (ag && (!tc_ok || a->splits > 1)) return kErrUnsupported;
+  if (a->epi_f32 && (!a->a_f32 || !a->b_f32 || !a->out_f32 || a->force_simt)) return kErrUnsupported;
+  if (a->a_f32 && a->b_f32 && a->out_f32 && !a->force_simt &&
+      (a->epi_f32 || !(a->residual || a->aux_out || a->aux_in || a->act)))
+    return gemm_f32(a, stream_v);
   if (!tc_ok) {
     p.tiles_m = p.tiles_n = p.num_kb = 0;
     p.splits = 1; p.kb_per_split = 0; p.ws = nullptr; p.counters = nullptr;

@@ -148,6 +148,7 @@ class GemmArgs(ctypes.Structure):
         ("bias_f32", c_int), ("out_f32", c_int), ("accumulate", c_int), ("act", c_int),
         ("alpha", c_float), ("force_simt", c_int), ("bn", c_int), ("splits", c_int),
         ("ws", c_void_p), ("ws_bytes", c_ll), ("counters", c_void_p), ("num_counters", c_int),
+        ("epi_f32", c_int),
     ]
 
 

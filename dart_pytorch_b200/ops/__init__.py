@@ -62,7 +62,8 @@ def linear(x, weight, bias=None, activation=None, residual=None):
 
 def mlp(x, w1, b1, w2, b2, activation="relu", residual=None):
     """Two-layer feed-forward ``act(x w1^T + b1) w2^T + b2 (+ residual)``."""
-    if _cuda(x) and w1.dtype == torch.bfloat16 and activation not in (None, "none"):
+    if _cuda(x) and (w1.dtype == torch.bfloat16 and activation not in (None, "none") or
+                     w1.dtype == w2.dtype == torch.float32 and activation in _cu().F32_ACTS):
         x = _match(x, w1)
         if residual is not None:
             residual = _match(residual, w1)

@@ -53,6 +53,14 @@ def _is_bf16(*ts) -> bool:
     return all(t is None or t.dtype == torch.bfloat16 for t in ts)
 
 
+F32_ACTS = ("relu", "gelu_tanh", "quick_gelu", "silu")     # what the fp32 GEMM's epilogue applies
+
+
+def _fused_f32(act, *ts) -> bool:
+    """Whether the fp32 GEMM takes everything after the product into its epilogue."""
+    return (not act or act in F32_ACTS) and all(t is None or t.dtype == torch.float32 for t in ts)
+
+
 # --------------------------------------------------------------------------- linear / mlp
 def _weight_grad(dy2: torch.Tensor, x2: torch.Tensor, w: torch.Tensor, needs: bool):
     """dW[N,K] = dy2^T @ x2, into the direct-grad buffer when there is one."""
@@ -163,18 +171,18 @@ def _bias_grad(dy2: torch.Tensor, b: Optional[torch.Tensor], needs: bool):
 
 
 class LinearFn(torch.autograd.Function):
-    """``act(x @ w.T + b) + residual`` with everything after the GEMM done in its epilogue (bf16)."""
+    """``act(x @ w.T + b) + residual`` with everything after the GEMM done in its epilogue."""
 
     @staticmethod
     def forward(ctx, x, w, b, act, residual):
         x2 = _as2d(x)
         M, Nn = x2.shape[0], w.shape[0]
         out = torch.empty(M, Nn, dtype=x.dtype, device=x.device)
-        fused = _is_bf16(x2, w, residual)
+        fused = _is_bf16(x2, w, residual) or _fused_f32(act, x2, w, residual)
         pre = None
         if fused:
             pre = torch.empty_like(out) if act else None
-            K.gemm(x2, w, out, trans_b=True, bias=None if b is None else b.view(-1), act=act, aux_out=pre,
+            K.gemm(x2, w, out, trans_b=True, bias=None if b is None else b.view(-1), act=act or None, aux_out=pre,
                    residual=None if residual is None else _as2d(residual))
         else:
             K.gemm(x2, w, out, trans_b=True, bias=None if b is None else b.view(-1))
@@ -226,7 +234,8 @@ class MLPFn(torch.autograd.Function):
         # same tanh), so the backward epilogue is one multiply; other activations save the pre-activation itself.
         pre = torch.empty(M, F, dtype=x.dtype, device=x.device)
         a = torch.empty_like(pre)
-        fwd_act = "gelu_tanh_d" if act == "gelu_tanh" else act
+        # (fp32 saves the pre-activation for it too: the derivative is recomputed at full precision.)
+        fwd_act = "gelu_tanh_d" if act == "gelu_tanh" and x.dtype == torch.bfloat16 else act
         K.gemm(x2, w1, a, trans_b=True, bias=None if b1 is None else b1.view(-1), act=fwd_act, aux_out=pre)
         out = torch.empty(M, D, dtype=x.dtype, device=x.device)
         K.gemm(a, w2, out, trans_b=True, bias=None if b2 is None else b2.view(-1),
@@ -246,7 +255,7 @@ class MLPFn(torch.autograd.Function):
         dpre = torch.empty_like(pre)
         fork = _ParamGradFork(dy2.device) if (_GRAD_SIDE and dy2.is_cuda) else None
         db2 = _bias_grad_fork(dy2, b2, ctx.needs_input_grad[4], fork)       # beside the next two GEMMs
-        K.gemm(dy2, w2, dpre, aux_in=pre, act_bwd="mul" if ctx.act == "gelu_tanh" else ctx.act)
+        K.gemm(dy2, w2, dpre, aux_in=pre, act_bwd="mul" if ctx.act == "gelu_tanh" and pre.dtype == torch.bfloat16 else ctx.act)
         dw2 = _weight_grad(dy2, a, w2, ctx.needs_input_grad[3])
         if fork is not None:
             fork.join()

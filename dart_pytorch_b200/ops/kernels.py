@@ -94,9 +94,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, trans_a: bool =
             raise ValueError("gemm: bias shorter than N")
         args.bias = bias.data_ptr()
         args.bias_f32 = int(bias.dtype == torch.float32)
+    extra = [t for t in (residual, aux_out, aux_in) if t is not None]
+    # an all-fp32 product takes fp32 per-element buffers too (and applies activations at fp32 precision)
+    args.epi_f32 = int(args.a_f32 and args.b_f32 and args.out_f32 and not force_simt and
+                       all(t.dtype == torch.float32 for t in extra))
     for name, t in (("residual", residual), ("aux_out", aux_out), ("aux_in", aux_in)):
         if t is not None:
-            if t.dtype != torch.bfloat16:
+            if t.dtype != torch.bfloat16 and not args.epi_f32:
                 raise TypeError(f"gemm: {name} must be bfloat16")
             if t.shape[0] != M or t.shape[1] < Nn:
                 raise ValueError(f"gemm: {name} has the wrong shape")
