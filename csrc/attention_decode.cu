@@ -1,10 +1,9 @@
-// Decode-time attention over a KV cache (one or a few new query tokens per sequence) and the fused rotary + cache
-// append that precedes it.
+// Decode-time attention over a KV cache (one or a few new query tokens per sequence).
 //
 // The reference keeps per-head K / V tensors on the device, re-uploads the whole cache after appending one row on the
 // host and materialises [1, T] score rows per head (reference: lib/core/nn/kv_cache.dart:22-84,
 // lib/core/nn/attention/multi_head_attention.dart:160-235, lib/core/tensor/concat.dart:51-90).  Here the cache is one
-// [B, capacity, Hkv * hd] buffer per layer, new rows are written in place by the kernel that also applies RoPE, and
+// [B, capacity, Hkv * hd] buffer per layer, new rows are written in place by the kernel that also applies RoPE (rope.cu), and
 // attention streams each KV row exactly once for all query heads that share it (grouped-query attention).
 //
 // attn_decode_kernel: grid (splits, Hkv, B * Sq).  A CTA owns one (sequence, query position, kv head) and a contiguous
@@ -26,6 +25,7 @@
 
 #include <initializer_list>
 
+#include "common/attn_args.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 #include "common/reduce.cuh"
@@ -49,6 +49,7 @@ struct DecodeArgs {
   const int* pos_ptr;        // when set: q_offset = *pos_ptr and Sk = q_offset + Sq (device-resident position, so a
                              // captured CUDA graph can be replayed as the sequence grows)
   int cap;                   // cache rows per sequence: no key at or beyond it is ever read
+  unsigned int* counters;    // one zeroed word per (query row, kv head), or null: the table below
   int fused_merge;           // the last split CTA of a (query row, kv head) merges the partials itself
   // windowed form
   const __nv_bfloat16* k_pool;   // [B, pool_rows, Hkv * dk]
@@ -96,7 +97,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 constexpr int kDecRound = 16;    // keys per round of a warp
 
 // Arrival counters of the split CTAs of one (query row, kv head): the last CTA to arrive merges the partials, so no
-// second kernel runs.  Zero at load, reset by the merging CTA; launches that use them must not overlap on two streams.
+// second kernel runs.  Zero at load, reset by the merging CTA.  Launches that share the table must not overlap on two streams; callers on several streams pass words of
+// their own.
 constexpr int kDecCounters = 1 << 16;
 __device__ unsigned int g_dec_counters[kDecCounters];
 constexpr int kDecMaxFusedSplits = 64;
@@ -324,7 +326,7 @@ attn_decode_kernel(const DecodeArgs a) {
   __threadfence();   // this thread's partials are visible device-wide before the CTA is counted
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned int* ctr = &g_dec_counters[bs * a.Hkv + g];
+    unsigned int* ctr = (a.counters ? a.counters : g_dec_counters) + bs * a.Hkv + g;
     const unsigned int prev = atomicAdd(ctr, 1u);
     s_last = prev == (unsigned int)a.splits - 1u ? 1u : 0u;
     if (s_last) *ctr = 0u;   // everyone has arrived: ready for the next launch
@@ -425,74 +427,9 @@ attn_decode_merge_kernel(const DecodeArgs a) {
   }
 }
 
-// Rotary embedding (half-split form) on the Q and K column blocks of a fused projection row, K / V written straight
-// into the cache at their absolute positions.  Grid: one CTA per (row, head) group; threads over the head dimension.
-//   qkv row layout: [Hq * hd | Hkv * hd | Hkv * hd];  q is rotated in place (the attention kernel reads it there).
-template <int HD>
-__global__ void __launch_bounds__(128)
-rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, __nv_bfloat16* __restrict__ kc,
-                      __nv_bfloat16* __restrict__ vc, long long ldkv, long long kv_batch_stride, int B, int S, int Hq,
-                      int Hkv, int pos0, int rotary_dim, float base, int cap, const int* __restrict__ pos_ptr) {
-  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
-  pdl_launch_dependents();
-  const int row = blockIdx.x;                // b * S + s
-  const int b = row / S, s = row % S;
-  const int pos = (pos_ptr ? *pos_ptr : pos0) + s;
-  if (pos >= cap) return;
-  __nv_bfloat16* r = qkv + (long long)row * ld;
-  const int half = rotary_dim / 2;
-  const int heads = Hq + 2 * Hkv;
-  // Thread -> one pair index i (angle computed once) and a strided subset of the heads.
-  constexpr int PAIRS = HD / 2;
-  const int i = threadIdx.x % PAIRS, hg = threadIdx.x / PAIRS, hstep = blockDim.x / PAIRS;
-  // pair (i, i + half) inside the rotary part; dims >= rotary_dim pass through as the pair
-  // (rotary_dim + 2 (i - half), + 1), so that every element is visited exactly once
-  int d0, d1;
-  float cs = 1.0f, sn = 0.0f;
-  if (i < half) {
-    d0 = i;
-    d1 = i + half;
-    const float inv = powf(base, -2.0f * (float)i / (float)rotary_dim);
-    sincosf((float)pos * inv, &sn, &cs);
-  } else {
-    d0 = rotary_dim + 2 * (i - half);
-    d1 = d0 + 1;
-  }
-  for (int h = hg; h < heads; h += hstep) {
-    __nv_bfloat16* src = r + (long long)h * HD;
-    const float x0 = __bfloat162float(src[d0]), x1 = __bfloat162float(src[d1]);
-    const bool is_v = h >= Hq + Hkv;
-    const float y0 = is_v ? x0 : x0 * cs - x1 * sn;
-    const float y1 = is_v ? x1 : x1 * cs + x0 * sn;
-    if (h < Hq) {
-      src[d0] = __float2bfloat16(y0);
-      src[d1] = __float2bfloat16(y1);
-    } else {
-      const int g = is_v ? h - Hq - Hkv : h - Hq;
-      __nv_bfloat16* dst = (is_v ? vc : kc) + (long long)b * kv_batch_stride + (long long)pos * ldkv + (long long)g * HD;
-      dst[d0] = __float2bfloat16(y0);
-      dst[d1] = __float2bfloat16(y1);
-    }
-  }
-}
-
 }  // namespace dptb
 
 using namespace dptb;
-
-struct DptbDecodeArgs {
-  const void* q;
-  const void* k;
-  const void* v;
-  void* o;
-  float* ws;
-  long long ws_floats;
-  long long ldq, ldkv, ldo, kv_batch_stride;
-  int B, Sq, Sk, Hq, Hkv, head_dim, splits, q_offset;
-  float scale;
-  const int* pos_ptr;
-  int cap;
-};
 
 // Floats of workspace needed for a given split count.
 extern "C" long long dptb_attn_decode_ws_floats(int B, int Sq, int Hq, int head_dim, int splits) {
@@ -561,7 +498,9 @@ extern "C" int dptb_attn_decode(const DptbDecodeArgs* h, void* stream) {
     return kErrTooLarge;
   dim3 grid(a.splits, a.Hkv, a.B * a.Sq);
   const int G = a.Hq / a.Hkv;
-  a.fused_merge = (a.splits > 1 && a.splits <= kDecMaxFusedSplits && (long long)a.B * a.Sq * a.Hkv <= kDecCounters) ? 1 : 0;
+  a.counters = h->counters;
+  const long long words = h->counters ? h->num_counters : kDecCounters;
+  a.fused_merge = (a.splits > 1 && a.splits <= kDecMaxFusedSplits && (long long)a.B * a.Sq * a.Hkv <= words) ? 1 : 0;
   const int gp = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;
   DPTB_CUDA_OK((h->head_dim == 128 ? decode_launch<128, false>(a, gp, grid, st) : decode_launch<64, false>(a, gp, grid, st)));
   DPTB_CUDA_OK(cudaGetLastError());
@@ -622,23 +561,4 @@ extern "C" int dptb_window_attn_decode(const DptbWindowDecodeArgs* h, void* stre
   const dim3 grid(a.splits, a.Hkv, a.B * a.Sq);
   const int gp = G <= 1 ? 1 : G <= 2 ? 2 : G <= 4 ? 4 : 8;
   return counted(1, (int)(HD == 128 ? decode_launch<128, true>(a, gp, grid, st) : decode_launch<64, true>(a, gp, grid, st)));
-}
-
-extern "C" int dptb_rope_kv_append(void* qkv, long long ld, void* kc, void* vc, long long ldkv,
-                                   long long kv_batch_stride, int B, int S, int Hq, int Hkv, int head_dim, int pos0,
-                                   int rotary_dim, float base, int cap, const int* pos_ptr, void* stream) {
-  auto st = static_cast<cudaStream_t>(stream);
-  if (B <= 0 || S <= 0) return 0;
-  if (rotary_dim < 0 || rotary_dim > head_dim || (rotary_dim & 1) || pos0 < 0 || (!pos_ptr && pos0 + S > cap))
-    return kErrBadShape;
-  auto* q = static_cast<__nv_bfloat16*>(qkv);
-  auto* k = static_cast<__nv_bfloat16*>(kc);
-  auto* v = static_cast<__nv_bfloat16*>(vc);
-  if (head_dim == 128)
-    DPTB_CUDA_OK(launch_k(rope_kv_append_kernel<128>, dim3(B * S), dim3(128), 0, st, q, ld, k, v, ldkv, kv_batch_stride, B, S, Hq, Hkv, pos0, rotary_dim, base, cap, pos_ptr));
-  else if (head_dim == 64)
-    DPTB_CUDA_OK(launch_k(rope_kv_append_kernel<64>, dim3(B * S), dim3(128), 0, st, q, ld, k, v, ldkv, kv_batch_stride, B, S, Hq, Hkv, pos0, rotary_dim, base, cap, pos_ptr));
-  else
-    return kErrUnsupported;
-  return counted(1, (int)cudaGetLastError());
 }

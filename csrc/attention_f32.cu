@@ -19,6 +19,7 @@
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
+#include "common/attn_args.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 
@@ -590,19 +591,6 @@ static int attn_f32_launch(const AttnF32Params& p, int backward, cudaStream_t st
 }  // namespace dptb
 
 using namespace dptb;
-
-struct DptbF32View {
-  float* p;
-  long long sb, ss, sh;
-};
-struct DptbAttnF32Args {
-  DptbF32View q, k, v, o, dout, dq, dk, dv;      // backward only: dout, dq, dk, dv
-  float* lse;      // [B, Hq, Sq]; forward: written unless null, backward: read
-  float* delta;    // backward scratch of the same size
-  int B, Sq, Sk, Hq, Hkv, hd, causal, q_offset;
-  float scale;
-  int backward;
-};
 
 extern "C" int dptb_attn_f32(const DptbAttnF32Args* a, void* stream) {
   if (a->B <= 0 || a->Sq <= 0 || a->Hq <= 0) return 0;

@@ -32,6 +32,7 @@
 
 #include <initializer_list>
 
+#include "common/attn_args.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 
@@ -552,20 +553,6 @@ static int encode_tmap_seq(CUtensorMap* map, const void* base, int heads, int hd
 }  // namespace dptb
 
 using namespace dptb;
-
-struct DptbAttnFwdArgs {
-  const void* q;
-  const void* k;
-  const void* v;
-  void* o;
-  float* lse;
-  long long ldq, ldk, ldv, ldo;
-  int B, Sq, Sk, Hq, Hkv, head_dim;
-  int causal, q_offset;
-  float scale;
-  long long kv_batch_rows;  // rows between consecutive batches of K / V (a cache's capacity); 0 = Sk
-  int precise;              // softmax weights as two bf16 parts
-};
 
 template <int HD, int NQ, int KST, int VST, bool PREC>
 static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {

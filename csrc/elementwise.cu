@@ -1,4 +1,4 @@
-// Elementwise, broadcast, reduction, transpose, RoPE, dropout, SwiGLU and sampling kernels.
+// Elementwise, broadcast, reduction, transpose, dropout, SwiGLU and sampling kernels.
 //
 // These keep the tensor-level API of the reference on the device (reference: lib/native/src/kernels/elementwise.cuh,
 // lib/native/src/kernels/transpose.cuh, lib/native/src/kernels/matmul.cuh:146-185, lib/native/src/engine.cu:65-88,575-596)
@@ -282,50 +282,6 @@ copy2d_kernel(const T* __restrict__ src, long long lds, T* __restrict__ dst, lon
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / cols, c = i % cols;
     dst[r * ldd + c] = src[r * lds + c];
-  }
-}
-
-// Half-split rotary embedding on rows laid out [tokens, heads, head_dim] inside a matrix with row stride `ld`:
-// element (t, h, d) sits at x[t*ld + h*head_dim + d].  Position of token t is pos_start + (t % seq_len), or
-// positions[t] when given.  `inverse` applies the transpose rotation (the backward).
-// inv_freq_i = base^(-2i/rotary_dim); dims >= rotary_dim pass through (reference: lib/core/nn/rotary.dart:95-201).
-template <typename T>
-__global__ void __launch_bounds__(kEwThreads)
-rope_kernel(const T* __restrict__ x, T* __restrict__ out, long long tokens, int heads, int head_dim, int rotary_dim,
-            int seq_len, int pos_start, float base, int inverse, const long long* __restrict__ positions,
-            long long ld_in, long long ld_out) {
-  const int half = rotary_dim / 2;
-  const long long per_tok = (long long)heads * half;
-  const long long n = tokens * per_tok;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_tok;
-    const int rem = (int)(i % per_tok);
-    const int h = rem / half, d = rem % half;
-    const float pos = positions ? (float)positions[t] : (float)(pos_start + (seq_len > 0 ? t % seq_len : t));
-    const float inv = powf(base, -2.0f * (float)d / (float)rotary_dim);
-    float sn, cs;
-    sincosf(pos * inv, &sn, &cs);
-    if (inverse) sn = -sn;
-    const long long oi = t * ld_in + (long long)h * head_dim + d;
-    const long long oo = t * ld_out + (long long)h * head_dim + d;
-    const float a = to_f32(x[oi]), b = to_f32(x[oi + half]);
-    out[oo] = from_f32<T>(a * cs - b * sn);
-    out[oo + half] = from_f32<T>(b * cs + a * sn);
-  }
-}
-// Pass-through copy of the non-rotated tail dims when out != x.
-template <typename T>
-__global__ void __launch_bounds__(kEwThreads)
-rope_tail_kernel(const T* __restrict__ x, T* __restrict__ out, long long tokens, int heads, int head_dim, int rotary_dim,
-                 long long ld_in, long long ld_out) {
-  const int tail = head_dim - rotary_dim;
-  const long long per_tok = (long long)heads * tail;
-  const long long n = tokens * per_tok;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_tok;
-    const int rem = (int)(i % per_tok);
-    const int h = rem / tail, d = rotary_dim + rem % tail;
-    out[t * ld_out + (long long)h * head_dim + d] = x[t * ld_in + (long long)h * head_dim + d];
   }
 }
 
@@ -702,25 +658,6 @@ extern "C" int dptb_copy2d(const void* src, long long lds, void* dst, long long 
   DPTB_BY_DTYPE(dtype,
                 (copy2d_kernel<__nv_bfloat16><<<ew_grid(rows * cols), kEwThreads, 0, st>>>((const __nv_bfloat16*)src, lds, (__nv_bfloat16*)dst, ldd, rows, cols)),
                 (copy2d_kernel<float><<<ew_grid(rows * cols), kEwThreads, 0, st>>>((const float*)src, lds, (float*)dst, ldd, rows, cols)));
-  return counted(1, (int)cudaGetLastError());
-}
-extern "C" int dptb_rope(const void* x, void* out, long long tokens, int heads, int head_dim, int rotary_dim,
-                         int seq_len, int pos_start, float base, int inverse, int dtype, long long ld_in,
-                         long long ld_out, const long long* positions, void* stream) {
-  if (tokens <= 0) return 0;
-  if (rotary_dim % 2 || rotary_dim > head_dim) return kErrBadShape;
-  auto st = static_cast<cudaStream_t>(stream);
-  const long long n = tokens * heads * (rotary_dim / 2);
-  DPTB_BY_DTYPE(dtype,
-                (rope_kernel<__nv_bfloat16><<<ew_grid(n), kEwThreads, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, tokens, heads, head_dim, rotary_dim, seq_len, pos_start, base, inverse, positions, ld_in, ld_out)),
-                (rope_kernel<float><<<ew_grid(n), kEwThreads, 0, st>>>((const float*)x, (float*)out, tokens, heads, head_dim, rotary_dim, seq_len, pos_start, base, inverse, positions, ld_in, ld_out)));
-  DPTB_CUDA_OK(cudaGetLastError());
-  if (x != out && rotary_dim < head_dim) {
-    const long long nt = tokens * heads * (head_dim - rotary_dim);
-    DPTB_BY_DTYPE(dtype,
-                  (rope_tail_kernel<__nv_bfloat16><<<ew_grid(nt), kEwThreads, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, tokens, heads, head_dim, rotary_dim, ld_in, ld_out)),
-                  (rope_tail_kernel<float><<<ew_grid(nt), kEwThreads, 0, st>>>((const float*)x, (float*)out, tokens, heads, head_dim, rotary_dim, ld_in, ld_out)));
-  }
   return counted(1, (int)cudaGetLastError());
 }
 extern "C" int dptb_dropout(const void* x, void* out, long long n, float p, unsigned long long seed,

@@ -80,6 +80,26 @@ class MHACache:
         self.__dict__.pop("_fills", None)
         return self.k_buf[:, :self.seq_len], self.v_buf[:, :self.seq_len]
 
+    def takes_rows(self, qkv: torch.Tensor) -> bool:
+        """Whether ``append_rows`` can write the K and V columns of this projection output straight into the buffers."""
+        if not qkv.is_cuda or qkv.requires_grad or qkv.dtype not in (torch.bfloat16, torch.float32) or qkv.stride(1) != 1:
+            return False
+        k, v = self.k_buf, self.v_buf
+        return k is None or (k.dtype == v.dtype == qkv.dtype and k.device == v.device == qkv.device and
+                             k.shape == v.shape and k.stride() == v.stride() and k.stride(2) == 1)
+
+    def append_rows(self, qkv: torch.Tensor, batch: int, n: int, heads: int, kv_heads: int, head_dim: int, rope=None,
+                    start_pos: int = 0):
+        """Append the K and V columns of ``qkv [batch * n, (heads + 2 kv_heads) hd]`` in one kernel, which also applies
+        ``rope`` to the keys on their way and to the queries in place; returns what ``append`` does."""
+        from ..ops import decode
+        self._ensure(batch, self.seq_len + n, kv_heads * head_dim, qkv)
+        decode.rows_to_cache(qkv, self.k_buf, self.v_buf, batch, n, heads, kv_heads, head_dim, start_pos,
+                             self.seq_len, 0 if rope is None else rope.rotary_dim, 1.0 if rope is None else rope.base)
+        self.seq_len += n
+        self.__dict__.pop("_fills", None)
+        return self.k_buf[:, :self.seq_len], self.v_buf[:, :self.seq_len]
+
     # Per-head accessors with the reference's shapes (``[T_seen, hd]``, batch 1).
     def _head(self, buf, h):
         hd = buf.shape[2] // self.num_kv_heads
@@ -230,8 +250,14 @@ class MultiHeadAttention(Module):
         qkv = F.linear(x2, self.w_qkv, self.b_qkv)  # [B*S, dq + 2 dkv]
         if self.rope is not None:
             self.rope.check_window(start_pos, S)
+        rows = cache is not None and cache.takes_rows(qkv)     # rotation and append in one kernel
+        if self.rope is not None and not rows:
             qkv = self._rope_qk(qkv, S, start_pos)
-        if cache is None and mask is None:
+        if rows:
+            past = cache.seq_len
+            k_all, v_all = cache.append_rows(qkv, B, S, H, Hkv, hd, self.rope, start_pos)
+            o = self._attend_tokens(qkv[:, :dq], k_all, v_all, B, S, past + S, causal, past, mask)
+        elif cache is None and mask is None:
             o = F.attention_packed(qkv, B, S, H, Hkv, hd, causal=causal)
         else:
             q = qkv[:, :dq]

@@ -17,9 +17,11 @@ class DecodeArgs(ctypes.Structure):
     _fields_ = [("q", c_void_p), ("k", c_void_p), ("v", c_void_p), ("o", c_void_p), ("ws", c_void_p),
                 ("ws_floats", c_ll), ("ldq", c_ll), ("ldkv", c_ll), ("ldo", c_ll), ("kv_batch_stride", c_ll),
                 ("B", c_int), ("Sq", c_int), ("Sk", c_int), ("Hq", c_int), ("Hkv", c_int), ("head_dim", c_int),
-                ("splits", c_int), ("q_offset", c_int), ("scale", c_float), ("pos_ptr", c_void_p), ("cap", c_int)]
+                ("splits", c_int), ("q_offset", c_int), ("scale", c_float), ("pos_ptr", c_void_p), ("cap", c_int),
+                ("num_counters", c_int), ("counters", c_void_p)]
 
 
+ERR_UNSUPPORTED = -5
 _declared = False
 
 
@@ -35,8 +37,8 @@ def _lib():
         lib.dptb_attn_decode_splits.restype = c_int
         lib.dptb_attn_decode_splits_hd.argtypes = [c_int] * 5
         lib.dptb_attn_decode_splits_hd.restype = c_int
-        lib.dptb_rope_kv_append.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll] + [c_int] * 7 + \
-            [c_float, c_int, c_void_p, c_void_p]
+        lib.dptb_rope_kv_append.argtypes = [c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_ll] + [c_int] * 8 + \
+            [c_float, c_int, c_void_p, c_int, c_void_p]
         lib.dptb_rope_kv_append.restype = c_int
         _declared = True
     return lib
@@ -62,11 +64,12 @@ def attn_decode_reference(q2, k_cache, v_cache, B, Sq, Sk, Hq, Hkv, hd, q_offset
 def attn_decode(q2: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, B: int, Sq: int, Sk: int, Hq: int,
                 Hkv: int, hd: int, q_offset: int, scale: Optional[float] = None, out: Optional[torch.Tensor] = None,
                 splits: int = 0, workspace: Optional[torch.Tensor] = None,
-                pos: Optional[torch.Tensor] = None) -> torch.Tensor:
+                pos: Optional[torch.Tensor] = None, counters: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of ``Sq`` new query rows per sequence over the first ``Sk`` cache rows (which already include the
     new tokens).  ``q2``: ``[B*Sq, >= Hq*hd]`` bf16; caches ``[B, cap, Hkv*hd]`` bf16.  Returns ``[B*Sq, Hq*hd]``.
     With ``pos`` (an int32 device scalar) the kernel takes ``q_offset = pos`` and ``Sk = pos + Sq`` from the device;
-    ``Sk`` then only sizes the split of the keys (pass the largest context that will be reached)."""
+    ``Sk`` then only sizes the split of the keys (pass the largest context that will be reached).  ``counters``: zeroed
+    int32 words of the current stream for the merge of the splits (without them calls on two streams must not overlap)."""
     if not q2.is_cuda:
         o = attn_decode_reference(q2, k_cache, v_cache, B, Sq, Sk, Hq, Hkv, hd, q_offset, scale).to(q2.dtype)
         if out is not None:
@@ -95,6 +98,8 @@ def attn_decode(q2: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     a.B, a.Sq, a.Sk, a.Hq, a.Hkv, a.head_dim = B, Sq, Sk, Hq, Hkv, hd
     a.splits, a.q_offset = splits, q_offset
     a.pos_ptr, a.cap = (pos.data_ptr() if pos is not None else None), k_cache.shape[1]
+    if counters is not None:
+        a.counters, a.num_counters = counters.data_ptr(), counters.numel()
     a.scale = 1.0 / math.sqrt(hd) if scale is None else scale
     N.check(lib.dptb_attn_decode(ctypes.byref(a), N.stream_ptr()), "attn_decode")
     return out
@@ -140,12 +145,19 @@ def rope_kv_append(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         raise ValueError(f"rope_kv_append: positions up to {pos0 + S} exceed the cache capacity {k_cache.shape[1]}")
     if not qkv.is_cuda:
         return rope_kv_append_reference(qkv, k_cache, v_cache, B, S, Hq, Hkv, hd, pos0, rotary_dim, base)
-    lib = _lib()
     if qkv.dtype != torch.bfloat16 or k_cache.dtype != torch.bfloat16 or v_cache.dtype != torch.bfloat16:
         raise TypeError("rope_kv_append: tensors must be bfloat16")
     if k_cache.stride() != v_cache.stride() or k_cache.stride(-1) != 1 or qkv.stride(-1) != 1:
         raise ValueError("rope_kv_append: unsupported layout")
-    N.check(lib.dptb_rope_kv_append(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
-                                    k_cache.stride(1), k_cache.stride(0), B, S, Hq, Hkv, hd, pos0, rotary_dim,
-                                    float(base), k_cache.shape[1], pos.data_ptr() if pos is not None else None,
-                                    N.stream_ptr()), "rope_kv_append")
+    if hd not in (64, 128):
+        N.check(ERR_UNSUPPORTED, "rope_kv_append")
+    rows_to_cache(qkv, k_cache, v_cache, B, S, Hq, Hkv, hd, pos0, pos0, rotary_dim, base, pos)
+
+
+def rows_to_cache(qkv, k_cache, v_cache, B, S, Hq, Hkv, hd, pos0, row0, rotary_dim, base=10000.0, pos=None) -> None:
+    """``rope_kv_append`` for fp32 or bf16 tensors of one dtype, any head size and separate starts of the positions and
+    of the cache rows; ``rotary_dim`` 0 only moves K and V."""
+    N.check(_lib().dptb_rope_kv_append(qkv.data_ptr(), qkv.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
+                                       k_cache.stride(1), k_cache.stride(0), B, S, Hq, Hkv, hd, pos0, row0, rotary_dim,
+                                       float(base), k_cache.shape[1], pos.data_ptr() if pos is not None else None,
+                                       N.dtype_code(qkv), N.stream_ptr()), "rope_kv_append")
