@@ -164,6 +164,13 @@ class SeparateAttentionFn(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None, None, None, None, None, None
 
 
+def attn_decode_rows(q2, k3, v3, B, Sk, H, Hkv, hd):
+    """One query row per sequence over all ``Sk`` rows of ``k3`` / ``v3 [B, Sk, Hkv hd]`` (cache views), no gradients."""
+    from . import decode
+    from .kernels import splitk_workspace
+    return decode.attn_decode(q2, k3, v3, B, 1, Sk, H, Hkv, hd, Sk - 1, counters=splitk_workspace(q2.device)[1])
+
+
 # ------------------------------------------------------------------------------------------------------------ fp32
 class F32View(ctypes.Structure):
     _fields_ = [("p", c_void_p), ("sb", c_ll), ("ss", c_ll), ("sh", c_ll)]
