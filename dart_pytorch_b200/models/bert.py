@@ -108,8 +108,34 @@ class BertModel(Module):
     def submodules(self):
         return [self.embeddings] + list(self.layers)
 
+    def _infer(self, tokens):
+        """The encoder without gradients as one native call; ``None`` when that does not stand for its modules."""
+        e = self.embeddings
+        if torch.is_grad_enabled() or not tokens.is_cuda or tokens.dim() not in (1, 2) or \
+                not 0 < tokens.shape[-1] <= e.max_len:
+            return None
+        from ..ops import stack
+        plain, layers = stack.plain, []
+        for b in self.layers:
+            m = b.attention
+            if not (plain(b, BertLayer) and plain(m, MultiHeadAttention) and plain(m.wo, Linear) and
+                    plain(b.attention_output_ln, LayerNorm) and plain(b.output_ln, LayerNorm) and
+                    plain(b.intermediate, Linear) and plain(b.output, Linear)) or \
+                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+                return None
+            layers.append(stack.Layer(m, b.attention_output_ln, b.output_ln, b.intermediate.weight, b.intermediate.bias,
+                                      b.output.weight, b.output.bias))
+        if not (plain(e, BertEmbeddings) and plain(e.layer_norm, LayerNorm)):
+            return None
+        return stack.run(layers, None, post_norm=True, act="gelu_tanh", tokens=tokens, table=e.word_embeddings.weight,
+                         pos_table=e.position_embeddings.weight, add_row=e.token_type_bias, embed_norm=e.layer_norm)
+
     def forward(self, tokens):
-        h = self.embeddings(_as_token_tensor(tokens, self.device))
+        tokens = _as_token_tensor(tokens, self.device)
+        h = self._infer(tokens)
+        if h is not None:
+            return h
+        h = self.embeddings(tokens)
         for layer in self.layers:
             h = layer(h)
         return h

@@ -113,6 +113,12 @@ class GPT(Module):
         n = tokens.shape[-1]
         if start_pos + n > self.config.max_ctx:
             raise ValueError(f"GPT: sequence of {start_pos + n} tokens exceeds maxCtx {self.config.max_ctx}")
+        if tokens.is_cuda and type(self.encoder) is TransformerEncoder and not (
+                self.embed_drop.training and self.embed_drop.p > 0):
+            h = self.encoder.infer(None, cache, n > 1, start_pos, tokens=tokens, table=self.token_emb.weight,
+                                   pos_table=self.pos_emb.table.weight, pos_start=start_pos)
+            if h is not None:
+                return h
         h = F.embedding(self.token_emb.weight, tokens, pos_table=self.pos_emb.table.weight, pos_start=start_pos)
         h = self.embed_drop(h)
         return self.encoder(h, cache=cache, causal=n > 1, start_pos=start_pos)

@@ -97,6 +97,27 @@ class Llama(Module):
     def head_weight(self):
         return self.embed_in.weight if self.untied_head is None else self.untied_head.weight
 
+    def _infer(self, x, start_pos, cache, n, **embedding):
+        """The stack without gradients as one native call; ``None`` when that does not stand for the blocks."""
+        if torch.is_grad_enabled():
+            return None
+        from ..ops import stack
+        plain, layers = stack.plain, []
+        for b in self.blocks:
+            m = b.attn
+            if not (plain(b, LlamaBlock) and plain(m, MultiHeadAttention) and plain(m.wo, Linear) and
+                    plain(b.attn_norm, RMSNorm) and plain(b.ffn_norm, RMSNorm) and plain(b.ffn, SwiGluFfn) and
+                    plain(b.ffn.down, Linear)) or \
+                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+                return None
+            layers.append(stack.Layer(m, b.attn_norm, b.ffn_norm, b.ffn.w_gate_up, None, b.ffn.down.weight,
+                                      b.ffn.down.bias))
+        if not plain(self.final_norm, RMSNorm) or cache is not None and not (
+                len(cache.layers) == len(layers) and all(type(c) is MHACache for c in cache.layers)):
+            return None
+        return stack.run(layers, x, rms=True, gated=True, causal=n > 1, start_pos=start_pos,
+                         caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)
+
     def hidden_from_embeddings(self, h, start_pos: int = 0, cache: Optional[EncoderCache] = None):
         """Run the decoder stack on precomputed input embeddings ``[N, D]`` / ``[B, N, D]``; returns the final-norm
         hidden states."""
@@ -105,6 +126,10 @@ class Llama(Module):
             raise ValueError(f"Llama: sequence of {start_pos + n} tokens exceeds maxCtx {self.config.max_ctx}")
         if cache is not None and len(cache.layers) != len(self.blocks):
             raise ValueError("Llama: cache has a different number of layers")
+        if h.is_cuda:
+            out = self._infer(h, start_pos, cache, n)
+            if out is not None:
+                return out
         for i, blk in enumerate(self.blocks):
             h = blk(h, cache=None if cache is None else cache.layers[i], start_pos=start_pos, causal=n > 1)
         return self.final_norm(h)
@@ -121,6 +146,11 @@ class Llama(Module):
     def hidden(self, tokens, start_pos: int = 0, cache: Optional[EncoderCache] = None):
         if tokens.dim() not in (1, 2):
             raise ValueError("Llama: tokens must be [N] or [B, N]")
+        n = tokens.shape[-1]
+        if tokens.is_cuda and start_pos + n <= self.config.max_ctx and type(self) is Llama:
+            h = self._infer(None, start_pos, cache, n, tokens=tokens, table=self.embed_in.weight)
+            if h is not None:
+                return h
         return self.hidden_from_embeddings(F.embedding(self.embed_in.weight, tokens), start_pos, cache)
 
     def forward(self, tokens, start_pos: int = 0, cache: Optional[EncoderCache] = None):

@@ -78,9 +78,36 @@ class TransformerEncoder(Module):
     def submodules(self):
         return list(self.blocks) + ([self.final_norm] if self.final_norm is not None else [])
 
+    def infer(self, x, cache: Optional[EncoderCache] = None, causal: bool = False, start_pos: int = 0, **embedding):
+        """The stack without gradients as one native call (on ``x``, or on the tokens and tables in ``embedding``); ``None``
+        when that does not stand for the blocks' own forward passes."""
+        if torch.is_grad_enabled() or not self.blocks:
+            return None
+        from ..ops import stack
+        plain = stack.plain
+        act, layers = self.blocks[0].activation, []
+        for b in self.blocks:
+            m = b.mha
+            if not (plain(b, TransformerBlock) and plain(m, MultiHeadAttention) and plain(b.ln1, LayerNorm) and
+                    plain(b.ln2, LayerNorm) and plain(b.ffn1, Linear) and plain(b.ffn2, Linear) and plain(m.wo, Linear)) or \
+                    b.activation != act or (b.training and b.dropout.p > 0) or \
+                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+                return None
+            layers.append(stack.Layer(m, b.ln1, b.ln2, b.ffn1.weight, b.ffn1.bias, b.ffn2.weight, b.ffn2.bias))
+        if self.final_norm is not None and not plain(self.final_norm, LayerNorm):
+            return None
+        if cache is not None and not (len(cache.layers) == len(layers) and all(type(c) is MHACache for c in cache.layers)):
+            return None
+        return stack.run(layers, x, act=activation_name(act), causal=causal, start_pos=start_pos,
+                         caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)
+
     def forward(self, x, mask=None, cache: Optional[EncoderCache] = None, causal: bool = False, start_pos: int = 0):
         if cache is not None and len(cache.layers) != len(self.blocks):
             raise ValueError("TransformerEncoder: cache has a different number of layers")
+        if mask is None and x.is_cuda:
+            out = self.infer(x, cache, causal, start_pos)
+            if out is not None:
+                return out
         for i, blk in enumerate(self.blocks):
             x = blk(x, mask=mask, cache=None if cache is None else cache.layers[i], causal=causal, start_pos=start_pos)
         return self.final_norm(x) if self.final_norm is not None else x
