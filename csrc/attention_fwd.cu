@@ -98,7 +98,8 @@ struct AttnFwdSmem {
   static_assert(kTotal <= 227 * 1024, "attention forward: shared memory budget");
 };
 
-template <int HD, int NQ, int KST, int VST, bool PREC, bool WIN>
+// SUB: heads of fewer than HD features (a multiple of 8), read through maps with an axis of heads.
+template <int HD, int NQ, int KST, int VST, bool PREC, bool WIN, bool SUB>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmPK,
@@ -205,7 +206,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_arrive_expect_tx(&q_full[t], L::kQBytes);
         for (int c = 0; c < kChunks; ++c) {
           uint8_t* dst = smem + L::kQOff + t * L::kQBytes + c * (kAttnBM * 128);
-          if constexpr (WIN) tma_load_4d(dst, &tmQ, &q_full[t], c * 64, head, q_row0 + t * kAttnBM, batch);
+          if constexpr (WIN || SUB) tma_load_4d(dst, &tmQ, &q_full[t], c * 64, head, q_row0 + t * kAttnBM, batch);
           else tma_load_3d(dst, &tmQ, &q_full[t], head * HD + c * 64, q_row0 + t * kAttnBM, batch);
         }
       }
@@ -219,6 +220,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if constexpr (WIN)
             tma_load_4d(dst, j < n_pool ? &tmPK : &tmK, &k_full[ks], c * 64, kv_head,
                         (j < n_pool ? j : j - n_pool + tile0) * kAttnBN, batch);
+          else if constexpr (SUB) tma_load_4d(dst, &tmK, &k_full[ks], c * 64, kv_head, j * kAttnBN, batch);
           else tma_load_3d(dst, &tmK, &k_full[ks], kv_head * HD + c * 64, j * kAttnBN, batch);
         }
         k_issued = j + 1;
@@ -229,6 +231,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if constexpr (WIN)
             tma_load_4d(dst, j < n_pool ? &tmPV : &tmV, &v_full[vs], c * 64, kv_head,
                         (j < n_pool ? j : j - n_pool + tile0) * kAttnBN, batch);
+          else if constexpr (SUB) tma_load_4d(dst, &tmV, &v_full[vs], c * 64, kv_head, j * kAttnBN, batch);
           else tma_load_3d(dst, &tmV, &v_full[vs], kv_head * HD + c * 64, j * kAttnBN, batch);
         }
         v_issued = j + 1;
@@ -487,7 +490,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // a row without any visible key keeps m_use = -inf (its polynomial exponentials are 2^-127, not 0)
         const bool any_key = l_run > 0.0f && m_use != -INFINITY;
         const float inv = any_key ? 1.0f / l_run : 0.0f;
-        const int dv = WIN ? p.dv : HD;
+        const int dv = WIN || SUB ? p.dv : HD;
         __nv_bfloat16* dst = p.o + ((long long)batch * p.Sq + (live ? q_row : 0)) * p.ldo + (long long)head * dv;
 #pragma unroll
         for (int c = 0; c < HD / 32; ++c) {
@@ -497,8 +500,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (live) {
 #pragma unroll
             for (int d = 0; d < 32; d += 8) {
-              if constexpr (WIN) {
+              if constexpr (WIN || SUB) {
                 if (c * 32 + d >= dv) break;
+              }
+              if constexpr (WIN) {
                 if (p.rot) {      // back by the query's position
                   const float4* cs = reinterpret_cast<const float4*>(p.rot + (long long)(p.pos + q_row) * (dv / 2) +
                                                                      (c * 32 + d) / 2);
@@ -550,20 +555,35 @@ static int encode_tmap_seq(CUtensorMap* map, const void* base, int heads, int hd
   return encode_tmap_nd_bf16(map, base, 3, dims, strides, box);
 }
 
+// dims: {hd, heads, seq, batch}: features past a head's own and rows past the end of a sequence read as zeros.
+static int encode_tmap_heads(CUtensorMap* map, const void* base, int heads, int hd, int seq, int batch, long long ld,
+                             int box_rows, long long batch_rows = 0) {
+  if (batch_rows <= 0) batch_rows = seq;
+  const uint64_t dims[4] = {(uint64_t)hd, (uint64_t)heads, (uint64_t)seq, (uint64_t)batch};
+  const uint64_t strides[3] = {(uint64_t)hd * 2, (uint64_t)ld * 2, (uint64_t)batch_rows * ld * 2};
+  const uint32_t box[4] = {64, 1, (uint32_t)box_rows, 1};
+  return encode_tmap_nd_bf16(map, base, 4, dims, strides, box);
+}
+
 }  // namespace dptb
 
 using namespace dptb;
 
-template <int HD, int NQ, int KST, int VST, bool PREC>
+template <int HD, int NQ, int KST, int VST, bool PREC, bool SUB>
 static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   using L = AttnFwdSmem<HD, NQ, KST, VST, PREC>;
   constexpr int kAttnBN = L::kBN;
   CUtensorMap tmQ, tmK, tmV;
-  int rc = encode_tmap_seq(&tmQ, a->q, a->Hq, HD, a->Sq, a->B, a->ldq, kAttnBM);
+  const int hd = a->head_dim;
+  auto encode = [&](CUtensorMap* map, const void* base, int heads, int seq, long long ld, int box_rows, long long batch_rows) {
+    return SUB ? encode_tmap_heads(map, base, heads, hd, seq, a->B, ld, box_rows, batch_rows)
+               : encode_tmap_seq(map, base, heads, HD, seq, a->B, ld, box_rows, batch_rows);
+  };
+  int rc = encode(&tmQ, a->q, a->Hq, a->Sq, a->ldq, kAttnBM, 0);
   if (rc) return rc;
-  rc = encode_tmap_seq(&tmK, a->k, a->Hkv, HD, a->Sk, a->B, a->ldk, kAttnBN, a->kv_batch_rows);
+  rc = encode(&tmK, a->k, a->Hkv, a->Sk, a->ldk, kAttnBN, a->kv_batch_rows);
   if (rc) return rc;
-  rc = encode_tmap_seq(&tmV, a->v, a->Hkv, HD, a->Sk, a->B, a->ldv, kAttnBN, a->kv_batch_rows);
+  rc = encode(&tmV, a->v, a->Hkv, a->Sk, a->ldv, kAttnBN, a->kv_batch_rows);
   if (rc) return rc;
   AttnFwdParams p = {};
   p.o = static_cast<__nv_bfloat16*>(a->o);
@@ -571,10 +591,11 @@ static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   p.ldo = a->ldo;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv;
   p.causal = a->causal;
+  p.dv = hd;
   p.q_offset = a->q_offset;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   p.num_q_blocks = (a->Sq + NQ * kAttnBM - 1) / (NQ * kAttnBM);
-  auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false>;
+  auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false, SUB>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
   dim3 grid(p.num_q_blocks, a->Hq, a->B);
   kern<<<grid, kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
@@ -601,12 +622,16 @@ extern "C" int dptb_attn_fwd(const DptbAttnFwdArgs* a, void* stream) {
   if ((a->ldq % 8) || (a->ldk % 8) || (a->ldv % 8) || (a->ldo % 8)) return kErrBadShape;
   if ((reinterpret_cast<uintptr_t>(a->o) & 15) != 0) return kErrBadShape;
   if (a->precise) {
-    if (a->head_dim == 64) return attn_fwd_launch<64, 2, 4, 4, true>(a, st);
-    if (a->head_dim == 128) return attn_fwd_launch<128, 2, 3, 3, true>(a, st);
+    if (a->head_dim == 64) return attn_fwd_launch<64, 2, 4, 4, true, false>(a, st);
+    if (a->head_dim == 128) return attn_fwd_launch<128, 2, 3, 3, true, false>(a, st);
     return kErrUnsupported;
   }
-  if (a->head_dim == 64) return attn_fwd_launch<64, 2, 2, 2, false>(a, st);
-  if (a->head_dim == 128) return attn_fwd_launch<128, 2, 2, 1, false>(a, st);
+  if (a->head_dim == 64) return attn_fwd_launch<64, 2, 2, 2, false, false>(a, st);
+  if (a->head_dim == 128) return attn_fwd_launch<128, 2, 2, 1, false, false>(a, st);
+  // Other sizes: the maps have an axis of heads, so a box of 64 features reads zeros behind a head's own.  Padding copies
+  // of Q, K and V cost more than the attention on them: 64 x 119 tokens, 12 heads of 32, B200, 74 us with them, 32 us so.
+  if (a->head_dim > 0 && a->head_dim % 8 == 0 && a->head_dim < 64) return attn_fwd_launch<64, 2, 2, 2, false, true>(a, st);
+  if (a->head_dim % 8 == 0 && a->head_dim > 64 && a->head_dim < 128) return attn_fwd_launch<128, 2, 2, 1, false, true>(a, st);
   return kErrUnsupported;
 }
 
@@ -623,24 +648,17 @@ struct DptbWindowFwdArgs {
   float scale;
 };
 
-static int encode_tmap_heads(CUtensorMap* map, const void* base, int heads, int d, int seq, int batch, int box_rows) {
-  const uint64_t dims[4] = {(uint64_t)d, (uint64_t)heads, (uint64_t)seq, (uint64_t)batch};
-  const uint64_t strides[3] = {(uint64_t)d * 2, (uint64_t)heads * d * 2, (uint64_t)seq * heads * d * 2};
-  const uint32_t box[4] = {64, 1, (uint32_t)box_rows, 1};
-  return encode_tmap_nd_bf16(map, base, 4, dims, strides, box);
-}
-
 template <int HD, int KST, int VST>
 static int window_fwd_launch(const DptbWindowFwdArgs* a, cudaStream_t st) {
   using L = AttnFwdSmem<HD, 2, KST, VST, true>;
   CUtensorMap tmQ, tmK, tmV, tmPK, tmPV;
-  int rc = encode_tmap_heads(&tmQ, a->q, a->H, a->dk, a->S, a->B, kAttnBM);
-  if (!rc) rc = encode_tmap_heads(&tmK, a->k, a->G, a->dk, a->rows, a->B, L::kBN);
-  if (!rc) rc = encode_tmap_heads(&tmV, a->v, a->G, a->dv, a->rows, a->B, L::kBN);
+  int rc = encode_tmap_heads(&tmQ, a->q, a->H, a->dk, a->S, a->B, (long long)a->H * a->dk, kAttnBM);
+  if (!rc) rc = encode_tmap_heads(&tmK, a->k, a->G, a->dk, a->rows, a->B, (long long)a->G * a->dk, L::kBN);
+  if (!rc) rc = encode_tmap_heads(&tmV, a->v, a->G, a->dv, a->rows, a->B, (long long)a->G * a->dv, L::kBN);
   tmPK = tmK;
   tmPV = tmV;
-  if (!rc && a->pool > 0) rc = encode_tmap_heads(&tmPK, a->k_pool, a->G, a->dk, a->pool_rows, a->B, L::kBN);
-  if (!rc && a->pool > 0) rc = encode_tmap_heads(&tmPV, a->v_pool, a->G, a->dv, a->pool_rows, a->B, L::kBN);
+  if (!rc && a->pool > 0) rc = encode_tmap_heads(&tmPK, a->k_pool, a->G, a->dk, a->pool_rows, a->B, (long long)a->G * a->dk, L::kBN);
+  if (!rc && a->pool > 0) rc = encode_tmap_heads(&tmPV, a->v_pool, a->G, a->dv, a->pool_rows, a->B, (long long)a->G * a->dv, L::kBN);
   if (rc) return rc;
   AttnFwdParams p = {};
   p.o = static_cast<__nv_bfloat16*>(a->o);
@@ -653,7 +671,7 @@ static int window_fwd_launch(const DptbWindowFwdArgs* a, cudaStream_t st) {
   p.window = a->window; p.pool = a->pool; p.pool_rows = a->pool_rows; p.pos = a->pos; p.dv = a->dv;
   p.sink = static_cast<const __nv_bfloat16*>(a->sink);
   p.rot = static_cast<const float2*>(a->rot);
-  auto kern = attn_fwd_kernel<HD, 2, KST, VST, true, true>;
+  auto kern = attn_fwd_kernel<HD, 2, KST, VST, true, true, false>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
   kern<<<dim3(p.num_q_blocks, a->H, a->B), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmPK, tmPV, p);
   return counted(1, (int)cudaGetLastError());

@@ -301,7 +301,7 @@ class MultiHeadAttention(Module):
                 # for all keys.  Faster at every length measured (B200): 4 heads of 64 on one key head, 1 x 65 keys,
                 # 6.6 -> 4.5 us; 16 heads of 128 on 4 key heads, 32 x 2049 keys, 153 -> 41 us.
                 return flash.attn_decode_rows(q2, k3, v3, B, Sk, H, Hkv, hd)
-            if flash.kernel_head_dim(hd) == hd:
+            if flash.kernel_head_dim(hd) is not None:
                 k2 = k3.reshape(-1, k3.shape[-1]) if k3.is_contiguous() else None
                 if k2 is not None:
                     o, _ = flash.attn_fwd(q2, k2, v3.reshape(-1, v3.shape[-1]), B, Sq, Sk, H, Hkv, hd, causal,

@@ -68,6 +68,16 @@ def _wants_grad(*tensors) -> bool:
     return torch.is_grad_enabled() and any(t.requires_grad for t in tensors)
 
 
+def _reads_rows(*tensors) -> bool:
+    """Rows in whole 16-byte pieces: what the tensor maps describe."""
+    return all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _raw_call() -> bool:
+    """Whether a kernel call stands for an autograd function without gradients: no forward-mode derivatives, no transforms."""
+    return torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+
+
 def _pad_heads(x2: torch.Tensor, heads: int, hd: int, to: int) -> torch.Tensor:
     """Token-major ``[rows, heads*hd]`` -> ``[rows, heads*to]`` with zeros behind every head's features."""
     return torch.nn.functional.pad(x2.reshape(x2.shape[0], heads, hd), (0, to - hd)).reshape(x2.shape[0], heads * to)
@@ -283,8 +293,8 @@ def attention_packed(qkv, batch, seq, heads, kv_heads, head_dim, causal=True):
 
 def attention_tokens(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causal=True, q_offset=0):
     """Token-major separate operands ``q2 [B*Sq, H hd]``, ``k2`` / ``v2`` ``[B*Sk, Hkv hd]`` (with a KV cache: cache
-    views) -> ``[B*Sq, H hd]``.  bf16 heads of 64 / 128 features run the tensor-core kernels as they are, other sizes
-    zero-padded to the next of the two; what the kernels do not cover (see ``kernel_head_dim``) runs the composed path."""
+    views) -> ``[B*Sq, H hd]``.  bf16 heads of 64 / 128 features run the tensor-core kernels as they are, other sizes as
+    they are without gradients and zero-padded to the next of the two with them; what the kernels do not cover (see ``kernel_head_dim``) runs the composed path."""
     hd_k = kernel_head_dim(head_dim, backward=_wants_grad(q2, k2, v2)) if q2.dtype == torch.bfloat16 else None
     if q2.dtype == torch.float32:
         o = attention_bhsd(_to_bhsd(q2, batch, sq, heads, head_dim), _to_bhsd(k2, batch, sk, kv_heads, head_dim),
@@ -296,6 +306,9 @@ def attention_tokens(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causa
         return o.transpose(1, 2).reshape(batch * sq, heads * head_dim)
     if hd_k == head_dim:
         return SeparateAttentionFn.apply(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causal, q_offset)
+    if not _wants_grad(q2, k2, v2) and _reads_rows(q2, k2, v2) and _raw_call():
+        # the forward kernel reads such heads as they are; only the backward one wants padded operands
+        return attn_fwd(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causal, q_offset=q_offset, need_lse=False)[0]
     o = SeparateAttentionFn.apply(_pad_heads(q2, heads, head_dim, hd_k), _pad_heads(k2, kv_heads, head_dim, hd_k),
                                   _pad_heads(v2, kv_heads, head_dim, hd_k), batch, sq, sk, heads, kv_heads, hd_k, causal,
                                   q_offset, 1.0 / math.sqrt(head_dim))

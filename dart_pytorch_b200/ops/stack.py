@@ -93,7 +93,7 @@ def run(layers: Sequence[Layer], x: Optional[torch.Tensor], *, post_norm=False, 
     if tokens is None and x.shape[-1] != D or max(B, H) > 65535:
         return None
     if bf16:
-        if hd not in (64, 128):
+        if hd <= 0 or hd > 128 or hd % 8:
             return None
     elif hd > 128:
         return None

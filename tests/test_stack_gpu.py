@@ -62,7 +62,7 @@ def test_gpt(monkeypatch, dtype, layers, shape, n):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("H,Hkv,hd", [(4, 1, 64), (4, 2, 128)])
+@pytest.mark.parametrize("H,Hkv,hd", [(4, 1, 64), (4, 2, 128), (4, 2, 32)])
 @pytest.mark.parametrize("shape,n", [((9,), 8), ((33, 20), 18)])
 def test_llama(monkeypatch, dtype, H, Hkv, hd, shape, n):
     m = Llama(LlamaConfig(vocab_size=97, max_ctx=64, embed_dim=H * hd, num_layers=3, num_heads=H, num_kv_heads=Hkv, ffn_dim=200,
@@ -72,7 +72,7 @@ def test_llama(monkeypatch, dtype, H, Hkv, hd, shape, n):
     _same(*_both(monkeypatch, lambda: _steps(m, m.new_cache(), toks, n)))
 
 
-@pytest.mark.parametrize("dtype,hd", [(torch.bfloat16, 64), (torch.float32, 32), (torch.float32, 24)])
+@pytest.mark.parametrize("dtype,hd", [(torch.bfloat16, 64), (torch.bfloat16, 32), (torch.bfloat16, 96), (torch.float32, 32), (torch.float32, 24)])
 @pytest.mark.parametrize("shape", [(5,), (1, 23), (6, 33)])
 def test_bert(monkeypatch, dtype, hd, shape):
     m = BertModel(BertConfig(vocab_size=97, max_position_embeddings=64, embed_dim=4 * hd, num_layers=3, num_heads=4,
