@@ -5,7 +5,7 @@
 //
 // Here the operands are swapped on the tensor core: a CTA owns 128 rows of W (the M = 128 side of tcgen05.mma, all
 // useful bytes) and one slice of K; x is the narrow N = 32 / 64 side.  Work units = (N / 128) x (K splits) are chosen
-// to fill the SMs once, each with an 8-stage TMA ring (128 KB of W in flight per SM).  D[128 weight rows, M] lands
+// to fill the SMs once, with TMA rings of 128 to 160 KB of W in flight per SM.  D[128 weight rows, M] lands
 // in 32 / 64 TMEM columns; a thread of the four epilogue warps owns one weight row = one output column.
 //   splits == 1: the epilogue writes out[m, n] directly (lanes = consecutive n, so stores coalesce);
 //   splits  > 1: fp32 partials go to a workspace, the last unit of a tile (per-tile counter) sums them in split order
@@ -35,7 +35,6 @@ __device__ unsigned long long g_skinny_prof[8];
 
 constexpr int kSkBM = 128;       // weight rows per CTA
 constexpr int kSkBK = 64;
-constexpr int kSkStages = 8;
 constexpr int kSkThreads = 192;  // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 
 struct SkinnyAr {
@@ -100,13 +99,13 @@ __device__ __forceinline__ uint4 ld_relaxed_sys_v4(const uint2* p) {
   return v;
 }
 
-template <int MP>
+template <int MP, int ST>
 struct SkinnySmem {
   static constexpr int kWBytes = kSkBM * kSkBK * 2;     // 16 KB
   static constexpr int kXBytes = MP * kSkBK * 2;        // 4 / 8 KB
   static constexpr int kStage = kWBytes + kXBytes;
-  static constexpr int kBarOff = kSkStages * kStage;
-  static constexpr int kTotal = kBarOff + (2 * kSkStages + 2) * 8 + 64 + 1024;
+  static constexpr int kBarOff = ST * kStage;
+  static constexpr int kTotal = kBarOff + (2 * ST + 2) * 8 + 64 + 1024;
 };
 
 // Final values of one tile -> output (non-tensor-parallel): thread = output column n, v[m] over the rows.
@@ -124,17 +123,17 @@ __device__ __forceinline__ void skinny_store(const SkinnyParams& p, int n, const
   }
 }
 
-template <int MP>
-__global__ void __launch_bounds__(kSkThreads, 1)
+template <int MP, int ST>
+__global__ void __launch_bounds__(kSkThreads, ST <= 5 ? 2 : 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                    const SkinnyParams p) {
-  using L = SkinnySmem<MP>;
+  using L = SkinnySmem<MP, ST>;
   constexpr int TMEM_COLS = MP < 32 ? 32 : MP;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* empty_bar = full_bar + kSkStages;
-  uint64_t* acc_full = empty_bar + kSkStages;
+  uint64_t* empty_bar = full_bar + ST;
+  uint64_t* acc_full = empty_bar + ST;
   uint64_t* drain_bar = acc_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -161,7 +160,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
   if (warp == 1) {
     if (lane == 0) {
-      for (int s = 0; s < kSkStages; ++s) {
+      for (int s = 0; s < ST; ++s) {
         mbar_init(&full_bar[s], 1);
         mbar_init(&empty_bar[s], 1);
       }
@@ -184,7 +183,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       // The weights do not depend on the kernel before this one: the first ring-full of weight tiles is requested at
       // once, then (programmatic dependent launch) the predecessor's completion is awaited, then the activation
       // tiles of those stages follow.  Every stage's barrier expects both tiles.
-      const int pre = max(0, min(kb1 - kb0, kSkStages));
+      const int pre = max(0, min(kb1 - kb0, ST));
       for (int i = 0; i < pre; ++i) {
         mbar_arrive_expect_tx(&full_bar[i], L::kStage);
         tma_load_2d(smem + i * L::kStage, &tmW, &full_bar[i], (kb0 + i) * kSkBK, n0);
@@ -194,8 +193,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tma_load_2d(smem + i * L::kStage + L::kWBytes, &tmX, &full_bar[i], (kb0 + i) * kSkBK, 0);
       int issued = pre;
       for (int kb = kb0 + pre; kb < kb1; ++kb, ++issued) {
-        const int s = issued % kSkStages;
-        const uint32_t ph = (issued / kSkStages) & 1;
+        const int s = issued % ST;
+        const uint32_t ph = (issued / ST) & 1;
         if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, kWaitEmptyTimeout)) break;
         mbar_arrive_expect_tx(&full_bar[s], L::kStage);
         uint8_t* w_dst = smem + s * L::kStage;
@@ -204,11 +203,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
       if (*abort_flag) {
         // Do not leave while a tile copy may still be writing this CTA's shared memory.
-        const int n = issued < kSkStages ? issued : kSkStages;
+        const int n = issued < ST ? issued : ST;
         const uint64_t t0 = global_timer_ns();
         for (int j = 0; j < n; ++j) {
           const int i = issued - 1 - j;
-          while (!mbar_try_wait(&full_bar[i % kSkStages], (i / kSkStages) & 1) &&
+          while (!mbar_try_wait(&full_bar[i % ST], (i / ST) & 1) &&
                  global_timer_ns() - t0 < kWaitLimitNs / 4) {}
         }
       }
@@ -220,8 +219,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       bool issued_any = false, ok = true;
       int consumed = 0;
       for (int kb = kb0; kb < kb1; ++kb, ++consumed) {
-        const int s = consumed % kSkStages;
-        const uint32_t ph = (consumed / kSkStages) & 1;
+        const int s = consumed % ST;
+        const uint32_t ph = (consumed / ST) & 1;
         if (!mbar_wait(&full_bar[s], ph, abort_flag, kWaitFullTimeout)) { ok = false; break; }
         SK_STAMP(2, blockIdx.x == 0 && kb == kb0);
         tc_fence_after_sync();
@@ -532,11 +531,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
-template <int MP>
+template <int MP, int ST>
 static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const SkinnyParams& p, int units,
                          cudaStream_t stream) {
-  using L = SkinnySmem<MP>;
-  auto kern = gemm_skinny_kernel<MP>;
+  using L = SkinnySmem<MP, ST>;
+  auto kern = gemm_skinny_kernel<MP, ST>;
   static bool configured = false;
   if (!configured) {
     DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
@@ -609,6 +608,7 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
   }
   const int mp = a->M <= 32 ? 32 : 64;
   const int tiles = (a->N + kSkBM - 1) / kSkBM;
+  const bool local = !ar && !os;
   const int num_kb = (a->K + kSkBK - 1) / kSkBK;
   // Split K so that the work units fill the SMs once, with at least 4 k-blocks each.
   int splits = a->splits >= 1 ? a->splits : 1;
@@ -619,7 +619,10 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
       return v > 0 ? v : 4;
     }();
     const int by_sm = sm_count() / tiles;
-    const int by_k = num_kb / min_kb;
+    // Writing and folding the partial tiles takes about 2 us, as long as 8 k-blocks and more: a local split has at least
+    // that many (B200, 32 rows: 768 x 768 in one piece 7.0 us, in three 8.9 us; 3072 x 2048 in 4 pieces 11.6 us, in 6 12.5 us;
+    // 2048 x 5504 in 8 pieces 13.9 us, in 18 16.7 us).
+    const int by_k = num_kb / (local && min_kb < 8 ? 8 : min_kb);
     splits = by_sm < by_k ? by_sm : by_k;
     if (splits < 1) splits = 1;
   }
@@ -673,5 +676,9 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
   rc = encode_tmap_2d_bf16(&tmX, a->A, (uint64_t)a->K, (uint64_t)a->M, (uint64_t)a->lda * 2, 64, (uint32_t)mp);
   if (rc) return rc;
   const int units = tiles * splits;
-  return mp == 32 ? launch_skinny<32>(tmW, tmX, p, units, stream) : launch_skinny<64>(tmW, tmX, p, units, stream);
+  // Two CTAs an SM with shorter rings beat one with 8 stages once there are more tiles than SMs: a second wave then fills in
+  // beside the first instead of after it (B200, 32 rows: 50257 x 768 31.6 -> 23.8 us, 32768 x 2048 32.2 -> 26.7 us, the same
+  // within 5 % for fewer tiles).  The collective forms keep one: their CTAs wait for peers.
+  if (local) return mp == 32 ? launch_skinny<32, 5>(tmW, tmX, p, units, stream) : launch_skinny<64, 4>(tmW, tmX, p, units, stream);
+  return mp == 32 ? launch_skinny<32, 8>(tmW, tmX, p, units, stream) : launch_skinny<64, 8>(tmW, tmX, p, units, stream);
 }
