@@ -166,6 +166,8 @@ attn_f32_fwd(const AttnF32Params p) {
   float* Vs = Ks + kFBN * LD;
   float* Ps = Vs + kFBN * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
+  pdl_launch_dependents();
   const int qt = p.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x;    // the longest rows start first
   const int h = blockIdx.y, b = blockIdx.z, hk = h / (p.Hq / p.Hkv), row0 = qt * kFBM;
   f32_load_tile<HD, kFBM>(Qs, p.q, b, h, row0, p.Sq, p.hd, p.vec);
@@ -246,6 +248,8 @@ attn_f32_decode(const AttnF32Params p) {
   const int nc = cluster.num_blocks(), rank = cluster.block_rank();
   const int hk = blockIdx.y, b = blockIdx.z, g = p.Hq / p.Hkv, rows = g * p.Sq;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_wait();
+  pdl_launch_dependents();
   // row r: query head hk * g + r / Sq, position r % Sq
   for (int i = tid; i < R * HD; i += kFThreads) {
     const int r = i / HD, d = i % HD;
@@ -566,18 +570,19 @@ static int attn_f32_launch(const AttnF32Params& p, int backward, cudaStream_t st
       cfg.blockDim = dim3(kFThreads);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = st;
-      cudaLaunchAttribute at[1];
+      cudaLaunchAttribute at[2];
       at[0].id = cudaLaunchAttributeClusterDimension;
       at[0].val.clusterDim.x = nc;
       at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
-      cfg.numAttrs = 1;
+      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.numAttrs = pdl_flag() ? 2 : 1;
       return counted(1, (int)cudaLaunchKernelEx(&cfg, attn_f32_decode<HD>, p));
     }
     const int smem = f32_smem<HD>(kFBM + 2 * kFBN, kFBM);
     DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_fwd<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attn_f32_fwd<HD><<<qgrid, kFThreads, smem, st>>>(p);
-    return counted(1, (int)cudaGetLastError());
+    return counted(1, (int)launch_k(attn_f32_fwd<HD>, qgrid, dim3(kFThreads), (size_t)smem, st, p));
   }
   const int smem_q = f32_smem<HD>(2 * kFBM + 2 * kFBN, kFBM), smem_kv = f32_smem<HD>(2 * kFBM + 2 * kFBN, 2 * kFBM);
   DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_dq<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));

@@ -108,9 +108,10 @@ inline int sm_count() {
 }
 
 // Whether the kernels that support it are launched as programmatic dependents of their predecessor on the stream
-// (see pdl_wait below).  Off by default; the tensor-parallel decode engine turns it on around its step.
+// (see pdl_wait below).  Off by default and a thread's own; the decode engines and short inference stacks turn it on around
+// their step.
 inline int& pdl_flag() {
-  static int on = 0;
+  static thread_local int on = 0;
   return on;
 }
 

@@ -125,7 +125,8 @@ struct F32Tile {
   static_assert(R * kF32BK / 4 % THREADS == 0, "whole 16-byte groups per thread");
   float4 v[kVecs];
 
-  __device__ __forceinline__ void load(const float* __restrict__ src, long long ld, int mn0, int mn_end, int k0, int k_end,
+  // Plain loads: a programmatic dependent starts before its input is complete, so no read may count as constant.
+  __device__ __forceinline__ void load(const float* src, long long ld, int mn0, int mn_end, int k0, int k_end,
                                        int vec) {
 #pragma unroll
     for (int i = 0; i < kVecs; ++i) {
@@ -136,24 +137,24 @@ struct F32Tile {
         const float* g = src + (long long)k * ld + mn;
         if (k < k_end) {
           if (vec && mn + 3 < mn_end) {
-            v[i] = __ldg(reinterpret_cast<const float4*>(g));
+            v[i] = *reinterpret_cast<const float4*>(g);
             continue;
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (mn + j < mn_end) e[j] = __ldg(g + j);
+            if (mn + j < mn_end) e[j] = g[j];
         }
       } else {
         const int mn = mn0 + idx / (kF32BK / 4), k = k0 + idx % (kF32BK / 4) * 4;
         const float* g = src + (long long)mn * ld + k;
         if (mn < mn_end) {
           if (vec && k + 3 < k_end) {
-            v[i] = __ldg(reinterpret_cast<const float4*>(g));
+            v[i] = *reinterpret_cast<const float4*>(g);
             continue;
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (k + j < k_end) e[j] = __ldg(g + j);
+            if (k + j < k_end) e[j] = g[j];
         }
       }
       v[i] = make_float4(e[0], e[1], e[2], e[3]);
@@ -190,6 +191,8 @@ gemm_f32_kernel(const GemmF32Params p) {
   __shared__ int s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tx = (warp % (TX / WX)) * WX + (lane & 7), ty = (warp / (TX / WX)) * 4 + (lane >> 3);
+  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
+  pdl_launch_dependents();
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const int k_begin = blockIdx.z * p.k_per_split;
   const int k_end = min(p.K, k_begin + p.k_per_split);
@@ -320,27 +323,35 @@ gemv_f32_kernel(const GemmF32Params p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group = warp / WPR, sub = warp % WPR;
   const int n0 = (blockIdx.x * GROUPS + group) * ROWS;
+  // The weights do not depend on the kernel before this one: as a programmatic dependent the first of them are under way
+  // while that one finishes.
+  constexpr int PRE = MR <= 4 ? 4 : 1, STEP = WPR * 128;
+  const float* w[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) w[r] = p.B + (long long)min(n0 + r, p.N - 1) * p.ldb;
+  const int kv = (p.vec_a && p.vec_b) ? p.K / 4 * 4 : 0, k_first = (sub * 32 + lane) * 4;
+  float4 pre[PRE][ROWS];
+#pragma unroll
+  for (int u = 0; u < PRE; ++u)
+    if (k_first + u * STEP < kv) {
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) pre[u][r] = __ldg(reinterpret_cast<const float4*>(w[r] + k_first + u * STEP));
+    }
+  pdl_wait();
+  pdl_launch_dependents();
   float acc[ROWS][MR];
 #pragma unroll
   for (int r = 0; r < ROWS; ++r)
 #pragma unroll
     for (int m = 0; m < MR; ++m) acc[r][m] = 0.0f;
   if (n0 < p.N) {
-    const float* w[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) w[r] = p.B + (long long)min(n0 + r, p.N - 1) * p.ldb;
     const float* x[MR];
 #pragma unroll
     for (int m = 0; m < MR; ++m) x[m] = p.A + (long long)min(m, p.M - 1) * p.lda;
-    const int kv = (p.vec_a && p.vec_b) ? p.K / 4 * 4 : 0;
-#pragma unroll 4
-    for (int k = (sub * 32 + lane) * 4; k < kv; k += WPR * 128) {
-      float4 wv[ROWS];
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) wv[r] = __ldg(reinterpret_cast<const float4*>(w[r] + k));
+    auto add = [&](const float4 (&wv)[ROWS], int k) {
 #pragma unroll
       for (int m = 0; m < MR; ++m) {
-        const float4 xv = __ldg(reinterpret_cast<const float4*>(x[m] + k));
+        const float4 xv = *reinterpret_cast<const float4*>(x[m] + k);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
           acc[r][m] = fmaf(wv[r].x, xv.x, acc[r][m]);
@@ -349,13 +360,23 @@ gemv_f32_kernel(const GemmF32Params p) {
           acc[r][m] = fmaf(wv[r].w, xv.w, acc[r][m]);
         }
       }
+    };
+#pragma unroll
+    for (int u = 0; u < PRE; ++u)
+      if (k_first + u * STEP < kv) add(pre[u], k_first + u * STEP);
+#pragma unroll 4
+    for (int k = k_first + PRE * STEP; k < kv; k += STEP) {
+      float4 wv[ROWS];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) wv[r] = __ldg(reinterpret_cast<const float4*>(w[r] + k));
+      add(wv, k);
     }
     for (int k = kv + sub * 32 + lane; k < p.K; k += WPR * 32) {
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
         const float wk = __ldg(w[r] + k);
 #pragma unroll
-        for (int m = 0; m < MR; ++m) acc[r][m] = fmaf(wk, __ldg(x[m] + k), acc[r][m]);
+        for (int m = 0; m < MR; ++m) acc[r][m] = fmaf(wk, x[m][k], acc[r][m]);
       }
     }
 #pragma unroll
@@ -381,26 +402,20 @@ gemv_f32_kernel(const GemmF32Params p) {
 }
 
 template <int MR, int ROWS>
-static void launch_gemv(const GemmF32Params& p, cudaStream_t st) {
+static cudaError_t launch_gemv(const GemmF32Params& p, cudaStream_t st) {
   // One warp per group of rows when that fills the SMs with at least two CTAs each, else four.
   const int groups = (p.N + ROWS - 1) / ROWS;
-  if (groups >= sm_count() * 16)
-    gemv_f32_kernel<MR, 1, ROWS><<<(groups + 7) / 8, kVecThreads, 0, st>>>(p);
-  else
-    gemv_f32_kernel<MR, 4, ROWS><<<(groups + 1) / 2, kVecThreads, 0, st>>>(p);
+  return groups >= sm_count() * 16 ? launch_k(gemv_f32_kernel<MR, 1, ROWS>, dim3((groups + 7) / 8), dim3(kVecThreads), 0, st, p)
+                                   : launch_k(gemv_f32_kernel<MR, 4, ROWS>, dim3((groups + 1) / 2), dim3(kVecThreads), 0, st, p);
 }
 
 template <int BM, int BN, int TM, int TN>
-static void launch_tiles(const GemmF32Params& p, bool amn, bool bmn, cudaStream_t st) {
+static cudaError_t launch_tiles(const GemmF32Params& p, bool amn, bool bmn, cudaStream_t st) {
   const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.splits);
   constexpr int T = (BM / TM) * (BN / TN);
-  if (amn) {
-    if (bmn) gemm_f32_kernel<BM, BN, TM, TN, true, true><<<grid, T, 0, st>>>(p);
-    else gemm_f32_kernel<BM, BN, TM, TN, true, false><<<grid, T, 0, st>>>(p);
-  } else {
-    if (bmn) gemm_f32_kernel<BM, BN, TM, TN, false, true><<<grid, T, 0, st>>>(p);
-    else gemm_f32_kernel<BM, BN, TM, TN, false, false><<<grid, T, 0, st>>>(p);
-  }
+  const auto kern = amn ? (bmn ? gemm_f32_kernel<BM, BN, TM, TN, true, true> : gemm_f32_kernel<BM, BN, TM, TN, true, false>)
+                        : (bmn ? gemm_f32_kernel<BM, BN, TM, TN, false, true> : gemm_f32_kernel<BM, BN, TM, TN, false, false>);
+  return launch_k(kern, grid, dim3(T), 0, st, p);
 }
 
 }  // namespace dptb
@@ -432,11 +447,8 @@ int gemm_f32(const DptbGemmArgs* a, void* stream_v) {
   const bool amn = a->trans_a != 0, bmn = a->trans_b == 0;
 
   if (a->M <= 8 && !amn && !bmn && a->bn == 0 && a->splits <= 1) {
-    if (a->M == 1) launch_gemv<1, 2>(p, st);
-    else if (a->M == 2) launch_gemv<2, 2>(p, st);
-    else if (a->M <= 4) launch_gemv<4, 2>(p, st);
-    else launch_gemv<8, 2>(p, st);
-    return counted(1, (int)cudaGetLastError());
+    return counted(1, (int)(a->M == 1 ? launch_gemv<1, 2>(p, st) : a->M == 2 ? launch_gemv<2, 2>(p, st)
+                          : a->M <= 4 ? launch_gemv<4, 2>(p, st) : launch_gemv<8, 2>(p, st)));
   }
 
   // Tile and split of K by a small model of an SM: the CTAs that land on the busiest one share its multiply-add
@@ -468,8 +480,6 @@ int gemm_f32(const DptbGemmArgs* a, void* stream_v) {
   p.splits = a->K > 0 ? (a->K + p.k_per_split - 1) / p.k_per_split : 1;   // every split non-empty
   if (p.k_per_split == 0) p.k_per_split = kF32BK;
   if ((a->M + kTiles[best].bm - 1) / kTiles[best].bm > 65535) return kErrBadShape;
-  if (best == 0) launch_tiles<128, 128, 8, 8>(p, amn, bmn, st);
-  else if (best == 1) launch_tiles<64, 64, 8, 4>(p, amn, bmn, st);
-  else launch_tiles<32, 64, 4, 4>(p, amn, bmn, st);
-  return counted(1, (int)cudaGetLastError());
+  return counted(1, (int)(best == 0 ? launch_tiles<128, 128, 8, 8>(p, amn, bmn, st)
+                        : best == 1 ? launch_tiles<64, 64, 8, 4>(p, amn, bmn, st) : launch_tiles<32, 64, 4, 4>(p, amn, bmn, st)));
 }

@@ -95,7 +95,7 @@ Layout layout(const DptbStackArgs* a) {
 
 extern "C" long long dptb_stack_ws_bytes(const DptbStackArgs* a) { return layout(a).total; }
 
-extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table, void* stream) {
+static int stack_launch(const DptbStackArgs* a, const void* const* table, void* stream) {
   const long long rows = (long long)a->B * a->S;
   if (rows <= 0 || a->layers <= 0) return kErrBadShape;
   if (rows > 0x7fffffffLL || a->H <= 0 || a->Hkv <= 0 || a->H % a->Hkv) return kErrBadShape;
@@ -237,4 +237,16 @@ extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table
   if (!a->post_norm && a->final_g) DPTB_STACK_OK(norm(cur, a->final_g, a->final_b, a->out, a->final_eps, a->rms));
 #undef DPTB_STACK_OK
   return 0;
+}
+
+// A step of few rows is a chain of short kernels: those that support it start as programmatic dependents of one another, so
+// their set-up (and the first weights of the matrix products) overlaps the end of the kernel before.
+constexpr long long kChainedRows = 64;
+extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table, void* stream) {
+  int& pdl = pdl_flag();
+  const int before = pdl;
+  if ((long long)a->B * a->S <= kChainedRows) pdl = 1;
+  const int rc = stack_launch(a, table, stream);
+  pdl = before;
+  return rc;
 }
