@@ -177,6 +177,7 @@ def _declare(lib: ctypes.CDLL) -> None:
     sig("dptb_mean_f32", P, L, P, F, P)
     sig("dptb_embedding_fwd", P, L, P, P, L, I, I, P, L, I, I, P)
     sig("dptb_embedding_bwd", P, L, P, P, P, P, L, I, I, P)
+    sig("dptb_embedding_bwd_scan", P, L, P, P, L, I, I, P)
     sig("dptb_pos_embedding_bwd", P, L, I, I, L, P, I, I, P)
     sig("dptb_sqnorm_parts", L)
     sig("dptb_grad_norm", P, L, I, P, P, F, I, P)

@@ -277,12 +277,19 @@ def embedding_fwd(table, idx, pos_table=None, pos_start: int = 0, seq_len: int =
     return out.view(*idx.shape, D)
 
 
+EMBED_SCAN_TOKENS = 4096      # index lists up to this long are scanned for equal entries, longer ones sorted (csrc/embed.cu)
+
+
 def embedding_bwd(dtable, idx, dout, deterministic: bool = True):
     """``dtable[idx[n]] += dout[n]`` in place."""
     lib = N.load()
     idx = idx.reshape(-1).contiguous()
     n, D = idx.numel(), dtable.shape[1]
     dout2 = dout.reshape(n, D).contiguous()
+    if deterministic and n <= EMBED_SCAN_TOKENS and dtable.shape[0] < 2 ** 31:
+        N.check(lib.dptb_embedding_bwd_scan(dtable.data_ptr(), dtable.shape[0], idx.data_ptr(), dout2.data_ptr(), n, D,
+                                            N.dtype_code(dtable), N.stream_ptr()), "embedding_bwd_scan")
+        return dtable
     sidx = perm = None
     if deterministic:
         sidx, perm = torch.sort(idx, stable=True)
