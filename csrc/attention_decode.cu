@@ -8,10 +8,9 @@
 //
 // attn_decode_kernel: grid (splits, Hkv, B * Sq).  A CTA owns one (sequence, query position, kv head) and a contiguous
 // chunk of the keys; its 4 warps take 16-key rounds round-robin, each through a private two-stage cp.async ring in
-// shared memory (the next round's K and V rows are in flight while this one is computed).  A key / value row is
-// covered by hd/8 lanes with 16 bytes each, scores of the G = Hq / Hkv grouped heads are reduced with shuffles inside
-// those lanes (packed fp32 multiply-adds), the softmax is computed per round and the round's probabilities are fetched
-// back by shuffle for the P.V accumulation.  Partial (max, sum, acc) per warp are merged in shared memory and, when
+// shared memory (the next round's K and V rows are in flight while this one is computed).  Scores
+// and P.V of the G = Hq / Hkv grouped heads are warp-level matrix products, the softmax is computed per round.  (The windowed
+// form, whose rows and heads have other sizes, covers a row by hd/8 lanes with packed multiply-adds and shuffles.)  Partial (max, sum, acc) per warp are merged in shared memory and, when
 // the keys are split across CTAs, through an fp32 workspace: the last CTA of a (query row, kv head) to finish merges
 // the splits itself (arrival counter), so one kernel runs per call (attn_decode_merge_kernel remains for shapes beyond
 // the counter table).
@@ -146,29 +145,6 @@ attn_decode_kernel(const DecodeArgs a) {
   __shared__ float s_m[kDecWarps][GP], s_l[kDecWarps][GP];
   __shared__ float s_acc[kDecWarps][GP][HD];
 
-  f32x2 qv[GP][4];
-  const __nv_bfloat16* qrow = a.q + (long long)bs * a.ldq + (long long)g * G * dk + sl * 8;
-  const f32x2 scale2 = f2_splat(a.scale);
-#pragma unroll
-  for (int h = 0; h < GP; ++h) {
-    if (h < G && (!WIN || sl * 8 < dk)) {
-      unpack_bf16x8_f2(*reinterpret_cast<const uint4*>(qrow + h * dk), qv[h]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) qv[h][e] = f2_mul(qv[h][e], scale2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) qv[h][e] = f2_splat(0.0f);
-    }
-  }
-  float m[GP], l[GP];
-  f32x2 acc[GP][4];
-#pragma unroll
-  for (int h = 0; h < GP; ++h) {
-    m[h] = -INFINITY;
-    l[h] = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[h][e] = f2_splat(0.0f);
-  }
   const __nv_bfloat16* kb = a.k + (long long)b * a.kv_batch_stride + (long long)g * HD;
   const __nv_bfloat16* vb = a.v + (long long)b * a.kv_batch_stride + (long long)g * HD;
   const int ldk = a.Hkv * dk, ldv = a.Hkv * dv;                // windowed form: rows of the ring and of the pooled blocks
@@ -200,13 +176,141 @@ attn_decode_kernel(const DecodeArgs a) {
         cp_async_16_or_zero(dst + kStageChunks + c, f < dv ? vr + f : vr, f < dv);
       } else {
         const long long off = (long long)key * a.ldkv + (c % LPK) * 8;
-        cp_async_16(dst + c, kb + off);
-        cp_async_16(dst + kStageChunks + c, vb + off);
+        const int at = c ^ (c / LPK & 7);       // 16-byte pieces of eight neighbouring rows fall on different banks
+        cp_async_16(dst + at, kb + off);
+        cp_async_16(dst + kStageChunks + at, vb + off);
       }
     }
     cp_async_commit();
   };
   if (warp < rounds) issue(warp, 0);
+  if constexpr (!WIN) {
+    // Scores^T and outputs^T by warp-level matrix instructions, the query heads of the group as their 8 columns: a round of 16 keys
+    // is about 150 instructions, where multiply-adds and shuffles took about 1000 (4 heads of 128) and bounded the kernel.
+    // The weights go in as three bf16 parts, which hold all 24 bits of them.
+    // Measured (B200, 32 sequences of 2049 keys, 16 heads of 128 on 4 key heads): 40.5 -> 32.0 us
+    // (20.5 us are the keys and values at copy speed); 8 heads on one key head 35.2 -> 25.3 us; one head a group: the same.
+    uint32_t qf[HD / 16][2];                  // Q^T: head lane / 4, features (lane % 4) * 2 and the next, and 8 further on
+    {
+      const int h = lane >> 2;
+      const __nv_bfloat16* qr = a.q + (long long)bs * a.ldq + (long long)(g * G + (h < G ? h : 0)) * HD + (lane & 3) * 2;
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k) {
+        qf[k][0] = h < G ? *reinterpret_cast<const uint32_t*>(qr + k * 16) : 0u;
+        qf[k][1] = h < G ? *reinterpret_cast<const uint32_t*>(qr + k * 16 + 8) : 0u;
+      }
+    }
+    float m2[2] = {-INFINITY, -INFINITY}, l2[2] = {0.0f, 0.0f};   // heads (lane % 4) * 2 and the next; l2: this lane's keys only
+    float o[HD / 16][4];                      // features i * 16 + lane / 4 (and 8 further on) of those heads
+#pragma unroll
+    for (int i = 0; i < HD / 16; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
+    const int mrow = lane & 7, mat = lane >> 3;
+    const int k_row = (mat & 1) * 8 + mrow, k_chunk = mat >> 1;   // this lane's row of the four 8 x 8 matrices of a load
+    const int v_row = (mat >> 1) * 8 + mrow, v_chunk = mat & 1;
+    int it_local = 0;
+    for (int t = warp; t < rounds; t += kDecWarps, ++it_local) {
+      const int stage = it_local & 1;
+      if (t + kDecWarps < rounds) {
+        issue(t + kDecWarps, stage ^ 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncwarp();
+      const uint32_t ks = smem_u32(ring + stage * 2 * kStageChunks), vs = ks + kStageChunks * 16;
+      float sc[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k) {
+        uint32_t kf[4];
+        ldmatrix_x4(kf, ks + (k_row * LPK + ((2 * k + k_chunk) ^ mrow)) * 16);
+        mma_bf16_16816(sc[k & 1], kf, qf[k][0], qf[k][1]);
+      }
+      const int key = j0 + t * kDecRound + (lane >> 2);
+      const bool live[2] = {key < j1, key + 8 < j1};
+      float p[2][2], corr[2];                 // [key, key + 8][head]
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float sv[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) sv[r] = live[r] ? (sc[0][2 * r + e] + sc[1][2 * r + e]) * a.scale : -INFINITY;
+        float mx = fmaxf(sv[0], sv[1]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float nm = fmaxf(m2[e], mx);
+        corr[e] = __expf(m2[e] - nm);         // 0 on the first round (m = -inf)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) p[r][e] = live[r] ? __expf(sv[r] - nm) : 0.0f;
+        l2[e] = l2[e] * corr[e] + (p[0][e] + p[1][e]);
+        m2[e] = nm;
+      }
+      // The parts of the weights (leading bits, next, rest), keys along a thread's pair.  Those of a positive weight stay
+      // positive, so that its product with an infinite value is infinite in each.
+      uint32_t pp[3][2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float rest[2] = {p[r][0], p[r][1]};
+#pragma unroll
+        for (int part = 0; part < 3; ++part) {
+          const uint32_t u0 = __float_as_uint(rest[0]), u1 = __float_as_uint(rest[1]);
+          pp[part][r] = movmatrix_trans((u0 >> 16) | (u1 & 0xffff0000u));
+          rest[0] = p[r][0] > 0.0f ? fmaxf(rest[0] - __uint_as_float(u0 & 0xffff0000u), 1.2e-38f) : 0.0f;
+          rest[1] = p[r][1] > 0.0f ? fmaxf(rest[1] - __uint_as_float(u1 & 0xffff0000u), 1.2e-38f) : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < HD / 16; ++i) {
+        uint32_t vf[4];
+        ldmatrix_x4_trans(vf, vs + (v_row * LPK + ((2 * i + v_chunk) ^ mrow)) * 16);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] *= corr[e & 1];
+#pragma unroll
+        for (int part = 0; part < 3; ++part) mma_bf16_16816(o[i], vf, pp[part][0], pp[part][1]);
+      }
+      __syncwarp();   // every lane has read this stage before the load two rounds ahead overwrites it
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int off = 4; off < 32; off <<= 1) l2[e] += __shfl_xor_sync(0xffffffffu, l2[e], off);
+      const int h = (lane & 3) * 2 + e;
+      if (h < GP) {
+        if (lane < 4) {
+          s_m[warp][h] = m2[e];
+          s_l[warp][h] = l2[e];
+        }
+#pragma unroll
+        for (int i = 0; i < HD / 16; ++i) {
+          s_acc[warp][h][i * 16 + (lane >> 2)] = o[i][e];
+          s_acc[warp][h][i * 16 + 8 + (lane >> 2)] = o[i][2 + e];
+        }
+      }
+    }
+  } else {
+  f32x2 qv[GP][4];
+  const __nv_bfloat16* qrow = a.q + (long long)bs * a.ldq + (long long)g * G * dk + sl * 8;
+  const f32x2 scale2 = f2_splat(a.scale);
+#pragma unroll
+  for (int h = 0; h < GP; ++h) {
+    if (h < G && (!WIN || sl * 8 < dk)) {
+      unpack_bf16x8_f2(*reinterpret_cast<const uint4*>(qrow + h * dk), qv[h]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) qv[h][e] = f2_mul(qv[h][e], scale2);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) qv[h][e] = f2_splat(0.0f);
+    }
+  }
+  float m[GP], l[GP];
+  f32x2 acc[GP][4];
+#pragma unroll
+  for (int h = 0; h < GP; ++h) {
+    m[h] = -INFINITY;
+    l[h] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[h][e] = f2_splat(0.0f);
+  }
   int it_local = 0;
   for (int t = warp; t < rounds; t += kDecWarps, ++it_local) {
     const int stage = it_local & 1;
@@ -287,6 +391,7 @@ attn_decode_kernel(const DecodeArgs a) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) s_acc[warp][h][lane * 8 + e] = af[e];
     }
+  }
   }
   __syncthreads();
   for (int idx = threadIdx.x; idx < G * HD; idx += blockDim.x) {
