@@ -27,8 +27,8 @@ def test_against_fp64(hd, H, Hkv, Sk, splits):
     k[:, Sk:], v[:, Sk:] = float("nan"), float("nan")               # rows nobody may read
     o = D.attn_decode(q, k, v, B, 1, Sk, H, Hkv, hd, Sk - 1, splits=splits)
     want = _want(q, k[:, :Sk], v[:, :Sk], H, Hkv, hd)
-    # weights and sums carry 24 bits: the result's own rounding (2^-9, root mean square half of that) is what shows
-    assert float((o.double() - want).norm() / want.norm()) < 2.0 ** -9
+    # weights and sums carry 24 bits: the result's own rounding is what shows, at most 2^-8 of each element
+    assert float((o.double() - want).norm() / want.norm()) < 2.0 ** -8
 
 
 def test_large_scores_and_infinite_values():
