@@ -19,11 +19,9 @@ __device__ __forceinline__ float group_sum(float v, float* scratch) {
   return block_sum(v, scratch);
 }
 
-// G threads cooperate on one row; a block of 256 threads handles 256 / G rows per iteration.  Bound by memory.  Rows of
-// more than 4 vectors per lane (V > 4) leave room for two blocks an SM only; there the next row is requested before this one is
-// reduced.  (Tried for shorter rows too: 16384 x 768 11.9 us without, 12.3 us with it.)
+// G threads cooperate on one row; a block of 256 threads handles 256 / G rows per iteration.
 template <typename T, int G, int V, bool RMS>
-__global__ void __launch_bounds__(kNormThreads, V > 4 ? 2 : 3)
+__global__ void __launch_bounds__(kNormThreads, 3)
 norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int D, float eps) {
   __shared__ float scratch[33];
@@ -32,18 +30,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
   constexpr int RPB = kNormThreads / G;
   const int g = threadIdx.x / G, t = threadIdx.x % G;
   const int nvec = D / 8;
-  const long long stride = (long long)gridDim.x * RPB;
-  constexpr bool kAhead = V > 4;
-  Raw8<T> next[V];
-  auto request = [&](long long r) {
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-      const int vi = t + i * G;
-      if (r < rows && vi < nvec) next[i].load(x + r * D + vi * 8);
-    }
-  };
-  if (kAhead) request((long long)blockIdx.x * RPB + g);
-  for (long long base = (long long)blockIdx.x * RPB; base < rows; base += stride) {
+  for (long long base = (long long)blockIdx.x * RPB; base < rows; base += (long long)gridDim.x * RPB) {
     const long long r = base + g;
     const bool live = r < rows;
     float v[V][8];
@@ -52,13 +39,11 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
     for (int i = 0; i < V; ++i) {
       const int vi = t + i * G;
       if (live && vi < nvec) {
-        if constexpr (kAhead) next[i].unpack(v[i]);
-        else Vec8<T>::load(x + r * D + vi * 8, v[i]);
+        Vec8<T>::load(x + r * D + vi * 8, v[i]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += RMS ? v[i][j] * v[i][j] : v[i][j];
       }
     }
-    if (kAhead) request(r + stride);
     s = group_sum<G>(s, scratch);
     float mean = 0.0f, rstd;
     if (RMS) {
@@ -344,14 +329,6 @@ static int norm_fwd_launch(const void* x, const void* gamma, const void* beta, v
     if (blocks > nsm * 8) blocks = nsm * 8;
     DPTB_NORM_DISPATCH_V((nvec + 31) / 32, (launch_k(norm_fwd_kernel<T, 32, V, RMS>, dim3((int)blocks), dim3(kNormThreads), 0, st,
                  (const T*)x, (const T*)gamma, (const T*)beta, (T*)y, mean, rstd, rows, D, eps)));
-  } else if (sizeof(T) == 2 && al && D % 8 == 0 && nvec <= 32 * 8 && rows >= nsm * 32) {
-    // bf16 rows of up to 2048 elements when every resident warp gets two of them: a warp per row needs no block barrier.
-    // B200, layer norm / RMS norm: 8192 x 2048 24.4 -> 17.7 / 17.9 -> 12.0 us, 8192 x 1536 23.8 -> 13.2 / 17.6 -> 8.8 us;
-    // 2000 x 2048 got slower (RMS 4.9 -> 5.4 us).
-    const long long blocks = nsm * 2;
-    using B = __nv_bfloat16;
-    launch_k(nvec <= 32 * 6 ? norm_fwd_kernel<B, 32, 6, RMS> : norm_fwd_kernel<B, 32, 8, RMS>, dim3((int)blocks),
-             dim3(kNormThreads), 0, st, (const B*)x, (const B*)gamma, (const B*)beta, (B*)y, mean, rstd, rows, D, eps);
   } else if (al && D % 8 == 0 && nvec <= 256 * kNormMaxVec) {
     long long blocks = rows < nsm * 8 ? rows : nsm * 8;
     DPTB_NORM_DISPATCH_V((nvec + 255) / 256, (launch_k(norm_fwd_kernel<T, 256, V, RMS>, dim3((int)blocks), dim3(kNormThreads), 0, st,
