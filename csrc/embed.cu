@@ -110,7 +110,8 @@ embedding_bwd_sorted_kernel(T* __restrict__ dtable, long long vocab, const long 
 // memory (32 keys a step, compared by ballot), blockIdx.y takes 256 features; up to four rows are loaded before they are added.
 // A sort of the list costs 25 us and more whatever its length.  Measured (B200, whole backward, against the one with the
 // sort): 603 tokens of 128 features 6.3 us, 33 us with it; 1024 tokens over 65 indices, 256 features, 12 and 38 us;
-// 4096 tokens over 50257 indices, 768 features, 39 and 42 us; 8192 of them 131 and 104 us, so lists stop at 4096.
+// 2048 tokens over 50257 indices, 768 features, 13 and 35 us;
+// 4096 of them 39 and 42 us, 8192 131 and 104 us, so lists stop at 2048.
 template <typename T>
 __global__ void __launch_bounds__(256)
 embedding_bwd_scan_kernel(T* __restrict__ dtable, int vocab, const long long* __restrict__ idx, const T* __restrict__ dout,
@@ -217,7 +218,7 @@ extern "C" int dptb_embedding_fwd(const void* table, long long vocab, const long
   return counted(1, (int)cudaGetLastError());
 }
 // The list as it is, at most kScanTokens long.
-constexpr int kScanTokens = 8192;
+constexpr int kScanTokens = 2048;
 extern "C" int dptb_embedding_bwd_scan(void* dtable, long long vocab, const long long* idx, const void* dout, long long n, int D,
                                        int dtype, void* stream) {
   if (n <= 0 || D <= 0) return 0;

@@ -277,7 +277,7 @@ def embedding_fwd(table, idx, pos_table=None, pos_start: int = 0, seq_len: int =
     return out.view(*idx.shape, D)
 
 
-EMBED_SCAN_TOKENS = 4096      # index lists up to this long are scanned for equal entries, longer ones sorted (csrc/embed.cu)
+EMBED_SCAN_TOKENS = 2048      # index lists up to this long are scanned for equal entries, longer ones sorted (csrc/embed.cu)
 
 
 def embedding_bwd(dtable, idx, dout, deterministic: bool = True):
