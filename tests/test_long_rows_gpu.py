@@ -1,4 +1,4 @@
-"""Norms over many rows (a warp per row, rows requested ahead) and long cross-entropy rows, against fp64."""
+"""Norms over many rows and long cross-entropy rows, against fp64."""
 import pytest
 import torch
 
