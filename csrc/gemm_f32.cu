@@ -49,7 +49,8 @@ struct GemmF32Params {
 __device__ __forceinline__ float act_f32(int act, float x) {
   switch (act) {
     case 1: return fmaxf(x, 0.0f);
-    case 2: return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+    case 2:
+    case 5: return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
     case 3: return x / (1.0f + expf(-1.702f * x));
     case 4: return x / (1.0f + expf(-x));
     default: return x;
@@ -74,10 +75,12 @@ __device__ __forceinline__ float act_grad_f32(int act, float x) {
     default: return 1.0f;
   }
 }
+// What goes to aux_out: the value before the activation, or (code 5) GELU's derivative there.
+__device__ __forceinline__ float aux_f32(int act, float x) { return act == 5 ? act_grad_f32(12, x) : x; }
 __device__ __forceinline__ void epilogue_f32(const GemmF32Params& p, long long row, int col, float v) {
   v *= p.alpha;
   if (p.bias) v += p.bias_f32 ? static_cast<const float*>(p.bias)[col] : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
-  if (p.aux_out) p.aux_out[row * p.ld_aux_out + col] = v;
+  if (p.aux_out) p.aux_out[row * p.ld_aux_out + col] = aux_f32(p.act, v);
   if (p.act >= 11) v *= act_grad_f32(p.act, p.aux_in[row * p.ld_aux_in + col]);
   else if (p.act) v = act_f32(p.act, v);
   if (p.residual) v += p.residual[row * p.ldr + col];
@@ -93,7 +96,9 @@ __device__ __forceinline__ void epilogue_f32x4(const GemmF32Params& p, long long
       v[j] += p.bias_f32 ? static_cast<const float*>(p.bias)[col + j]
                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + j]);
   }
-  if (p.aux_out) *reinterpret_cast<float4*>(p.aux_out + row * p.ld_aux_out + col) = make_float4(v[0], v[1], v[2], v[3]);
+  if (p.aux_out)
+    *reinterpret_cast<float4*>(p.aux_out + row * p.ld_aux_out + col) =
+        make_float4(aux_f32(p.act, v[0]), aux_f32(p.act, v[1]), aux_f32(p.act, v[2]), aux_f32(p.act, v[3]));
   if (p.act >= 11) {
     const float4 x = *reinterpret_cast<const float4*>(p.aux_in + row * p.ld_aux_in + col);
     v[0] *= act_grad_f32(p.act, x.x); v[1] *= act_grad_f32(p.act, x.y);
