@@ -292,9 +292,9 @@ class MultiHeadAttention(Module):
         return torch.cat([rot.reshape(-1, n_rot), qkv[:, n_rot:]], dim=1)
 
     def _attend_tokens(self, q2, k3, v3, B, Sq, Sk, causal, q_offset, mask):
+        from ..ops import flash
         H, Hkv, hd = self.num_heads, self.num_kv_heads, self.head_dim
-        if q2.is_cuda and mask is None and q2.dtype == torch.bfloat16 and not q2.requires_grad:
-            from ..ops import flash
+        if q2.is_cuda and mask is None and q2.dtype == torch.bfloat16 and not q2.requires_grad and flash._raw_call():
             if Sq == 1 and hd in (64, 128) and H // Hkv <= 8 and _decode_layout(q2, k3, v3):
                 # One query row per sequence: the keys are split over the SMs and read once for all query heads of a
                 # group; the prompt kernel fills a 128-row tile with it and reads them once per query head, one CTA
@@ -315,7 +315,6 @@ class MultiHeadAttention(Module):
                                       kv_batch_rows=cap)
                 return o
         if q2.is_cuda and mask is None and q2.dtype == torch.bfloat16:
-            from ..ops import flash
             return flash.attention_tokens(q2, k3.reshape(B * Sk, Hkv * hd), v3.reshape(B * Sk, Hkv * hd), B, Sq, Sk, H,
                                           Hkv, hd, causal, q_offset)
         q = q2.reshape(B, Sq, H, hd).transpose(1, 2)

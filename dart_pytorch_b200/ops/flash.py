@@ -272,7 +272,7 @@ class AttentionF32Fn(torch.autograd.Function):
 
 
 def _attention_f32(q4, k4, v4, causal, q_offset):
-    if _wants_grad(q4, k4, v4):
+    if _wants_grad(q4, k4, v4) or not _raw_call():     # (the function refuses derivatives and transforms that it does not have)
         return AttentionF32Fn.apply(q4, k4, v4, causal, q_offset)
     o = torch.empty(q4.shape, dtype=q4.dtype, device=q4.device)
     attn_f32(_f32_rows(q4), _f32_rows(k4), _f32_rows(v4), o, causal, q_offset)
