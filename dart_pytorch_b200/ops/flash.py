@@ -322,7 +322,10 @@ def attention_bhsd(q, k, v, causal=False, mask=None, q_offset=0):
     B, H, Sq, hd = q.shape
     Hkv, Sk = k.shape[1], k.shape[2]
     if q.dtype == torch.float32 and mask is None:
-        if _f32_covers(B, Sq, Sk, H, Hkv, hd, q_offset):
+        # keys and values of the queries' batch, head size and device; others (values of a size of their own among them) are
+        # computed, or refused, by the composed path
+        if _f32_covers(B, Sq, Sk, H, Hkv, hd, q_offset) and k.shape == v.shape == (B, Hkv, Sk, hd) and \
+                all(t.device == q.device and t.dtype in (torch.float32, torch.bfloat16) for t in (k, v)):
             q4, k4, v4 = (t.to(q.dtype).transpose(1, 2) for t in (q, k, v))
             return _attention_f32(q4, k4, v4, causal, q_offset).transpose(1, 2)
     if q.dtype == torch.bfloat16 and mask is None and supported_head_dim(hd, backward=_wants_grad(q, k, v)):
