@@ -306,7 +306,8 @@ def attention_tokens(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causa
         return o.transpose(1, 2).reshape(batch * sq, heads * head_dim)
     if hd_k == head_dim:
         return SeparateAttentionFn.apply(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causal, q_offset)
-    if not _wants_grad(q2, k2, v2) and _reads_rows(q2, k2, v2) and _raw_call():
+    if q2.shape == (batch * sq, heads * head_dim) and k2.shape == v2.shape == (batch * sk, kv_heads * head_dim) and \
+            not _wants_grad(q2, k2, v2) and _reads_rows(q2, k2, v2) and _raw_call():
         # the forward kernel reads such heads as they are; only the backward one wants padded operands
         return attn_fwd(q2, k2, v2, batch, sq, sk, heads, kv_heads, head_dim, causal, q_offset=q_offset, need_lse=False)[0]
     o = SeparateAttentionFn.apply(_pad_heads(q2, heads, head_dim, hd_k), _pad_heads(k2, kv_heads, head_dim, hd_k),

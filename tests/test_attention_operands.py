@@ -1,4 +1,4 @@
-"""fp32 attention on keys and values that do not go with the queries: never by the kernel, which takes their sizes from them."""
+"""Attention on keys and values that do not go with the queries: never by a kernel, which takes their sizes from them."""
 import pytest
 import torch
 
@@ -38,6 +38,22 @@ def test_other_devices_and_types(calls):
     for t in (torch.randn(2, 2, 7, 16), torch.randn(2, 2, 7, 16).bfloat16()):
         A.attention_bhsd(q, t, t, True)
     assert calls == ["kernel"] * 2
+
+
+def test_bf16_rows_of_another_width(monkeypatch):
+    """Heads that are no kernel size of their own: rows of another width than the heads take up are refused."""
+    seen = []
+    monkeypatch.setattr(A, "attn_fwd", lambda q, *a, **k: (seen.append(1), (q, None))[1])
+
+    def rows(n, width):
+        return torch.zeros(n, width, dtype=torch.bfloat16)
+    with torch.no_grad():
+        for widths in ((4 * 24, 2 * 16, 2 * 24), (4 * 24, 2 * 24, 2 * 32), (4 * 16, 2 * 24, 2 * 24), (4 * 32, 2 * 24, 2 * 24)):
+            with pytest.raises(RuntimeError):
+                A.attention_tokens(rows(10, widths[0]), rows(14, widths[1]), rows(14, widths[2]), 2, 5, 7, 4, 2, 24, False)
+        assert not seen
+        A.attention_tokens(rows(10, 96), rows(14, 48), rows(14, 48), 2, 5, 7, 4, 2, 24, False)
+        assert seen == [1]
 
 
 @pytest.mark.gpu
