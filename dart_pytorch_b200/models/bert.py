@@ -11,6 +11,8 @@ from dataclasses import dataclass
 import torch
 
 from .. import ops as F
+from ..ops import stack
+from ..ops.stack import plain
 from ..nn.attention import MultiHeadAttention
 from ..nn.layers import Embedding, LayerNorm, Linear
 from ..nn.module import Module, make_param
@@ -112,21 +114,18 @@ class BertModel(Module):
         """The encoder without gradients as one native call; ``None`` when that does not stand for its modules."""
         e = self.embeddings
         if torch.is_grad_enabled() or not tokens.is_cuda or tokens.dim() not in (1, 2) or \
-                not 0 < tokens.shape[-1] <= e.max_len:
+                not (plain(e, BertEmbeddings) and plain(e.layer_norm, LayerNorm)) or not 0 < tokens.shape[-1] <= e.max_len:
             return None
-        from ..ops import stack
-        plain, layers = stack.plain, []
+        layers = []
         for b in self.layers:
+            if not plain(b, BertLayer):
+                return None
             m = b.attention
-            if not (plain(b, BertLayer) and plain(m, MultiHeadAttention) and plain(m.wo, Linear) and
-                    plain(b.attention_output_ln, LayerNorm) and plain(b.output_ln, LayerNorm) and
-                    plain(b.intermediate, Linear) and plain(b.output, Linear)) or \
-                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.attention_output_ln, LayerNorm) and
+                    plain(b.output_ln, LayerNorm) and plain(b.intermediate, Linear) and plain(b.output, Linear)):
                 return None
             layers.append(stack.Layer(m, b.attention_output_ln, b.output_ln, b.intermediate.weight, b.intermediate.bias,
                                       b.output.weight, b.output.bias))
-        if not (plain(e, BertEmbeddings) and plain(e.layer_norm, LayerNorm)):
-            return None
         return stack.run(layers, None, post_norm=True, act="gelu_tanh", tokens=tokens, table=e.word_embeddings.weight,
                          pos_table=e.position_embeddings.weight, add_row=e.token_type_bias, embed_norm=e.layer_norm)
 

@@ -15,6 +15,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from .. import ops as F
+from ..ops.stack import plain
 from ..nn.attention import EncoderCache
 from ..nn.layers import Dropout, Embedding, LearnedPositionalEmbedding, Linear
 from ..nn.module import Module
@@ -113,8 +114,8 @@ class GPT(Module):
         n = tokens.shape[-1]
         if start_pos + n > self.config.max_ctx:
             raise ValueError(f"GPT: sequence of {start_pos + n} tokens exceeds maxCtx {self.config.max_ctx}")
-        if tokens.is_cuda and type(self.encoder) is TransformerEncoder and not (
-                self.embed_drop.training and self.embed_drop.p > 0):
+        if tokens.is_cuda and not torch.is_grad_enabled() and plain(self.encoder, TransformerEncoder) and \
+                plain(self.embed_drop, Dropout) and not (self.embed_drop.training and self.embed_drop.p > 0):
             h = self.encoder.infer(None, cache, n > 1, start_pos, tokens=tokens, table=self.token_emb.weight,
                                    pos_table=self.pos_emb.table.weight, pos_start=start_pos)
             if h is not None:

@@ -14,6 +14,8 @@ from typing import List, Optional, Sequence
 import torch
 
 from .. import ops as F
+from ..ops import stack
+from ..ops.stack import plain
 from ..nn.attention import EncoderCache, MHACache, MultiHeadAttention, RopeCache
 from ..nn.layers import Embedding, Linear, RMSNorm, SwiGluFfn
 from ..nn.module import Module
@@ -101,14 +103,13 @@ class Llama(Module):
         """The stack without gradients as one native call; ``None`` when that does not stand for the blocks."""
         if torch.is_grad_enabled():
             return None
-        from ..ops import stack
-        plain, layers = stack.plain, []
+        layers = []
         for b in self.blocks:
+            if not plain(b, LlamaBlock):
+                return None
             m = b.attn
-            if not (plain(b, LlamaBlock) and plain(m, MultiHeadAttention) and plain(m.wo, Linear) and
-                    plain(b.attn_norm, RMSNorm) and plain(b.ffn_norm, RMSNorm) and plain(b.ffn, SwiGluFfn) and
-                    plain(b.ffn.down, Linear)) or \
-                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.attn_norm, RMSNorm) and plain(b.ffn_norm, RMSNorm) and
+                    plain(b.ffn, SwiGluFfn) and plain(b.ffn.down, Linear)):
                 return None
             layers.append(stack.Layer(m, b.attn_norm, b.ffn_norm, b.ffn.w_gate_up, None, b.ffn.down.weight,
                                       b.ffn.down.bias))
@@ -147,7 +148,7 @@ class Llama(Module):
         if tokens.dim() not in (1, 2):
             raise ValueError("Llama: tokens must be [N] or [B, N]")
         n = tokens.shape[-1]
-        if tokens.is_cuda and start_pos + n <= self.config.max_ctx and type(self) is Llama:
+        if tokens.is_cuda and start_pos + n <= self.config.max_ctx and plain(self, Llama):
             h = self._infer(None, start_pos, cache, n, tokens=tokens, table=self.embed_in.weight)
             if h is not None:
                 return h

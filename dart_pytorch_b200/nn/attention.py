@@ -13,6 +13,7 @@ from typing import List, Optional
 import torch
 
 from .. import ops as F
+from ..ops.stack import plain
 from .layers import Dropout, Linear
 from .module import Module, make_param, uniform_, normal_
 
@@ -280,6 +281,13 @@ class MultiHeadAttention(Module):
         if self.attn_dropout is not None:
             out = self.attn_dropout(out)
         return out.reshape(*x.shape[:-1], self.embed_dim)
+
+    def stock(self) -> bool:
+        """Whether the layer and its parts are what this file defines, with no dropout at work: the native stack stands for it."""
+        drop = self.attn_dropout
+        return plain(self, MultiHeadAttention) and plain(self.wo, Linear) and \
+            (self.rope is None or plain(self.rope, RopeCache)) and \
+            (drop is None or plain(drop, Dropout) and not (drop.training and drop.p > 0))
 
     def _rope_qk(self, qkv, S, start_pos):
         """Rotate the Q and K column blocks of the fused projection output."""

@@ -12,6 +12,8 @@ from typing import List, Optional
 import torch
 
 from .. import ops as F
+from ..ops import stack
+from ..ops.stack import plain
 from .attention import EncoderCache, MHACache, MultiHeadAttention, MultiHeadCrossAttention, RopeCache
 from .layers import Dropout, LayerNorm, Linear, activation_name
 from .module import Module
@@ -83,15 +85,14 @@ class TransformerEncoder(Module):
         when that does not stand for the blocks' own forward passes."""
         if torch.is_grad_enabled() or not self.blocks:
             return None
-        from ..ops import stack
-        plain = stack.plain
-        act, layers = self.blocks[0].activation, []
+        act, layers = None, []
         for b in self.blocks:
-            m = b.mha
-            if not (plain(b, TransformerBlock) and plain(m, MultiHeadAttention) and plain(b.ln1, LayerNorm) and
-                    plain(b.ln2, LayerNorm) and plain(b.ffn1, Linear) and plain(b.ffn2, Linear) and plain(m.wo, Linear)) or \
-                    b.activation != act or (b.training and b.dropout.p > 0) or \
-                    (m.attn_dropout is not None and m.attn_dropout.training and m.attn_dropout.p > 0):
+            if not plain(b, TransformerBlock):
+                return None
+            m, act = b.mha, act if layers else b.activation
+            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.ln1, LayerNorm) and plain(b.ln2, LayerNorm) and
+                    plain(b.ffn1, Linear) and plain(b.ffn2, Linear)) or \
+                    b.activation != act or (b.training and b.dropout.p > 0):
                 return None
             layers.append(stack.Layer(m, b.ln1, b.ln2, b.ffn1.weight, b.ffn1.bias, b.ffn2.weight, b.ffn2.bias))
         if self.final_norm is not None and not plain(self.final_norm, LayerNorm):

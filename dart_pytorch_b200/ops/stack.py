@@ -6,6 +6,7 @@ own forward passes then run (and raise their errors)."""
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -37,9 +38,14 @@ class Layer:
         self.up_w, self.up_b, self.down_w, self.down_b = up_w, up_b, down_w, down_b
 
 
-def plain(module, cls) -> bool:
-    """A module of exactly this class whose forward nobody has replaced on the object."""
-    return type(module) is cls and "forward" not in module.__dict__
+@functools.lru_cache(maxsize=None)
+def _names(cls) -> frozenset:
+    return frozenset(dir(cls))
+
+
+def plain(obj, cls) -> bool:
+    """An object of exactly this class, none of whose methods has been replaced on the object."""
+    return type(obj) is cls and _names(cls).isdisjoint(obj.__dict__)
 
 
 def eligible(t: torch.Tensor) -> bool:
