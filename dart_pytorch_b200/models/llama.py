@@ -114,7 +114,7 @@ class Llama(Module):
             layers.append(stack.Layer(m, b.attn_norm, b.ffn_norm, b.ffn.w_gate_up, None, b.ffn.down.weight,
                                       b.ffn.down.bias))
         if not plain(self.final_norm, RMSNorm) or cache is not None and not (
-                len(cache.layers) == len(layers) and all(type(c) is MHACache for c in cache.layers)):
+                len(cache.layers) == len(layers) and all(plain(c, MHACache) for c in cache.layers)):
             return None
         return stack.run(layers, x, rms=True, gated=True, causal=n > 1, start_pos=start_pos,
                          caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)

@@ -171,6 +171,12 @@ def _decode_layout(q2, k3, v3) -> bool:
         q2.data_ptr() % 16 == 0 and k3.data_ptr() % 16 == 0 and v3.data_ptr() % 16 == 0
 
 
+def _rows_layout(q2, k3, v3, hd, Hkv) -> bool:
+    """The same for the prompt kernel on heads that are no kernel size of their own, whose rows a cache of any class hands
+    over: also of the heads' width, and sequences a whole number of rows apart."""
+    return _decode_layout(q2, k3, v3) and k3.shape == v3.shape and k3.shape[2] == Hkv * hd and k3.stride(0) % k3.stride(1) == 0
+
+
 class MultiHeadAttention(Module):
     """Self-attention with grouped-query sharing, optional RoPE and KV cache
     (reference: lib/core/nn/attention/multi_head_attention.dart:27-253).
@@ -258,7 +264,8 @@ class MultiHeadAttention(Module):
         qkv = F.linear(x2, self.w_qkv, self.b_qkv)  # [B*S, dq + 2 dkv]
         if self.rope is not None:
             self.rope.check_window(start_pos, S)
-        rows = cache is not None and cache.takes_rows(qkv)     # rotation and append in one kernel
+        # rotation and append in one kernel; another class of cache (or a replaced append) gets its rows by `append`
+        rows = plain(cache, MHACache) and cache.takes_rows(qkv)
         if self.rope is not None and not rows:
             qkv = self._rope_qk(qkv, S, start_pos)
         if rows:
@@ -309,7 +316,7 @@ class MultiHeadAttention(Module):
                 # for all keys.  Faster at every length measured (B200): 4 heads of 64 on one key head, 1 x 65 keys,
                 # 6.6 -> 4.5 us; 16 heads of 128 on 4 key heads, 32 x 2049 keys, 153 -> 41 us.
                 return flash.attn_decode_rows(q2, k3, v3, B, Sk, H, Hkv, hd)
-            if flash.kernel_head_dim(hd) is not None:
+            if flash.kernel_head_dim(hd) == hd or flash.kernel_head_dim(hd) is not None and _rows_layout(q2, k3, v3, hd, Hkv):
                 k2 = k3.reshape(-1, k3.shape[-1]) if k3.is_contiguous() else None
                 if k2 is not None:
                     o, _ = flash.attn_fwd(q2, k2, v3.reshape(-1, v3.shape[-1]), B, Sq, Sk, H, Hkv, hd, causal,

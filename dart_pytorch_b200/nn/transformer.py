@@ -97,7 +97,7 @@ class TransformerEncoder(Module):
             layers.append(stack.Layer(m, b.ln1, b.ln2, b.ffn1.weight, b.ffn1.bias, b.ffn2.weight, b.ffn2.bias))
         if self.final_norm is not None and not plain(self.final_norm, LayerNorm):
             return None
-        if cache is not None and not (len(cache.layers) == len(layers) and all(type(c) is MHACache for c in cache.layers)):
+        if cache is not None and not (len(cache.layers) == len(layers) and all(plain(c, MHACache) for c in cache.layers)):
             return None
         return stack.run(layers, x, act=activation_name(act), causal=causal, start_pos=start_pos,
                          caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)
