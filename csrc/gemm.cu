@@ -374,6 +374,14 @@ extern "C" int dptb_tp_wait_ready(const void* ready, const void* epoch, int worl
   return counted(1, (int)cudaGetLastError());
 }
 
+// The capture that is under way on a stream, or 0.
+extern "C" unsigned long long dptb_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) return 0;
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 // Status word access ------------------------------------------------------------------------------
 // Folds the blocks of all translation units: the first non-zero code (with its detail) and the total number of
 // waits that ran out.

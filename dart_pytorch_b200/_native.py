@@ -163,6 +163,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     sig("dptb_gemm", ctypes.POINTER(GemmArgs), P)
     sig("dptb_gemm_skinny", ctypes.POINTER(GemmArgs), P, P)
     sig("dptb_attn_f32", P, P)
+    sig("dptb_capture_id", P)
+    lib.dptb_capture_id.restype = ctypes.c_ulonglong
     sig("dptb_status_read", ctypes.POINTER(c_int * 4))
     sig("dptb_status_clear")
     sig("dptb_layernorm_fwd", P, P, P, P, P, P, L, I, F, I, P)

@@ -26,7 +26,7 @@ def _lead(t: torch.Tensor) -> int:
     return t.stride(0) if t.shape[0] > 1 else max(t.shape[1], t.stride(0))
 
 
-_SPLITK_WS = {}
+_SPLITK_WS, _SPLITK_GRAPH_WS = {}, {}
 SPLITK_WS_BYTES = 64 << 20
 SKINNY_MAX_ROWS = 64      # rows up to which x @ W^T takes the weight-streaming kernel (csrc/gemm_skinny.cu)
 _SKINNY_ON = os.environ.get("DPTB200_SKINNY_GEMM", "1") != "0"
@@ -37,15 +37,20 @@ SPLITK_COUNTERS = 4096
 def splitk_workspace(device: torch.device):
     """Scratch of the split-K GEMM path, one per (device, stream): an fp32 partial-tile buffer and zeroed per-tile
     counters.  Launches on one stream reuse it in order (the counters return to zero at the end of every launch);
-    GEMMs launched on another stream (weight gradients beside the data-gradient chain) get their own."""
+    GEMMs launched on another stream (weight gradients beside the data-gradient chain) get their own.  So does every
+    CUDA graph for each stream of its capture, because graphs that were captured on one stream may be replayed on several
+    at once: its scratch comes from the graph's memory pool, and the graph zeroes the counters itself."""
     dev = device.index if device.index is not None else torch.cuda.current_device()
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream)
-    ws = _SPLITK_WS.get(key)
-    if ws is None:
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    key = (dev, stream)
+    capture = N.load().dptb_capture_id(stream) if torch.cuda.is_current_stream_capturing() else 0
+    held = _SPLITK_GRAPH_WS if capture else _SPLITK_WS      # (of the graphs, the newest of a stream; an older one is its graph's alone)
+    ws = held.get(key)
+    if ws is None or ws[2] != capture:
         ws = (torch.empty(SPLITK_WS_BYTES, dtype=torch.uint8, device=device),
-              torch.zeros(SPLITK_COUNTERS, dtype=torch.int32, device=device))
-        _SPLITK_WS[key] = ws
-    return ws
+              torch.zeros(SPLITK_COUNTERS, dtype=torch.int32, device=device), capture)
+        held[key] = ws
+    return ws[:2]
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, trans_a: bool = False, trans_b: bool = False,
