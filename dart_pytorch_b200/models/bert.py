@@ -13,7 +13,7 @@ import torch
 from .. import ops as F
 from ..ops import stack
 from ..ops.stack import plain
-from ..nn.attention import MultiHeadAttention
+from ..nn.attention import MultiHeadAttention, stock_attention
 from ..nn.layers import Embedding, LayerNorm, Linear
 from ..nn.module import Module, make_param
 from .gpt import _as_token_tensor
@@ -121,7 +121,7 @@ class BertModel(Module):
             if not plain(b, BertLayer):
                 return None
             m = b.attention
-            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.attention_output_ln, LayerNorm) and
+            if not (stock_attention(m) and plain(b.attention_output_ln, LayerNorm) and
                     plain(b.output_ln, LayerNorm) and plain(b.intermediate, Linear) and plain(b.output, Linear)):
                 return None
             layers.append(stack.Layer(m, b.attention_output_ln, b.output_ln, b.intermediate.weight, b.intermediate.bias,

@@ -16,7 +16,7 @@ import torch
 from .. import ops as F
 from ..ops import stack
 from ..ops.stack import plain
-from ..nn.attention import EncoderCache, MHACache, MultiHeadAttention, RopeCache
+from ..nn.attention import EncoderCache, MHACache, MultiHeadAttention, RopeCache, stock_attention, stock_cache
 from ..nn.layers import Embedding, Linear, RMSNorm, SwiGluFfn
 from ..nn.module import Module
 from .gpt import _as_token_tensor
@@ -108,13 +108,13 @@ class Llama(Module):
             if not plain(b, LlamaBlock):
                 return None
             m = b.attn
-            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.attn_norm, RMSNorm) and plain(b.ffn_norm, RMSNorm) and
+            if not (stock_attention(m) and plain(b.attn_norm, RMSNorm) and plain(b.ffn_norm, RMSNorm) and
                     plain(b.ffn, SwiGluFfn) and plain(b.ffn.down, Linear)):
                 return None
             layers.append(stack.Layer(m, b.attn_norm, b.ffn_norm, b.ffn.w_gate_up, None, b.ffn.down.weight,
                                       b.ffn.down.bias))
         if not plain(self.final_norm, RMSNorm) or cache is not None and not (
-                len(cache.layers) == len(layers) and all(plain(c, MHACache) for c in cache.layers)):
+                len(cache.layers) == len(layers) and all(stock_cache(c) for c in cache.layers)):
             return None
         return stack.run(layers, x, rms=True, gated=True, causal=n > 1, start_pos=start_pos,
                          caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)
@@ -148,7 +148,8 @@ class Llama(Module):
         if tokens.dim() not in (1, 2):
             raise ValueError("Llama: tokens must be [N] or [B, N]")
         n = tokens.shape[-1]
-        if tokens.is_cuda and start_pos + n <= self.config.max_ctx and plain(self, Llama):
+        if tokens.is_cuda and start_pos + n <= self.config.max_ctx and plain(self, Llama) and \
+                "hidden_from_embeddings" not in self.__dict__:
             h = self._infer(None, start_pos, cache, n, tokens=tokens, table=self.embed_in.weight)
             if h is not None:
                 return h

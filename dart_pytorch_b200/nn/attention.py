@@ -143,6 +143,11 @@ class MHACache:
         self.__dict__.pop("_fills", None)
 
 
+def stock_cache(cache) -> bool:
+    """A cache of exactly this class whose ``append`` nobody has replaced on the object."""
+    return type(cache) is MHACache and "append" not in cache.__dict__
+
+
 class EncoderCache:
     """One ``MHACache`` per layer (reference: lib/core/nn/kv_cache.dart:66-84)."""
 
@@ -265,7 +270,7 @@ class MultiHeadAttention(Module):
         if self.rope is not None:
             self.rope.check_window(start_pos, S)
         # rotation and append in one kernel; another class of cache (or a replaced append) gets its rows by `append`
-        rows = plain(cache, MHACache) and cache.takes_rows(qkv)
+        rows = stock_cache(cache) and cache.takes_rows(qkv)
         if self.rope is not None and not rows:
             qkv = self._rope_qk(qkv, S, start_pos)
         if rows:
@@ -288,13 +293,6 @@ class MultiHeadAttention(Module):
         if self.attn_dropout is not None:
             out = self.attn_dropout(out)
         return out.reshape(*x.shape[:-1], self.embed_dim)
-
-    def stock(self) -> bool:
-        """Whether the layer and its parts are what this file defines, with no dropout at work: the native stack stands for it."""
-        drop = self.attn_dropout
-        return plain(self, MultiHeadAttention) and plain(self.wo, Linear) and \
-            (self.rope is None or plain(self.rope, RopeCache)) and \
-            (drop is None or plain(drop, Dropout) and not (drop.training and drop.p > 0))
 
     def _rope_qk(self, qkv, S, start_pos):
         """Rotate the Q and K column blocks of the fused projection output."""
@@ -337,6 +335,16 @@ class MultiHeadAttention(Module):
         v = v3.reshape(B, Sk, Hkv, hd).transpose(1, 2)
         o = F.attention(q, k, v, causal=causal, mask=mask, q_offset=q_offset)
         return o.transpose(1, 2).reshape(B * Sq, H * hd)
+
+
+def stock_attention(m) -> bool:
+    """Whether the layer and its parts are what this file defines, with no dropout at work: the native stack stands for it."""
+    if not plain(m, MultiHeadAttention):
+        return False
+    own, rope, drop = m.__dict__, m.rope, m.attn_dropout
+    return "_attend_tokens" not in own and "_rope_qk" not in own and plain(m.wo, Linear) and \
+        (rope is None or type(rope) is RopeCache and "check_window" not in rope.__dict__) and \
+        (drop is None or plain(drop, Dropout) and not (drop.training and drop.p > 0))
 
 
 class MultiHeadCrossAttention(Module):

@@ -14,7 +14,8 @@ import torch
 from .. import ops as F
 from ..ops import stack
 from ..ops.stack import plain
-from .attention import EncoderCache, MHACache, MultiHeadAttention, MultiHeadCrossAttention, RopeCache
+from .attention import (EncoderCache, MHACache, MultiHeadAttention, MultiHeadCrossAttention, RopeCache, stock_attention,
+                        stock_cache)
 from .layers import Dropout, LayerNorm, Linear, activation_name
 from .module import Module
 
@@ -90,14 +91,14 @@ class TransformerEncoder(Module):
             if not plain(b, TransformerBlock):
                 return None
             m, act = b.mha, act if layers else b.activation
-            if not (type(m) is MultiHeadAttention and m.stock() and plain(b.ln1, LayerNorm) and plain(b.ln2, LayerNorm) and
+            if not (stock_attention(m) and plain(b.ln1, LayerNorm) and plain(b.ln2, LayerNorm) and
                     plain(b.ffn1, Linear) and plain(b.ffn2, Linear)) or \
                     b.activation != act or (b.training and b.dropout.p > 0):
                 return None
             layers.append(stack.Layer(m, b.ln1, b.ln2, b.ffn1.weight, b.ffn1.bias, b.ffn2.weight, b.ffn2.bias))
         if self.final_norm is not None and not plain(self.final_norm, LayerNorm):
             return None
-        if cache is not None and not (len(cache.layers) == len(layers) and all(plain(c, MHACache) for c in cache.layers)):
+        if cache is not None and not (len(cache.layers) == len(layers) and all(stock_cache(c) for c in cache.layers)):
             return None
         return stack.run(layers, x, act=activation_name(act), causal=causal, start_pos=start_pos,
                          caches=None if cache is None else cache.layers, final_norm=self.final_norm, **embedding)

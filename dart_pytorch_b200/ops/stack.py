@@ -6,7 +6,6 @@ own forward passes then run (and raise their errors)."""
 from __future__ import annotations
 
 import ctypes
-import functools
 from typing import Optional, Sequence
 
 import torch
@@ -38,14 +37,12 @@ class Layer:
         self.up_w, self.up_b, self.down_w, self.down_b = up_w, up_b, down_w, down_b
 
 
-@functools.lru_cache(maxsize=None)
-def _names(cls) -> frozenset:
-    return frozenset(dir(cls))
-
-
-def plain(obj, cls) -> bool:
-    """An object of exactly this class, none of whose methods has been replaced on the object."""
-    return type(obj) is cls and _names(cls).isdisjoint(obj.__dict__)
+def plain(module, cls) -> bool:
+    """A module of exactly this class, neither of whose forward methods has been replaced on the object."""
+    if type(module) is not cls:
+        return False
+    own = module.__dict__
+    return "forward" not in own and "with_residual" not in own
 
 
 def eligible(t: torch.Tensor) -> bool:
