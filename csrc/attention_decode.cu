@@ -562,13 +562,9 @@ extern "C" int dptb_attn_decode_splits_hd(int B, int Sq, int Hkv, int Sk, int he
 template <int HD, int GP, bool WIN>
 static cudaError_t decode_launch_gp(const DecodeArgs& a, dim3 grid, cudaStream_t st) {
   constexpr int kRing = kDecWarps * 4 * kDecRound * HD * 2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<HD, GP, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kRing);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(reinterpret_cast<const void*>(attn_decode_kernel<HD, GP, WIN>), kRing);
+  if (e != cudaSuccess) return e;
   return launch_k(attn_decode_kernel<HD, GP, WIN>, grid, dim3(kDecWarps * 32), kRing, st, a);
 }
 template <int HD, bool WIN>

@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include "smem_limit.h"
+
 namespace dptb {
 
 // Return codes of every extern "C" entry point: 0 = ok, > 0 = cudaError_t, < 0 = library error.

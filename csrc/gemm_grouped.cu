@@ -335,11 +335,8 @@ template <int BN, int STAGES>
 static int launch_grouped(const CUtensorMap* tm, const GroupedParams& p, int max_tiles, cudaStream_t st) {
   using L = GroupedSmem<BN, STAGES>;
   auto kern = gemm_grouped_kernel<BN, STAGES>;
-  static bool configured = false;
-  if (!configured) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-    configured = true;
-  }
+  static SmemLimit limit;
+  DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   const int grid = max_tiles < sm_count() ? max_tiles : sm_count();
   return counted(1, (int)launch_k(kern, dim3(grid), dim3(kGgThreads), L::kTotal, st, tm[0], tm[1], tm[2], tm[3], p));
 }

@@ -536,11 +536,8 @@ static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const S
                          cudaStream_t stream) {
   using L = SkinnySmem<MP, ST>;
   auto kern = gemm_skinny_kernel<MP, ST>;
-  static bool configured = false;
-  if (!configured) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-    configured = true;
-  }
+  static SmemLimit limit;
+  DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   return counted(1, (int)launch_k(kern, dim3(units), dim3(kSkThreads), L::kTotal, stream, tmW, tmX, p));
 }
 

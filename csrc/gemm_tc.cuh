@@ -1443,11 +1443,8 @@ template <bool A_MN, bool B_MN, int BN, int STAGES>
 static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES>;
   auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES>;
-  static bool configured = false;
-  if (!configured) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-    configured = true;
-  }
+  static SmemLimit limit;
+  DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   kern<<<grid, kGemmThreads, L::kTotal, stream>>>(tmA, tmB, NoPeerMaps{}, EpiMaps{}, p);
@@ -1459,12 +1456,16 @@ constexpr int kPairStages256 = 5;   // 32 KB per stage and CTA, 64 KB of epilogu
 constexpr int kPairStages128 = 6;   // 24 KB per stage and CTA
 template <bool A_MN, bool B_MN, int BN, int STAGES>
 static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
-  // Clusters of this kernel that can be resident at once (a persistent grid must not exceed it), once per process.
+  // Clusters of this kernel that can be resident at once (a persistent grid must not exceed it), once per device.
   using L = GemmSmem<BN, STAGES, BN / 2, 2>;
   auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true>;
-  static int cached = -1;
+  static SmemLimit limit;
+  static std::atomic<int> counts[64];      // one more than the number; 0: not asked for yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+  int cached = counts[dev].load(std::memory_order_relaxed) - 1;
   if (cached < 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal) != cudaSuccess) return 0;
+    if (limit.raise(reinterpret_cast<const void*>(kern), L::kTotal) != cudaSuccess) return 0;
     cfg->gridDim = dim3(2 * (sm_count() / 2));
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, cfg) != cudaSuccess || n <= 0) {
@@ -1472,6 +1473,7 @@ static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
       n = 0;
     }
     cached = n;
+    counts[dev].store(n + 1, std::memory_order_relaxed);
     if (getenv("DPTB_GEMM_VERBOSE")) fprintf(stderr, "gemm pair BN=%d: %d clusters of 2 CTAs can be resident\n", BN, n);
   }
   (void)attr;
@@ -1506,11 +1508,8 @@ template <int BN, int STAGES>
 static int launch_tc_ag(const TmapSet& peers, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES>;
   auto kern = gemm_tc_kernel<false, false, BN, STAGES, true>;
-  static bool configured = false;
-  if (!configured) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-    configured = true;
-  }
+  static SmemLimit limit;
+  DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   const int tiles = p.tiles_m * p.tiles_n;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   kern<<<grid, kGemmThreads, L::kTotal, stream>>>(peers.m[p.ag.rank], tmB, peers, EpiMaps{}, p);

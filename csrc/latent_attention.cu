@@ -452,11 +452,7 @@ template <int MAXP>
 static int launch_latent_mma(const LatentAttnParams& p, dim3 grid, cudaStream_t st) {
   auto kern = latent_attn_mma_kernel<MAXP>;
   const int bytes = la_smem_bytes(p.R);
-  static int configured = 0;
-  if (configured < bytes) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    configured = bytes;
-  }
+  DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   const int rc = counted(1, (int)launch_k(kern, grid, dim3(kLaThreads), (size_t)bytes, st, p));
   if (rc || p.splits == 1) return rc;
   return counted(1, (int)launch_k(latent_attn_merge_kernel, dim3((unsigned)(p.B * p.S * p.H)), dim3(128), (size_t)0, st, p));

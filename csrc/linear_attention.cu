@@ -767,12 +767,9 @@ template <int DK, int DV>
 static int launch_chunks(const LinearParams& p, cudaStream_t st) {
   using L1 = LinSmem<DK, DV, false>;
   using L2 = LinSmem<DK, DV, true>;
-  static bool configured = false;
-  if (!configured) {
-    DPTB_CUDA_OK(cudaFuncSetAttribute(linear_chunk_kernel<DK, DV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, L1::kTotal));
-    DPTB_CUDA_OK(cudaFuncSetAttribute(linear_chunk_kernel<DK, DV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, L2::kTotal));
-    configured = true;
-  }
+  static SmemLimit limit1, limit2;
+  DPTB_CUDA_OK(limit1.raise(reinterpret_cast<const void*>(linear_chunk_kernel<DK, DV, false>), L1::kTotal));
+  DPTB_CUDA_OK(limit2.raise(reinterpret_cast<const void*>(linear_chunk_kernel<DK, DV, true>), L2::kTotal));
   const unsigned gy = p.H * ((p.dv + DV - 1) / DV);
   if (p.segments > 1) {
     const int rc = counted(1, (int)launch_k(linear_chunk_kernel<DK, DV, false>, dim3(p.segments - 1, gy, p.B), dim3(L1::kThreads),
