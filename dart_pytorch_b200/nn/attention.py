@@ -97,6 +97,7 @@ class MHACache:
         self._ensure(batch, self.seq_len + n, kv_heads * head_dim, qkv)
         decode.rows_to_cache(qkv, self.k_buf, self.v_buf, batch, n, heads, kv_heads, head_dim, start_pos,
                              self.seq_len, 0 if rope is None else rope.rotary_dim, 1.0 if rope is None else rope.base)
+        torch.autograd.graph.increment_version((self.k_buf, self.v_buf))     # written in place, as by `append`
         self.seq_len += n
         self.__dict__.pop("_fills", None)
         return self.k_buf[:, :self.seq_len], self.v_buf[:, :self.seq_len]

@@ -177,6 +177,7 @@ def run(layers: Sequence[Layer], x: Optional[torch.Tensor], *, post_norm=False, 
     a.ws, a.out = scratch.data_ptr(), out.data_ptr()
     N.check(lib.dptb_stack_infer(ctypes.byref(a), (c_void_p * len(ptrs))(*ptrs), N.stream_ptr()), "stack_infer")
     if caches is not None:
+        torch.autograd.graph.increment_version([t for c in caches for t in (c.k_buf, c.v_buf)])     # written in place
         for c in caches:
             c.seq_len += S
             c.__dict__.pop("_fills", None)
