@@ -148,7 +148,7 @@ def run(layers: Sequence[Layer], x: Optional[torch.Tensor], *, post_norm=False, 
             if c.seq_len != past or k is not None and (
                     k.dtype != dtype or v.dtype != dtype or k.device != dev or v.device != dev or
                     k.shape[0] != B or k.shape[2] != width or not k.is_contiguous() or not v.is_contiguous() or
-                    k.shape != v.shape):
+                    k.shape != v.shape or bf16 and (k.data_ptr() | v.data_ptr()) % 16):     # (bf16 rows go in 16-byte pieces)
                 return None
         if len({id(c) for c in caches}) != len(caches):
             return None
