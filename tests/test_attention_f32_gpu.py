@@ -52,7 +52,10 @@ def test_attention_f32(B, H, Hkv, Sq, Sk, hd, causal, off, layout):
     ref = _exact(*d, causal, off)
     want = torch.autograd.grad(ref, d, do.double())
     for a, b in zip((o.detach(), *got), (ref.detach(), *want)):
-        assert float((a.double() - b).norm() / (b.norm() + 1e-30)) < 3e-6 or float(b.norm()) < 1e-6
+        if float(b.norm()) < 1e-6:      # one key: its weight is 1 whatever the score, and the exact dQ and dK are zero
+            assert float(a.abs().max()) < 1e-6
+        else:
+            assert float((a.double() - b).norm() / b.norm()) < 3e-6
 
 
 @pytest.mark.parametrize("B,S,H,Hkv,hd", [(2, 96, 4, 2, 32), (1, 33, 3, 3, 20)])

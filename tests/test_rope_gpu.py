@@ -32,7 +32,8 @@ def _close(got, want, dtype, pos_max):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens,heads,hd,rot,pad", [(1, 1, 2, 2, 0), (7, 3, 20, 12, 1), (33, 5, 64, 64, 8), (900, 4, 128, 128, 0),
-                                                     (5000, 2, 64, 16, 0), (9, 1, 1200, 1100, 0)])
+                                                     (5000, 2, 64, 16, 0), (9, 1, 1200, 1100, 0),
+                                                     (5000, 1, 1200, 1100, 0)])
 @pytest.mark.parametrize("inverse", [False, True])
 @pytest.mark.parametrize("seq_len,start", [(0, 3), (4, 11)])
 def test_rope(dtype, tokens, heads, hd, rot, pad, inverse, seq_len, start):
