@@ -10,7 +10,8 @@
 // chunk of the keys; its 4 warps take 16-key rounds round-robin, each through a private two-stage cp.async ring in
 // shared memory (the next round's K and V rows are in flight while this one is computed).  Scores
 // and P.V of the G = Hq / Hkv grouped heads are warp-level matrix products, the softmax is computed per round.  (The windowed
-// form, whose rows and heads have other sizes, covers a row by hd/8 lanes with packed multiply-adds and shuffles.)  Partial (max, sum, acc) per warp are merged in shared memory and, when
+// form, whose rows and heads have other sizes, covers a row by hd/8 lanes with packed multiply-adds and shuffles.)
+// Partial (max, sum, acc) per warp are merged in shared memory and, when
 // the keys are split across CTAs, through an fp32 workspace: the last CTA of a (query row, kv head) to finish merges
 // the splits itself (arrival counter), so one kernel runs per call (attn_decode_merge_kernel remains for shapes beyond
 // the counter table).
@@ -75,13 +76,10 @@ __device__ __forceinline__ void unpack_bf16x8_f2(const uint4& u, f32x2 (&f)[4]) 
   for (int i = 0; i < 4; ++i) f[i] = f2_pack(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
 
-// GP = grouped query heads padded to a power of two (heads >= G carry zero queries).  A key row is covered by
-// LPK = HD / 8 lanes with 16 bytes each.  Every warp streams its keys in rounds of 16 through a private two-stage ring in
-// shared memory filled by cp.async (16 bytes per lane and instruction): the K and V rows of the next round are in
-// flight while this round is computed, so the loads of the resident warps overlap their arithmetic instead of
-// alternating with it, and no register holds data in flight.  Within a round sub-group sg (LPK lanes) owns keys
-// sg * KS + u, u < KS = LPK / 2; lane u of the sub-group ends up holding that key's scores, the round's softmax is two
-// warp reductions per head and the probabilities are fetched back by shuffle for P.V.
+// GP = grouped query heads padded to a power of two (heads >= G carry zero queries).  Every warp streams its keys in rounds of 16
+// through a private two-stage ring in shared memory filled by cp.async (16 bytes per lane and instruction; a row is LPK = HD / 8
+// of them): the K and V rows of the next round are in flight while this round is computed, so the loads of the resident warps
+// overlap their arithmetic instead of alternating with it, and no register holds data in flight.
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
@@ -96,8 +94,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 constexpr int kDecRound = 16;    // keys per round of a warp
 
 // Arrival counters of the split CTAs of one (query row, kv head): the last CTA to arrive merges the partials, so no
-// second kernel runs.  Zero at load, reset by the merging CTA.  Launches that share the table must not overlap on two streams; callers on several streams pass words of
-// their own.
+// second kernel runs.  Zero at load, reset by the merging CTA.  Launches that share the table must not overlap on two streams;
+// callers on several streams pass words of their own.
 constexpr int kDecCounters = 1 << 16;
 __device__ unsigned int g_dec_counters[kDecCounters];
 constexpr int kDecMaxFusedSplits = 64;
@@ -288,110 +286,113 @@ attn_decode_kernel(const DecodeArgs a) {
       }
     }
   } else {
-  f32x2 qv[GP][4];
-  const __nv_bfloat16* qrow = a.q + (long long)bs * a.ldq + (long long)g * G * dk + sl * 8;
-  const f32x2 scale2 = f2_splat(a.scale);
-#pragma unroll
-  for (int h = 0; h < GP; ++h) {
-    if (h < G && (!WIN || sl * 8 < dk)) {
-      unpack_bf16x8_f2(*reinterpret_cast<const uint4*>(qrow + h * dk), qv[h]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) qv[h][e] = f2_mul(qv[h][e], scale2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) qv[h][e] = f2_splat(0.0f);
-    }
-  }
-  float m[GP], l[GP];
-  f32x2 acc[GP][4];
-#pragma unroll
-  for (int h = 0; h < GP; ++h) {
-    m[h] = -INFINITY;
-    l[h] = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[h][e] = f2_splat(0.0f);
-  }
-  int it_local = 0;
-  for (int t = warp; t < rounds; t += kDecWarps, ++it_local) {
-    const int stage = it_local & 1;
-    if (t + kDecWarps < rounds) {
-      issue(t + kDecWarps, stage ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncwarp();
-    const uint4* ks = ring + stage * 2 * kStageChunks;
-    const uint4* vs = ks + kStageChunks;
-    // ---- scores: lane u of a sub-group keeps the scores of key sg * KS + u of this round
-    float sc[GP];
-#pragma unroll
-    for (int h = 0; h < GP; ++h) sc[h] = -INFINITY;
-#pragma unroll
-    for (int u = 0; u < KS; ++u) {
-      f32x2 kf[4];
-      unpack_bf16x8_f2(ks[(sg * KS + u) * LPK + sl], kf);
-#pragma unroll
-      for (int h = 0; h < GP; ++h) {
-        f32x2 d2 = f2_mul(qv[h][0], kf[0]);
-#pragma unroll
-        for (int e = 1; e < 4; ++e) d2 = f2_fma(qv[h][e], kf[e], d2);
-        float dlo, dhi;
-        f2_unpack(d2, dlo, dhi);
-        float d = dlo + dhi;
-#pragma unroll
-        for (int o = LPK / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (sl == u) sc[h] = d;
-      }
-    }
-    const bool live = sl < KS && j0 + t * kDecRound + sg * KS + sl < j1;
-    // ---- round softmax statistics and rescale
-    float p[GP];
-#pragma unroll
+    // The windowed form, by multiply-adds: a key row is covered by LPK lanes with 16 bytes each.  Within a round sub-group sg (LPK
+    // lanes) owns keys sg * KS + u, u < KS = LPK / 2; lane u of the sub-group ends up holding that key's scores, the round's
+    // softmax is two warp reductions per head and the probabilities are fetched back by shuffle for P.V.
+    f32x2 qv[GP][4];
+    const __nv_bfloat16* qrow = a.q + (long long)bs * a.ldq + (long long)g * G * dk + sl * 8;
+    const f32x2 scale2 = f2_splat(a.scale);
+  #pragma unroll
     for (int h = 0; h < GP; ++h) {
-      const float s = live ? sc[h] : -INFINITY;
-      const float nm = fmaxf(m[h], warp_max(s));
-      const float corr = __expf(m[h] - nm);             // 0 on the first round (m = -inf)
-      p[h] = live ? __expf(s - nm) : 0.0f;
-      l[h] = l[h] * corr + warp_sum(p[h]);
-      m[h] = nm;
-      const f32x2 corr2 = f2_splat(corr);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[h][e] = f2_mul(acc[h][e], corr2);
-    }
-    // ---- P.V: every sub-group accumulates its own keys; the sub-groups are folded once at the end
-#pragma unroll
-    for (int u = 0; u < KS; ++u) {
-      f32x2 vf[4];
-      unpack_bf16x8_f2(vs[(sg * KS + u) * LPK + sl], vf);
-#pragma unroll
-      for (int h = 0; h < GP; ++h) {
-        const f32x2 pj = f2_splat(__shfl_sync(0xffffffffu, p[h], sg0 + u));
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[h][e] = f2_fma(pj, vf[e], acc[h][e]);
+      if (h < G && sl * 8 < dk) {
+        unpack_bf16x8_f2(*reinterpret_cast<const uint4*>(qrow + h * dk), qv[h]);
+  #pragma unroll
+        for (int e = 0; e < 4; ++e) qv[h][e] = f2_mul(qv[h][e], scale2);
+      } else {
+  #pragma unroll
+        for (int e = 0; e < 4; ++e) qv[h][e] = f2_splat(0.0f);
       }
     }
-    __syncwarp();   // every lane has read this stage before the load two rounds ahead overwrites it
-  }
-  // ---- fold the sub-groups of the warp, then the warps of the CTA (fixed order)
-#pragma unroll
-  for (int h = 0; h < GP; ++h) {
-    float af[8];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) f2_unpack(acc[h][e], af[2 * e], af[2 * e + 1]);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-      for (int o = 16; o >= LPK; o >>= 1) af[e] += __shfl_xor_sync(0xffffffffu, af[e], o);
-    if (lane == 0) {
-      s_m[warp][h] = m[h];
-      s_l[warp][h] = l[h];
+    float m[GP], l[GP];
+    f32x2 acc[GP][4];
+  #pragma unroll
+    for (int h = 0; h < GP; ++h) {
+      m[h] = -INFINITY;
+      l[h] = 0.0f;
+  #pragma unroll
+      for (int e = 0; e < 4; ++e) acc[h][e] = f2_splat(0.0f);
     }
-    if (lane < LPK) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s_acc[warp][h][lane * 8 + e] = af[e];
+    int it_local = 0;
+    for (int t = warp; t < rounds; t += kDecWarps, ++it_local) {
+      const int stage = it_local & 1;
+      if (t + kDecWarps < rounds) {
+        issue(t + kDecWarps, stage ^ 1);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      __syncwarp();
+      const uint4* ks = ring + stage * 2 * kStageChunks;
+      const uint4* vs = ks + kStageChunks;
+      // ---- scores: lane u of a sub-group keeps the scores of key sg * KS + u of this round
+      float sc[GP];
+  #pragma unroll
+      for (int h = 0; h < GP; ++h) sc[h] = -INFINITY;
+  #pragma unroll
+      for (int u = 0; u < KS; ++u) {
+        f32x2 kf[4];
+        unpack_bf16x8_f2(ks[(sg * KS + u) * LPK + sl], kf);
+  #pragma unroll
+        for (int h = 0; h < GP; ++h) {
+          f32x2 d2 = f2_mul(qv[h][0], kf[0]);
+  #pragma unroll
+          for (int e = 1; e < 4; ++e) d2 = f2_fma(qv[h][e], kf[e], d2);
+          float dlo, dhi;
+          f2_unpack(d2, dlo, dhi);
+          float d = dlo + dhi;
+  #pragma unroll
+          for (int o = LPK / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+          if (sl == u) sc[h] = d;
+        }
+      }
+      const bool live = sl < KS && j0 + t * kDecRound + sg * KS + sl < j1;
+      // ---- round softmax statistics and rescale
+      float p[GP];
+  #pragma unroll
+      for (int h = 0; h < GP; ++h) {
+        const float s = live ? sc[h] : -INFINITY;
+        const float nm = fmaxf(m[h], warp_max(s));
+        const float corr = __expf(m[h] - nm);             // 0 on the first round (m = -inf)
+        p[h] = live ? __expf(s - nm) : 0.0f;
+        l[h] = l[h] * corr + warp_sum(p[h]);
+        m[h] = nm;
+        const f32x2 corr2 = f2_splat(corr);
+  #pragma unroll
+        for (int e = 0; e < 4; ++e) acc[h][e] = f2_mul(acc[h][e], corr2);
+      }
+      // ---- P.V: every sub-group accumulates its own keys; the sub-groups are folded once at the end
+  #pragma unroll
+      for (int u = 0; u < KS; ++u) {
+        f32x2 vf[4];
+        unpack_bf16x8_f2(vs[(sg * KS + u) * LPK + sl], vf);
+  #pragma unroll
+        for (int h = 0; h < GP; ++h) {
+          const f32x2 pj = f2_splat(__shfl_sync(0xffffffffu, p[h], sg0 + u));
+  #pragma unroll
+          for (int e = 0; e < 4; ++e) acc[h][e] = f2_fma(pj, vf[e], acc[h][e]);
+        }
+      }
+      __syncwarp();   // every lane has read this stage before the load two rounds ahead overwrites it
     }
-  }
+    // ---- fold the sub-groups of the warp, then the warps of the CTA (fixed order)
+  #pragma unroll
+    for (int h = 0; h < GP; ++h) {
+      float af[8];
+  #pragma unroll
+      for (int e = 0; e < 4; ++e) f2_unpack(acc[h][e], af[2 * e], af[2 * e + 1]);
+  #pragma unroll
+      for (int e = 0; e < 8; ++e)
+  #pragma unroll
+        for (int o = 16; o >= LPK; o >>= 1) af[e] += __shfl_xor_sync(0xffffffffu, af[e], o);
+      if (lane == 0) {
+        s_m[warp][h] = m[h];
+        s_l[warp][h] = l[h];
+      }
+      if (lane < LPK) {
+  #pragma unroll
+        for (int e = 0; e < 8; ++e) s_acc[warp][h][lane * 8 + e] = af[e];
+      }
+    }
   }
   __syncthreads();
   for (int idx = threadIdx.x; idx < G * HD; idx += blockDim.x) {

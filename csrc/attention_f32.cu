@@ -5,7 +5,7 @@
 // [batch, seq, head, hd] views (a fused projection output, a cache, separate tensors), head size up to 128, grouped queries.
 //
 //   attn_f32_fwd     CTA = 32 query rows of one (batch, head), walks tiles of 64 keys with a running maximum and sum.  Four CTAs
-//                    fit an SM (48 KB each at heads of 64): what a launch of the composed chain cost in gaps, neighbours now hide.
+//                    fit an SM (51 KB each at heads of 64): what a launch of the composed chain cost in gaps, neighbours now hide.
 //   attn_f32_decode  few query rows over a long history: a cluster of up to 8 CTAs shares the keys of one (batch, kv head), each
 //                    streams its own tiles, and the partial results meet in distributed shared memory (no workspace, fixed order)
 //   attn_f32_dq      CTA = 32 query rows, walks the keys: delta = rowsum(dO O), dQ

@@ -575,8 +575,8 @@ patchify_kernel(const TIn* __restrict__ img, TOut* __restrict__ out, int B, int 
 
 // The same for C channels known at compile time, P and W multiples of 8 and 16-byte aligned buffers: a thread takes eight
 // neighbouring pixels of one image row in every channel, which are 8 * C consecutive features of a patch row.  One index
-// computation and whole 16-byte accesses instead of eight divisions per element: 128 images of 3 x 224 x 224, P = 16, bf16 on
-// B200: 148 us before, 13.8 us.
+// computation and whole 16-byte accesses instead of eight divisions per element: 128 images of 3 x 224 x 224, P = 16, on B200,
+// four batches in turn: bf16 136 us before, 14.7 us; fp32 137 and 35 us.
 template <typename TIn, typename TOut, int C>
 __global__ void __launch_bounds__(kEwThreads)
 patchify_vec8_kernel(const TIn* __restrict__ img, TOut* __restrict__ out, long long groups, int H, int W, int P) {

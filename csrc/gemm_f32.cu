@@ -7,7 +7,7 @@
 // splits are added in order.  (reference: lib/native/src/kernels/matmul.cuh:27-63, one
 // 32x32 shared-memory tile and a separate kernel for each step of the epilogue.)
 //
-// Three kernels by the number of rows:
+// Two kernels by the number of rows:
 //   M <= 8   x W^T only: one pass over W at memory speed, a warp (or four) per pair of weight rows, no tiles.
 //   else     tiles of 128x128 (8x8 outputs per thread), 64x64 (8x4) or 32x64 (4x4), double-buffered through shared
 //            memory; operands are kept k-major there, swizzled so that both a K-contiguous operand (transposed on the
@@ -24,6 +24,11 @@
 namespace dptb {
 
 constexpr int kF32BK = 16;
+// Below this many terms every output is one run of fma over K whatever the number of rows, so a row's bits do not depend on which
+// others are computed with it (a decoder of width below 256 gives the same bits for some rows as for all).  From here on the
+// streaming kernel, the tiles and each split add in an order of their own.  The line is where that property is given up for speed,
+// not where the speed begins.  Measured (B200): 1 x 768 x K, K = 64 / 128 / 256: tiles 3.8 / 5.7 / 10 us, streaming 2.3 / 2.3 / 2.4 us;
+// 8 rows 4.2 / 6.1 / 10 and 2.9 / 3.0 / 3.1 us; 256 x 256 x K, K = 128 / 192 / 256: one run 6.2 / 8.1 / 10.1 us, split 6.7 / 7.0 / 7.4 us.
 constexpr int kOneRunK = 256;
 
 struct GemmF32Params {
@@ -455,16 +460,15 @@ static int product_f32(const DptbGemmArgs* a, cudaStream_t st) {
   p.k_per_split = (a->K + kF32BK - 1) / kF32BK * kF32BK;
   const bool amn = a->trans_a != 0, bmn = a->trans_b == 0;
 
-  // Below kOneRunK terms every output is one run of fma over K whatever the number of rows, so a row's bits do not depend on
-  // which others are computed with it; the streaming kernel and the splits start where their gain is (1 x 768 x 768: 3.1 us
-  // against 8 to 10 us by tiles).
   if (a->M <= 8 && a->K >= kOneRunK && !amn && !bmn && a->bn == 0 && a->splits <= 1) {
     return counted(1, (int)(a->M == 1 ? launch_gemv<1, 2>(p, st) : a->M == 2 ? launch_gemv<2, 2>(p, st)
                           : a->M <= 4 ? launch_gemv<4, 2>(p, st) : launch_gemv<8, 2>(p, st)));
   }
 
   // Tile and split of K by a small model of an SM: the CTAs that land on the busiest one share its multiply-add
-  // units, which 16 resident warps keep busy; `rate` is the share of their peak that the tile's inner loop reaches.
+  // units, which 16 resident warps keep busy; `rate` is the share of their peak that the tile's inner loop reaches, between what
+  // 4096 x 4096 x K gives in one run at K = 2048 (B200: 51.4, 46.2 and 33.8 of 74.5 TFLOP/s: 0.69, 0.62, 0.45) and at K = 256 (0.63,
+  // 0.58, 0.43).
   struct Tile { int bm, bn, warps; double rate; };
   static const Tile kTiles[3] = {{128, 128, 8, 0.70}, {64, 64, 4, 0.57}, {32, 64, 4, 0.42}};
   const int sms = sm_count();

@@ -43,7 +43,8 @@ __device__ __forceinline__ void row_online_max_sum(const T* __restrict__ xr, int
 #pragma unroll
         for (int j = 0; j < 8; ++j) lm = fmaxf(lm, v[j]);
       }
-      const float base = lm == -INFINITY ? 0.0f : lm;      // all -inf: no weight; a NaN among them still shows in ls
+      // all -inf: no weight.  A NaN shows in ls, and stays unless nothing finite has been seen by then (see online_combine).
+      const float base = lm == -INFINITY ? 0.0f : lm;
       float ls = 0.0f;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
