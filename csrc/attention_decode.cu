@@ -80,10 +80,6 @@ __device__ __forceinline__ void unpack_bf16x8_f2(const uint4& u, f32x2 (&f)[4]) 
 // through a private two-stage ring in shared memory filled by cp.async (16 bytes per lane and instruction; a row is LPK = HD / 8
 // of them): the K and V rows of the next round are in flight while this round is computed, so the loads of the resident warps
 // overlap their arithmetic instead of alternating with it, and no register holds data in flight.
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async_16_or_zero(void* smem_dst, const void* gsrc, bool valid) {
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(valid ? 16 : 0) : "memory");
@@ -155,7 +151,7 @@ attn_decode_kernel(const DecodeArgs a) {
   uint4* ring = dec_ring + warp * kWarpChunks;   // [stage][K | V][16 rows][LPK chunks]
   const int sg = lane / LPK;
   const int rounds = (j1 - j0 + kDecRound - 1) / kDecRound;   // of this CTA; warp w takes rounds w, w + 4, ...
-  // Rows past the end of the range are fetched from the last valid row (finite data) and masked in the softmax.
+  // Rows past the end of the range are zeros (the windowed form fetches the last valid row) and masked in the softmax.
   auto issue = [&](int t, int stage) {
     const int key0 = j0 + t * kDecRound;
     uint4* dst = ring + stage * 2 * kStageChunks;
@@ -175,8 +171,9 @@ attn_decode_kernel(const DecodeArgs a) {
       } else {
         const long long off = (long long)key * a.ldkv + (c % LPK) * 8;
         const int at = c ^ (c / LPK & 7);       // 16-byte pieces of eight neighbouring rows fall on different banks
-        cp_async_16(dst + at, kb + off);
-        cp_async_16(dst + kStageChunks + at, vb + off);
+        const bool live = key0 + c / LPK < j1;  // (a weight of zero times a value that is not finite would be NaN)
+        cp_async_16_or_zero(dst + at, kb + off, live);
+        cp_async_16_or_zero(dst + kStageChunks + at, vb + off, live);
       }
     }
     cp_async_commit();
@@ -236,10 +233,10 @@ attn_decode_kernel(const DecodeArgs a) {
         float mx = fmaxf(sv[0], sv[1]);
 #pragma unroll
         for (int off = 4; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const float nm = fmaxf(m2[e], mx);
-        corr[e] = __expf(m2[e] - nm);         // 0 on the first round (m = -inf)
+        const float nm = fmaxf(m2[e], mx), sub = nm == -INFINITY ? 0.0f : nm;     // nothing but -inf so far: no weight
+        corr[e] = __expf(m2[e] - sub);        // 0 on the first round (m = -inf)
 #pragma unroll
-        for (int r = 0; r < 2; ++r) p[r][e] = live[r] ? __expf(sv[r] - nm) : 0.0f;
+        for (int r = 0; r < 2; ++r) p[r][e] = live[r] ? __expf(sv[r] - sub) : 0.0f;
         l2[e] = l2[e] * corr[e] + (p[0][e] + p[1][e]);
         m2[e] = nm;
       }
@@ -415,7 +412,7 @@ attn_decode_kernel(const DecodeArgs a) {
       }
       decode_store_windowed(a, bs, g * G + h, d, q_pos, oo / ll);
     } else if (a.splits == 1) {
-      a.o[(long long)bs * a.ldo + (long long)(g * G + h) * HD + d] = __float2bfloat16(ll > 0.0f ? oo / ll : 0.0f);
+      a.o[(long long)bs * a.ldo + (long long)(g * G + h) * HD + d] = __float2bfloat16(ll == 0.0f ? 0.0f : oo / ll);
     } else {
       float* w = a.ws + ((((long long)bs * a.Hkv + g) * a.splits + split) * G + h) * (HD + 2);
       w[d] = oo;
@@ -506,7 +503,7 @@ attn_decode_kernel(const DecodeArgs a) {
       decode_store_windowed(a, bs, g * G + hh[k], idx % HD, q_pos, oo[k] / ll[k]);
     } else {
       a.o[(long long)bs * a.ldo + (long long)(g * G + idx / HD) * HD + idx % HD] =
-          __float2bfloat16(ll[k] > 0.0f ? oo[k] / ll[k] : 0.0f);
+          __float2bfloat16(ll[k] == 0.0f ? 0.0f : oo[k] / ll[k]);
     }
   }
 }
@@ -529,7 +526,7 @@ attn_decode_merge_kernel(const DecodeArgs a) {
       ll += base[s * stride + HD + 1] * c;
       oo += base[s * stride + d] * c;
     }
-    a.o[(long long)bs * a.ldo + (long long)hq * HD + d] = __float2bfloat16(ll > 0.0f ? oo / ll : 0.0f);
+    a.o[(long long)bs * a.ldo + (long long)hq * HD + d] = __float2bfloat16(ll == 0.0f ? 0.0f : oo / ll);
   }
 }
 
