@@ -1,7 +1,7 @@
 // Embedding gather (optionally fused with a learned position table) and its scatter-add backward.
 //
 // Out-of-range indices read as a zero row and are skipped in the backward, as in the reference
-// (lib/native/src/kernels/embedding.cuh:19-48).  The backward comes in two forms: a sorted,
+// (lib/native/src/kernels/embedding.cuh:19-48).  The backward comes in three forms: a sorted,
 // segmented sum (one warp per distinct index, rows added in ascending order -> bit-reproducible), a form
 // for short index lists that finds the equal indices itself instead of having them sorted (the same additions in the same
 // order), and an atomic form.
