@@ -82,3 +82,33 @@ def test_non_finite_scores_behave_as_softmax_does():
     ref = _exact(q, k, v, True, 0)
     assert torch.equal(o.isnan(), ref.isnan())
     assert torch.allclose(o[~ref.isnan()], ref[~ref.isnan()], rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("Sq,Sk,causal", [(1, 2, True), (1, 65, True), (1, 700, True), (4, 130, False), (40, 130, False)])
+@pytest.mark.parametrize("H,Hkv,hd", [(2, 1, 64), (2, 2, 24)])
+@pytest.mark.parametrize("what", ["value inf", "value -inf", "value nan", "key nan", "key inf", "scores -inf", "most scores -inf"])
+@pytest.mark.parametrize("at", [0, -1, "middle"])
+def test_non_finite_operands(Sq, Sk, causal, H, Hkv, hd, what, at):
+    """Every key that these queries see, in the split form and in the tiles."""
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v = (torch.randn(1, h, s, hd, device="cuda", generator=g) for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    q[..., 3] = 1.0
+    j = Sk // 2 if at == "middle" else at
+    kind, x = what.rsplit(" ", 1)
+    if kind == "value":
+        v[:, :, j, 5] = float(x)
+    elif kind == "key":
+        k[:, :, j, 3] = float(x)
+    elif kind == "scores":
+        k[:, :, j, 3] = float("-inf")
+    else:
+        keep = k[:, :, j].clone()
+        k[..., 3] = float("-inf")
+        k[:, :, j] = keep
+    o = A.attention_bhsd(q, k, v, causal, None, Sk - Sq)
+    d = [t.double() for t in (q, k, v)]
+    s = d[0] @ d[1].repeat_interleave(H // Hkv, 1).transpose(-1, -2) / math.sqrt(hd)
+    ref = s.softmax(-1) @ d[2].repeat_interleave(H // Hkv, 1)
+    assert torch.equal(o.isnan(), ref.isnan()) and torch.equal(o.isinf(), ref.isinf())
+    fin = ref.isfinite()
+    assert torch.equal(o[ref.isinf()].double(), ref[ref.isinf()]) and torch.allclose(o[fin].double(), ref[fin], rtol=1e-5, atol=1e-5)
