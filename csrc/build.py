@@ -33,7 +33,7 @@ NVCC_FLAGS = [
 ]
 
 COMPONENTS = {
-    "serve": ["gemm", "gemm_f32", "gemm_nt", "gemm_skinny", "gemm_grouped", "attention_fwd", "attention_decode", "attention_f32", "latent_attention",
+    "serve": ["gemm", "gemm_f32", "gemm_f32_tc", "gemm_nt", "gemm_skinny", "gemm_grouped", "attention_fwd", "attention_decode", "attention_f32", "latent_attention",
               "window_attention", "recurrent", "linear_attention", "moe_local", "stream_norm", "branch_norm", "rope", "elementwise"],
 }
 

@@ -1,25 +1,27 @@
-// fp32 GEMM on the CUDA cores' packed multiply-adds, every operand layout, with a fused fp32 epilogue:
+// fp32 GEMM, every operand layout, with a fused fp32 epilogue:
 //
 //   C[M,N] = epilogue( op(A)[M,K] * op(B)[K,N] ),   epilogue: *alpha, +bias, aux_out <- value, act, *act'(aux_in),
 //                                                             +residual, (+C)
 //
-// The products stay in 32 bits: every multiply-add is an IEEE fma into one accumulator per output and split of K, the
-// splits are added in order.  (reference: lib/native/src/kernels/matmul.cuh:27-63, one
-// 32x32 shared-memory tile and a separate kernel for each step of the epilogue.)
+// (reference: lib/native/src/kernels/matmul.cuh:27-63, one 32x32 shared-memory tile and a separate kernel for each step of the
+// epilogue.)
 //
-// Two kernels by the number of rows:
+// The kernels of this file are multiply-adds: every one an IEEE fma into one accumulator per output and split of K, the splits
+// added in order.  Two by the number of rows:
 //   M <= 8   x W^T only: one pass over W at memory speed, a warp (or four) per pair of weight rows, no tiles.
 //   else     tiles of 128x128 (8x8 outputs per thread), 64x64 (8x4) or 32x64 (4x4), double-buffered through shared
 //            memory; operands are kept k-major there, swizzled so that both a K-contiguous operand (transposed on the
 //            way in) and an M/N-contiguous one are stored and read without bank conflicts.
 // What bounds the tiles is the issue of multiply-adds: fma.rn.f32x2 does two per instruction, which leaves issue slots
-// for the shared-memory loads beside them.
+// for the shared-memory loads beside them.  From 256 terms on, where a tile's multiply-adds outweigh its launch, the tensor cores
+// take over (gemm_f32_tc.cu).
 #include <cuda_bf16.h>
 
 #include "common/gemm_args.h"
 #include "common/host.h"
 #include "common/ptx.cuh"
 #include "common/reduce.cuh"
+#include "gemm_f32.cuh"
 
 namespace dptb {
 
@@ -30,94 +32,6 @@ constexpr int kF32BK = 16;
 // not where the speed begins.  Measured (B200): 1 x 768 x K, K = 64 / 128 / 256: tiles 3.8 / 5.7 / 10 us, streaming 2.3 / 2.3 / 2.4 us;
 // 8 rows 4.2 / 6.1 / 10 and 2.9 / 3.0 / 3.1 us; 256 x 256 x K, K = 128 / 192 / 256: one run 6.2 / 8.1 / 10.1 us, split 6.7 / 7.0 / 7.4 us.
 constexpr int kOneRunK = 256;
-
-struct GemmF32Params {
-  const float* A;
-  const float* B;
-  float* C;
-  const void* bias;
-  const float* residual;
-  float* aux_out;
-  const float* aux_in;
-  long long lda, ldb, ldc, ldr, ld_aux_out, ld_aux_in;
-  int M, N, K;
-  int bias_f32, accumulate, act;
-  float alpha;
-  int vec_a, vec_b, vec_c;   // 16-byte accesses allowed (base and leading dimension)
-  int splits, k_per_split;   // k_per_split is a multiple of kF32BK
-  float* ws;
-  int* counters;
-};
-
-// Activations as the elementwise kernels compute them (accurate tanh / exp): the values do not depend on whether the
-// activation is fused.
-__device__ __forceinline__ float act_f32(int act, float x) {
-  switch (act) {
-    case 1: return fmaxf(x, 0.0f);
-    case 2: return 0.5f * x * (1.0f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
-    case 3: return x / (1.0f + expf(-1.702f * x));
-    case 4: return x / (1.0f + expf(-x));
-    default: return x;
-  }
-}
-__device__ __forceinline__ float act_grad_f32(int act, float x) {
-  switch (act) {
-    case 11: return x > 0.0f ? 1.0f : 0.0f;
-    case 12: {
-      const float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
-      return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * x * x);
-    }
-    case 13: {
-      const float s = 1.0f / (1.0f + expf(-1.702f * x));
-      return s + 1.702f * x * s * (1.0f - s);
-    }
-    case 14: {
-      const float s = 1.0f / (1.0f + expf(-x));
-      return s * (1.0f + x * (1.0f - s));
-    }
-    case 15: return x;
-    default: return 1.0f;
-  }
-}
-__device__ __forceinline__ void epilogue_f32(const GemmF32Params& p, long long row, int col, float v) {
-  v *= p.alpha;
-  if (p.bias) v += p.bias_f32 ? static_cast<const float*>(p.bias)[col] : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col]);
-  if (p.aux_out) p.aux_out[row * p.ld_aux_out + col] = v;
-  if (p.act >= 11) v *= act_grad_f32(p.act, p.aux_in[row * p.ld_aux_in + col]);
-  else if (p.act) v = act_f32(p.act, v);
-  if (p.residual) v += p.residual[row * p.ldr + col];
-  float* c = p.C + row * p.ldc + col;
-  *c = p.accumulate ? *c + v : v;
-}
-// Four neighbouring columns; every buffer takes 16-byte accesses (vec_c).
-__device__ __forceinline__ void epilogue_f32x4(const GemmF32Params& p, long long row, int col, float4 v4) {
-  float v[4] = {v4.x * p.alpha, v4.y * p.alpha, v4.z * p.alpha, v4.w * p.alpha};
-  if (p.bias) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      v[j] += p.bias_f32 ? static_cast<const float*>(p.bias)[col + j]
-                         : __bfloat162float(static_cast<const __nv_bfloat16*>(p.bias)[col + j]);
-  }
-  if (p.aux_out) *reinterpret_cast<float4*>(p.aux_out + row * p.ld_aux_out + col) = make_float4(v[0], v[1], v[2], v[3]);
-  if (p.act >= 11) {
-    const float4 x = *reinterpret_cast<const float4*>(p.aux_in + row * p.ld_aux_in + col);
-    v[0] *= act_grad_f32(p.act, x.x); v[1] *= act_grad_f32(p.act, x.y);
-    v[2] *= act_grad_f32(p.act, x.z); v[3] *= act_grad_f32(p.act, x.w);
-  } else if (p.act) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = act_f32(p.act, v[j]);
-  }
-  if (p.residual) {
-    const float4 r = *reinterpret_cast<const float4*>(p.residual + row * p.ldr + col);
-    v[0] += r.x; v[1] += r.y; v[2] += r.z; v[3] += r.w;
-  }
-  float4* c = reinterpret_cast<float4*>(p.C + row * p.ldc + col);
-  if (p.accumulate) {
-    const float4 o = *c;
-    v[0] = o.x + v[0]; v[1] = o.y + v[1]; v[2] = o.z + v[2]; v[3] = o.w + v[3];
-  }
-  *c = make_float4(v[0], v[1], v[2], v[3]);
-}
 
 // Position of element `mn` of k-row `k` in a shared tile of `R` elements per k-row: bits 3-4 are flipped by k / 4.  The
 // four k-groups that a warp stores at once from a K-contiguous operand then fall on different banks, and 4-element
@@ -490,6 +404,18 @@ static int product_f32(const DptbGemmArgs* a, cudaStream_t st) {
       // the fold: each split's tile leaves and comes back through L2
       const double fold = sp > 1 ? 2500.0 + area * 4.0 * sp / 64.0 : 0.0;
       if (clocks + fold < best_cost) { best_cost = clocks + fold; best = t; best_sp = sp; }
+    }
+  }
+  // Tensor cores where they are expected to be faster (1.8 us: what the model above leaves out, launch and first loads).  Not below
+  // kOneRunK, and not for forced tiles.
+  if ((a->bn == 0 && a->splits < 1 && a->K >= kOneRunK) || a->bn == 1064 || a->bn == 1128) {
+    int bn = a->bn - 1000, sp = a->splits < 1 ? 1 : a->splits;
+    if (a->bn || f32_tc_plan(a->M, a->N, a->K, &bn, &sp) < best_cost / 1900.0 + 1.8) {
+      const int kb = (a->K + kF32TcBK - 1) / kF32TcBK, per = kb > 0 ? (kb + sp - 1) / sp : 1;
+      p.k_per_split = per * kF32TcBK;
+      p.splits = kb > 0 ? (kb + per - 1) / per : 1;
+      if (p.splits > 8 || (a->M + 127) / 128 > 65535) return kErrBadShape;
+      return counted(1, (int)launch_f32_tc(p, bn, amn, bmn, st));
     }
   }
   p.k_per_split = ((a->K + best_sp - 1) / best_sp + kF32BK - 1) / kF32BK * kF32BK;
