@@ -9,14 +9,16 @@
 // output needs no split / permute, and O is written as [B*Sq, Hq*hd] ready for the output projection.
 // Grouped-query attention: query head h reads KV head h / (Hq / Hkv).
 //
-// One CTA owns NQ query tiles of 128 rows of one (batch, head) and walks the KV sequence in tiles of 128 keys:
+// One persistent CTA an SM works through units of NQ query tiles of 128 rows of one (batch, head), heavy ones first, and walks the
+// unit's keys in tiles of 128:
 //   warps 0-3 / 4-7  softmax warpgroups, one per query tile, one thread per query row: pull the whole S row (128
 //                    scores) from TMEM into registers in one go and hand the S columns straight back to the tensor
 //                    core, so S_t(j+1) = Q_t K_{j+1}^T is computed while this tile's softmax runs; then max / exp2 /
 //                    sum and P (bf16) into shared memory in the tensor core's K-major swizzled layout
-//   warp 8           TMA producer (Q once, K / V through rings)
-//   warp 9           MMA issuer: S_t = Q_t K_j^T, and O_t += P_t V_j accumulated in TMEM
-// The output accumulator never leaves TMEM during the loop.  The running maximum is lazy: a row keeps exponentiating
+//   warp 8           TMA producer (Q once a unit, K / V through rings); it runs ahead into the next unit
+//   warps 9, 10      MMA issuers, one per query tile: S_t = Q_t K_j^T, and O_t += P_t V_j accumulated in TMEM
+// The two query tiles meet nowhere but at the rings: with one issuer for both, which waits for them in turn, the softmax
+// warpgroups ran in step and wanted the special-function unit at the same time.  The output accumulator never leaves TMEM during the loop.  The running maximum is lazy: a row keeps exponentiating
 // against an older maximum until the true one has grown by more than 8 (a factor 256 of headroom in fp32 / bf16);
 // only then (decided per warp) O is pulled out, rescaled and stored back, which after the first tiles is rare.
 //
@@ -93,7 +95,7 @@ struct AttnFwdSmem {
   static constexpr int kVOff = kKOff + KST * kKVBytes;
   static constexpr int kPOff = kVOff + VST * kKVBytes;
   static constexpr int kBarOff = kPOff + NQ * kPBytes;
-  static constexpr int kNumBars = NQ + 2 * KST + 2 * VST + 4 * NQ + 1;
+  static constexpr int kNumBars = 2 * NQ + 2 * KST + 2 * VST + 5 * NQ;
   static constexpr int kTotal = kBarOff + kNumBars * 8 + 16 + 1024;
   static_assert(kTotal <= 227 * 1024, "attention forward: shared memory budget");
 };
@@ -114,7 +116,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
   uint64_t* q_full = bars;                          // [NQ]
-  uint64_t* k_full = q_full + NQ;                   // [KST]
+  uint64_t* q_empty = q_full + NQ;                  // [NQ] every S_t of the unit has been computed
+  uint64_t* k_full = q_empty + NQ;                  // [KST]
   uint64_t* k_empty = k_full + KST;
   uint64_t* v_full = k_empty + KST;                 // [VST]
   uint64_t* v_empty = v_full + VST;
@@ -122,44 +125,56 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* s_empty = s_full + NQ;                  // [NQ] S_t(j) has been copied to registers
   uint64_t* p_full = s_empty + NQ;                  // [NQ] P_t(j) is in shared memory (and O_t is rescaled)
   uint64_t* o_full = p_full + NQ;                   // [NQ] O_t += P_t(j) V_j has completed
-  uint64_t* drain_bar = o_full + NQ;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  uint64_t* drain_bar = o_full + NQ;                // [NQ]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + NQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Heavy (late) query blocks first when causal.
-  const int qb = p.causal ? (p.num_q_blocks - 1 - (int)blockIdx.x) : (int)blockIdx.x;
-  const int head = blockIdx.y, batch = blockIdx.z;
-  const int kv_head = head / (p.Hq / p.Hkv);
-  const int q_row0 = qb * (NQ * kAttnBM);
-
-  // Number of KV tiles each query tile needs; with a window they start with n_pool tiles of pooled rows, and the first token
-  // tile is tile0.
-  int n_tiles[NQ];
-  int n_max = 0, n_pool = 0, tile0 = 0;
   auto pooled_rows = [&](int row) {     // pooled rows that query `row` sees
     const int left = p.pos + row - p.window + 1;
     return p.pool > 0 && left >= p.pool ? min(left / p.pool, p.pool_rows) : 0;
   };
-  if constexpr (WIN) {
-    n_pool = (pooled_rows(min(q_row0 + NQ * kAttnBM, p.Sq) - 1) + kAttnBN - 1) / kAttnBN;
-    tile0 = max(0, q_row0 + p.q_offset - p.window + 1) / kAttnBN;
-  }
-#pragma unroll
-  for (int t = 0; t < NQ; ++t) {
-    const int r0 = q_row0 + t * kAttnBM;
-    int n = 0;
-    if (r0 < p.Sq) {
-      int last_key = p.Sk - 1;
-      if (p.causal) {
-        const int r_last = min(r0 + kAttnBM - 1, p.Sq - 1);
-        last_key = min(last_key, r_last + p.q_offset);
-      }
-      n = last_key >= 0 ? last_key / kAttnBN + 1 - tile0 + n_pool : 0;
+  // The unit of round `r` of this CTA.  Causal units are ordered heavy (late query rows) first and handed out back and forth, so that
+  // a CTA's sum of work stays near the mean (16 x 12 heads x 1024 queries: the largest is 1.09 of it, 1.16 if every round went the
+  // same way).
+  struct Unit {
+    int q_row0, head, batch, kv_head;
+    int n_tiles[NQ];                    // KV tiles each query tile needs (0: it has no rows, or none that sees a key)
+    int n_max, n_pool, tile0;           // with a window they start with n_pool tiles of pooled rows; first token tile
+  };
+  const int per_block = p.Hq * p.B, num_units = p.num_q_blocks * per_block;
+  const int num_rounds = (num_units + (int)gridDim.x - 1) / (int)gridDim.x;
+  auto get_unit = [&](int r, Unit& w) -> bool {
+    const int u = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    if (u >= num_units) return false;
+    const int qb = p.causal ? p.num_q_blocks - 1 - u / per_block : u % p.num_q_blocks;
+    const int rest = p.causal ? u % per_block : u / p.num_q_blocks;
+    w.head = rest % p.Hq;
+    w.batch = rest / p.Hq;
+    w.kv_head = w.head / (p.Hq / p.Hkv);
+    w.q_row0 = qb * (NQ * kAttnBM);
+    w.n_max = w.n_pool = w.tile0 = 0;
+    if constexpr (WIN) {
+      w.n_pool = (pooled_rows(min(w.q_row0 + NQ * kAttnBM, p.Sq) - 1) + kAttnBN - 1) / kAttnBN;
+      w.tile0 = max(0, w.q_row0 + p.q_offset - p.window + 1) / kAttnBN;
     }
-    n_tiles[t] = n;
-    n_max = max(n_max, n);
-  }
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) {
+      const int r0 = w.q_row0 + t * kAttnBM;
+      int n = 0;
+      if (r0 < p.Sq) {
+        int last_key = p.Sk - 1;
+        if (p.causal) {
+          const int r_last = min(r0 + kAttnBM - 1, p.Sq - 1);
+          last_key = min(last_key, r_last + p.q_offset);
+        }
+        n = last_key >= 0 ? last_key / kAttnBN + 1 - w.tile0 + w.n_pool : 0;
+      }
+      w.n_tiles[t] = n;
+      w.n_max = max(w.n_max, n);
+    }
+    return true;
+  };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -171,20 +186,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) {
       for (int t = 0; t < NQ; ++t) {
         mbar_init(&q_full[t], 1);
+        mbar_init(&q_empty[t], 1);
         mbar_init(&s_full[t], 1);
         mbar_init(&s_empty[t], kAttnBM);
         mbar_init(&p_full[t], kAttnBM);
         mbar_init(&o_full[t], 1);
+        mbar_init(&drain_bar[t], 1);
       }
       for (int s = 0; s < KST; ++s) {
         mbar_init(&k_full[s], 1);
-        mbar_init(&k_empty[s], 1);
+        mbar_init(&k_empty[s], NQ);        // both issuers let go of a stage
       }
       for (int s = 0; s < VST; ++s) {
         mbar_init(&v_full[s], 1);
-        mbar_init(&v_empty[s], 1);
+        mbar_init(&v_empty[s], NQ);
       }
-      mbar_init(drain_bar, 1);
       mbar_fence_init();
     }
     __syncwarp();
@@ -201,126 +217,139 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      for (int t = 0; t < NQ; ++t) {
-        if (n_tiles[t] == 0) continue;
-        mbar_arrive_expect_tx(&q_full[t], L::kQBytes);
-        for (int c = 0; c < kChunks; ++c) {
-          uint8_t* dst = smem + L::kQOff + t * L::kQBytes + c * (kAttnBM * 128);
-          if constexpr (WIN || SUB) tma_load_4d(dst, &tmQ, &q_full[t], c * 64, head, q_row0 + t * kAttnBM, batch);
-          else tma_load_3d(dst, &tmQ, &q_full[t], head * HD + c * 64, q_row0 + t * kAttnBM, batch);
+      int q_issued[NQ] = {}, k_issued = 0, v_issued = 0;
+      Unit w;
+      bool ok = true;
+      for (int r = 0; r < num_rounds && ok; ++r) {
+        if (!get_unit(r, w)) break;
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) {
+          if (w.n_tiles[t] == 0 || !ok) continue;
+          ok = mbar_wait(&q_empty[t], (q_issued[t] & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&q_full[t], L::kQBytes);
+          for (int c = 0; c < kChunks; ++c) {
+            uint8_t* dst = smem + L::kQOff + t * L::kQBytes + c * (kAttnBM * 128);
+            if constexpr (WIN || SUB) tma_load_4d(dst, &tmQ, &q_full[t], c * 64, w.head, w.q_row0 + t * kAttnBM, w.batch);
+            else tma_load_3d(dst, &tmQ, &q_full[t], w.head * HD + c * 64, w.q_row0 + t * kAttnBM, w.batch);
+          }
+          ++q_issued[t];
         }
-      }
-      int k_issued = 0, v_issued = 0;
-      for (int j = 0; j < n_max; ++j) {
-        const int ks = j % KST, vs = j % VST;
-        if (!mbar_wait(&k_empty[ks], ((j / KST) & 1) ^ 1, abort_flag, kWaitEmptyTimeout)) break;
-        mbar_arrive_expect_tx(&k_full[ks], L::kKVBytes);
-        for (int c = 0; c < kChunks; ++c) {
-          uint8_t* dst = smem + L::kKOff + ks * L::kKVBytes + c * (kAttnBN * 128);
-          if constexpr (WIN)
-            tma_load_4d(dst, j < n_pool ? &tmPK : &tmK, &k_full[ks], c * 64, kv_head,
-                        (j < n_pool ? j : j - n_pool + tile0) * kAttnBN, batch);
-          else if constexpr (SUB) tma_load_4d(dst, &tmK, &k_full[ks], c * 64, kv_head, j * kAttnBN, batch);
-          else tma_load_3d(dst, &tmK, &k_full[ks], kv_head * HD + c * 64, j * kAttnBN, batch);
+        for (int j = 0; j < w.n_max && ok; ++j) {
+          const int ks = k_issued % KST, vs = v_issued % VST;
+          ok = mbar_wait(&k_empty[ks], ((k_issued / KST) & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&k_full[ks], L::kKVBytes);
+          for (int c = 0; c < kChunks; ++c) {
+            uint8_t* dst = smem + L::kKOff + ks * L::kKVBytes + c * (kAttnBN * 128);
+            if constexpr (WIN)
+              tma_load_4d(dst, j < w.n_pool ? &tmPK : &tmK, &k_full[ks], c * 64, w.kv_head,
+                          (j < w.n_pool ? j : j - w.n_pool + w.tile0) * kAttnBN, w.batch);
+            else if constexpr (SUB) tma_load_4d(dst, &tmK, &k_full[ks], c * 64, w.kv_head, j * kAttnBN, w.batch);
+            else tma_load_3d(dst, &tmK, &k_full[ks], w.kv_head * HD + c * 64, j * kAttnBN, w.batch);
+          }
+          ++k_issued;
+          ok = mbar_wait(&v_empty[vs], ((v_issued / VST) & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+          if (!ok) break;
+          mbar_arrive_expect_tx(&v_full[vs], L::kKVBytes);
+          for (int c = 0; c < kChunks; ++c) {
+            uint8_t* dst = smem + L::kVOff + vs * L::kKVBytes + c * (kAttnBN * 128);
+            if constexpr (WIN)
+              tma_load_4d(dst, j < w.n_pool ? &tmPV : &tmV, &v_full[vs], c * 64, w.kv_head,
+                          (j < w.n_pool ? j : j - w.n_pool + w.tile0) * kAttnBN, w.batch);
+            else if constexpr (SUB) tma_load_4d(dst, &tmV, &v_full[vs], c * 64, w.kv_head, j * kAttnBN, w.batch);
+            else tma_load_3d(dst, &tmV, &v_full[vs], w.kv_head * HD + c * 64, j * kAttnBN, w.batch);
+          }
+          ++v_issued;
         }
-        k_issued = j + 1;
-        if (!mbar_wait(&v_empty[vs], ((j / VST) & 1) ^ 1, abort_flag, kWaitEmptyTimeout)) break;
-        mbar_arrive_expect_tx(&v_full[vs], L::kKVBytes);
-        for (int c = 0; c < kChunks; ++c) {
-          uint8_t* dst = smem + L::kVOff + vs * L::kKVBytes + c * (kAttnBN * 128);
-          if constexpr (WIN)
-            tma_load_4d(dst, j < n_pool ? &tmPV : &tmV, &v_full[vs], c * 64, kv_head,
-                        (j < n_pool ? j : j - n_pool + tile0) * kAttnBN, batch);
-          else if constexpr (SUB) tma_load_4d(dst, &tmV, &v_full[vs], c * 64, kv_head, j * kAttnBN, batch);
-          else tma_load_3d(dst, &tmV, &v_full[vs], kv_head * HD + c * 64, j * kAttnBN, batch);
-        }
-        v_issued = j + 1;
       }
       if (*abort_flag) {
         // Wait (bounded) for copies that may still be landing in this CTA's shared memory.
         const uint64_t t0 = global_timer_ns();
         for (int t = 0; t < NQ; ++t)
-          while (n_tiles[t] && !mbar_try_wait(&q_full[t], 0) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+          while (q_issued[t] && !mbar_try_wait(&q_full[t], (q_issued[t] - 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
         for (int j = max(0, k_issued - KST); j < k_issued; ++j)
           while (!mbar_try_wait(&k_full[j % KST], (j / KST) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
         for (int j = max(0, v_issued - VST); j < v_issued; ++j)
           while (!mbar_try_wait(&v_full[j % VST], (j / VST) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
       }
     }
-  } else if (warp == 9) {
-    // ------------------------------------------------------------------ MMA issuer
+  } else if (warp < 9 + NQ) {
+    // ------------------------------------------------------------------ MMA issuer of query tile t
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(kAttnBM, kAttnBN, false, false);
       constexpr uint32_t idesc_o = make_idesc_bf16(kAttnBM, HD, false, true);
+      const int t = warp - 9;
+      const uint32_t qa = smem_u32(smem + L::kQOff + t * L::kQBytes);
+      const uint32_t pa = smem_u32(smem + L::kPOff + t * L::kPBytes);
       bool issued_any = false;
       bool ok = true;
-      auto issue_s = [&](int t, int j) {
-        const uint32_t qa = smem_u32(smem + L::kQOff + t * L::kQBytes);
-        const uint32_t kb = smem_u32(smem + L::kKOff + (j % KST) * L::kKVBytes);
+      int kv = 0;            // KV tiles before this unit, of either query tile
+      int tiles = 0;         // tiles of this query tile whose S has been issued
+      int done = 0;          // ... and whose P V has been
+      int units = 0;
+      Unit w;
+      for (int r = 0; r < num_rounds && ok; ++r) {
+        if (!get_unit(r, w)) break;
+        const int n = t == 0 ? w.n_tiles[0] : w.n_tiles[NQ - 1];
+        if (n > 0) {
+          ok = mbar_wait(&q_full[t], units & 1, abort_flag, kWaitFullTimeout);
+          ++units;
+        }
+        // Before tile j's P V, S of tile j + 1 as soon as the softmax warpgroup has copied the one before out of TMEM.
+        for (int j = -1; j < w.n_max && ok; ++j) {
+          if (j + 1 < w.n_max) {
+            const int ks = (kv + j + 1) % KST;
+            ok = mbar_wait(&k_full[ks], ((kv + j + 1) / KST) & 1, abort_flag, kWaitFullTimeout);
+            if (ok && j + 1 < n) {
+              if (tiles > 0) ok = mbar_wait(&s_empty[t], (tiles - 1) & 1, abort_flag, kWaitTmemEmptyTimeout);
+              if (!ok) break;
+              tc_fence_after_sync();
+              const uint32_t kb = smem_u32(smem + L::kKOff + ks * L::kKVBytes);
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t q_off = (kk / 4) * (kAttnBM * 128) + (kk % 4) * 32;
-          const uint32_t k_off = (kk / 4) * (kAttnBN * 128) + (kk % 4) * 32;
-          umma_bf16(tmem_base + kSCol + t * 128, make_smem_desc(qa + q_off, 16, 1024),
-                    make_smem_desc(kb + k_off, 16, 1024), idesc_s, kk != 0);
-        }
-        umma_commit(&s_full[t]);
-        issued_any = true;
-      };
-      // Prologue: S_t(0) for every query tile.
-      if (n_max > 0) {
-        ok = mbar_wait(&k_full[0], 0, abort_flag, kWaitFullTimeout);
-        for (int t = 0; t < NQ && ok; ++t) {
-          if (n_tiles[t] == 0) continue;
-          ok = mbar_wait(&q_full[t], 0, abort_flag, kWaitFullTimeout);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_s(t, 0);
-        }
-        if (ok) umma_commit(&k_empty[0]);
-      }
-      for (int j = 0; j < n_max && ok; ++j) {
-        // (a) S_t(j+1) as soon as the softmax warpgroup has copied S_t(j) out of TMEM.
-        if (j + 1 < n_max) {
-          const int ks1 = (j + 1) % KST;
-          ok = mbar_wait(&k_full[ks1], ((j + 1) / KST) & 1, abort_flag, kWaitFullTimeout);
-          for (int t = 0; t < NQ && ok; ++t) {
-            if (j + 1 >= n_tiles[t]) continue;
-            ok = mbar_wait(&s_empty[t], j & 1, abort_flag, kWaitTmemEmptyTimeout);
+              for (int kk = 0; kk < HD / 16; ++kk) {
+                const uint32_t q_off = (kk / 4) * (kAttnBM * 128) + (kk % 4) * 32;
+                const uint32_t k_off = (kk / 4) * (kAttnBN * 128) + (kk % 4) * 32;
+                umma_bf16(tmem_base + kSCol + t * 128, make_smem_desc(qa + q_off, 16, 1024),
+                          make_smem_desc(kb + k_off, 16, 1024), idesc_s, kk != 0);
+              }
+              umma_commit(&s_full[t]);
+              if (j + 1 == n - 1) umma_commit(&q_empty[t]);
+              issued_any = true;
+              ++tiles;
+            }
+            if (!ok) break;
+            umma_commit(&k_empty[ks]);
+          }
+          if (j < 0) continue;
+          const int vs = (kv + j) % VST;
+          ok = mbar_wait(&v_full[vs], ((kv + j) / VST) & 1, abort_flag, kWaitFullTimeout);
+          if (ok && j < n) {
+            // O_t += P_t(j) V_j once P_t(j) is in shared memory (and, for j = 0, the unit before has been read out of O_t)
+            ok = mbar_wait(&p_full[t], done & 1, abort_flag, kWaitFlagTimeout);
             if (!ok) break;
             tc_fence_after_sync();
-            issue_s(t, j + 1);
-          }
-          if (!ok) break;
-          umma_commit(&k_empty[ks1]);
-        }
-        // (b) O_t += P_t(j) V_j once P_t(j) is in shared memory.
-        const int vs = j % VST;
-        ok = mbar_wait(&v_full[vs], (j / VST) & 1, abort_flag, kWaitFullTimeout);
-        for (int t = 0; t < NQ && ok; ++t) {
-          if (j >= n_tiles[t]) continue;
-          ok = mbar_wait(&p_full[t], j & 1, abort_flag, kWaitFlagTimeout);
-          if (!ok) break;
-          tc_fence_after_sync();
-          const uint32_t pa = smem_u32(smem + L::kPOff + t * L::kPBytes);
-          const uint32_t vb = smem_u32(smem + L::kVOff + vs * L::kKVBytes);
+            const uint32_t vb = smem_u32(smem + L::kVOff + vs * L::kKVBytes);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {     // 128 keys, or the high and then the low parts of 64
-            const uint32_t aoff = (kk / 4) * (kAttnBM * 128) + (kk % 4) * 32;
-            umma_bf16(tmem_base + kOCol + t * HD, make_smem_desc(pa + aoff, 16, 1024),
-                      make_smem_desc(vb + (PREC ? kk % 4 : kk) * 2048, kAttnBN * 128, 1024), idesc_o,
-                      (j != 0 || kk != 0) ? 1u : 0u);
+            for (int kk = 0; kk < 8; ++kk) {     // 128 keys, or the high and then the low parts of 64
+              const uint32_t aoff = (kk / 4) * (kAttnBM * 128) + (kk % 4) * 32;
+              umma_bf16(tmem_base + kOCol + t * HD, make_smem_desc(pa + aoff, 16, 1024),
+                        make_smem_desc(vb + (PREC ? kk % 4 : kk) * 2048, kAttnBN * 128, 1024), idesc_o,
+                        (j != 0 || kk != 0) ? 1u : 0u);
+            }
+            umma_commit(&o_full[t]);
+            issued_any = true;
+            ++done;
           }
-          umma_commit(&o_full[t]);
-          issued_any = true;
+          if (!ok) break;
+          umma_commit(&v_empty[vs]);
         }
-        if (!ok) break;
-        umma_commit(&v_empty[vs]);
+        kv += w.n_max;
       }
       if (*abort_flag && issued_any) {
-        umma_commit(drain_bar);
+        umma_commit(&drain_bar[t]);
         const uint64_t t0 = global_timer_ns();
-        while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+        while (!mbar_try_wait(&drain_bar[t], 0) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
       }
     }
   }
@@ -330,13 +359,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int t = warp >> 2;
     const int q = warp & 3;
     const int row_in_tile = q * 32 + lane;
-    const int q_row = q_row0 + t * kAttnBM + row_in_tile;         // row inside the sequence
-    const int n = n_tiles[t];
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t s_addr = lane_addr + kSCol + t * 128;
     const uint32_t o_addr = lane_addr + kOCol + t * HD;
     uint8_t* p_tile = smem + L::kPOff + t * L::kPBytes;
 
+    int tiles = 0;             // tiles of this warpgroup before the present one
+    bool ok = true;
+    Unit w;
+#ifdef DPTB_ATTN_PROFILE
+    long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const long long prof_begin = clock64();
+#endif
+    for (int r = 0; r < num_rounds && ok; ++r) {
+    if (!get_unit(r, w)) break;
+    const int q_row = w.q_row0 + t * kAttnBM + row_in_tile;       // row inside the sequence
+    const int n = t == 0 ? w.n_tiles[0] : w.n_tiles[NQ - 1];
+    const int head = w.head, batch = w.batch;
     float m_use = -INFINITY;   // the maximum the stored exponentials are relative to (lags the true maximum)
     float l_run = 0.0f;
     int pool_limit = -1;       // last visible pooled row
@@ -348,15 +387,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
     const int key_limit = p.causal ? min(p.Sk - 1, q_row + p.q_offset) : p.Sk - 1;  // last visible key of this row
-    bool ok = true;
-#ifdef DPTB_ATTN_PROFILE
-    long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const long long prof_begin = clock64();
-#endif
-
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n && ok; ++j, ++tiles) {
       ATTN_PROF_MARK(pt0);
-      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], j & 1, abort_flag, kWaitTmemFullTimeout));
+      ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], tiles & 1, abort_flag, kWaitTmemFullTimeout));
       if (!ok) break;
       ATTN_PROF_MARK(pt1);
       tc_fence_after_sync();
@@ -369,8 +402,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ATTN_PROF_MARK(pt2);
 
       if constexpr (WIN) {
-        const bool pooled = j < n_pool;
-        const int key0 = (pooled ? j : j - n_pool + tile0) * kAttnBN;
+        const bool pooled = j < w.n_pool;
+        const int key0 = (pooled ? j : j - w.n_pool + w.tile0) * kAttnBN;
         const int hi = pooled ? pool_limit : key_limit, lo = pooled ? 0 : q_row + p.q_offset - p.window + 1;
         if (key0 + kAttnBN - 1 > hi || key0 < lo) {
 #pragma unroll
@@ -402,7 +435,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const float m_new = fmaxf(m_use, m_tile);
         const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_use - m_new);   // m_use = -inf -> 0
         if (j > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (j - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
           if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
@@ -423,12 +456,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ATTN_PROF_MARK(pt4);
       // The previous P_t must have been consumed before it is overwritten (it nearly always has been by now).
       if (j > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (j - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
         if (!ok) break;
       }
       ATTN_PROF_MARK(pt5);
       // Probabilities -> bf16 -> shared memory (K-major, 128-byte swizzle), row sum.
-      float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f, l3 = 0.0f;
+      f32x2 l01 = 0ull, l23 = 0ull;
+      const f32x2 scale2 = f2_splat(p.scale_log2), neg_m2 = f2_splat(-m_sub);
 #pragma unroll
       for (int c = 0; c < kAttnBN / 32; ++c) {
         uint32_t packed[16], low[16];
@@ -438,11 +472,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           // against 102 us at B16 H12 S1024 hd64; the softmax warps are bound by issue slots, not by the
           // special-function unit.  Taking the exponentials two at a time in bf16, ex2.approx.bf16x2, was slower as
           // well, 115 us, for the unpacking its row sum needs.)
-          const float a = fast_exp2(fmaf(__uint_as_float(s[c * 32 + i + 0]), p.scale_log2, -m_sub));
-          const float b = fast_exp2(fmaf(__uint_as_float(s[c * 32 + i + 1]), p.scale_log2, -m_sub));
-          const float e = fast_exp2(fmaf(__uint_as_float(s[c * 32 + i + 2]), p.scale_log2, -m_sub));
-          const float f = fast_exp2(fmaf(__uint_as_float(s[c * 32 + i + 3]), p.scale_log2, -m_sub));
-          l0 += a; l1 += b; l2 += e; l3 += f;
+          float a, b, e, f;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(s[c * 32 + i]), __uint_as_float(s[c * 32 + i + 1])), scale2, neg_m2), a, b);
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(s[c * 32 + i + 2]), __uint_as_float(s[c * 32 + i + 3])), scale2, neg_m2), e, f);
+          a = fast_exp2(a); b = fast_exp2(b); e = fast_exp2(e); f = fast_exp2(f);
+          l01 = f2_add(l01, f2_pack(a, b));
+          l23 = f2_add(l23, f2_pack(e, f));
           packed[(i >> 1) + 0] = pack_bf16x2(a, b);
           packed[(i >> 1) + 1] = pack_bf16x2(e, f);
           if constexpr (PREC) {
@@ -463,6 +498,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 make_uint4(low[i * 4 + 0], low[i * 4 + 1], low[i * 4 + 2], low[i * 4 + 3]);
         }
       }
+      float l0, l1, l2, l3;
+      f2_unpack(l01, l0, l1);
+      f2_unpack(l23, l2, l3);
       l_run += (l0 + l1) + (l2 + l3);
       fence_proxy_async_smem();
       tc_fence_before_sync();
@@ -475,15 +513,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ATTN_PROF_ADD(4, pt4, pt5);
       ATTN_PROF_ADD(5, pt5, pt6);
     }
-#ifdef DPTB_ATTN_PROFILE
-    if (threadIdx.x == 0) {
-      prof_acc[6] = clock64() - prof_begin;
-      prof_acc[7] = n;
-      for (int i = 0; i < 8; ++i) atomicAdd(&g_attn_prof[i], (unsigned long long)prof_acc[i]);
-    }
-#endif
     if (ok && n > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (n - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
       if (ok) {
         tc_fence_after_sync();
         const bool live = q_row < p.Sq;
@@ -535,6 +566,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     }
+    }
+#ifdef DPTB_ATTN_PROFILE
+    if (threadIdx.x == 0) {
+      prof_acc[6] = clock64() - prof_begin;
+      prof_acc[7] = tiles;
+      for (int i = 0; i < 8; ++i) atomicAdd(&g_attn_prof[i], (unsigned long long)prof_acc[i]);
+    }
+#endif
   }
 
   tc_fence_before_sync();
@@ -563,6 +602,12 @@ static int encode_tmap_heads(CUtensorMap* map, const void* base, int heads, int 
   const uint64_t strides[3] = {(uint64_t)hd * 2, (uint64_t)ld * 2, (uint64_t)batch_rows * ld * 2};
   const uint32_t box[4] = {64, 1, (uint32_t)box_rows, 1};
   return encode_tmap_nd_bf16(map, base, 4, dims, strides, box);
+}
+
+// One CTA an SM (shared memory and TMEM allow no more), or one a unit.
+static int attn_grid(const AttnFwdParams& p) {
+  const long long units = (long long)p.num_q_blocks * p.Hq * p.B;
+  return units < sm_count() ? (int)units : sm_count();
 }
 
 }  // namespace dptb
@@ -597,8 +642,7 @@ static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   p.num_q_blocks = (a->Sq + NQ * kAttnBM - 1) / (NQ * kAttnBM);
   auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false, SUB>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  dim3 grid(p.num_q_blocks, a->Hq, a->B);
-  kern<<<grid, kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
+  kern<<<attn_grid(p), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
   return counted(1, (int)cudaGetLastError());
 }
 
@@ -673,7 +717,7 @@ static int window_fwd_launch(const DptbWindowFwdArgs* a, cudaStream_t st) {
   p.rot = static_cast<const float2*>(a->rot);
   auto kern = attn_fwd_kernel<HD, 2, KST, VST, true, true, false>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  kern<<<dim3(p.num_q_blocks, a->H, a->B), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmPK, tmPV, p);
+  kern<<<attn_grid(p), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmPK, tmPV, p);
   return counted(1, (int)cudaGetLastError());
 }
 

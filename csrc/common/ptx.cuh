@@ -401,6 +401,11 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ f32x2 f2_splat(float x) { return f2_pack(x, x); }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
