@@ -5,8 +5,8 @@
 // lib/core/tensor/mat_mul.dart:56-74).  Here one kernel recomputes the probabilities tile by tile and produces
 // dQ, dK and dV without any [N, N] tensor in HBM.
 //
-// One CTA owns one tile of 128 keys of one (batch, KV head) and loops over the query heads of its group and over the
-// query tiles that can see those keys.  Per query tile, five tensor-core products:
+// One persistent CTA an SM works through units: one tile of 128 keys of one (batch, KV head), with a loop over the query heads of
+// its group and over the query tiles that can see those keys.  Per query tile, five tensor-core products:
 //   S  = Q K^T          dP = dO V^T                       (into TMEM, rows = queries)
 //   dV += P^T dO        dK += dS^T Q                      (accumulate in TMEM across the whole loop, rows = keys)
 //   dQ  = dS K                                            (TMEM -> shared staging -> fp32 reduction into dq_acc)
@@ -14,9 +14,9 @@
 // layout that serves both as a K-major operand (dS K) and, transposed, as an MN-major operand (P^T dO, dS^T Q).
 //   warps 0-7  two compute warpgroups: thread = one query row x one half (64 keys) of the S / dP tiles.  A thread pulls
 //              its 64 scores and 64 dP values from TMEM in one go and hands the columns straight back, so the tensor core
-//              computes S / dP of the next query tile while P / dS of this one are formed; it then drains its quarter
-//              of the previous tile's dQ (TMEM -> shared staging -> fp32 reduction into dq_acc)
-//   warp 8     TMA producer      warp 9     MMA issuer      (warps 10-11 only take part in the register hand-over)
+//              computes S / dP of the next query tile while P / dS of this one are formed
+//   warps 8-11 drain dQ of the tile before (TMEM -> shared staging -> fp32 reduction into dq_acc)
+//   warp 12    TMA producer      warp 13    MMA issuer      (warps 14-15 only take part in the register hand-over)
 #include <cuda_bf16.h>
 
 #include "common/host.h"
@@ -47,7 +47,7 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 
 // Opt-in phase timers (compile with -DDPTB_ATTN_PROFILE), SM clock cycles summed over all CTAs:
 //   compute thread 0:  [0] wait S/dP  [1] TMEM -> registers  [2] P / dS math  [3] wait for the previous products
-//                      [4] stores + signal  [5] dQ drain  [6] loop total  [7] iterations
+//                      [4] stores + signal  [5] dK / dV out  [6] loop total  [7] iterations
 //   MMA issuer:        [8] wait Q/dO  [9] wait S/dP drained  [10] wait P/dS  [11] wait dQ drained  [12] loop total
 #ifdef DPTB_ATTN_PROFILE
 __device__ unsigned long long g_attn_bwd_prof[16];
@@ -60,11 +60,13 @@ __device__ unsigned long long g_attn_bwd_prof[16];
 
 constexpr int kBwdHD = 64;
 constexpr int kBwdTile = 128;
-constexpr int kBwdThreads = 384;
-// Registers per thread after the hand-over (the CTA starts with 384 x 168 and the pool does not grow).
-constexpr int kBwdComputeRegs = 216;
+constexpr int kBwdThreads = 512;
+// Registers per thread after the hand-over (the CTA starts with 512 x 128 and the pool does not grow).
+constexpr int kBwdComputeRegs = 168;
+constexpr int kBwdDrainRegs = 96;
 constexpr int kBwdProducerRegs = 72;
-static_assert(2 * 128 * kBwdComputeRegs + 128 * kBwdProducerRegs <= kBwdThreads * 168, "register hand-over must balance");
+static_assert(2 * 128 * kBwdComputeRegs + 128 * kBwdDrainRegs + 128 * kBwdProducerRegs <= kBwdThreads * 128,
+              "register hand-over must balance");
 constexpr int kBwdStages = 2;
 constexpr int kDqStride = 68;  // floats per staged dQ row (padding keeps 16-byte accesses conflict-free)
 
@@ -80,7 +82,7 @@ struct AttnBwdSmem {
   static constexpr int kDqOff = kDSOff + kPBytes;
   static constexpr int kDqBytes = kBwdTile * kDqStride * 4;
   static constexpr int kBarOff = kDqOff + kDqBytes;
-  static constexpr int kNumBars = 1 + 2 * kBwdStages + 7;
+  static constexpr int kNumBars = 2 + 2 * kBwdStages + 8;
   static constexpr int kTotal = kBarOff + kNumBars * 8 + 16 + 1024;
 };
 
@@ -96,31 +98,47 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = kv_full + 1;               // [stages]
+  uint64_t* kv_empty = kv_full + 1;               // every product of the unit has read K and V
+  uint64_t* qdo_full = kv_empty + 1;              // [stages]
   uint64_t* qdo_empty = qdo_full + kBwdStages;    // [stages]
   uint64_t* sdp_full = qdo_empty + kBwdStages;    // S and dP of the current query tile are in TMEM
   uint64_t* sdp_empty = sdp_full + 1;             // ... and have been copied to registers by all 256 compute threads
   uint64_t* pds_full = sdp_empty + 1;             // P and dS are in shared memory
-  uint64_t* dq_full = pds_full + 1;
+  uint64_t* dq_full = pds_full + 1;               // dQ of the tile is in TMEM, and every product that reads P / dS is done
   uint64_t* dq_empty = dq_full + 1;
   uint64_t* dkv_full = dq_empty + 1;
-  uint64_t* drain_bar = dkv_full + 1;
+  uint64_t* dkv_empty = dkv_full + 1;             // dK / dV of the unit have been copied to registers
+  uint64_t* drain_bar = dkv_empty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, kv_head = blockIdx.y, batch = blockIdx.z;
-  const int key0 = kt * kBwdTile;
   const int group = p.Hq / p.Hkv;
   const int n_q_tiles = (p.Sq + kBwdTile - 1) / kBwdTile;
-  // First query tile with a row that can see key0 (causal: i + q_offset >= key0).
-  int i_start = 0;
-  if (p.causal) {
-    const int first_row = key0 - p.q_offset;
-    i_start = first_row > 0 ? first_row / kBwdTile : 0;
-  }
-  const int tiles_per_head = n_q_tiles > i_start ? n_q_tiles - i_start : 0;
-  const int total_iters = tiles_per_head * group;
+  // The unit of round `r` of this CTA: causal ones heavy (early keys) first, handed out back and forth so that a CTA's sum of work
+  // stays near the mean.
+  struct Unit {
+    int key0, kv_head, batch;
+    int i_start, iters;      // first query tile with a row that sees key0; tiles over all heads of the group
+  };
+  const int n_k_tiles = (p.Sk + kBwdTile - 1) / kBwdTile;
+  const int per_tile = p.Hkv * p.B, num_units = n_k_tiles * per_tile;
+  const int num_rounds = (num_units + (int)gridDim.x - 1) / (int)gridDim.x;
+  auto get_unit = [&](int r, Unit& w) -> bool {
+    const int u = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    if (u >= num_units) return false;
+    const int rest = p.causal ? u % per_tile : u / n_k_tiles;
+    w.key0 = (p.causal ? u / per_tile : u % n_k_tiles) * kBwdTile;
+    w.kv_head = rest % p.Hkv;
+    w.batch = rest / p.Hkv;
+    w.i_start = 0;
+    if (p.causal) {          // causal: row i sees keys up to i + q_offset
+      const int first_row = w.key0 - p.q_offset;
+      w.i_start = first_row > 0 ? first_row / kBwdTile : 0;
+    }
+    w.iters = (n_q_tiles > w.i_start ? n_q_tiles - w.i_start : 0) * group;
+    return true;
+  };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -129,9 +147,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
   }
-  if (warp == 9) {
+  if (warp == 13) {
     if (lane == 0) {
       mbar_init(kv_full, 1);
+      mbar_init(kv_empty, 1);
       for (int s = 0; s < kBwdStages; ++s) {
         mbar_init(&qdo_full[s], 1);
         mbar_init(&qdo_empty[s], 1);
@@ -140,8 +159,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_init(sdp_empty, 2 * kBwdTile);
       mbar_init(pds_full, 2 * kBwdTile);
       mbar_init(dq_full, 1);
-      mbar_init(dq_empty, 2 * kBwdTile);
+      mbar_init(dq_empty, kBwdTile);
       mbar_init(dkv_full, 1);
+      mbar_init(dkv_empty, 2 * kBwdTile);
       mbar_init(drain_bar, 1);
       mbar_fence_init();
     }
@@ -153,47 +173,63 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp >= 8) {
+  if (warp >= 12) {
     warpgroup_reg_dec<kBwdProducerRegs>();
-  if (warp == 8) {
+  if (warp == 12) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && total_iters > 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * L::kTileBytes);
-      tma_load_3d(smem + L::kKOff, &tmK, kv_full, kv_head * HD, key0, batch);
-      tma_load_3d(smem + L::kVOff, &tmV, kv_full, kv_head * HD, key0, batch);
-      int it = 0;
-      for (int g = 0; g < group && !*abort_flag; ++g) {
-        const int head = kv_head * group + g;
-        for (int i = i_start; i < n_q_tiles; ++i, ++it) {
-          const int s = it % kBwdStages;
-          const uint32_t ph = (it / kBwdStages) & 1;
-          if (!mbar_wait(&qdo_empty[s], ph ^ 1, abort_flag, kWaitEmptyTimeout)) break;
-          mbar_arrive_expect_tx(&qdo_full[s], 2 * L::kTileBytes);
-          tma_load_3d(smem + L::kQOff + s * L::kTileBytes, &tmQ, &qdo_full[s], head * HD, i * kBwdTile, batch);
-          tma_load_3d(smem + L::kDOOff + s * L::kTileBytes, &tmDO, &qdo_full[s], head * HD, i * kBwdTile, batch);
+    if (lane == 0) {
+      int it = 0, units = 0;
+      Unit w;
+      bool ok = true;
+      for (int r = 0; r < num_rounds && ok; ++r) {
+        if (!get_unit(r, w)) break;
+        if (w.iters == 0) continue;
+        for (int g = 0; g < group && ok; ++g) {
+          const int head = w.kv_head * group + g;
+          for (int i = w.i_start; i < n_q_tiles; ++i, ++it) {
+            const int s = it % kBwdStages;
+            ok = mbar_wait(&qdo_empty[s], ((it / kBwdStages) & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&qdo_full[s], 2 * L::kTileBytes);
+            tma_load_3d(smem + L::kQOff + s * L::kTileBytes, &tmQ, &qdo_full[s], head * HD, i * kBwdTile, w.batch);
+            tma_load_3d(smem + L::kDOOff + s * L::kTileBytes, &tmDO, &qdo_full[s], head * HD, i * kBwdTile, w.batch);
+            if (g == 0 && i == w.i_start) {
+              // K and V after the first query tile, whose stage is free before the unit ahead has let go of its keys.
+              ok = mbar_wait(kv_empty, (units & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+              if (!ok) { ++it; break; }
+              mbar_arrive_expect_tx(kv_full, 2 * L::kTileBytes);
+              tma_load_3d(smem + L::kKOff, &tmK, kv_full, w.kv_head * HD, w.key0, w.batch);
+              tma_load_3d(smem + L::kVOff, &tmV, kv_full, w.kv_head * HD, w.key0, w.batch);
+              ++units;
+            }
+          }
         }
       }
       if (*abort_flag) {
+        // Wait (bounded) for copies that may still be landing in this CTA's shared memory.
         const uint64_t t0 = global_timer_ns();
-        while (!mbar_try_wait(kv_full, 0) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+        while (units > 0 && !mbar_try_wait(kv_full, (units - 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
         for (int j = max(0, it - kBwdStages); j < it; ++j)
           while (!mbar_try_wait(&qdo_full[j % kBwdStages], (j / kBwdStages) & 1) &&
                  global_timer_ns() - t0 < kWaitLimitNs / 4) {}
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == 13) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && total_iters > 0) {
+    if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(kBwdTile, kBwdTile, false, false);   // S, dP
       constexpr uint32_t idesc_kv = make_idesc_bf16(kBwdTile, HD, true, true);          // dV, dK
       constexpr uint32_t idesc_q = make_idesc_bf16(kBwdTile, HD, false, true);          // dQ
       const uint32_t k_addr = smem_u32(smem + L::kKOff), v_addr = smem_u32(smem + L::kVOff);
       const uint32_t p_addr = smem_u32(smem + L::kPOff), ds_addr = smem_u32(smem + L::kDSOff);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, kWaitFullTimeout);
-      bool issued_any = false;
-      // S = Q K^T and dP = dO V^T of query tile `it` (operands in stage it % stages).
-      auto issue_sdp = [&](int it) {
-        const int s = it % kBwdStages;
+      bool ok = true, issued_any = false;
+      int it = 0, units = 0;             // query tiles and units before the present one
+      // S = Q K^T and dP = dO V^T of query tile `n` once its operands have landed and the tile before has been copied out.
+      auto issue_sdp = [&](int n) -> bool {
+        const int s = n % kBwdStages;
+        if (!mbar_wait(&qdo_full[s], (n / kBwdStages) & 1, abort_flag, kWaitFullTimeout)) return false;
+        if (n > 0 && !mbar_wait(sdp_empty, (n - 1) & 1, abort_flag, kWaitTmemEmptyTimeout)) return false;
+        tc_fence_after_sync();
         const uint32_t q_addr = smem_u32(smem + L::kQOff + s * L::kTileBytes);
         const uint32_t do_addr = smem_u32(smem + L::kDOOff + s * L::kTileBytes);
 #pragma unroll
@@ -206,73 +242,72 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                     make_smem_desc(v_addr + kk * 32, 16, 1024), idesc_s, kk != 0);
         umma_commit(sdp_full);
         issued_any = true;
+        return true;
       };
-      if (ok) ok = mbar_wait(&qdo_full[0], 0, abort_flag, kWaitFullTimeout);
-      if (ok) {
-        tc_fence_after_sync();
-        issue_sdp(0);
-      }
 #ifdef DPTB_ATTN_PROFILE
       long long prof_acc[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
       const long long prof_begin = clock64();
 #endif
-      for (int it = 0; it < total_iters && ok; ++it) {
-        const int s = it % kBwdStages;
-        const uint32_t q_addr = smem_u32(smem + L::kQOff + s * L::kTileBytes);
-        const uint32_t do_addr = smem_u32(smem + L::kDOOff + s * L::kTileBytes);
-        // (a) S / dP of the next query tile, as soon as the compute warps have copied this tile's out of TMEM.
-        if (it + 1 < total_iters) {
-          const int s1 = (it + 1) % kBwdStages;
+      Unit w;
+      for (int r = 0; r < num_rounds && ok; ++r) {
+        if (!get_unit(r, w)) break;
+        if (w.iters == 0) continue;
+        ok = mbar_wait(kv_full, units & 1, abort_flag, kWaitFullTimeout) && issue_sdp(it);
+        for (int n = 0; n < w.iters && ok; ++n, ++it) {
+          const int s = it % kBwdStages;
+          const uint32_t q_addr = smem_u32(smem + L::kQOff + s * L::kTileBytes);
+          const uint32_t do_addr = smem_u32(smem + L::kDOOff + s * L::kTileBytes);
+          // (a) S / dP of the next query tile, as soon as the compute warps have copied this tile's out of TMEM.
           BWD_PROF_MARK(m0);
-          ok = mbar_wait(&qdo_full[s1], ((it + 1) / kBwdStages) & 1, abort_flag, kWaitFullTimeout);
-          BWD_PROF_MARK(m1);
-          if (ok) ok = mbar_wait(sdp_empty, it & 1, abort_flag, kWaitTmemEmptyTimeout);
+          if (n + 1 < w.iters) ok = issue_sdp(it + 1);
           BWD_PROF_MARK(m2);
-          BWD_PROF_ADD(8, m0, m1);
-          BWD_PROF_ADD(9, m1, m2);
+          BWD_PROF_ADD(9, m0, m2);
+          if (!ok) break;
+          // (b) the three products that consume P / dS of this tile.
+          BWD_PROF_MARK(m3);
+          ok = mbar_wait(pds_full, it & 1, abort_flag, kWaitFlagTimeout);
+          if (ok && n == 0 && units > 0)       // dK / dV of the unit ahead have left TMEM
+            ok = mbar_wait(dkv_empty, (units - 1) & 1, abort_flag, kWaitTmemEmptyTimeout);
+          BWD_PROF_MARK(m4);
+          BWD_PROF_ADD(10, m3, m4);
           if (!ok) break;
           tc_fence_after_sync();
-          issue_sdp(it + 1);
+          // dV += P^T dO ; dK += dS^T Q    (A: [q rows][keys] read as MN-major, B: [q rows][hd] read as MN-major)
+#pragma unroll
+          for (int kk = 0; kk < kBwdTile / 16; ++kk)
+            umma_bf16(tmem_base + kDVCol, make_smem_desc(p_addr + kk * 2048, kBwdTile * 128, 1024),
+                      make_smem_desc(do_addr + kk * 2048, kBwdTile * 128, 1024), idesc_kv, (n | kk) != 0);
+#pragma unroll
+          for (int kk = 0; kk < kBwdTile / 16; ++kk)
+            umma_bf16(tmem_base + kDKCol, make_smem_desc(ds_addr + kk * 2048, kBwdTile * 128, 1024),
+                      make_smem_desc(q_addr + kk * 2048, kBwdTile * 128, 1024), idesc_kv, (n | kk) != 0);
+          if (it > 0) {
+            BWD_PROF_MARK(m5);
+            ok = mbar_wait(dq_empty, (it - 1) & 1, abort_flag, kWaitFlagTimeout);
+            BWD_PROF_MARK(m6);
+            BWD_PROF_ADD(11, m5, m6);
+            if (!ok) break;
+            tc_fence_after_sync();
+          }
+          // dQ = dS K   (A: dS K-major over keys, B: K tile [keys][hd] read as MN-major)
+#pragma unroll
+          for (int kk = 0; kk < kBwdTile / 16; ++kk)
+            umma_bf16(tmem_base + kDQCol,
+                      make_smem_desc(ds_addr + (kk / 4) * (kBwdTile * 128) + (kk % 4) * 32, 16, 1024),
+                      make_smem_desc(k_addr + kk * 2048, kBwdTile * 128, 1024), idesc_q, kk != 0);
+          umma_commit(dq_full);
+          umma_commit(&qdo_empty[s]);
+          issued_any = true;
         }
-        // (b) the three products that consume P / dS of this tile.
-        BWD_PROF_MARK(m3);
-        ok = mbar_wait(pds_full, it & 1, abort_flag, kWaitFlagTimeout);
-        BWD_PROF_MARK(m4);
-        BWD_PROF_ADD(10, m3, m4);
         if (!ok) break;
-        tc_fence_after_sync();
-        // dV += P^T dO ; dK += dS^T Q    (A: [q rows][keys] read as MN-major, B: [q rows][hd] read as MN-major)
-#pragma unroll
-        for (int kk = 0; kk < kBwdTile / 16; ++kk)
-          umma_bf16(tmem_base + kDVCol, make_smem_desc(p_addr + kk * 2048, kBwdTile * 128, 1024),
-                    make_smem_desc(do_addr + kk * 2048, kBwdTile * 128, 1024), idesc_kv, (it | kk) != 0);
-#pragma unroll
-        for (int kk = 0; kk < kBwdTile / 16; ++kk)
-          umma_bf16(tmem_base + kDKCol, make_smem_desc(ds_addr + kk * 2048, kBwdTile * 128, 1024),
-                    make_smem_desc(q_addr + kk * 2048, kBwdTile * 128, 1024), idesc_kv, (it | kk) != 0);
-        if (it > 0) {
-          BWD_PROF_MARK(m5);
-          ok = mbar_wait(dq_empty, (it - 1) & 1, abort_flag, kWaitFlagTimeout);
-          BWD_PROF_MARK(m6);
-          BWD_PROF_ADD(11, m5, m6);
-          if (!ok) break;
-          tc_fence_after_sync();
-        }
-        // dQ = dS K   (A: dS K-major over keys, B: K tile [keys][hd] read as MN-major)
-#pragma unroll
-        for (int kk = 0; kk < kBwdTile / 16; ++kk)
-          umma_bf16(tmem_base + kDQCol,
-                    make_smem_desc(ds_addr + (kk / 4) * (kBwdTile * 128) + (kk % 4) * 32, 16, 1024),
-                    make_smem_desc(k_addr + kk * 2048, kBwdTile * 128, 1024), idesc_q, kk != 0);
-        umma_commit(dq_full);
-        umma_commit(&qdo_empty[s]);
-        issued_any = true;
+        umma_commit(kv_empty);
+        umma_commit(dkv_full);
+        ++units;
       }
 #ifdef DPTB_ATTN_PROFILE
       prof_acc[12] = clock64() - prof_begin;
       for (int i = 8; i < 13; ++i) atomicAdd(&g_attn_bwd_prof[i], (unsigned long long)prof_acc[i]);
 #endif
-      if (ok) umma_commit(dkv_full);
       if (*abort_flag && issued_any) {
         umma_commit(drain_bar);
         const uint64_t t0 = global_timer_ns();
@@ -280,6 +315,53 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   }
+  } else if (warp >= 8) {
+    // ------------------------------------------------------------------ dQ: TMEM -> staging -> fp32 reduction
+    warpgroup_reg_dec<kBwdDrainRegs>();
+    const int q = warp & 3;              // TMEM lane quarter: rows [32 q, 32 q + 32) of the query tile
+    const uint32_t dq_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kDQCol;
+    float* stage = reinterpret_cast<float*>(smem + L::kDqOff) + q * 32 * kDqStride;
+    int it = 0;
+    Unit w;
+    bool ok = true;
+    for (int r = 0; r < num_rounds && ok; ++r) {
+      if (!get_unit(r, w)) break;
+      if (w.iters == 0) continue;
+      for (int g = 0; g < group && ok; ++g) {
+        const int head = w.kv_head * group + g;
+        for (int i = w.i_start; i < n_q_tiles; ++i, ++it) {
+          ok = __all_sync(0xffffffffu, mbar_wait(dq_full, it & 1, abort_flag, kWaitTmemFullTimeout));
+          if (!ok) break;
+          tc_fence_after_sync();
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(dq_addr, r0);
+          tmem_ld_32x32(dq_addr + 32, r1);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          mbar_arrive(dq_empty);
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            *reinterpret_cast<float4*>(stage + lane * kDqStride + e) =
+                make_float4(__uint_as_float(r0[e]), __uint_as_float(r0[e + 1]), __uint_as_float(r0[e + 2]), __uint_as_float(r0[e + 3]));
+            *reinterpret_cast<float4*>(stage + lane * kDqStride + 32 + e) =
+                make_float4(__uint_as_float(r1[e]), __uint_as_float(r1[e + 1]), __uint_as_float(r1[e + 2]), __uint_as_float(r1[e + 3]));
+          }
+          __syncwarp();
+          // 2 rows of 256 bytes per instruction
+          const int col = (lane & 15) * 4;
+          float* dst = p.dq_acc + ((long long)w.batch * p.Sq + i * kBwdTile + q * 32) * ((long long)p.Hq * HD) + (long long)head * HD + col;
+#pragma unroll
+          for (int rr = 0; rr < 32; rr += 2) {
+            const int r_loc = rr + (lane >> 4);
+            if (i * kBwdTile + q * 32 + r_loc < p.Sq) {
+              const float4 v = *reinterpret_cast<const float4*>(stage + r_loc * kDqStride + col);
+              red_add_v4(dst + (long long)r_loc * p.Hq * HD, v.x, v.y, v.z, v.w);
+            }
+          }
+          __syncwarp();
+        }
+      }
+    }
   } else {
     // ------------------------------------------------------------------ compute warpgroups
     warpgroup_reg_inc<kBwdComputeRegs>();
@@ -289,49 +371,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     uint8_t* p_tile = smem + L::kPOff + half * (kBwdTile * 128);     // 64-key block `half` of the K-major tiles
     uint8_t* ds_tile = smem + L::kDSOff + half * (kBwdTile * 128);
-    float* dq_stage = reinterpret_cast<float*>(smem + L::kDqOff);
     bool ok = true;
-
-    // Drains this thread's part of dQ of iteration `itp` (head hp, query tile ip): TMEM -> staging -> fp32 reduction.
-    // Its phase of dq_full has been waited for by the caller.
-    auto flush_dq = [&](int hp, int ip) {
-      tc_fence_after_sync();
-      uint32_t r[32];
-      tmem_ld_32x32(lane_addr + kDQCol + half * 32, r);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      mbar_arrive(dq_empty);
-#pragma unroll
-      for (int i = 0; i < 32; i += 4)
-        *reinterpret_cast<float4*>(dq_stage + row * kDqStride + half * 32 + i) =
-            make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
-                        __uint_as_float(r[i + 3]));
-      __syncwarp();
-      // This warp staged rows [q*32, q*32+32) x columns [half*32, half*32+32) and reduces exactly that block:
-      // 4 rows of 128 bytes per instruction.
-#pragma unroll
-      for (int rr = 0; rr < 32; rr += 4) {
-        const int r_loc = q * 32 + rr + (lane >> 3);
-        const int col = half * 32 + (lane & 7) * 4;
-        const int qi = ip * kBwdTile + r_loc;
-        if (qi < p.Sq) {
-          const float4 v = *reinterpret_cast<const float4*>(dq_stage + r_loc * kDqStride + col);
-          float* dst = p.dq_acc + ((long long)batch * p.Sq + qi) * ((long long)p.Hq * HD) + (long long)hp * HD + col;
-          red_add_v4(dst, v.x, v.y, v.z, v.w);
-        }
-      }
-      __syncwarp();
-    };
-
-    int it = 0;
-    int prev_h = 0, prev_i = 0;
+    int it = 0, units = 0;
+    Unit w;
 #ifdef DPTB_ATTN_PROFILE
     long long prof_acc[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const long long prof_begin = clock64();
 #endif
+    const f32x2 scale2 = f2_splat(p.scale), scale_log2_2 = f2_splat(p.scale_log2);
+    for (int r = 0; r < num_rounds && ok; ++r) {
+    if (!get_unit(r, w)) break;
+    const int key0 = w.key0, kv_head = w.kv_head, batch = w.batch;
     for (int g = 0; g < group && ok; ++g) {
       const int head = kv_head * group + g;
-      for (int i = i_start; i < n_q_tiles && ok; ++i, ++it) {
+      for (int i = w.i_start; i < n_q_tiles && ok; ++i, ++it) {
         const int qi = i * kBwdTile + row;
         const bool row_ok = qi < p.Sq;
         const long long stat = ((long long)batch * p.Hq + head) * p.Sq + (row_ok ? qi : 0);
@@ -357,16 +410,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         BWD_PROF_MARK(c2);
         uint32_t pk_p[32], pk_ds[32];
         const bool need_mask = kbase + 63 > key_limit;
+        const f32x2 neg_lse2 = f2_splat(-lse2), neg_delta2 = f2_splat(-delta);
 #pragma unroll
         for (int e = 0; e < 64; e += 2) {
-          float p0 = fast_exp2_b(fmaf(__uint_as_float(rs[e]), p.scale_log2, -lse2));
-          float p1 = fast_exp2_b(fmaf(__uint_as_float(rs[e + 1]), p.scale_log2, -lse2));
+          float p0, p1, d0, d1;
+          f2_unpack(f2_fma(f2_pack(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), scale_log2_2, neg_lse2), p0, p1);
+          p0 = fast_exp2_b(p0);
+          p1 = fast_exp2_b(p1);
           if (need_mask) {
             if (kbase + e > key_limit) p0 = 0.0f;
             if (kbase + e + 1 > key_limit) p1 = 0.0f;
           }
-          const float d0 = p0 * (__uint_as_float(rp[e]) - delta) * p.scale;
-          const float d1 = p1 * (__uint_as_float(rp[e + 1]) - delta) * p.scale;
+          const f32x2 dd = f2_add(f2_pack(__uint_as_float(rp[e]), __uint_as_float(rp[e + 1])), neg_delta2);
+          f2_unpack(f2_mul(f2_mul(f2_pack(p0, p1), dd), scale2), d0, d1);
           pk_p[e >> 1] = pack_bf16x2(p0, p1);
           pk_ds[e >> 1] = pack_bf16x2(d0, d1);
         }
@@ -388,33 +444,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc_fence_before_sync();
         mbar_arrive(pds_full);
         BWD_PROF_MARK(c5);
-        if (it > 0) flush_dq(prev_h, prev_i);
-        BWD_PROF_MARK(c6);
         BWD_PROF_ADD(0, c0, c1);
         BWD_PROF_ADD(1, c1, c2);
         BWD_PROF_ADD(2, c2, c3);
         BWD_PROF_ADD(3, c3, c4);
         BWD_PROF_ADD(4, c4, c5);
-        BWD_PROF_ADD(5, c5, c6);
-        prev_h = head;
-        prev_i = i;
       }
     }
-#ifdef DPTB_ATTN_PROFILE
-    if (threadIdx.x == 0) {
-      prof_acc[6] = clock64() - prof_begin;
-      prof_acc[7] = it;
-      for (int i = 0; i < 8; ++i) atomicAdd(&g_attn_bwd_prof[i], (unsigned long long)prof_acc[i]);
-    }
-#endif
-    if (ok && total_iters > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(dq_full, (total_iters - 1) & 1, abort_flag, kWaitTmemFullTimeout));
-      if (ok) flush_dq(prev_h, prev_i);
-    }
+    if (!ok) break;
+    BWD_PROF_MARK(c6);
 
     // dK / dV of this key tile.
     const int key = key0 + row;
-    if (total_iters == 0) {
+    if (w.iters == 0) {
       if (key < p.Sk) {
         __nv_bfloat16* dkp = p.dk + ((long long)batch * p.Sk + key) * p.lddk + (long long)kv_head * HD;
         __nv_bfloat16* dvp = p.dv + ((long long)batch * p.Sk + key) * p.lddv + (long long)kv_head * HD;
@@ -423,39 +465,50 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           *reinterpret_cast<uint4*>(dvp + d) = make_uint4(0, 0, 0, 0);
         }
       }
-    } else if (ok && __all_sync(0xffffffffu, mbar_wait(dkv_full, 0, abort_flag, kWaitTmemFullTimeout))) {
+    } else {
+      ok = __all_sync(0xffffffffu, mbar_wait(dkv_full, units & 1, abort_flag, kWaitTmemFullTimeout));
+      if (!ok) break;
+      ++units;
       tc_fence_after_sync();
+      uint32_t rv[32], rk[32];               // each compute warpgroup writes 32 of the 64 columns
+      tmem_ld_32x32(lane_addr + kDVCol + half * 32, rv);
+      tmem_ld_32x32(lane_addr + kDKCol + half * 32, rk);
+      tmem_ld_wait();
+      tc_fence_before_sync();
+      mbar_arrive(dkv_empty);
+      if (key < p.Sk) {
 #pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        __nv_bfloat16* base = which == 0 ? p.dv : p.dk;
-        const long long ld = which == 0 ? p.lddv : p.lddk;
-        const uint32_t col0 = which == 0 ? kDVCol : kDKCol;
-        {
-          const int c = half;   // each compute warpgroup writes 32 of the 64 columns
-          uint32_t r[32];
-          tmem_ld_32x32(lane_addr + col0 + c * 32, r);
-          tmem_ld_wait();
-          if (key < p.Sk) {
-            __nv_bfloat16* dst = base + ((long long)batch * p.Sk + key) * ld + (long long)kv_head * HD + c * 32;
+        for (int which = 0; which < 2; ++which) {
+          const uint32_t (&r)[32] = which == 0 ? rv : rk;
+          __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + ((long long)batch * p.Sk + key) * (which == 0 ? p.lddv : p.lddk) +
+                               (long long)kv_head * HD + half * 32;
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 u;
-              u.x = pack_bf16x2(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
-              u.y = pack_bf16x2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
-              u.z = pack_bf16x2(__uint_as_float(r[e + 4]), __uint_as_float(r[e + 5]));
-              u.w = pack_bf16x2(__uint_as_float(r[e + 6]), __uint_as_float(r[e + 7]));
-              *reinterpret_cast<uint4*>(dst + e) = u;
-            }
+          for (int e = 0; e < 32; e += 8) {
+            uint4 u;
+            u.x = pack_bf16x2(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+            u.y = pack_bf16x2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
+            u.z = pack_bf16x2(__uint_as_float(r[e + 4]), __uint_as_float(r[e + 5]));
+            u.w = pack_bf16x2(__uint_as_float(r[e + 6]), __uint_as_float(r[e + 7]));
+            *reinterpret_cast<uint4*>(dst + e) = u;
           }
         }
       }
-      tc_fence_before_sync();
     }
+    BWD_PROF_MARK(c7);
+    BWD_PROF_ADD(5, c6, c7);
+    }
+#ifdef DPTB_ATTN_PROFILE
+    if (threadIdx.x == 0) {
+      prof_acc[6] = clock64() - prof_begin;
+      prof_acc[7] = it;
+      for (int i = 0; i < 8; ++i) atomicAdd(&g_attn_bwd_prof[i], (unsigned long long)prof_acc[i]);
+    }
+#endif
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 13) {
     tc_fence_after_sync();
     tmem_dealloc<TMEM_COLS>(tmem_base);
   }
@@ -583,7 +636,9 @@ extern "C" int dptb_attn_bwd(const DptbAttnBwdArgs* a, void* stream) {
   p.scale = a->scale;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   DPTB_CUDA_OK(cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  dim3 grid((a->Sk + kBwdTile - 1) / kBwdTile, a->Hkv, a->B);
+  // one CTA an SM (shared memory and TMEM allow no more), or one a unit
+  const long long units = (long long)((a->Sk + kBwdTile - 1) / kBwdTile) * a->Hkv * a->B;
+  const int grid = units < sm_count() ? (int)units : sm_count();
   attn_bwd_kernel<<<grid, kBwdThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmDO, p);
   DPTB_CUDA_OK(cudaGetLastError());
   const long long rows = (long long)a->B * a->Sq;
