@@ -90,12 +90,14 @@ struct AttnFwdSmem {
   static constexpr int kQBytes = kAttnBM * HD * 2;
   static constexpr int kKVBytes = kBN * HD * 2;
   static constexpr int kPBytes = kAttnBM * 128 * 2;     // 128 keys, or 64 keys twice
+  // Two P tiles per query tile where they fit (heads of 64): the softmax of tile j + 1 then does not wait for P V of tile j.
+  static constexpr int kPBufs = HD == 64 && KST == 2 && VST == 2 ? 2 : 1;
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + NQ * kQBytes;
   static constexpr int kVOff = kKOff + KST * kKVBytes;
   static constexpr int kPOff = kVOff + VST * kKVBytes;
-  static constexpr int kBarOff = kPOff + NQ * kPBytes;
-  static constexpr int kNumBars = 2 * NQ + 2 * KST + 2 * VST + 5 * NQ;
+  static constexpr int kBarOff = kPOff + NQ * kPBufs * kPBytes;
+  static constexpr int kNumBars = 2 * NQ + 2 * KST + 2 * VST + 3 * NQ + 2 * NQ * kPBufs;
   static constexpr int kTotal = kBarOff + kNumBars * 8 + 16 + 1024;
   static_assert(kTotal <= 227 * 1024, "attention forward: shared memory budget");
 };
@@ -123,9 +125,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* v_empty = v_full + VST;
   uint64_t* s_full = v_empty + VST;                 // [NQ] S_t(j) is in TMEM
   uint64_t* s_empty = s_full + NQ;                  // [NQ] S_t(j) has been copied to registers
-  uint64_t* p_full = s_empty + NQ;                  // [NQ] P_t(j) is in shared memory (and O_t is rescaled)
-  uint64_t* o_full = p_full + NQ;                   // [NQ] O_t += P_t(j) V_j has completed
-  uint64_t* drain_bar = o_full + NQ;                // [NQ]
+  uint64_t* p_full = s_empty + NQ;                  // [NQ][P buffers] P_t(j) is in shared memory (and O_t is rescaled)
+  uint64_t* o_full = p_full + NQ * L::kPBufs;                   // [NQ][P buffers] O_t += P_t(j) V_j has completed
+  uint64_t* drain_bar = o_full + NQ * L::kPBufs;    // [NQ]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + NQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -189,8 +191,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         mbar_init(&q_empty[t], 1);
         mbar_init(&s_full[t], 1);
         mbar_init(&s_empty[t], kAttnBM);
-        mbar_init(&p_full[t], kAttnBM);
-        mbar_init(&o_full[t], 1);
+        for (int b = t * L::kPBufs; b < (t + 1) * L::kPBufs; ++b) {
+          mbar_init(&p_full[b], kAttnBM);
+          mbar_init(&o_full[b], 1);
+        }
         mbar_init(&drain_bar[t], 1);
       }
       for (int s = 0; s < KST; ++s) {
@@ -281,7 +285,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       constexpr uint32_t idesc_o = make_idesc_bf16(kAttnBM, HD, false, true);
       const int t = warp - 9;
       const uint32_t qa = smem_u32(smem + L::kQOff + t * L::kQBytes);
-      const uint32_t pa = smem_u32(smem + L::kPOff + t * L::kPBytes);
       bool issued_any = false;
       bool ok = true;
       int kv = 0;            // KV tiles before this unit, of either query tile
@@ -326,10 +329,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           ok = mbar_wait(&v_full[vs], ((kv + j) / VST) & 1, abort_flag, kWaitFullTimeout);
           if (ok && j < n) {
             // O_t += P_t(j) V_j once P_t(j) is in shared memory (and, for j = 0, the unit before has been read out of O_t)
-            ok = mbar_wait(&p_full[t], done & 1, abort_flag, kWaitFlagTimeout);
+            const int pb = t * L::kPBufs + done % L::kPBufs;
+            ok = mbar_wait(&p_full[pb], (done / L::kPBufs) & 1, abort_flag, kWaitFlagTimeout);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t vb = smem_u32(smem + L::kVOff + vs * L::kKVBytes);
+            const uint32_t pa = smem_u32(smem + L::kPOff + pb * L::kPBytes);
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk) {     // 128 keys, or the high and then the low parts of 64
               const uint32_t aoff = (kk / 4) * (kAttnBM * 128) + (kk % 4) * 32;
@@ -337,7 +342,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                         make_smem_desc(vb + (PREC ? kk % 4 : kk) * 2048, kAttnBN * 128, 1024), idesc_o,
                         (j != 0 || kk != 0) ? 1u : 0u);
             }
-            umma_commit(&o_full[t]);
+            umma_commit(&o_full[pb]);
             issued_any = true;
             ++done;
           }
@@ -362,9 +367,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const uint32_t s_addr = lane_addr + kSCol + t * 128;
     const uint32_t o_addr = lane_addr + kOCol + t * HD;
-    uint8_t* p_tile = smem + L::kPOff + t * L::kPBytes;
 
     int tiles = 0;             // tiles of this warpgroup before the present one
+    // O_t += P V of tile `n` (counted over all units) has completed.  Each P buffer has barriers of its own: as one
+    // side may be two tiles ahead of the other, a shared one could pass two phases, and so look as if it had passed none.
+    auto pv_done = [&](int n) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait(&o_full[t * L::kPBufs + n % L::kPBufs], (n / L::kPBufs) & 1, abort_flag,
+                                               kWaitTmemFullTimeout));
+    };
     bool ok = true;
     Unit w;
 #ifdef DPTB_ATTN_PROFILE
@@ -435,7 +445,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const float m_new = fmaxf(m_use, m_tile);
         const float alpha = (m_new == -INFINITY) ? 1.0f : fast_exp2(m_use - m_new);   // m_use = -inf -> 0
         if (j > 0) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+          ok = pv_done(tiles - 1);
           if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
@@ -454,11 +464,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float m_sub = (m_use == -INFINITY) ? 0.0f : m_use;
       ATTN_PROF_MARK(pt4);
-      // The previous P_t must have been consumed before it is overwritten (it nearly always has been by now).
-      if (j > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+      // The P_t that was last in this buffer must have been consumed before it is overwritten.
+      if (j >= L::kPBufs) {
+        ok = pv_done(tiles - L::kPBufs);
         if (!ok) break;
       }
+      uint8_t* p_tile = smem + L::kPOff + (t * L::kPBufs + tiles % L::kPBufs) * L::kPBytes;
       ATTN_PROF_MARK(pt5);
       // Probabilities -> bf16 -> shared memory (K-major, 128-byte swizzle), row sum.
       f32x2 l01 = 0ull, l23 = 0ull;
@@ -504,7 +515,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       l_run += (l0 + l1) + (l2 + l3);
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(&p_full[t]);
+      mbar_arrive(&p_full[t * L::kPBufs + tiles % L::kPBufs]);
       ATTN_PROF_MARK(pt6);
       ATTN_PROF_ADD(0, pt0, pt1);
       ATTN_PROF_ADD(1, pt1, pt2);
@@ -514,7 +525,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ATTN_PROF_ADD(5, pt5, pt6);
     }
     if (ok && n > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], (tiles - 1) & 1, abort_flag, kWaitTmemFullTimeout));
+      ok = pv_done(tiles - 1);
       if (ok) {
         tc_fence_after_sync();
         const bool live = q_row < p.Sq;
