@@ -9,13 +9,13 @@
 // its group and over the query tiles that can see those keys.  Per query tile, five tensor-core products:
 //   S  = Q K^T          dP = dO V^T                       (into TMEM, rows = queries)
 //   dV += P^T dO        dK += dS^T Q                      (accumulate in TMEM across the whole loop, rows = keys)
-//   dQ  = dS K                                            (TMEM -> shared staging -> fp32 reduction into dq_acc)
+//   dQ  = dS K                                            (TMEM -> shared memory -> fp32 reduction into dq_acc)
 // with P = exp2(S*c - lse) and dS = scale * P * (dP - delta) computed in between and written to shared memory in a
 // layout that serves both as a K-major operand (dS K) and, transposed, as an MN-major operand (P^T dO, dS^T Q).
 //   warps 0-7  two compute warpgroups: thread = one query row x one half (64 keys) of the S / dP tiles.  A thread pulls
 //              its 64 scores and 64 dP values from TMEM in one go and hands the columns straight back, so the tensor core
 //              computes S / dP of the next query tile while P / dS of this one are formed
-//   warps 8-11 drain dQ of the tile before (TMEM -> shared staging -> fp32 reduction into dq_acc)
+//   warps 8-11 drain dQ of the tile before (TMEM -> shared staging -> TMA reduction into dq_acc)
 //   warp 12    TMA producer      warp 13    MMA issuer      (warps 14-15 only take part in the register hand-over)
 #include <cuda_bf16.h>
 
@@ -27,7 +27,6 @@ namespace dptb {
 struct AttnBwdParams {
   const float* lse;      // [B, Hq, Sq] natural log
   const float* delta;    // [B, Hq, Sq] rowsum(dO * O)
-  float* dq_acc;         // [B*Sq, Hq*64] fp32, zero-initialised
   __nv_bfloat16* dk;     // [B*Sk, lddk]
   __nv_bfloat16* dv;
   long long lddk, lddv;
@@ -41,10 +40,6 @@ __device__ __forceinline__ float fast_exp2_b(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // Opt-in phase timers (compile with -DDPTB_ATTN_PROFILE), SM clock cycles summed over all CTAs:
 //   compute thread 0:  [0] wait S/dP  [1] TMEM -> registers  [2] P / dS math  [3] wait for the previous products
 //                      [4] stores + signal  [5] dK / dV out  [6] loop total  [7] iterations
@@ -67,8 +62,9 @@ constexpr int kBwdDrainRegs = 96;
 constexpr int kBwdProducerRegs = 72;
 static_assert(2 * 128 * kBwdComputeRegs + 128 * kBwdDrainRegs + 128 * kBwdProducerRegs <= kBwdThreads * 128,
               "register hand-over must balance");
-constexpr int kBwdStages = 2;
-constexpr int kDqStride = 68;  // floats per staged dQ row (padding keeps 16-byte accesses conflict-free)
+// Three query tiles of Q and dO: a stage is free when the last products of its tile are done, which is when the tile after next
+// should start; with two its load (1500 clocks) stood in the chain.
+constexpr int kBwdStages = 3;
 
 struct AttnBwdSmem {
   static constexpr int kTileBytes = kBwdTile * kBwdHD * 2;       // 16 KB: one [128 x 64] bf16 tile
@@ -80,16 +76,16 @@ struct AttnBwdSmem {
   static constexpr int kPOff = kDOOff + kBwdStages * kTileBytes;
   static constexpr int kDSOff = kPOff + kPBytes;
   static constexpr int kDqOff = kDSOff + kPBytes;
-  static constexpr int kDqBytes = kBwdTile * kDqStride * 4;
-  static constexpr int kBarOff = kDqOff + kDqBytes;
+  static constexpr int kBarOff = kDqOff + kBwdTile * kBwdHD * 4;
   static constexpr int kNumBars = 2 + 2 * kBwdStages + 8;
   static constexpr int kTotal = kBarOff + kNumBars * 8 + 16 + 1024;
+  static_assert(kTotal <= 227 * 1024, "attention backward: shared memory budget");
 };
 
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
   using L = AttnBwdSmem;
   constexpr int HD = kBwdHD;
   constexpr int TMEM_COLS = 512;
@@ -146,6 +142,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
+    tma_prefetch_desc(&tmDQ);
   }
   if (warp == 13) {
     if (lane == 0) {
@@ -316,11 +313,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   }
   } else if (warp >= 8) {
-    // ------------------------------------------------------------------ dQ: TMEM -> staging -> fp32 reduction
+    // ------------------------------------------------------------------ dQ: TMEM -> shared memory -> fp32 reduction
+    // Two boxes of 32 rows x 32 columns a warp, rewritten once the copy engine has read them.  (Reductions straight from the registers,
+    // 32 bytes of 16 rows an instruction: 1050 us instead of 950 at 2 x 12 heads x 8192 causal.)
     warpgroup_reg_dec<kBwdDrainRegs>();
     const int q = warp & 3;              // TMEM lane quarter: rows [32 q, 32 q + 32) of the query tile
     const uint32_t dq_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kDQCol;
-    float* stage = reinterpret_cast<float*>(smem + L::kDqOff) + q * 32 * kDqStride;
+    uint8_t* stage = smem + L::kDqOff + q * 8192;
     int it = 0;
     Unit w;
     bool ok = true;
@@ -333,35 +332,36 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           ok = __all_sync(0xffffffffu, mbar_wait(dq_full, it & 1, abort_flag, kWaitTmemFullTimeout));
           if (!ok) break;
           tc_fence_after_sync();
-          uint32_t r0[32], r1[32];
-          tmem_ld_32x32(dq_addr, r0);
-          tmem_ld_32x32(dq_addr + 32, r1);
-          tmem_ld_wait();
-          tc_fence_before_sync();
-          mbar_arrive(dq_empty);
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            *reinterpret_cast<float4*>(stage + lane * kDqStride + e) =
-                make_float4(__uint_as_float(r0[e]), __uint_as_float(r0[e + 1]), __uint_as_float(r0[e + 2]), __uint_as_float(r0[e + 3]));
-            *reinterpret_cast<float4*>(stage + lane * kDqStride + 32 + e) =
-                make_float4(__uint_as_float(r1[e]), __uint_as_float(r1[e + 1]), __uint_as_float(r1[e + 2]), __uint_as_float(r1[e + 3]));
-          }
+          if (lane == 0) bulk_wait_read_all();
           __syncwarp();
-          // 2 rows of 256 bytes per instruction
-          const int col = (lane & 15) * 4;
-          float* dst = p.dq_acc + ((long long)w.batch * p.Sq + i * kBwdTile + q * 32) * ((long long)p.Hq * HD) + (long long)head * HD + col;
 #pragma unroll
-          for (int rr = 0; rr < 32; rr += 2) {
-            const int r_loc = rr + (lane >> 4);
-            if (i * kBwdTile + q * 32 + r_loc < p.Sq) {
-              const float4 v = *reinterpret_cast<const float4*>(stage + r_loc * kDqStride + col);
-              red_add_v4(dst + (long long)r_loc * p.Hq * HD, v.x, v.y, v.z, v.w);
+          for (int c = 0; c < 2; ++c) {
+            uint32_t v[32];
+            tmem_ld_32x32(dq_addr + c * 32, v);
+            tmem_ld_wait();
+            if (c == 1) {
+              tc_fence_before_sync();
+              mbar_arrive(dq_empty);
+            }
+            uint8_t* row = stage + c * 4096 + lane * 128;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              *reinterpret_cast<uint4*>(row + ((e ^ (lane & 7)) << 4)) = make_uint4(v[e * 4], v[e * 4 + 1], v[e * 4 + 2], v[e * 4 + 3]);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const int y = i * kBwdTile + q * 32;
+            if (y < p.Sq) {                  // (rows from Sq on are dropped)
+              tma_reduce_add_3d(&tmDQ, stage, head * HD, y, w.batch);
+              tma_reduce_add_3d(&tmDQ, stage + 4096, head * HD + 32, y, w.batch);
+              bulk_commit_group();
             }
           }
-          __syncwarp();
         }
       }
     }
+    if (lane == 0) bulk_wait_all();
   } else {
     // ------------------------------------------------------------------ compute warpgroups
     warpgroup_reg_inc<kBwdComputeRegs>();
@@ -628,7 +628,15 @@ extern "C" int dptb_attn_bwd(const DptbAttnBwdArgs* a, void* stream) {
   rc = encode_tmap_seq_b(&tmDO, a->dout, a->Hq, kBwdHD, a->Sq, a->B, a->lddo);
   if (rc) return rc;
   AttnBwdParams p;
-  p.lse = a->lse; p.delta = a->delta; p.dq_acc = a->dq_acc;
+  CUtensorMap tmDQ;
+  {
+    const uint64_t dims[3] = {(uint64_t)a->Hq * kBwdHD, (uint64_t)a->Sq, (uint64_t)a->B};
+    const uint64_t strides[2] = {dims[0] * 4, dims[0] * dims[1] * 4};
+    const uint32_t box[3] = {32, 32, 1};
+    rc = encode_tmap_nd(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a->dq_acc, 3, dims, strides, box);
+    if (rc) return rc;
+  }
+  p.lse = a->lse; p.delta = a->delta;
   p.dk = static_cast<__nv_bfloat16*>(a->dk); p.dv = static_cast<__nv_bfloat16*>(a->dv);
   p.lddk = a->lddk; p.lddv = a->lddv;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv;
@@ -639,7 +647,7 @@ extern "C" int dptb_attn_bwd(const DptbAttnBwdArgs* a, void* stream) {
   // one CTA an SM (shared memory and TMEM allow no more), or one a unit
   const long long units = (long long)((a->Sk + kBwdTile - 1) / kBwdTile) * a->Hkv * a->B;
   const int grid = units < sm_count() ? (int)units : sm_count();
-  attn_bwd_kernel<<<grid, kBwdThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmDO, p);
+  attn_bwd_kernel<<<grid, kBwdThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmDO, tmDQ, p);
   DPTB_CUDA_OK(cudaGetLastError());
   const long long rows = (long long)a->B * a->Sq;
   const int cols = a->Hq * kBwdHD;

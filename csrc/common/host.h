@@ -62,10 +62,10 @@ inline int encode_tmap_2d_bf16(CUtensorMap* map, const void* base, uint64_t inne
   return r == CUDA_SUCCESS ? 0 : kErrTensorMap;
 }
 
-// Rank-N (N <= 5) bf16 tensor map with 128-byte swizzle: dims[0] is contiguous; strides[i] (bytes) is the stride of
+// Rank-N (N <= 5) tensor map with 128-byte swizzle: dims[0] is contiguous; strides[i] (bytes) is the stride of
 // dims[i+1].  The rank must equal the dimensionality of the copy instruction that uses the map.
-inline int encode_tmap_nd_bf16(CUtensorMap* map, const void* base, int rank, const uint64_t* dims_in,
-                               const uint64_t* strides_bytes, const uint32_t* box_in) {
+inline int encode_tmap_nd(CUtensorMap* map, CUtensorMapDataType type, const void* base, int rank, const uint64_t* dims_in,
+                          const uint64_t* strides_bytes, const uint32_t* box_in) {
   EncodeTiledFn fn = get_encode_tiled();
   if (!fn) return kErrNoDriver;
   if (rank < 1 || rank > 5 || (reinterpret_cast<uintptr_t>(base) & 15)) return kErrBadShape;
@@ -81,10 +81,15 @@ inline int encode_tmap_nd_bf16(CUtensorMap* map, const void* base, int rank, con
     if (strides_bytes[i] & 15) return kErrBadShape;
     strides[i] = strides_bytes[i];
   }
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = fn(map, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : kErrTensorMap;
+}
+
+inline int encode_tmap_nd_bf16(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                               const uint32_t* box) {
+  return encode_tmap_nd(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, dims, strides_bytes, box);
 }
 
 // Number of kernels this library has launched since the last reset (host-side bookkeeping for benchmarks).
