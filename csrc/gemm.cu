@@ -72,6 +72,8 @@ using namespace dptb;
 
 int gemm_f32(const DptbGemmArgs* a, void* stream);   // gemm_f32.cu
 
+constexpr long long kHotOperandBytes = 24ll << 20, kBandBytes = 12ll << 20;   // shares of the 126 MB L2, which two dies halve
+
 // Peer-memory description of the all-gather prologue (see TpAg): every rank's shard of A, [rows_per_rank, lda] each.
 struct DptbTpAgArgs {
   int world, rank;
@@ -131,8 +133,9 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
       (a->epi_f32 || !(a->residual || a->aux_out || a->aux_in || a->act)))
     return gemm_f32(a, stream_v);
   if (!tc_ok) {
-    p.tiles_m = p.tiles_n = p.num_kb = 0;
-    p.splits = 1; p.kb_per_split = 0; p.ws = nullptr; p.counters = nullptr;
+    p.tiles_m = p.tiles_n = p.num_kb = p.band = p.last_band = 0;
+    p.by_tiles = p.by_band = p.by_rows = p.by_last_rows = make_fast_div(1);
+    p.splits = 1; p.kb_per_split = p.fold_all = 0; p.ws = nullptr; p.counters = nullptr;
     dim3 grid((unsigned)((a->N + 63) / 64), (unsigned)((a->M + 63) / 64));
     const long long sam = a->trans_a ? 1 : a->lda, sak = a->trans_a ? a->lda : 1;
     const long long sbk = a->trans_b ? 1 : a->ldb, sbn = a->trans_b ? a->ldb : 1;
@@ -159,11 +162,11 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
     const char* e = getenv("DPTB_GEMM_PAIR");
     return !(e && e[0] == '0');
   }();
-  // A pair's epilogue leaves through tile stores: bf16 output, every per-element buffer describable by a tensor map
-  // (16-byte aligned, strides multiples of 16 bytes), at most one per-element input, and a pre-activation copy not
+  // A pair's epilogue leaves through tile stores (but for the last columns of a width that is no multiple of 8): bf16 output,
+  // every per-element buffer describable by a tensor map (16-byte aligned, strides multiples of 16 bytes), at most one per-element input, and a pre-activation copy not
   // combined with an input (a warp's two staging blocks cover either case).
   const int epi_inputs = (p.act >= 11 ? 1 : 0) + (p.residual ? 1 : 0) + (p.accumulate ? 1 : 0);
-  const bool tile_store_ok = !p.out_f32 && p.vec_ok && !(p.bias && p.bias_f32) && (a->N % 8) == 0 && epi_inputs <= 1 &&
+  const bool tile_store_ok = !p.out_f32 && p.vec_ok && !(p.bias && p.bias_f32) && epi_inputs <= 1 &&
                              !(epi_inputs == 1 && p.aux_out);
   const bool pair = pairs_enabled && !ar && !ag && tm >= 2 && tile_store_ok;
   // Work units run on `sms` CTAs, or on sms / 2 pairs, each pair taking two row tiles at a time.
@@ -171,6 +174,7 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
   const int tm_sched = pair ? (tm + 1) / 2 : tm;
   int bn = a->bn, splits = a->splits;
   {
+    const bool by_rows = a->trans_a && !a->trans_b;
     double best = 1e30;
     int best_bn = 128, best_sp = 1;
     for (int cand_bn = 128; cand_bn <= 256; cand_bn += 128) {
@@ -178,22 +182,24 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
       if (cand_bn == 256 && a->N <= 128) continue;
       const int tiles = tm * ((a->N + cand_bn - 1) / cand_bn);
       const int sched_tiles = tm_sched * ((a->N + cand_bn - 1) / cand_bn);
-      for (int sp = 1; sp <= 8; ++sp) {
+      for (int sp = 1; sp <= kMaxSplits; ++sp) {
         if (a->splits >= 1 && sp != a->splits) continue;
         if ((ar || ag) && sp > 1) break;
+        const long long units = (long long)sched_tiles * sp;
         if (sp > 1) {
           if (!a->ws || !a->counters || tiles > a->num_counters) break;
           if ((long long)tiles * sp * cand_bn * kBM * 4 > a->ws_bytes) break;
           if (num_kb / sp < 4) break;
         }
         const int kbs = (num_kb + sp - 1) / sp;
-        const long long units = (long long)sched_tiles * sp;
         const double waves = (double)((units + sms - 1) / sms);
-        const double per_kb = cand_bn == 256 ? 1.0 : 0.75;
-        // (the fold of a 256-wide tile is serial in its last CTA: measured on 768 x 768 x 16384, 8 splits of 256-wide tiles
-        // took 48 us against 42 us for 4 splits of 128-wide ones)
+        // Sums over the rows of both operands (weight gradients): a k-block of a 128-wide tile takes as long as one of 256 (768 x 768 x
+        // 16384 without splits 83.6 and 83.4 us), and rounds of split units wait for their folds (5632 x 1024 x 6124, 88 tiles of 256:
+        // 70 us whole, 106 us in three rounds of halves).  768 x 768 x 16384, bn x splits: 256x8 26 us, 128x4 33, 256x4 36; 1024 x
+        // 1024 x 6124: 256x4 24, 128x2 30.
+        const double per_kb = cand_bn == 256 || by_rows ? 1.0 : 0.75;
         const double fixed = (cand_bn == 256 ? 8.0 : 5.0) + (sp > 1 ? (cand_bn == 256 ? 8.0 + 2.5 * sp : 4.0 + 1.0 * sp) : 0.0);
-        const double cost = waves * (kbs * per_kb + fixed);
+        const double cost = waves * (kbs * per_kb + fixed) + (by_rows && sp > 1 ? waves - 1.0 : 0.0);
         if (cost < best) { best = cost; best_bn = cand_bn; best_sp = sp; }
       }
     }
@@ -203,7 +209,23 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
   p.tiles_m = tm;
   p.tiles_n = (a->N + bn - 1) / bn;
   p.num_kb = num_kb;
+  // Order of the tiles: what is read again must still be in L2.  A small B stays there by itself, and one row tile after the other
+  // reads A once; else a band of row tiles whose A takes up to 12 MB stays while B passes, once a band.  Columns outermost for
+  // all: 16384 x 768 x 3072 66 us (61 so), 25216 x 768 x 3072 112 us (95), 16384 x 768 x 50264 1029 us (980).
+  // The order of the tensor-parallel forms is their own.
+  const long long row_bytes = (long long)(pair ? 2 : 1) * kBM * a->K * 2;
+  p.band = tm_sched;
+  if (!ar && !ag) {
+    const long long fit = (long long)a->N * a->K * 2 <= kHotOperandBytes ? 1 : kBandBytes / row_bytes;
+    p.band = fit < 1 ? 1 : fit < tm_sched ? (int)fit : tm_sched;
+  }
+  p.last_band = (tm_sched - 1) / p.band;
+  p.by_tiles = make_fast_div(tm_sched * p.tiles_n);
+  p.by_band = make_fast_div(p.band * p.tiles_n);
+  p.by_rows = make_fast_div(p.band);
+  p.by_last_rows = make_fast_div(tm_sched - p.last_band * p.band);
   p.splits = splits;
+  p.fold_all = 0;
   p.kb_per_split = (num_kb + splits - 1) / splits;
   if ((long long)(splits - 1) * p.kb_per_split >= num_kb) {  // keep every split non-empty
     splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;
