@@ -72,8 +72,6 @@ using namespace dptb;
 
 int gemm_f32(const DptbGemmArgs* a, void* stream);   // gemm_f32.cu
 
-constexpr long long kHotOperandBytes = 24ll << 20, kBandBytes = 12ll << 20;   // shares of the 126 MB L2, which two dies halve
-
 // Peer-memory description of the all-gather prologue (see TpAg): every rank's shard of A, [rows_per_rank, lda] each.
 struct DptbTpAgArgs {
   int world, rank;
@@ -209,21 +207,8 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
   p.tiles_m = tm;
   p.tiles_n = (a->N + bn - 1) / bn;
   p.num_kb = num_kb;
-  // Order of the tiles: what is read again must still be in L2.  A small B stays there by itself, and one row tile after the other
-  // reads A once; else a band of row tiles whose A takes up to 12 MB stays while B passes, once a band.  Columns outermost for
-  // all: 16384 x 768 x 3072 66 us (61 so), 25216 x 768 x 3072 112 us (95), 16384 x 768 x 50264 1029 us (980).
-  // The order of the tensor-parallel forms is their own.
-  const long long row_bytes = (long long)(pair ? 2 : 1) * kBM * a->K * 2;
-  p.band = tm_sched;
-  if (!ar && !ag) {
-    const long long fit = (long long)a->N * a->K * 2 <= kHotOperandBytes ? 1 : kBandBytes / row_bytes;
-    p.band = fit < 1 ? 1 : fit < tm_sched ? (int)fit : tm_sched;
-  }
-  p.last_band = (tm_sched - 1) / p.band;
-  p.by_tiles = make_fast_div(tm_sched * p.tiles_n);
-  p.by_band = make_fast_div(p.band * p.tiles_n);
-  p.by_rows = make_fast_div(p.band);
-  p.by_last_rows = make_fast_div(tm_sched - p.last_band * p.band);
+  // (the order of the tensor-parallel forms is their own)
+  order_tiles(p, tm_sched, (long long)(pair ? 2 : 1) * kBM * a->K * 2, (long long)a->N * a->K * 2, !ar && !ag);
   p.splits = splits;
   p.fold_all = 0;
   p.kb_per_split = (num_kb + splits - 1) / splits;

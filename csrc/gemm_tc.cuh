@@ -882,7 +882,9 @@ template <> struct PeerMaps<true> { using type = TmapSet; };
 // rows [128 r, 128 r + 128) of the A tile and columns [BN/2 r, BN/2 r + BN/2) of the B tile, the leader's (r = 0)
 // issuer thread runs the MMAs of both tensor cores, each CTA's epilogue warps drain their own 128 x BN accumulator.
 // Work units are then pairs of row tiles; `tile` below stays the index of this CTA's own 128-row tile.
-template <bool A_MN, bool B_MN, int BN, int STAGES, bool AG = false, bool PAIR = false>
+// GLU (pairs, x W^T): W holds F rows of gates and then F rows of values.  A tile's columns are 128 gates, staged by the first CTA, and
+// the 128 values that go with them, staged by the second; both CTAs' accumulators have both, and what leaves is silu(gate) * value.
+template <bool A_MN, bool B_MN, int BN, int STAGES, bool AG = false, bool PAIR = false, bool GLU = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ typename PeerMaps<AG>::type peers, const __grid_constant__ EpiMaps em,
@@ -967,7 +969,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         tile_of_unit(p, stile, smi, ni);
         const int mi = PAIR ? smi * 2 + (int)cta_rank : (p.ar.world > 0 || p.ag.world > 0) ? tile_row_index(p, stile) : smi;
         const int m0 = mi * kBM;
-        const int n0 = ni * BN + (PAIR ? (int)cta_rank * BROWS : 0);
+        const int n0 = GLU ? ni * BROWS + (int)cta_rank * p.N : ni * BN + (PAIR ? (int)cta_rank * BROWS : 0);
         const CUtensorMap* a_map = &tmA;
         int a_row = m0;
         if constexpr (AG) {
@@ -1261,6 +1263,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       }
       const long long row0 = (long long)m0 + q * 32;
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
+      if constexpr (GLU) {
+        const long long col0 = (long long)ni * BROWS + half * 64;
+        if (row0 < p.M && col0 < p.N) {    // warp-uniform
+          uint8_t* buf = stage + (epi_blk & 1) * 4096;
+          if (lane == 0) bulk_wait_read_1();
+          __syncwarp();
+#pragma unroll 1
+          for (int col = 0; col < 64; col += 32) {
+            uint32_t g[32], u[32];
+            tmem_ld_32x32(t_row + half * 64 + col, g);
+            tmem_ld_32x32(t_row + BROWS + half * 64 + col, u);
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              float v[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                // both rounded to bf16 first, as where the product is stored and gated by a kernel of its own
+                const float z = __bfloat162float(__float2bfloat16(__uint_as_float(g[k * 8 + e])));
+                v[e] = z / (1.0f + __expf(-z)) * __bfloat162float(__float2bfloat16(__uint_as_float(u[k * 8 + e])));
+              }
+              *reinterpret_cast<uint4*>(buf + lane * 128 + (((col / 8 + k) ^ (lane & 7)) << 4)) = pack8(v);
+            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&em.c, buf, (int)col0, (int)row0);
+            bulk_commit_group();
+          }
+          ++epi_blk;
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) release_acc(acc);
+        continue;
+      }
       if (!PAIR && p.ar.world > 0) {
         // Partial tile -> this rank's partial buffer (each thread writes its row's 128 bytes of a 64-column block as
         // whole sectors); flag the owner.  The CTA-wide barrier orders every warp's stores before the one
@@ -1542,11 +1581,11 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams 
 // CTA-pair variant: clusters of two CTAs, one 256-row tile per pair (see the kernel's PAIR parameter).
 constexpr int kPairStages256 = 5;   // 32 KB per stage and CTA, 64 KB of epilogue staging
 constexpr int kPairStages128 = 6;   // 24 KB per stage and CTA
-template <bool A_MN, bool B_MN, int BN, int STAGES>
+template <bool A_MN, bool B_MN, int BN, int STAGES, bool GLU>
 static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
   // Clusters of this kernel that can be resident at once (a persistent grid must not exceed it), once per device.
   using L = GemmSmem<BN, STAGES, BN / 2, 2>;
-  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true>;
+  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true, GLU>;
   static SmemLimit limit;
   static std::atomic<int> counts[64];      // one more than the number; 0: not asked for yet
   int dev = 0;
@@ -1567,11 +1606,11 @@ static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
   (void)attr;
   return cached;
 }
-template <bool A_MN, bool B_MN, int BN, int STAGES>
+template <bool A_MN, bool B_MN, int BN, int STAGES, bool GLU = false>
 static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& em, GemmParams p,
                           cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES, BN / 2, 2>;
-  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true>;
+  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true, GLU>;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
@@ -1583,7 +1622,7 @@ static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int max_clusters = pair_clusters<A_MN, B_MN, BN, STAGES>(&cfg, attr);
+  const int max_clusters = pair_clusters<A_MN, B_MN, BN, STAGES, GLU>(&cfg, attr);
   if (max_clusters <= 0) return kErrUnsupported;
   const int units = ((p.tiles_m + 1) / 2) * p.tiles_n * p.splits;
   const int clusters = units < max_clusters ? units : max_clusters;
@@ -1603,6 +1642,20 @@ static int launch_tc_ag(const TmapSet& peers, const CUtensorMap& tmB, const Gemm
   const int grid = tiles < sm_count() ? tiles : sm_count();
   kern<<<grid, kGemmThreads, L::kTotal, stream>>>(peers.m[p.ag.rank], tmB, peers, EpiMaps{}, p);
   return counted(1, (int)cudaGetLastError());
+}
+
+// Order of the tiles: what is read again must still be in L2.  A small B stays there by itself, and one row tile after the other reads A
+// once; else a band of row tiles whose A takes up to 12 MB stays while B passes, once a band.  Columns outermost for all:
+// 16384 x 768 x 3072 66 us (59 so), 25216 x 768 x 3072 112 us (93), 16384 x 768 x 50264 1029 us (980).
+constexpr long long kHotOperandBytes = 24ll << 20, kBandBytes = 12ll << 20;   // shares of the 126 MB L2, which two dies halve
+inline void order_tiles(GemmParams& p, int sched_tiles_m, long long row_tile_bytes, long long b_bytes, bool bands) {
+  const long long fit = b_bytes <= kHotOperandBytes ? 1 : kBandBytes / row_tile_bytes;
+  p.band = !bands ? sched_tiles_m : fit < 1 ? 1 : fit < sched_tiles_m ? (int)fit : sched_tiles_m;
+  p.last_band = (sched_tiles_m - 1) / p.band;
+  p.by_tiles = make_fast_div(sched_tiles_m * p.tiles_n);
+  p.by_band = make_fast_div(p.band * p.tiles_n);
+  p.by_rows = make_fast_div(p.band);
+  p.by_last_rows = make_fast_div(sched_tiles_m - p.last_band * p.band);
 }
 
 // One layout's entry point: CTA pairs or single CTAs, 128- or 256-wide tiles.

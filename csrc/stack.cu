@@ -17,6 +17,7 @@ using namespace dptb;
 extern "C" {
 int dptb_gemm(const DptbGemmArgs*, void*);
 int dptb_gemm_skinny(const DptbGemmArgs*, const DptbTpArArgs*, void*);
+int dptb_gemm_swiglu(const DptbGemmArgs*, void*);
 int dptb_attn_fwd(const DptbAttnFwdArgs*, void*);
 int dptb_attn_f32(const DptbAttnF32Args*, void*);
 int dptb_attn_decode(const DptbDecodeArgs*, void*);
@@ -127,6 +128,21 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
     }
     return dptb_gemm(&g, stream);
   };
+  // The two products of a gated unit and the gate: one kernel where it exists, else the product of both and a pass over it.
+  auto gated = [&](const void* x, const void* w, const void* bias, char* up, void* y) {
+    if (a->bf16 && !bias && M > a->skinny_rows) {
+      DptbGemmArgs g;
+      memset(&g, 0, sizeof(g));
+      g.A = x; g.B = w; g.C = y;
+      g.lda = g.ldb = D; g.ldc = a->F;
+      g.M = M; g.N = a->F; g.K = D;
+      g.trans_b = 1; g.alpha = 1.0f;
+      const int rc = dptb_gemm_swiglu(&g, stream);
+      if (rc != kErrUnsupported) return rc;
+    }
+    const int rc = linear(x, D, w, bias, 2 * a->F, up, 0, nullptr);
+    return rc ? rc : dptb_swiglu_fwd(up, 2LL * a->F, up + a->F * esz, 2LL * a->F, y, a->F, rows, a->F, a->bf16, stream);
+  };
   auto attend = [&](char* qkv, const void* kc, const void* vc, void* o) {
     const int Sk = a->cached ? a->past + a->S : a->S;
     const char* k = a->cached ? static_cast<const char*>(kc) : qkv + dq * esz;
@@ -214,9 +230,7 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
     }
     const void* f = ws + l.up;
     if (a->gated) {
-      DPTB_STACK_OK(linear(y, D, t[kUpW], t[kUpB], 2 * a->F, ws + l.up, 0, nullptr));
-      DPTB_STACK_OK(dptb_swiglu_fwd(ws + l.up, 2LL * a->F, ws + l.up + a->F * esz, 2LL * a->F, ws + l.act, a->F, rows, a->F,
-                                    a->bf16, stream));
+      DPTB_STACK_OK(gated(y, t[kUpW], t[kUpB], ws + l.up, ws + l.act));
       f = ws + l.act;
     } else {
       DPTB_STACK_OK(linear(y, D, t[kUpW], t[kUpB], a->F, ws + l.up, a->act, nullptr));
