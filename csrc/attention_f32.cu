@@ -38,6 +38,10 @@ struct AttnF32Params {
   int causal, q_offset;   // causal: key j is visible to query i when j <= i + q_offset
   float scale;
   int vec;                // every row starts on a 16-byte boundary and hd is a multiple of 4
+  // Decoding only: the keys and values of the rows from `appended` on (Sk: none) are read from kn / vn (row 0 there) and written to
+  // k / v, the caches.
+  F32View kn, vn;
+  int appended;
 };
 
 constexpr int kFBM = 32, kFBN = 64, kFThreads = 128;
@@ -300,9 +304,23 @@ attn_f32_decode(const AttnF32Params p) {
   for (int t = rank; t < tiles; t += nc) {
     const int key0 = t * kFBN;
     __syncthreads();
-    f32_load_tile<HD, kFBN>(Ks, p.k, b, hk, key0, p.Sk, p.hd, p.vec);
-    f32_load_tile<HD, kFBN>(Vs, p.v, b, hk, key0, p.Sk, p.hd, p.vec);
+    f32_load_tile<HD, kFBN>(Ks, p.k, b, hk, key0, p.appended, p.hd, p.vec);
+    f32_load_tile<HD, kFBN>(Vs, p.v, b, hk, key0, p.appended, p.hd, p.vec);
     __syncthreads();
+    if (key0 + kFBN > p.appended && p.appended < p.Sk) {
+      // A tile is one CTA's alone, so that one appends its rows.
+      const int first = max(key0, p.appended), count = min(p.Sk, key0 + kFBN) - first;
+      for (int i = tid; i < count * p.hd; i += kFThreads) {
+        const int key = first + i / p.hd, d = i % p.hd;
+        const float x = p.kn.p[b * p.kn.sb + (key - p.appended) * p.kn.ss + hk * p.kn.sh + d];
+        const float y = p.vn.p[b * p.vn.sb + (key - p.appended) * p.vn.ss + hk * p.vn.sh + d];
+        Ks[(key - key0) * LD + d] = x;
+        Vs[(key - key0) * LD + d] = y;
+        p.k.p[b * p.k.sb + key * p.k.ss + hk * p.k.sh + d] = x;
+        p.v.p[b * p.v.sb + key * p.v.ss + hk * p.v.sh + d] = y;
+      }
+      __syncthreads();
+    }
     // scores: two threads per key, alternate 16-byte pieces
     const int key = tid >> 1;
     float s[R];
@@ -628,7 +646,7 @@ static int attn_f32_launch(const AttnF32Params& p, int backward, cudaStream_t st
 
 using namespace dptb;
 
-extern "C" int dptb_attn_f32(const DptbAttnF32Args* a, void* stream) {
+static int attn_f32(const DptbAttnF32Args* a, const DptbF32View* kn, const DptbF32View* vn, void* stream) {
   if (a->B <= 0 || a->Sq <= 0 || a->Hq <= 0) return 0;
   if (a->hd <= 0 || a->hd > 128) return kErrUnsupported;
   if (a->Sk <= 0 || a->Hkv <= 0 || a->Hq % a->Hkv || a->q_offset < 0) return kErrBadShape;
@@ -644,6 +662,9 @@ extern "C" int dptb_attn_f32(const DptbAttnF32Args* a, void* stream) {
     if (!in[i]->p) return kErrBadShape;
     if ((reinterpret_cast<uintptr_t>(in[i]->p) & 15) || (in[i]->sb | in[i]->ss | in[i]->sh) % 4) p.vec = 0;
   }
+  p.kn = kn ? F32View{kn->p, kn->sb, kn->ss, kn->sh} : F32View{};
+  p.vn = vn ? F32View{vn->p, vn->sb, vn->ss, vn->sh} : F32View{};
+  p.appended = kn ? a->Sk - a->Sq : a->Sk;
   p.lse = a->lse;
   p.delta = a->delta;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv; p.hd = a->hd;
@@ -655,4 +676,14 @@ extern "C" int dptb_attn_f32(const DptbAttnF32Args* a, void* stream) {
   if (a->hd <= 32) return attn_f32_launch<32>(p, a->backward, st);
   if (a->hd <= 64) return attn_f32_launch<64>(p, a->backward, st);
   return attn_f32_launch<128>(p, a->backward, st);
+}
+extern "C" int dptb_attn_f32(const DptbAttnF32Args* a, void* stream) { return attn_f32(a, nullptr, nullptr, stream); }
+
+// Decoding with the cache append in the same kernel: k and v are caches, the last Sq of their Sk rows come from kn and vn.  A step of few
+// rows is a chain of short kernels: GPT-2 124M, one token over 509, spent 3.5 us a layer in the copy alone.  kErrUnsupported where the
+// rows are too many for the decode kernel: the caller appends, then attends.
+extern "C" int dptb_attn_f32_append(const DptbAttnF32Args* a, const DptbF32View* kn, const DptbF32View* vn, void* stream) {
+  if (a->backward || a->Hkv <= 0 || a->Hq % a->Hkv || a->Hq / a->Hkv * a->Sq > kFDecRows || a->Sk < a->Sq || !kn->p || !vn->p)
+    return kErrUnsupported;
+  return attn_f32(a, kn, vn, stream);
 }

@@ -18,6 +18,7 @@ extern "C" {
 int dptb_gemm(const DptbGemmArgs*, void*);
 int dptb_gemm_skinny(const DptbGemmArgs*, const DptbTpArArgs*, void*);
 int dptb_gemm_swiglu(const DptbGemmArgs*, void*);
+int dptb_attn_f32_append(const DptbAttnF32Args*, const DptbF32View*, const DptbF32View*, void*);
 int dptb_attn_fwd(const DptbAttnFwdArgs*, void*);
 int dptb_attn_f32(const DptbAttnF32Args*, void*);
 int dptb_attn_decode(const DptbDecodeArgs*, void*);
@@ -143,7 +144,7 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
     const int rc = linear(x, D, w, bias, 2 * a->F, up, 0, nullptr);
     return rc ? rc : dptb_swiglu_fwd(up, 2LL * a->F, up + a->F * esz, 2LL * a->F, y, a->F, rows, a->F, a->bf16, stream);
   };
-  auto attend = [&](char* qkv, const void* kc, const void* vc, void* o) {
+  auto attend = [&](char* qkv, const void* kc, const void* vc, void* o, bool append) {
     const int Sk = a->cached ? a->past + a->S : a->S;
     const char* k = a->cached ? static_cast<const char*>(kc) : qkv + dq * esz;
     const char* v = a->cached ? static_cast<const char*>(vc) : qkv + (dq + dkv) * esz;
@@ -158,7 +159,10 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
       f.o = {static_cast<float*>(o), (long long)a->S * dq, dq, hd};
       f.B = a->B; f.Sq = a->S; f.Sk = Sk; f.Hq = a->H; f.Hkv = a->Hkv; f.hd = hd;
       f.causal = a->causal; f.q_offset = a->cached ? a->past : 0; f.scale = scale;
-      return dptb_attn_f32(&f, stream);
+      if (!append) return dptb_attn_f32(&f, stream);
+      const DptbF32View kn = {reinterpret_cast<float*>(qkv) + dq, (long long)a->S * ldqkv, ldqkv, hd};
+      const DptbF32View vn = {reinterpret_cast<float*>(qkv) + dq + dkv, (long long)a->S * ldqkv, ldqkv, hd};
+      return dptb_attn_f32_append(&f, &kn, &vn, stream);
     }
     if (l.dec_splits > 0) {
       DptbDecodeArgs d;
@@ -210,15 +214,22 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
       x = ws + l.norm;
     }
     DPTB_STACK_OK(linear(x, D, t[kQkvW], t[kQkvB], ldqkv, qkv, 0, nullptr));
-    if (a->cached) {
-      DPTB_STACK_OK(dptb_rope_kv_append(qkv, ldqkv, const_cast<void*>(t[kKCache]), const_cast<void*>(t[kVCache]), a->ldkv,
-                                        a->kv_batch_stride, a->B, a->S, a->H, a->Hkv, hd, a->start_pos, a->past,
-                                        a->rotary_dim, a->rope_base, a->cap, nullptr, a->bf16, stream));
-    } else if (a->rotary_dim > 0) {
-      DPTB_STACK_OK(dptb_rope(qkv, qkv, rows, a->H + a->Hkv, hd, a->rotary_dim, a->S, a->start_pos, a->rope_base, 0, a->bf16,
-                              ldqkv, ldqkv, nullptr, stream));
+    // Few fp32 rows that are not turned: the attention appends them to the caches itself.
+    int attended = kErrUnsupported;
+    if (a->cached && !a->bf16 && a->rotary_dim == 0 && a->past + a->S <= a->cap)
+      attended = attend(qkv, t[kKCache], t[kVCache], ws + l.attn, true);
+    if (attended == kErrUnsupported) {
+      if (a->cached) {
+        DPTB_STACK_OK(dptb_rope_kv_append(qkv, ldqkv, const_cast<void*>(t[kKCache]), const_cast<void*>(t[kVCache]), a->ldkv,
+                                          a->kv_batch_stride, a->B, a->S, a->H, a->Hkv, hd, a->start_pos, a->past,
+                                          a->rotary_dim, a->rope_base, a->cap, nullptr, a->bf16, stream));
+      } else if (a->rotary_dim > 0) {
+        DPTB_STACK_OK(dptb_rope(qkv, qkv, rows, a->H + a->Hkv, hd, a->rotary_dim, a->S, a->start_pos, a->rope_base, 0, a->bf16,
+                                ldqkv, ldqkv, nullptr, stream));
+      }
+      attended = attend(qkv, t[kKCache], t[kVCache], ws + l.attn, false);
     }
-    DPTB_STACK_OK(attend(qkv, t[kKCache], t[kVCache], ws + l.attn));
+    DPTB_STACK_OK(attended);
     DPTB_STACK_OK(linear(ws + l.attn, dq, t[kWoW], t[kWoB], D, mid, 0, cur));          // mid = attention + residual
     const void* y = ws + l.norm;
     const void* res = mid;

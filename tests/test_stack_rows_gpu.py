@@ -1,0 +1,75 @@
+"""Few fp32 rows through the native stack (norms inside the products, the cache append inside the attention) against the modules' own
+forward passes: the same bits, in the hidden states and in the caches."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+import dart_pytorch_b200 as dp
+from dart_pytorch_b200.models.llama import Llama, LlamaConfig
+from dart_pytorch_b200.nn.attention import EncoderCache
+from dart_pytorch_b200.nn.transformer import Activation
+from dart_pytorch_b200.ops import stack
+
+
+def _steps(model, cache, toks, n):
+    with torch.no_grad():
+        out = [model.hidden(toks[:, :n], 0, cache)]
+        for i in range(n, toks.shape[1]):
+            out.append(model.hidden(toks[:, i:i + 1], i, cache))
+    return out + [c.k_buf for c in cache.layers] + [c.v_buf for c in cache.layers]
+
+
+def _both(monkeypatch, fn):
+    native = fn()
+    with monkeypatch.context() as m:
+        m.setattr(stack, "run", lambda *a, **k: None)
+        plain = fn()
+    for x, y in zip(native, plain, strict=True):
+        assert torch.equal(x, y)
+
+
+# rows up to 8 stream the weights and from 256 terms on take the norm with them (9 rows and 1032 columns do not); tokens go past a tile
+# of 64 keys, and 3 at a time into it
+@pytest.mark.parametrize("width,heads", [(256, 4), (264, 3), (1024, 8), (1032, 12)])
+@pytest.mark.parametrize("B,n", [(1, 62), (3, 1), (8, 126), (9, 3)])
+def test_gpt(monkeypatch, width, heads, B, n):
+    m = dp.GPT(dp.GPTConfig(vocab_size=97, max_ctx=300, embed_dim=width, num_layers=2, num_heads=heads, ffn_dim=300, attn_bias=True,
+                            activation=Activation.geluTanh, device="cuda", dtype=torch.float32, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (B, n + 4), device="cuda")
+    _both(monkeypatch, lambda: _steps(m, EncoderCache.empty(2, heads, max_len=300), toks, n))
+
+
+@pytest.mark.parametrize("B,n,S", [(1, 63, 3), (2, 5, 4), (1, 0, 2)])
+def test_several_tokens_a_step(monkeypatch, B, n, S):
+    m = dp.GPT(dp.GPTConfig(vocab_size=97, max_ctx=300, embed_dim=256, num_layers=2, num_heads=4, ffn_dim=300, attn_bias=False,
+                            activation=Activation.relu, device="cuda", dtype=torch.float32, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (B, n + S), device="cuda")
+
+    def run():
+        cache = EncoderCache.empty(2, 4, max_len=300)
+        with torch.no_grad():
+            out = [m.hidden(toks[:, :n], 0, cache)] if n else []
+            out.append(m.hidden(toks[:, n:], n, cache))
+        return out + [c.k_buf for c in cache.layers] + [c.v_buf for c in cache.layers]
+    _both(monkeypatch, run)
+
+
+@pytest.mark.parametrize("B", [1, 8, 9])
+def test_llama(monkeypatch, B):
+    m = Llama(LlamaConfig(vocab_size=97, max_ctx=300, embed_dim=512, num_layers=2, num_heads=8, num_kv_heads=2, ffn_dim=264,
+                          device="cuda", dtype=torch.float32, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (B, 68), device="cuda")
+    _both(monkeypatch, lambda: _steps(m, m.new_cache(), toks, 62))
+
+
+def test_infinities_and_nan(monkeypatch):
+    m = dp.GPT(dp.GPTConfig(vocab_size=97, max_ctx=300, embed_dim=256, num_layers=1, num_heads=4, ffn_dim=300, attn_bias=True,
+                            activation=Activation.relu, device="cuda", dtype=torch.float32, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (3, 6), device="cuda")
+    with torch.no_grad():
+        table = m.parameters()[0].data
+        table[toks[0, 5], 3], table[toks[1, 5], 4] = float("inf"), float("nan")
+    def run():
+        return [t.nan_to_num(1.5) for t in _steps(m, EncoderCache.empty(1, 4, max_len=300), toks, 5)]
+    _both(monkeypatch, run)
