@@ -116,8 +116,13 @@ attn_decode_kernel(const DecodeArgs a) {
   constexpr int kStageChunks = kDecRound * LPK;            // 16-byte chunks of one K (or V) stage
   constexpr int kWarpChunks = 4 * kStageChunks;            // two stages of K and V
   extern __shared__ uint4 dec_ring[];
-  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
-  pdl_launch_dependents();
+  // As a programmatic dependent a warp requests its first keys before the kernel ahead (which appends this step's rows) is done, if
+  // they are rows of earlier steps; the windowed form and a position on the device wait first.
+  const bool known = !WIN && !a.pos_ptr;
+  if (!known) {
+    pdl_wait();              // (programmatic dependent launch: no-ops in an ordinary launch)
+    pdl_launch_dependents();
+  }
   const int split = blockIdx.x, g = blockIdx.y, bs = blockIdx.z;
   const int b = bs / a.Sq, sq = bs % a.Sq;
   const int G = a.Hq / a.Hkv;
@@ -178,7 +183,13 @@ attn_decode_kernel(const DecodeArgs a) {
     }
     cp_async_commit();
   };
-  if (warp < rounds) issue(warp, 0);
+  const bool early = known && j0 + (warp + 1) * kDecRound <= q_off;
+  if (early && warp < rounds) issue(warp, 0);
+  if (known) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
+  if (!early && warp < rounds) issue(warp, 0);
   if constexpr (!WIN) {
     // Scores^T and outputs^T by warp-level matrix instructions, the query heads of the group as their 8 columns: a round of 16 keys
     // is about 150 instructions, where multiply-adds and shuffles took about 1000 (4 heads of 128) and bounded the kernel.

@@ -283,6 +283,14 @@ attn_f32_decode(const AttnF32Params p) {
   const int nc = cluster.num_blocks(), rank = cluster.block_rank();
   const int hk = blockIdx.y, b = blockIdx.z, g = p.Hq / p.Hkv, rows = g * p.Sq;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tiles = (p.Sk + kFBN - 1) / kFBN;
+  // With rows to append, those that the caches have are older than the kernel ahead (the projection): this CTA's first tile of them is
+  // requested before the wait for it.
+  const bool ahead = p.appended < p.Sk && rank < tiles;
+  if (ahead) {
+    f32_request_tile<HD, kFBN>(Ks, p.k, b, hk, rank * kFBN, p.appended, p.hd, p.vec);
+    f32_request_tile<HD, kFBN>(Vs, p.v, b, hk, rank * kFBN, p.appended, p.hd, p.vec);
+  }
   pdl_wait();
   pdl_launch_dependents();
   // row r: query head hk * g + r / Sq, position r % Sq
@@ -299,13 +307,16 @@ attn_f32_decode(const AttnF32Params p) {
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-  const int tiles = (p.Sk + kFBN - 1) / kFBN;
   const int c4 = tid % C4, kg = tid / C4;
   for (int t = rank; t < tiles; t += nc) {
     const int key0 = t * kFBN;
-    __syncthreads();
-    f32_load_tile<HD, kFBN>(Ks, p.k, b, hk, key0, p.appended, p.hd, p.vec);
-    f32_load_tile<HD, kFBN>(Vs, p.v, b, hk, key0, p.appended, p.hd, p.vec);
+    if (ahead && t == rank) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+      __syncthreads();
+      f32_load_tile<HD, kFBN>(Ks, p.k, b, hk, key0, p.appended, p.hd, p.vec);
+      f32_load_tile<HD, kFBN>(Vs, p.v, b, hk, key0, p.appended, p.hd, p.vec);
+    }
     __syncthreads();
     if (key0 + kFBN > p.appended && p.appended < p.Sk) {
       // A tile is one CTA's alone, so that one appends its rows.
