@@ -7,14 +7,20 @@
 // useful bytes) and one slice of K; x is the narrow N = 32 / 64 side.  Work units = (N / 128) x (K splits) are chosen
 // to fill the SMs once, with TMA rings of 128 to 160 KB of W in flight per SM.  D[128 weight rows, M] lands
 // in 32 / 64 TMEM columns; a thread of the four epilogue warps owns one weight row = one output column.
-//   splits == 1: the epilogue writes out[m, n] directly (lanes = consecutive n, so stores coalesce);
-//   splits  > 1: fp32 partials go to a workspace, the last unit of a tile (per-tile counter) sums them in split order
-//                (deterministic) and runs the epilogue.
+// The K splits of a tile (up to 8) are the CTAs of a cluster: each leaves its fp32 sums in its own shared memory and every one adds
+// an equal share of the outputs, in split order, and runs the epilogue on it.  Through a workspace in global memory, with the last
+// unit of a tile folding all of it, a split product took about 2 us more.
+// GLU: W holds F rows of gates and then F rows of values; a CTA's 128 rows are 64 gates and the 64 values that go with them.
+//
+// In a tensor-parallel group (gemm_skinny_kernel) fp32 partials go to a workspace, the last unit of a tile (per-tile counter) sums
+// them in split order (deterministic) and runs the epilogue.
 // Row-parallel Linear of a tensor-parallel group (all-reduce over ranks, + bias, + residual) is fused the same way as
 // in the big GEMM: the finished local tile goes to this rank's symmetric partial buffer, the tile's owner rank is
 // flagged, the owner reduces over the ranks (multimem.ld_reduce through the NVSwitch, else peer loads) and writes the
 // result into every rank's output (multimem.st, else peer stores); the last CTA runs the end-of-kernel handshake.
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "common/gemm_args.h"
 #include "common/host.h"
@@ -74,7 +80,6 @@ struct SkinnyParams {
   const __nv_bfloat16* residual;    // [M, ldr] or null
   long long ldr;
   int num_kb, splits, kb_per_split;
-  int vec_out;                      // C / residual 16-byte aligned, leading dimensions and N multiples of 8
   float* ws;                        // [tile][split][MP][128] fp32
   int* counters;                    // per tile, zero between launches
   SkinnyAr ar;
@@ -99,6 +104,22 @@ __device__ __forceinline__ uint4 ld_relaxed_sys_v4(const uint2* p) {
   return v;
 }
 
+constexpr int kSkMaxSplits = 8;      // CTAs of a cluster
+struct SkinnyLocalParams {
+  int M, N;                          // N: output columns (GLU: half the weight rows)
+  __nv_bfloat16* C;
+  long long ldc, ldr;
+  const __nv_bfloat16* bias;
+  const __nv_bfloat16* residual;
+  int num_kb, splits, kb_per_split;
+  int vec_out;                       // 16-byte stores, and loads of the residual
+};
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 template <int MP, int ST>
 struct SkinnySmem {
   static constexpr int kWBytes = kSkBM * kSkBK * 2;     // 16 KB
@@ -108,23 +129,203 @@ struct SkinnySmem {
   static constexpr int kTotal = kBarOff + (2 * ST + 2) * 8 + 64 + 1024;
 };
 
-// Final values of one tile -> output (non-tensor-parallel): thread = output column n, v[m] over the rows.
-template <int MP>
-__device__ __forceinline__ void skinny_store(const SkinnyParams& p, int n, const float (&v)[MP]) {
-  if (n >= p.N) return;
-  const float b = p.bias ? __bfloat162float(p.bias[n]) : 0.0f;
-#pragma unroll
-  for (int m = 0; m < MP; ++m) {
-    if (m < p.M) {
-      float o = v[m] + b;
-      if (p.residual) o += __bfloat162float(p.residual[(long long)m * p.ldr + n]);
-      p.C[(long long)m * p.ldc + n] = __float2bfloat16(o);
+// This rank's product alone, out = x W^T (+ bias) (+ residual), or with GLU out = silu(x Wg^T) * (x Wu^T): see the head of the file.
+template <int MP, int ST, bool GLU>
+__global__ void __launch_bounds__(kSkThreads, 2)
+gemm_skinny_local_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const SkinnyLocalParams p) {
+  using L = SkinnySmem<MP, ST>;
+  constexpr int TMEM_COLS = MP < 32 ? 32 : MP;
+  constexpr int COLS = GLU ? kSkBM / 2 : kSkBM;            // output columns of a tile
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
+  uint64_t* empty_bar = full_bar + ST;
+  uint64_t* acc_full = empty_bar + ST;
+  uint64_t* drain_bar = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* sums = reinterpret_cast<float*>(smem);            // [MP][128], once the ring is idle
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = p.splits > 1 ? (int)cluster_cta_rank() : 0;
+  const int n0 = (int)(p.splits > 1 ? blockIdx.x / p.splits : blockIdx.x) * COLS;
+  const int kb0 = split * p.kb_per_split;
+  const int kb1 = min(p.num_kb, kb0 + p.kb_per_split);     // (never empty)
+  pdl_launch_dependents();   // the small kernel after this one waits for this grid's completion at its own top
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    if (lane == 0) *abort_flag = 0;
+    if (lane < 2 * ST + 2) mbar_init(full_bar + lane, 1);
+    mbar_fence_init();
+    __syncwarp();
+    tmem_alloc<TMEM_COLS>(tmem_slot);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      auto load_w = [&](int s, int kb) {
+        uint8_t* dst = smem + s * L::kStage;
+        tma_load_2d(dst, &tmW, &full_bar[s], kb * kSkBK, n0);
+        if constexpr (GLU) tma_load_2d(dst + L::kWBytes / 2, &tmW, &full_bar[s], kb * kSkBK, p.N + n0);
+      };
+      // The weights do not depend on the kernel before this one: the first ring-full of weight tiles is requested at once, then
+      // (programmatic dependent launch) the predecessor's completion is awaited, then the activation tiles of those stages follow.
+      const int pre = min(kb1 - kb0, ST);
+      for (int i = 0; i < pre; ++i) {
+        mbar_arrive_expect_tx(&full_bar[i], L::kStage);
+        load_w(i, kb0 + i);
+      }
+      pdl_wait();
+      for (int i = 0; i < pre; ++i)
+        tma_load_2d(smem + i * L::kStage + L::kWBytes, &tmX, &full_bar[i], (kb0 + i) * kSkBK, 0);
+      int issued = pre;
+      for (int kb = kb0 + pre; kb < kb1; ++kb, ++issued) {
+        const int s = issued % ST;
+        if (!mbar_wait(&empty_bar[s], ((issued / ST) & 1) ^ 1, abort_flag, kWaitEmptyTimeout)) break;
+        mbar_arrive_expect_tx(&full_bar[s], L::kStage);
+        load_w(s, kb);
+        tma_load_2d(smem + s * L::kStage + L::kWBytes, &tmX, &full_bar[s], kb * kSkBK, 0);
+      }
+      if (*abort_flag) {
+        // Do not leave while a tile copy may still be writing this CTA's shared memory.
+        const int n = issued < ST ? issued : ST;
+        const uint64_t t0 = global_timer_ns();
+        for (int j = 0; j < n; ++j) {
+          const int i = issued - 1 - j;
+          while (!mbar_try_wait(&full_bar[i % ST], (i / ST) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+        }
+      }
     }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(kSkBM, MP, false, false);
+      bool issued_any = false, ok = true;
+      int consumed = 0;
+      for (int kb = kb0; kb < kb1; ++kb, ++consumed) {
+        const int s = consumed % ST;
+        if (!mbar_wait(&full_bar[s], (consumed / ST) & 1, abort_flag, kWaitFullTimeout)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint32_t w_addr = smem_u32(smem + s * L::kStage);
+        const uint32_t x_addr = w_addr + L::kWBytes;
+#pragma unroll
+        for (int k = 0; k < kSkBK / 16; ++k)
+          umma_bf16(tmem_base, make_smem_desc(w_addr + k * 32, 16, 1024), make_smem_desc(x_addr + k * 32, 16, 1024),
+                    idesc, (kb != kb0 || k != 0) ? 1u : 0u);
+        issued_any = true;
+        umma_commit(&empty_bar[s]);
+      }
+      if (ok) umma_commit(acc_full);
+      if (*abort_flag && issued_any) {
+        umma_commit(drain_bar);
+        const uint64_t t0 = global_timer_ns();
+        while (!mbar_try_wait(drain_bar, 0) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ accumulator -> shared memory, a weight row a thread
+    pdl_wait();   // nothing below may touch global memory before the predecessor has completed
+    const int q = warp & 3, row = q * 32 + lane;
+    if (__all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, kWaitTmemFullTimeout))) {
+      tc_fence_after_sync();
+#pragma unroll
+      for (int c = 0; c < MP; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sums[(c + i) * kSkBM + row] = __uint_as_float(r[i]);
+      }
+    }
+  }
+  tc_fence_before_sync();
+  if (p.splits > 1) cluster_sync_all();
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc<TMEM_COLS>(tmem_base);
+  }
+  if (warp >= 2) {
+    // Eight neighbouring outputs of a row a thread.  In a CTA that gave up the sums are worthless.
+    const int et = threadIdx.x - 64;
+    auto add = [&](const float* at, float (&f)[8]) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = 0.0f;
+      if (p.splits > 1) {
+        float4 part[kSkMaxSplits][2];                      // all requested before the first is used
+#pragma unroll
+        for (int s = 0; s < kSkMaxSplits; ++s)
+          if (s < p.splits) {
+            const uint32_t a = map_to_cta(at, s);
+            part[s][0] = ld_cluster_v4(a);
+            part[s][1] = ld_cluster_v4(a + 16);
+          }
+#pragma unroll
+        for (int s = 0; s < kSkMaxSplits; ++s)
+          if (s < p.splits) {
+            f[0] += part[s][0].x; f[1] += part[s][0].y; f[2] += part[s][0].z; f[3] += part[s][0].w;
+            f[4] += part[s][1].x; f[5] += part[s][1].y; f[6] += part[s][1].z; f[7] += part[s][1].w;
+          }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] += at[e];
+      }
+    };
+    for (int i = split * 128 + et; i < p.M * (COLS / 8); i += p.splits * 128) {
+      const int m = i / (COLS / 8), c = i % (COLS / 8) * 8, col = n0 + c;
+      if (col >= p.N) continue;
+      float f[8];
+      add(sums + m * kSkBM + c, f);
+      __nv_bfloat16* dst = p.C + (long long)m * p.ldc + col;
+      if constexpr (GLU) {
+        float u[8];
+        add(sums + m * kSkBM + COLS + c, u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          // both rounded to bf16 first, as where the product is stored and gated by a kernel of its own
+          const float z = __bfloat162float(__float2bfloat16(f[e]));
+          f[e] = z / (1.0f + __expf(-z)) * __bfloat162float(__float2bfloat16(u[e]));
+        }
+      } else if (p.bias) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (col + e < p.N) f[e] += __bfloat162float(p.bias[col + e]);
+      }
+      if (p.vec_out) {
+        if (!GLU && p.residual) {
+          const uint4 r = *reinterpret_cast<const uint4*>(p.residual + (long long)m * p.ldr + col);
+          const float2 r0 = unpack_bf16x2(r.x), r1 = unpack_bf16x2(r.y), r2 = unpack_bf16x2(r.z), r3 = unpack_bf16x2(r.w);
+          f[0] += r0.x; f[1] += r0.y; f[2] += r1.x; f[3] += r1.y; f[4] += r2.x; f[5] += r2.y; f[6] += r3.x; f[7] += r3.y;
+        }
+        *reinterpret_cast<uint4*>(dst) =
+            make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+      } else {
+        for (int e = 0; e < 8 && col + e < p.N; ++e) {
+          float o = f[e];
+          if (!GLU && p.residual) o += __bfloat162float(p.residual[(long long)m * p.ldr + col + e]);
+          dst[e] = __float2bfloat16(o);
+        }
+      }
+    }
+  }
+  if (p.splits > 1) {        // no CTA leaves while another reads its sums
+    __syncwarp();
+    cluster_sync_all();
   }
 }
 
 template <int MP, int ST>
-__global__ void __launch_bounds__(kSkThreads, ST <= 5 ? 2 : 1)
+__global__ void __launch_bounds__(kSkThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                    const SkinnyParams p) {
   using L = SkinnySmem<MP, ST>;
@@ -323,37 +524,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
     SK_STAMP(6, tile == 0 && have_tile && et == 0);
-    if (have_tile && p.ar.world == 0 && p.os.world == 0 && p.vec_out) {
-      // Transpose through shared memory (the ring is idle by now) so that the output leaves as 16-byte vectors:
-      // fp32 [MP][128] staging, then 16 lanes per output row.
-      float* tile_s = reinterpret_cast<float*>(smem);
-      const float b = (p.bias && n0 + n_local < p.N) ? __bfloat162float(p.bias[n0 + n_local]) : 0.0f;
-#pragma unroll
-      for (int m = 0; m < MP; ++m) tile_s[m * kSkBM + n_local] = v[m] + b;
-      ok = epi_sync();
-      const int cg = et & 15;
-      const int col = n0 + cg * 8;
-      if (ok && col < p.N) {
-        for (int m = et >> 4; m < p.M; m += 8) {
-          const float4 lo = *reinterpret_cast<const float4*>(tile_s + m * kSkBM + cg * 8);
-          const float4 hi = *reinterpret_cast<const float4*>(tile_s + m * kSkBM + cg * 8 + 4);
-          float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-          if (p.residual) {
-            const uint4 r = *reinterpret_cast<const uint4*>(p.residual + (long long)m * p.ldr + col);
-            const float2 r0 = unpack_bf16x2(r.x), r1 = unpack_bf16x2(r.y), r2 = unpack_bf16x2(r.z), r3 = unpack_bf16x2(r.w);
-            f[0] += r0.x; f[1] += r0.y; f[2] += r1.x; f[3] += r1.y;
-            f[4] += r2.x; f[5] += r2.y; f[6] += r3.x; f[7] += r3.y;
-          }
-          uint4 o;
-          o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
-          o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-          *reinterpret_cast<uint4*>(p.C + (long long)m * p.ldc + col) = o;
-        }
-      }
-      SK_STAMP(7, tile == 0 && et == 0);
-    } else if (have_tile && p.ar.world == 0 && p.os.world == 0) {
-      skinny_store<MP>(p, n0 + n_local, v);
-    } else if (have_tile && p.os.world > 0) {
+    if (have_tile && p.os.world > 0) {
       // ---- one-shot all-reduce, flag-in-data: every value travels as one 8-byte store {fp32 bits, launch number}
       // into slot [parity][this rank][tile] of EVERY rank; a receiver polls the slots of all ranks in its own memory
       // until every word carries this launch's number and sums them in rank order.  No fence, no separate flag.
@@ -540,6 +711,34 @@ static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, const S
   DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   return counted(1, (int)launch_k(kern, dim3(units), dim3(kSkThreads), L::kTotal, stream, tmW, tmX, p));
 }
+template <int MP, int ST, bool GLU>
+static int launch_skinny_local(const CUtensorMap& tmW, const CUtensorMap& tmX, const SkinnyLocalParams& p, int tiles, cudaStream_t stream) {
+  using L = SkinnySmem<MP, ST>;
+  auto kern = gemm_skinny_local_kernel<MP, ST, GLU>;
+  static SmemLimit limit;
+  DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (p.splits > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = p.splits;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl_flag()) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.splits);
+  cfg.blockDim = dim3(kSkThreads);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  return counted(1, (int)cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p));
+}
 
 }  // namespace dptb
 
@@ -582,6 +781,16 @@ extern "C" int dptb_gemm_skinny_oneshot(const DptbGemmArgs* a, const DptbTpOneSh
   if (!os) return kErrBadShape;
   return skinny_impl(a, nullptr, os, stream_v);
 }
+// Out = silu(x Wg^T) * (x Wu^T), W = [gates; values] [2N, K], without bias or residual.
+static int skinny_local(const DptbGemmArgs* a, bool glu, cudaStream_t stream);
+extern "C" int dptb_gemm_skinny_swiglu(const DptbGemmArgs* a, void* stream_v) {
+  if (a->M <= 0 || a->N <= 0) return 0;
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (a->M > 64 || a->K <= 0 || a->trans_a || !a->trans_b || a->a_f32 || a->b_f32 || a->out_f32 || a->accumulate || a->act || a->aux_out ||
+      a->aux_in || a->alpha != 1.0f || a->bias || a->residual || !al16(a->A) || !al16(a->B) || (a->lda % 8) || (a->ldb % 8))
+    return kErrUnsupported;
+  return skinny_local(a, true, static_cast<cudaStream_t>(stream_v));
+}
 static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTpOneShotArgs* os, void* stream_v) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   if (a->M <= 0 || a->N <= 0) return 0;
@@ -603,9 +812,9 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
         (a->residual && (!al16(a->residual) || a->ldr % 8)))
       return kErrUnsupported;
   }
+  if (!ar && !os) return skinny_local(a, false, stream);
   const int mp = a->M <= 32 ? 32 : 64;
   const int tiles = (a->N + kSkBM - 1) / kSkBM;
-  const bool local = !ar && !os;
   const int num_kb = (a->K + kSkBK - 1) / kSkBK;
   // Split K so that the work units fill the SMs once, with at least 4 k-blocks each.
   int splits = a->splits >= 1 ? a->splits : 1;
@@ -616,10 +825,7 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
       return v > 0 ? v : 4;
     }();
     const int by_sm = sm_count() / tiles;
-    // Writing and folding the partial tiles takes about 2 us, as long as 8 k-blocks and more: a local split has at least
-    // that many (B200, 32 rows: 768 x 768 in one piece 7.0 us, in three 8.9 us; 3072 x 2048 in 4 pieces 11.6 us, in 6 12.5 us;
-    // 2048 x 5504 in 8 pieces 13.9 us, in 18 16.7 us).
-    const int by_k = num_kb / (local && min_kb < 8 ? 8 : min_kb);
+    const int by_k = num_kb / min_kb;
     splits = by_sm < by_k ? by_sm : by_k;
     if (splits < 1) splits = 1;
   }
@@ -636,8 +842,6 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
   p.bias = static_cast<const __nv_bfloat16*>(a->bias);
   p.residual = static_cast<const __nv_bfloat16*>(a->residual); p.ldr = a->ldr;
   p.num_kb = num_kb; p.splits = splits; p.kb_per_split = kb_per_split;
-  p.vec_out = (al16(a->C) && a->ldc % 8 == 0 && a->N % 8 == 0 &&
-               (!a->residual || (al16(a->residual) && a->ldr % 8 == 0))) ? 1 : 0;
   p.ws = static_cast<float*>(a->ws);
   p.counters = a->counters;
   p.ar.world = 0;
@@ -673,9 +877,43 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
   rc = encode_tmap_2d_bf16(&tmX, a->A, (uint64_t)a->K, (uint64_t)a->M, (uint64_t)a->lda * 2, 64, (uint32_t)mp);
   if (rc) return rc;
   const int units = tiles * splits;
+  // (one CTA an SM: they wait for peers)
+  return mp == 32 ? launch_skinny<32, 8>(tmW, tmX, p, units, stream) : launch_skinny<64, 8>(tmW, tmX, p, units, stream);
+}
+static int skinny_local(const DptbGemmArgs* a, bool glu, cudaStream_t stream) {
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const int cols = glu ? kSkBM / 2 : kSkBM;
+  const int tiles = (a->N + cols - 1) / cols;
+  const int num_kb = (a->K + kSkBK - 1) / kSkBK;
+  // Splits of K: of 8 k-blocks and more as many as two CTAs an SM take (what counts is bytes in flight), shorter ones of 3 and more only
+  // while all CTAs stay within two thirds of the SMs (what counts is the chain; a meeting of many CTAs gets longer).  Measured (B200, 32
+  // rows, weights from HBM), splits: us: 768 x 768 1: 7.2, 2: 6.4, 4: 5.6, 8: 5.6; 2304 x 768 1: 7.7, 4: 6.4, 8: 6.7; 2048 x 2048 1:
+  // 13.6, 4: 8.1, 6: 8.2, 8: 9.2; 3072 x 2048 4: 8.6, 6: 10.1; 2048 x 5504 4: 12.7, 6: 11.4, 8: 12.2; 11008 x 2048 1: 15.4, 3: 13.9, 4: 19.2;
+  // 32768 x 2048 1: 27.9, 2: 33.8.  Partial tiles through global memory took 11.7 (2048 x 2048), 15.0 (2048 x 5504) and 15.3 us (11008 x 2048).
+  int splits = a->splits;
+  if (splits < 1) {
+    const int sms = sm_count();
+    const int loads = std::min(2 * sms / tiles, num_kb / 8), chain = std::min(2 * sms / (3 * tiles), num_kb / 3);
+    splits = std::max(loads, chain);
+  }
+  splits = splits < 1 ? 1 : splits > kSkMaxSplits ? kSkMaxSplits : splits;
+  SkinnyLocalParams p;
+  p.M = a->M; p.N = a->N;
+  p.C = static_cast<__nv_bfloat16*>(a->C); p.ldc = a->ldc;
+  p.bias = static_cast<const __nv_bfloat16*>(a->bias);
+  p.residual = static_cast<const __nv_bfloat16*>(a->residual); p.ldr = a->ldr;
+  p.num_kb = num_kb;
+  p.kb_per_split = (num_kb + splits - 1) / splits;
+  p.splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;   // every split non-empty
+  p.vec_out = al16(a->C) && a->ldc % 8 == 0 && a->N % 8 == 0 && (!a->residual || (al16(a->residual) && a->ldr % 8 == 0));
+  const bool wide = a->M > 32;
+  CUtensorMap tmW, tmX;
+  int rc = encode_tmap_2d_bf16(&tmW, a->B, (uint64_t)a->K, (uint64_t)a->N * (glu ? 2 : 1), (uint64_t)a->ldb * 2, 64, (uint32_t)cols);
+  if (!rc) rc = encode_tmap_2d_bf16(&tmX, a->A, (uint64_t)a->K, (uint64_t)a->M, (uint64_t)a->lda * 2, 64, wide ? 64u : 32u);
+  if (rc) return rc;
   // Two CTAs an SM with shorter rings beat one with 8 stages once there are more tiles than SMs: a second wave then fills in
   // beside the first instead of after it (B200, 32 rows: 50257 x 768 31.6 -> 23.8 us, 32768 x 2048 32.2 -> 26.7 us, the same
-  // within 5 % for fewer tiles).  The collective forms keep one: their CTAs wait for peers.
-  if (local) return mp == 32 ? launch_skinny<32, 5>(tmW, tmX, p, units, stream) : launch_skinny<64, 4>(tmW, tmX, p, units, stream);
-  return mp == 32 ? launch_skinny<32, 8>(tmW, tmX, p, units, stream) : launch_skinny<64, 8>(tmW, tmX, p, units, stream);
+  // within 5 % for fewer tiles).
+  if (glu) return wide ? launch_skinny_local<64, 4, true>(tmW, tmX, p, tiles, stream) : launch_skinny_local<32, 5, true>(tmW, tmX, p, tiles, stream);
+  return wide ? launch_skinny_local<64, 4, false>(tmW, tmX, p, tiles, stream) : launch_skinny_local<32, 5, false>(tmW, tmX, p, tiles, stream);
 }

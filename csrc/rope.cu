@@ -63,8 +63,13 @@ struct RopeVec<__nv_bfloat16, 8> {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kRopeThreads)
 rope_kernel(const RopeParams p) {
-  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
-  pdl_launch_dependents();
+  // As a programmatic dependent the first angles are worked out before the kernel ahead is done, unless positions come from the device.
+  bool waits = !p.pos_ptr && !p.positions;
+  auto wait = [&] {
+    pdl_wait();              // (no-ops in an ordinary launch)
+    pdl_launch_dependents();
+  };
+  if (!waits) wait();
   __shared__ float2 table[kRopeTable];
   using V = RopeVec<T, VEC>;
   const long long t0 = (long long)blockIdx.x * p.tokens_per_block;
@@ -105,6 +110,8 @@ rope_kernel(const RopeParams p) {
       sincosf(pos * inv, &sn, &cs);
       table[i] = make_float2(cs, p.inverse ? -sn : sn);
     }
+    if (waits) wait();
+    waits = false;
     __syncthreads();
     const int groups = n / VEC, per_tok = turned * groups;
     for (int i = threadIdx.x; i < nt * per_tok; i += kRopeThreads) {
@@ -127,6 +134,7 @@ rope_kernel(const RopeParams p) {
       V::store(o + d0 + g + half, b);
     }
   }
+  if (waits) wait();
   // What passes through: the dimensions beyond rotary_dim of heads that move, and the values.
   const int first = cache ? p.heads : 0, tail = p.head_dim - p.rotary_dim;
   const bool moves = cache || x != out;

@@ -18,6 +18,7 @@ extern "C" {
 int dptb_gemm(const DptbGemmArgs*, void*);
 int dptb_gemm_skinny(const DptbGemmArgs*, const DptbTpArArgs*, void*);
 int dptb_gemm_swiglu(const DptbGemmArgs*, void*);
+int dptb_gemm_skinny_swiglu(const DptbGemmArgs*, void*);
 int dptb_attn_f32_append(const DptbAttnF32Args*, const DptbF32View*, const DptbF32View*, void*);
 int dptb_attn_fwd(const DptbAttnFwdArgs*, void*);
 int dptb_attn_f32(const DptbAttnF32Args*, void*);
@@ -131,14 +132,14 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
   };
   // The two products of a gated unit and the gate: one kernel where it exists, else the product of both and a pass over it.
   auto gated = [&](const void* x, const void* w, const void* bias, char* up, void* y) {
-    if (a->bf16 && !bias && M > a->skinny_rows) {
+    if (a->bf16 && !bias) {
       DptbGemmArgs g;
       memset(&g, 0, sizeof(g));
       g.A = x; g.B = w; g.C = y;
       g.lda = g.ldb = D; g.ldc = a->F;
       g.M = M; g.N = a->F; g.K = D;
       g.trans_b = 1; g.alpha = 1.0f;
-      const int rc = dptb_gemm_swiglu(&g, stream);
+      const int rc = M <= a->skinny_rows ? dptb_gemm_skinny_swiglu(&g, stream) : dptb_gemm_swiglu(&g, stream);
       if (rc != kErrUnsupported) return rc;
     }
     const int rc = linear(x, D, w, bias, 2 * a->F, up, 0, nullptr);
