@@ -148,8 +148,12 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
-  pdl_launch_dependents();
+  // As a programmatic dependent an x W^T product requests its first weights, which no kernel of a chain writes, before the wait.
+  constexpr bool kAhead = !AMN && !BMN;
+  if (!kAhead || warp == kTcThreads / 32) {
+    pdl_wait();              // (programmatic dependent launch: no-ops in an ordinary launch)
+    pdl_launch_dependents();
+  }
 
   const int m0 = blockIdx.y * kTcBM, n0 = blockIdx.x * BN;
   const int k_begin = blockIdx.z * p.k_per_split;
@@ -212,8 +216,12 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
       return true;
     };
 
-    ta.load(p.A, p.lda, m0, p.M, k_begin, k_end, p.vec_a);
     tb.load(p.B, p.ldb, n0, p.N, k_begin, k_end, p.vec_b);
+    if (kAhead) {
+      pdl_wait();
+      pdl_launch_dependents();
+    }
+    ta.load(p.A, p.lda, m0, p.M, k_begin, k_end, p.vec_a);
     bool ok = true;
     for (int i = 0; i < blocks && ok; ++i) {
       // (stage i & 1 is free: `collect` of block i - 2 has waited for the MMAs that read it)
