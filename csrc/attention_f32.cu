@@ -42,6 +42,7 @@ struct AttnF32Params {
   // k / v, the caches.
   F32View kn, vn;
   int appended;
+  int key_ctas;           // forward tiles: CTAs that share the keys of a row tile
 };
 
 constexpr int kFBM = 32, kFBN = 64, kFThreads = 128;
@@ -174,13 +175,14 @@ __device__ __forceinline__ float half_warp_sum(float x) {
 }
 
 // Key tiles that the rows [row0, row0 + 32) can see.
-__device__ __forceinline__ int f32_key_tiles(const AttnF32Params& p, int row0) {
+__host__ __device__ __forceinline__ int f32_key_tiles(const AttnF32Params& p, int row0) {
   int last = p.Sk - 1;
-  if (p.causal) last = min(last, min(row0 + kFBM, p.Sq) - 1 + p.q_offset);
+  const int end = row0 + kFBM < p.Sq ? row0 + kFBM : p.Sq;
+  if (p.causal && end - 1 + p.q_offset < last) last = end - 1 + p.q_offset;
   return last < 0 ? 0 : last / kFBN + 1;
 }
 
-template <int HD>
+template <int HD, bool SHARED>
 __global__ void __launch_bounds__(kFThreads)
 attn_f32_fwd(const AttnF32Params p) {
   extern __shared__ float4 sm4[];
@@ -192,8 +194,13 @@ attn_f32_fwd(const AttnF32Params p) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
   pdl_launch_dependents();
-  const int qt = p.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x;    // the longest rows start first
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / (p.Hq / p.Hkv), row0 = qt * kFBM;
+  // The key tiles of the rows are dealt out to the CTAs of a cluster (one, two or four).  The units go by the length of their rows, all
+  // heads of the longest first, so that the last ones to find an SM are the shortest (B200, causal, 12 heads of 64: 509 tokens 41.5 us
+  // with the rows of each head together, 31.1 us so; 1024 tokens 96.5 and 80.3 us).
+  const int nc = SHARED ? p.key_ctas : 1, rank = SHARED ? blockIdx.x % nc : 0, unit = blockIdx.x / nc;
+  const int qx = unit / (p.B * p.Hq), bh = unit - qx * p.B * p.Hq;
+  const int qt = p.causal ? (p.Sq + kFBM - 1) / kFBM - 1 - qx : qx;     // the longest rows of all heads start first
+  const int b = bh / p.Hq, h = bh - b * p.Hq, hk = h / (p.Hq / p.Hkv), row0 = qt * kFBM;
   f32_load_tile<HD, kFBM>(Qs, p.q, b, h, row0, p.Sq, p.hd, p.vec);
   float m[4], l[4], o[4][N];
 #pragma unroll
@@ -207,18 +214,19 @@ attn_f32_fwd(const AttnF32Params p) {
   // K and V have a buffer each; a tile is requested as soon as its buffer has been read, so that it arrives under the other
   // product.  (The time of a key tile was that of fetching it: B200, causal, 12 heads of 64, 509 tokens: 51.6 us with
   // plain loads between two barriers, 42.3 us so; 256 tokens 22.3 and 16.3 us; 6 heads of 128, 509 tokens 73.5 and 49.0 us.)
-  if (tiles > 0) {
-    f32_request_tile<HD, kFBN>(Ks, p.k, b, hk, 0, p.Sk, p.hd, p.vec);
-    f32_request_tile<HD, kFBN>(Vs, p.v, b, hk, 0, p.Sk, p.hd, p.vec);
+  if (rank < tiles) {
+    f32_request_tile<HD, kFBN>(Ks, p.k, b, hk, rank * kFBN, p.Sk, p.hd, p.vec);
+    f32_request_tile<HD, kFBN>(Vs, p.v, b, hk, rank * kFBN, p.Sk, p.hd, p.vec);
   }
-  for (int t = 0; t < tiles; ++t) {
-    const int key0 = t * kFBN;
+  for (int t = rank; t < tiles; t += nc) {
+    const int key0 = t * kFBN, next0 = key0 + nc * kFBN;
+    const bool more = t + nc < tiles;
     asm volatile("cp.async.wait_group 1;" ::: "memory");      // all but the V tile
     __syncthreads();
     float s[4][4];
     f32_tile_dot<HD>(Qs, Ks, ty, tx, s);
     __syncthreads();
-    if (t + 1 < tiles) f32_request_tile<HD, kFBN>(Ks, p.k, b, hk, key0 + kFBN, p.Sk, p.hd, p.vec);
+    if (more) f32_request_tile<HD, kFBN>(Ks, p.k, b, hk, next0, p.Sk, p.hd, p.vec);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = row0 + ty * 4 + i;
@@ -243,12 +251,47 @@ attn_f32_fwd(const AttnF32Params p) {
         Ps[(ty * 4 + i) * LW + tx + 16 * j] = e;
       }
     }
-    if (t + 1 < tiles) asm volatile("cp.async.wait_group 1;" ::: "memory");      // all but the next K tile
+    if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");      // all but the next K tile
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();       // (a row's weights are written and read by the same half warp)
     f32_tile_acc<HD>(Ps, Vs, ty, tx, o);
     __syncthreads();
-    if (t + 1 < tiles) f32_request_tile<HD, kFBN>(Vs, p.v, b, hk, key0 + kFBN, p.Sk, p.hd, p.vec);
+    if (more) f32_request_tile<HD, kFBN>(Vs, p.v, b, hk, next0, p.Sk, p.hd, p.vec);
+  }
+  if constexpr (SHARED) {
+    // Each CTA leaves its weighted sums, maxima and sums in shared memory (the tiles are idle by now); every one finishes an equal share
+    // of the rows, in the order of the CTAs.
+    cg::cluster_group cluster = cg::this_cluster();
+    float* Os = Ks;                    // [kFBM][LD]
+    float* Ms = Os + kFBM * LD;        // [kFBM] maximum, [kFBM] sum
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = ty * 4 + i;
+#pragma unroll
+      for (int c = 0; c < N; ++c) Os[r * LD + f32_col<HD>(tx, c)] = o[i][c];
+      const float sum = half_warp_sum(l[i]);
+      if (tx == 0) {
+        Ms[r] = m[i];
+        Ms[kFBM + r] = sum;
+      }
+    }
+    cluster.sync();
+    for (int i = rank * kFThreads + threadIdx.x; i < kFBM * HD; i += nc * kFThreads) {
+      const int r = i / HD, d = i % HD, row = row0 + r;
+      if (row >= p.Sq || d >= p.hd) continue;
+      float mx = -INFINITY, x = 0.f, sum = 0.f;
+      for (int c = 0; c < nc; ++c) mx = fmaxf(mx, cluster.map_shared_rank(Ms, c)[r]);
+      const float sub = mx == -INFINITY ? 0.f : mx;
+      for (int c = 0; c < nc; ++c) {
+        const float w = expf(cluster.map_shared_rank(Ms, c)[r] - sub);
+        x = fmaf(w, cluster.map_shared_rank(Os, c)[r * LD + d], x);
+        sum = fmaf(w, cluster.map_shared_rank(Ms, c)[kFBM + r], sum);
+      }
+      p.o.p[b * p.o.sb + row * p.o.ss + h * p.o.sh + d] = x * (1.f / sum);
+      if (p.lse && d == 0) p.lse[((long long)b * p.Hq + h) * p.Sq + row] = mx + logf(sum);
+    }
+    cluster.sync();                    // nobody leaves while its shared memory is being read
+    return;
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -613,6 +656,17 @@ template <int HD> constexpr int f32_smem(int hd_rows, int w_rows) {
   return (hd_rows * f32_ld<HD>() + w_rows * (kFBN + 4)) * 4;
 }
 
+// CTAs for the keys of a row tile: 1, 2 or 4, by what the longest rows weigh in even shares of the key tiles (see the launch).
+static int f32_key_ctas(const AttnF32Params& p, bool wide) {
+  const int qtiles = (p.Sq + kFBM - 1) / kFBM, longest = f32_key_tiles(p, (qtiles - 1) * kFBM);
+  const long long heads = (long long)p.Hq * p.B, room = (long long)longest * sm_count();
+  if (longest < 4 || heads * qtiles > room) return 1;
+  long long work = 0;
+  for (int t = 0; t < qtiles; ++t) work += heads * f32_key_tiles(p, t * kFBM);
+  if (room >= 2 * work) return 4;
+  return longest >= 8 && (wide ? 4 * room >= 5 * work : room >= work) ? 2 : 1;
+}
+
 template <int HD>
 static int attn_f32_launch(const AttnF32Params& p, int backward, cudaStream_t st) {
   const dim3 qgrid((p.Sq + kFBM - 1) / kFBM, p.Hq, p.B);
@@ -641,8 +695,36 @@ static int attn_f32_launch(const AttnF32Params& p, int backward, cudaStream_t st
       return counted(1, (int)cudaLaunchKernelEx(&cfg, attn_f32_decode<HD>, p));
     }
     const int smem = f32_smem<HD>(kFBM + 2 * kFBN, kFBM);
-    DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_fwd<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    return counted(1, (int)launch_k(attn_f32_fwd<HD>, qgrid, dim3(kFThreads), (size_t)smem, st, p));
+    // The time of a launch is that of the SM with the most key tiles: one CTA keeps an SM's shared memory busy, two at once take twice as
+    // long (3.1 us a tile at heads of 64).  Where the longest rows weigh as much as an SM's even share of the tiles, two CTAs divide
+    // them, and four where they weigh twice as much; each CTA more costs 2 to 3 us of meeting, so that shorter rows stay whole.  B200,
+    // one / two / four CTAs, causal: 12 heads of 64, 509 tokens 31.1 / 28.5 / 32.2 us (longest rows 1.4 even shares), 256 tokens
+    // 16.0 / 17.3 / 14.2 (2.5), 2 x 512 tokens 43.0 / 47.9 / 52.2 (0.7); 8 heads of 32, 512 tokens 19.7 / 16.4 / 13.6 (2.1); heads of
+    // 128, of which an SM holds two: 2 heads, 1024 tokens 92.4 / 58.8 / 38.8 (4.3), 10 heads, 512 tokens 51.6 / 46.6 / 58.5 (1.6),
+    // 16 heads 60.4 / 70.2 / 85.0 (1.0).
+    AttnF32Params s = p;
+    s.key_ctas = f32_key_ctas(p, HD > 64);
+    const long long ctas = (long long)qgrid.x * qgrid.y * qgrid.z;
+    const dim3 grid((unsigned)(ctas * s.key_ctas));
+    if (s.key_ctas == 1) {
+      DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_fwd<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      return counted(1, (int)launch_k(attn_f32_fwd<HD, false>, grid, dim3(kFThreads), (size_t)smem, st, s));
+    }
+    DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_fwd<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kFThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = s.key_ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl_flag() ? 2 : 1;
+    return counted(1, (int)cudaLaunchKernelEx(&cfg, attn_f32_fwd<HD, true>, s));
   }
   const int smem_q = f32_smem<HD>(2 * kFBM + 2 * kFBN, kFBM), smem_kv = f32_smem<HD>(2 * kFBM + 2 * kFBN, 2 * kFBM);
   DPTB_CUDA_OK(cudaFuncSetAttribute(attn_f32_dq<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));
@@ -676,6 +758,7 @@ static int attn_f32(const DptbAttnF32Args* a, const DptbF32View* kn, const DptbF
   p.kn = kn ? F32View{kn->p, kn->sb, kn->ss, kn->sh} : F32View{};
   p.vn = vn ? F32View{vn->p, vn->sb, vn->ss, vn->sh} : F32View{};
   p.appended = kn ? a->Sk - a->Sq : a->Sk;
+  p.key_ctas = 1;
   p.lse = a->lse;
   p.delta = a->delta;
   p.B = a->B; p.Sq = a->Sq; p.Sk = a->Sk; p.Hq = a->Hq; p.Hkv = a->Hkv; p.hd = a->hd;

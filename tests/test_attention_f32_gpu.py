@@ -112,3 +112,45 @@ def test_non_finite_operands(Sq, Sk, causal, H, Hkv, hd, what, at):
     assert torch.equal(o.isnan(), ref.isnan()) and torch.equal(o.isinf(), ref.isinf())
     fin = ref.isfinite()
     assert torch.equal(o[ref.isinf()].double(), ref[ref.isinf()]) and torch.allclose(o[fin].double(), ref[fin], rtol=1e-5, atol=1e-5)
+
+
+# Row tiles whose keys several CTAs divide: four (few rows; the first causal rows leave some without a key tile) and two (as many
+# rows as the chip has SMs), the fewest tiles that are divided, ragged ends, offsets and odd head sizes.  The bound is that above: the
+# parts meet in at most four more products and sums.
+@pytest.mark.parametrize("B,H,Hkv,Sq,Sk,hd,causal,off", [
+    (1, 2, 2, 193, 193, 64, True, 0), (1, 2, 1, 257, 257, 32, False, 0), (2, 3, 3, 64, 450, 10, True, 386), (1, 1, 1, 33, 511, 128, False, 0),
+    (1, 12, 12, 481, 481, 64, True, 0), (1, 10, 5, 509, 513, 64, False, 0), (1, 6, 2, 1000, 1000, 128, True, 0), (1, 16, 16, 449, 449, 16, True, 0)])
+@pytest.mark.parametrize("what", ["finite", "value inf", "value -inf", "key nan", "scores -inf", "most scores -inf"])
+def test_rows_with_shared_keys(B, H, Hkv, Sq, Sk, hd, causal, off, what):
+    g = torch.Generator(device="cuda").manual_seed(Sk)
+    q, k, v = (torch.randn(B, h, s, hd, device="cuda", generator=g) for h, s in ((H, Sq), (Hkv, Sk), (Hkv, Sk)))
+    q[..., 3] = 1.0
+    kind, _, x = what.rpartition(" ")
+    if kind == "value":
+        v[:, :, Sk // 2, 5] = float(x)
+    elif kind == "key":
+        k[:, :, Sk // 2, 3] = float(x)
+    elif kind == "scores":
+        k[:, :, 0, 3] = float("-inf")
+    elif kind:
+        k[:, :, 70:, 3] = float("-inf")
+    o = A.attention_bhsd(q, k, v, causal, None, off)
+    ref = _exact(q.double(), k.double(), v.double(), causal, off)
+    if kind == "value":      # a weight of zero times the value: rows that do not see the key are exact without it
+        i = torch.arange(Sq, device="cuda") + off
+        seen = i >= Sk // 2 if causal else torch.ones_like(i, dtype=torch.bool)
+        v[:, :, Sk // 2, 5] = 0.0
+        ref = _exact(q.double(), k.double(), v.double(), causal, off)
+        assert torch.equal(o[:, :, seen, 5], torch.full_like(o[:, :, seen, 5], float(x)))
+        o, ref = o.clone(), ref.clone()
+        o[..., 5] = ref[..., 5].float()
+    assert torch.equal(o.isnan(), ref.isnan())
+    fin = ref.isfinite()
+    assert float((o.double() - ref)[fin].norm()) <= 3e-6 * float(ref[fin].norm())
+    if what == "finite":
+        a = [t.requires_grad_(True) for t in (q, k, v)]
+        d = [t.detach().double().requires_grad_(True) for t in a]
+        do = torch.randn(o.shape, device="cuda", generator=g)
+        got = torch.autograd.grad(A.attention_bhsd(*a, causal, None, off), a, do)
+        for x, y in zip(got, torch.autograd.grad(_exact(*d, causal, off), d, do.double())):
+            assert float((x.double() - y).norm() / y.norm()) < 3e-6
