@@ -18,7 +18,10 @@
 //   warp 8           TMA producer (Q once a unit, K / V through rings); it runs ahead into the next unit
 //   warps 9, 10      MMA issuers, one per query tile: S_t = Q_t K_j^T, and O_t += P_t V_j accumulated in TMEM
 // The two query tiles meet nowhere but at the rings: with one issuer for both, which waits for them in turn, the softmax
-// warpgroups ran in step and wanted the special-function unit at the same time.  The output accumulator never leaves TMEM during the loop.  The running maximum is lazy: a row keeps exponentiating
+// warpgroups ran in step and wanted the special-function unit at the same time.  B200, a layer, one CTA a unit and one issuer / persistent
+// and two: 16 x 1024 causal, 12 heads of 64 93.4 / 69.6 us, 128 x 197 105 / 78 us, 4 x 2048 causal, 16 heads of 128 131 / 89 us.  What bounds
+// it now is the softmax of a tile: 1024 clocks of the special-function unit a warpgroup, two to a scheduler, beside conversions
+// and shared-memory stores.  The output accumulator never leaves TMEM during the loop.  The running maximum is lazy: a row keeps exponentiating
 // against an older maximum until the true one has grown by more than 8 (a factor 256 of headroom in fp32 / bf16);
 // only then (decided per warp) O is pulled out, rescaled and stored back, which after the first tiles is rare.
 //
@@ -103,12 +106,15 @@ struct AttnFwdSmem {
 };
 
 // SUB: heads of fewer than HD features (a multiple of 8), read through maps with an axis of heads.
-template <int HD, int NQ, int KST, int VST, bool PREC, bool WIN, bool SUB>
+// HEADS: sequences of at most one query tile; the two query tiles of a unit are two heads, each with a K and a V stage and a producer
+// (warps 8 and 11) of its own, so that neither softmax warpgroup idles and neither head waits for the other.
+template <int HD, int NQ, int KST, int VST, bool PREC, bool WIN, bool SUB, bool HEADS>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmPK,
                 const __grid_constant__ CUtensorMap tmPV, const AttnFwdParams p) {
   using L = AttnFwdSmem<HD, NQ, KST, VST, PREC>;
+  static_assert(!HEADS || (!WIN && KST == NQ && VST == NQ), "a K and a V stage for each head");
   constexpr int kAttnBN = L::kBN;
   constexpr int kChunks = HD / 64;            // 64-column (128-byte) chunks per head row
   constexpr int TMEM_COLS = 512;
@@ -144,11 +150,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     int n_tiles[NQ];                    // KV tiles each query tile needs (0: it has no rows, or none that sees a key)
     int n_max, n_pool, tile0;           // with a window they start with n_pool tiles of pooled rows; first token tile
   };
-  const int per_block = p.Hq * p.B, num_units = p.num_q_blocks * per_block;
+  const int per_block = p.Hq * p.B, num_units = HEADS ? (per_block + 1) / 2 : p.num_q_blocks * per_block;
   const int num_rounds = (num_units + (int)gridDim.x - 1) / (int)gridDim.x;
-  auto get_unit = [&](int r, Unit& w) -> bool {
+  auto get_unit = [&](int r, int t_own, Unit& w) -> bool {       // (t_own: the role's query tile, which with HEADS decides the head)
     const int u = r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
     if (u >= num_units) return false;
+    if constexpr (HEADS) {
+      const int bh = 2 * u + t_own;
+      w.batch = bh / p.Hq;
+      w.head = bh - w.batch * p.Hq;
+      w.kv_head = w.head / (p.Hq / p.Hkv);
+      w.q_row0 = -t_own * kAttnBM;
+      const int last_key = p.causal ? min(p.Sk - 1, p.Sq - 1 + p.q_offset) : p.Sk - 1;
+      w.n_max = bh < per_block && last_key >= 0 ? last_key / kAttnBN + 1 : 0;
+      w.n_pool = w.tile0 = 0;
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) w.n_tiles[t] = w.n_max;
+      return true;
+    }
     const int qb = p.causal ? p.num_q_blocks - 1 - u / per_block : u % p.num_q_blocks;
     const int rest = p.causal ? u % per_block : u / p.num_q_blocks;
     w.head = rest % p.Hq;
@@ -199,11 +218,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       for (int s = 0; s < KST; ++s) {
         mbar_init(&k_full[s], 1);
-        mbar_init(&k_empty[s], NQ);        // both issuers let go of a stage
+        mbar_init(&k_empty[s], HEADS ? 1 : NQ);        // both issuers let go of a stage
       }
       for (int s = 0; s < VST; ++s) {
         mbar_init(&v_full[s], 1);
-        mbar_init(&v_empty[s], NQ);
+        mbar_init(&v_empty[s], HEADS ? 1 : NQ);
       }
       mbar_fence_init();
     }
@@ -218,14 +237,58 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   static_assert(NQ == 2, "warp roles assume two softmax warpgroups");
   if (warp >= 8) {
     warpgroup_reg_dec<kProducerRegs>();
-  if (warp == 8) {
+  if (HEADS && (warp == 8 || warp == 11)) {
+    // ------------------------------------------------------------------ TMA producer of one head
+    if (lane == 0) {
+      const int t = warp == 8 ? 0 : 1;
+      int units = 0, tiles = 0;
+      Unit w;
+      bool ok = true;
+      auto load = [&](const CUtensorMap* map, uint64_t* bar, int off, int bytes, int rows, int head, int row, int batch) {
+        mbar_arrive_expect_tx(bar, bytes);
+        for (int c = 0; c < kChunks; ++c) {
+          uint8_t* dst = smem + off + t * bytes + c * (rows * 128);
+          if constexpr (SUB) tma_load_4d(dst, map, bar, c * 64, head, row, batch);
+          else tma_load_3d(dst, map, bar, head * HD + c * 64, row, batch);
+        }
+      };
+      bool k_last = false, v_last = false;      // copies of the last tile have been requested
+      for (int r = 0; r < num_rounds && ok; ++r) {
+        if (!get_unit(r, t, w)) break;
+        if (w.n_max == 0) continue;
+        ok = mbar_wait(&q_empty[t], (units & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+        if (!ok) break;
+        load(&tmQ, &q_full[t], L::kQOff, L::kQBytes, kAttnBM, w.head, 0, w.batch);
+        ++units;
+        for (int j = 0; j < w.n_max; ++j, ++tiles) {
+          k_last = v_last = false;
+          ok = mbar_wait(&k_empty[t], (tiles & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+          if (!ok) break;
+          load(&tmK, &k_full[t], L::kKOff, L::kKVBytes, kAttnBN, w.kv_head, j * kAttnBN, w.batch);
+          k_last = true;
+          ok = mbar_wait(&v_empty[t], (tiles & 1) ^ 1, abort_flag, kWaitEmptyTimeout);
+          if (!ok) break;
+          load(&tmV, &v_full[t], L::kVOff, L::kKVBytes, kAttnBN, w.kv_head, j * kAttnBN, w.batch);
+          v_last = true;
+        }
+      }
+      if (*abort_flag) {
+        // As below.  `tiles` counts whole tiles: one whose K alone was requested is the one after them.
+        const uint64_t t0 = global_timer_ns();
+        const int nk = tiles + (k_last && !v_last ? 1 : 0);
+        while (units && !mbar_try_wait(&q_full[t], (units - 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+        while (nk && !mbar_try_wait(&k_full[t], (nk - 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+        while (tiles && !mbar_try_wait(&v_full[t], (tiles - 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
+      }
+    }
+  } else if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       int q_issued[NQ] = {}, k_issued = 0, v_issued = 0;
       Unit w;
       bool ok = true;
       for (int r = 0; r < num_rounds && ok; ++r) {
-        if (!get_unit(r, w)) break;
+        if (!get_unit(r, 0, w)) break;
 #pragma unroll
         for (int t = 0; t < NQ; ++t) {
           if (w.n_tiles[t] == 0 || !ok) continue;
@@ -293,7 +356,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int units = 0;
       Unit w;
       for (int r = 0; r < num_rounds && ok; ++r) {
-        if (!get_unit(r, w)) break;
+        if (!get_unit(r, t, w)) break;
         const int n = t == 0 ? w.n_tiles[0] : w.n_tiles[NQ - 1];
         if (n > 0) {
           ok = mbar_wait(&q_full[t], units & 1, abort_flag, kWaitFullTimeout);
@@ -302,8 +365,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         // Before tile j's P V, S of tile j + 1 as soon as the softmax warpgroup has copied the one before out of TMEM.
         for (int j = -1; j < w.n_max && ok; ++j) {
           if (j + 1 < w.n_max) {
-            const int ks = (kv + j + 1) % KST;
-            ok = mbar_wait(&k_full[ks], ((kv + j + 1) / KST) & 1, abort_flag, kWaitFullTimeout);
+            const int ks = HEADS ? t : (kv + j + 1) % KST;
+            ok = mbar_wait(&k_full[ks], HEADS ? tiles & 1 : ((kv + j + 1) / KST) & 1, abort_flag, kWaitFullTimeout);
             if (ok && j + 1 < n) {
               if (tiles > 0) ok = mbar_wait(&s_empty[t], (tiles - 1) & 1, abort_flag, kWaitTmemEmptyTimeout);
               if (!ok) break;
@@ -325,8 +388,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             umma_commit(&k_empty[ks]);
           }
           if (j < 0) continue;
-          const int vs = (kv + j) % VST;
-          ok = mbar_wait(&v_full[vs], ((kv + j) / VST) & 1, abort_flag, kWaitFullTimeout);
+          const int vs = HEADS ? t : (kv + j) % VST;
+          ok = mbar_wait(&v_full[vs], HEADS ? done & 1 : ((kv + j) / VST) & 1, abort_flag, kWaitFullTimeout);
           if (ok && j < n) {
             // O_t += P_t(j) V_j once P_t(j) is in shared memory (and, for j = 0, the unit before has been read out of O_t)
             const int pb = t * L::kPBufs + done % L::kPBufs;
@@ -382,7 +445,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const long long prof_begin = clock64();
 #endif
     for (int r = 0; r < num_rounds && ok; ++r) {
-    if (!get_unit(r, w)) break;
+    if (!get_unit(r, t, w)) break;
     const int q_row = w.q_row0 + t * kAttnBM + row_in_tile;       // row inside the sequence
     const int n = t == 0 ? w.n_tiles[0] : w.n_tiles[NQ - 1];
     const int head = w.head, batch = w.batch;
@@ -482,7 +545,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           // (Computing half of the exponentials as cubic polynomials on the FMA pipe was measured slower here: 117 us
           // against 102 us at B16 H12 S1024 hd64; the softmax warps are bound by issue slots, not by the
           // special-function unit.  Taking the exponentials two at a time in bf16, ex2.approx.bf16x2, was slower as
-          // well, 115 us, for the unpacking its row sum needs.)
+          // well, 115 us, for the unpacking its row sum needs.  Both with one issuer for the two query tiles.)
           float a, b, e, f;
           f2_unpack(f2_fma(f2_pack(__uint_as_float(s[c * 32 + i]), __uint_as_float(s[c * 32 + i + 1])), scale2, neg_m2), a, b);
           f2_unpack(f2_fma(f2_pack(__uint_as_float(s[c * 32 + i + 2]), __uint_as_float(s[c * 32 + i + 3])), scale2, neg_m2), e, f);
@@ -616,8 +679,8 @@ static int encode_tmap_heads(CUtensorMap* map, const void* base, int heads, int 
 }
 
 // One CTA an SM (shared memory and TMEM allow no more), or one a unit.
-static int attn_grid(const AttnFwdParams& p) {
-  const long long units = (long long)p.num_q_blocks * p.Hq * p.B;
+static int attn_grid(const AttnFwdParams& p, bool heads = false) {
+  const long long units = heads ? ((long long)p.Hq * p.B + 1) / 2 : (long long)p.num_q_blocks * p.Hq * p.B;
   return units < sm_count() ? (int)units : sm_count();
 }
 
@@ -625,7 +688,7 @@ static int attn_grid(const AttnFwdParams& p) {
 
 using namespace dptb;
 
-template <int HD, int NQ, int KST, int VST, bool PREC, bool SUB>
+template <int HD, int NQ, int KST, int VST, bool PREC, bool SUB, bool HEADS = false>
 static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   using L = AttnFwdSmem<HD, NQ, KST, VST, PREC>;
   constexpr int kAttnBN = L::kBN;
@@ -651,9 +714,9 @@ static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   p.q_offset = a->q_offset;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   p.num_q_blocks = (a->Sq + NQ * kAttnBM - 1) / (NQ * kAttnBM);
-  auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false, SUB>;
+  auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false, SUB, HEADS>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  kern<<<attn_grid(p), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
+  kern<<<attn_grid(p, HEADS), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
   return counted(1, (int)cudaGetLastError());
 }
 
@@ -681,10 +744,17 @@ extern "C" int dptb_attn_fwd(const DptbAttnFwdArgs* a, void* stream) {
     if (a->head_dim == 128) return attn_fwd_launch<128, 2, 3, 3, true, false>(a, st);
     return kErrUnsupported;
   }
+  // Sequences of one query tile: two heads a CTA once there are more heads than SMs; below, each has an SM to itself.  (There is no room
+  // for a second V stage beside heads of 128.)  A unit is one chain of loads, scores, softmax and P V, of which the other warpgroup saw
+  // nothing.  B200, one head a CTA (which then came and went) / two: 64 x 119 tokens, 12 heads of 32 31.1 / 16.6 us (26.5 with one
+  // head in the persistent form), of 64 33.6 / 19.9; 200 x 64, 8 heads of 64 58.6 / 28.2; 13 x 17, 12 heads of 32 10.3 / 7.2 us.
+  const bool heads = a->Sq <= kAttnBM && (long long)a->Hq * a->B > sm_count();
+  if (a->head_dim == 64 && heads) return attn_fwd_launch<64, 2, 2, 2, false, false, true>(a, st);
   if (a->head_dim == 64) return attn_fwd_launch<64, 2, 2, 2, false, false>(a, st);
   if (a->head_dim == 128) return attn_fwd_launch<128, 2, 2, 1, false, false>(a, st);
   // Other sizes: the maps have an axis of heads, so a box of 64 features reads zeros behind a head's own.  Padding copies
   // of Q, K and V cost more than the attention on them: 64 x 119 tokens, 12 heads of 32, B200, 74 us with them, 32 us so.
+  if (a->head_dim > 0 && a->head_dim % 8 == 0 && a->head_dim < 64 && heads) return attn_fwd_launch<64, 2, 2, 2, false, true, true>(a, st);
   if (a->head_dim > 0 && a->head_dim % 8 == 0 && a->head_dim < 64) return attn_fwd_launch<64, 2, 2, 2, false, true>(a, st);
   if (a->head_dim % 8 == 0 && a->head_dim > 64 && a->head_dim < 128) return attn_fwd_launch<128, 2, 2, 1, false, true>(a, st);
   return kErrUnsupported;
@@ -726,7 +796,7 @@ static int window_fwd_launch(const DptbWindowFwdArgs* a, cudaStream_t st) {
   p.window = a->window; p.pool = a->pool; p.pool_rows = a->pool_rows; p.pos = a->pos; p.dv = a->dv;
   p.sink = static_cast<const __nv_bfloat16*>(a->sink);
   p.rot = static_cast<const float2*>(a->rot);
-  auto kern = attn_fwd_kernel<HD, 2, KST, VST, true, true, false>;
+  auto kern = attn_fwd_kernel<HD, 2, KST, VST, true, true, false, false>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
   kern<<<attn_grid(p), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmPK, tmPV, p);
   return counted(1, (int)cudaGetLastError());

@@ -133,7 +133,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Launches `kern`, as a programmatic dependent of the previous kernel on the stream when pdl_flag() is set.  Such a
 // kernel calls pdl_wait() before its first global access and pdl_launch_dependents() after it, never before: the kernel
 // after it must not start while the kernel two places back is still running.  Two exceptions.  The weight-streaming products
-// (gemm_skinny.cu, the rows of gemm_f32.cu) request their second operand before the wait.  So no kernel of a chain may write what
+// (gemm_skinny.cu, gemm_f32_tc.cu, the rows of gemm_f32.cu) request their second operand before the wait.  So no kernel of a chain may write what
 // a product in it takes as weight; a caller whose second operand is computed leaves the flag off around it.  And decoding attention
 // requests cache rows before this step's own (attention_decode.cu, the appending form of attention_f32.cu): they are written at least
 // two kernels before it.
