@@ -270,14 +270,13 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
 // stacks of 3 layers, widths 128 to 2048, 1 to 64 rows as one prompt and as one token each over 100 (B200, one graph a step):
 //   bf16   1.0 to 1.15 times as fast up to 64 rows, where the weight-streaming products end; from 65 to 1024 rows the products and
 //          the attention are no dependents, and the time is the same within 1 %.
-//   fp32   1.02 to 1.17 times as fast up to 8 rows (the streaming products).  With more rows a product is tiles and splits of K, which
-//          wait without having requested anything: 1.02 to 1.11 times as fast where they are few (widths 128 and 256 up to 64 rows, 384
-//          up to 32), but 0.94 with 48 and 64 rows of width 384 and 0.85 to 1.03 from width 512 on (24 rows of width 768: 0.86 as a
-//          prompt, 0.92 as one token each).
-constexpr long long kChainedRows = 64, kStreamedRowsF32 = 8;
+//   fp32   (stacks of 4 layers, as called) 1.05 to 1.37 times as fast at 1 to 64 rows of widths 128 to 1024, since the products on tensor
+//          cores request their first weights before the wait; 1.18 to 1.28 at 72 to 128 rows of widths up to 768, 1.20 at 256 rows of
+//          384; then less: 1.03 (a prompt) and 1.14 (one token each) at 256 rows of 768, 0.91 and 1.07 at 509.
+constexpr long long kChainedRows = 64, kChainedRowsF32 = 256, kChainedAreaF32 = 128 * 1024;
 static bool chained(const DptbStackArgs* a) {
   const long long rows = (long long)a->B * a->S;
-  return rows <= kChainedRows && (a->bf16 || rows <= kStreamedRowsF32 || (a->D <= 384 && rows * a->D <= 16384));
+  return a->bf16 ? rows <= kChainedRows : rows <= kChainedRows || (rows <= kChainedRowsF32 && rows * a->D <= kChainedAreaF32);
 }
 extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table, void* stream) {
   int& pdl = pdl_flag();

@@ -1,4 +1,4 @@
-"""Few fp32 rows through the native stack (norms inside the products, the cache append inside the attention) against the modules' own
+"""Few fp32 rows through the native stack (a chain of dependent launches, the cache append inside the attention) against the modules' own
 forward passes: the same bits, in the hidden states and in the caches."""
 import pytest
 import torch
@@ -61,6 +61,20 @@ def test_llama(monkeypatch, B):
                           device="cuda", dtype=torch.float32, init_std=0.05)).eval()
     toks = torch.randint(0, 97, (B, 68), device="cuda")
     _both(monkeypatch, lambda: _steps(m, m.new_cache(), toks, 62))
+
+
+# Both ends of the chained steps; every repetition gives the same bits.
+@pytest.mark.parametrize("width,heads", [(128, 2), (512, 8), (1024, 16)])
+@pytest.mark.parametrize("B,n", [(1, 24), (33, 1), (1, 64), (5, 13), (128, 1), (1, 129), (2, 128), (257, 1)])
+def test_chained_steps(monkeypatch, width, heads, B, n):
+    m = dp.GPT(dp.GPTConfig(vocab_size=97, max_ctx=300, embed_dim=width, num_layers=3, num_heads=heads, ffn_dim=4 * width, attn_bias=True,
+                            activation=Activation.geluTanh, device="cuda", dtype=torch.float32, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (B, n + 2), device="cuda")
+    run = lambda: _steps(m, EncoderCache.empty(3, heads, max_len=300), toks, n)
+    _both(monkeypatch, run)
+    first = run()
+    for _ in range(10):
+        assert all(torch.equal(x, y) for x, y in zip(first, run()))
 
 
 def test_infinities_and_nan(monkeypatch):
