@@ -233,6 +233,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                // (programmatic dependent launch: no-ops in an ordinary launch)
+  pdl_launch_dependents();
 
   static_assert(NQ == 2, "warp roles assume two softmax warpgroups");
   if (warp >= 8) {
@@ -716,8 +718,7 @@ static int attn_fwd_launch(const DptbAttnFwdArgs* a, cudaStream_t st) {
   p.num_q_blocks = (a->Sq + NQ * kAttnBM - 1) / (NQ * kAttnBM);
   auto kern = attn_fwd_kernel<HD, NQ, KST, VST, PREC, false, SUB, HEADS>;
   DPTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  kern<<<attn_grid(p, HEADS), kAttnThreads, L::kTotal, st>>>(tmQ, tmK, tmV, tmK, tmV, p);
-  return counted(1, (int)cudaGetLastError());
+  return counted(1, (int)launch_k(kern, dim3(attn_grid(p, HEADS)), dim3(kAttnThreads), (size_t)L::kTotal, st, tmQ, tmK, tmV, tmK, tmV, p));
 }
 
 // Phase timers (see DPTB_ATTN_PROFILE): copies the 8 counters out and zeroes them; -5 when not compiled in.

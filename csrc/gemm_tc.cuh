@@ -946,6 +946,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   else __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // Programmatic dependent launch (no-ops in an ordinary one).  The forms with a collective are launched as usual and let nobody start
+  // early: the kernel after them may read the protocol's counters before its own wait.
+  pdl_wait();
+  if (!AG && p.ar.world == 0) pdl_launch_dependents();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -1574,6 +1578,8 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams 
   const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   p.fold_all = p.splits > 1 && tiles <= grid;
+  if (p.ar.world == 0)
+    return counted(1, (int)launch_k(kern, dim3(grid), dim3(kGemmThreads), (size_t)L::kTotal, stream, tmA, tmB, NoPeerMaps{}, EpiMaps{}, p));
   kern<<<grid, kGemmThreads, L::kTotal, stream>>>(tmA, tmB, NoPeerMaps{}, EpiMaps{}, p);
   return counted(1, (int)cudaGetLastError());
 }
@@ -1611,7 +1617,7 @@ static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
                           cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES, BN / 2, 2>;
   auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true, GLU>;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -1628,6 +1634,9 @@ static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   const int clusters = units < max_clusters ? units : max_clusters;
   cfg.gridDim = dim3(2 * clusters);
   p.fold_all = p.splits > 1 && units <= clusters;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  if (pdl_flag()) cfg.numAttrs = 2;
   return counted(1, (int)cudaLaunchKernelEx(&cfg, kern, tmA, tmB, NoPeerMaps{}, em, p));
 }
 

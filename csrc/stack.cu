@@ -265,18 +265,19 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
   return 0;
 }
 
-// A step of few rows is a chain of short kernels: those that support it start as programmatic dependents of one another, so
-// their set-up (and the first weights of the matrix products) overlaps the end of the kernel before.  Which steps gain was measured on
-// stacks of 3 layers, widths 128 to 2048, 1 to 64 rows as one prompt and as one token each over 100 (B200, one graph a step):
-//   bf16   1.0 to 1.15 times as fast up to 64 rows, where the weight-streaming products end; from 65 to 1024 rows the products and
-//          the attention are no dependents, and the time is the same within 1 %.
-//   fp32   (stacks of 4 layers, as called) 1.05 to 1.37 times as fast at 1 to 64 rows of widths 128 to 1024, since the products on tensor
-//          cores request their first weights before the wait; 1.18 to 1.28 at 72 to 128 rows of widths up to 768, 1.20 at 256 rows of
-//          384; then less: 1.03 (a prompt) and 1.14 (one token each) at 256 rows of 768, 0.91 and 1.07 at 509.
-constexpr long long kChainedRows = 64, kChainedRowsF32 = 256, kChainedAreaF32 = 128 * 1024;
+// The kernels of a step start as programmatic dependents of one another, so that their set-up, and the first weights of the products of few
+// rows, overlap the end of the kernel before.  Which steps gain was measured as called, with and without (B200):
+//   bf16   1.0 to 1.15 times as fast up to 64 rows (stacks of 3 layers, widths 128 to 2048, a prompt and one token each); beyond, products
+//          and attention wait at their top: 64 x 119 tokens of width 384 693 -> 606 us, 300 tokens of width 2048 946 -> 832, 128 tokens
+//          over 300 each 737 -> 607, 256 x 119 of width 384 1730 -> 1673, but 4 x 2048 of width 2048 4545 -> 4568.
+//   fp32   (stacks of 4 layers) 1.05 to 1.37 times as fast at 1 to 64 rows of widths 128 to 1024, 1.18 to 1.28 at 72 to 128 rows of widths
+//          up to 768; sequences of up to 128: 1.15 at 8 x 119 rows of 384, 1.07 at 509 tokens, one each, of 768.  Longer sequences: 1.18
+//          at 256 rows of 384, but 0.91 at 509 of 768, where all rows have the same keys: CTAs that start where an SM is free crowd on the
+//          first ones.  Causal rows, the longest first, stand that better: 1.03.
+constexpr long long kChainedArea = 12 << 20, kChainedAreaF32 = 384 << 10, kChainedAreaF32Long = 128 << 10;
 static bool chained(const DptbStackArgs* a) {
-  const long long rows = (long long)a->B * a->S;
-  return a->bf16 ? rows <= kChainedRows : rows <= kChainedRows || (rows <= kChainedRowsF32 && rows * a->D <= kChainedAreaF32);
+  const long long area = (long long)a->B * a->S * a->D;
+  return area <= (a->bf16 ? kChainedArea : a->causal || a->S <= 128 ? kChainedAreaF32 : kChainedAreaF32Long);
 }
 extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table, void* stream) {
   int& pdl = pdl_flag();

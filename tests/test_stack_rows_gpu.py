@@ -1,4 +1,4 @@
-"""Few fp32 rows through the native stack (a chain of dependent launches, the cache append inside the attention) against the modules' own
+"""Steps through the native stack (a chain of dependent launches, the cache append inside the attention) against the modules' own
 forward passes: the same bits, in the hidden states and in the caches."""
 import pytest
 import torch
@@ -75,6 +75,23 @@ def test_chained_steps(monkeypatch, width, heads, B, n):
     first = run()
     for _ in range(10):
         assert all(torch.equal(x, y) for x, y in zip(first, run()))
+
+
+# bf16 prompts on both sides of the longest chain (12 M activations): tiled products and attention as dependents, several query tiles and
+# two heads a CTA.
+@pytest.mark.parametrize("width,heads,B,n", [(384, 12, 8, 119), (384, 6, 1, 300), (768, 12, 3, 65), (1024, 16, 16, 128), (2048, 16, 47, 128)])
+def test_chained_bf16_prompts(monkeypatch, width, heads, B, n):
+    m = dp.GPT(dp.GPTConfig(vocab_size=97, max_ctx=300, embed_dim=width, num_layers=3, num_heads=heads, ffn_dim=2 * width, attn_bias=True,
+                            activation=Activation.geluTanh, device="cuda", dtype=torch.bfloat16, init_std=0.05)).eval()
+    toks = torch.randint(0, 97, (B, n), device="cuda")
+
+    def run():
+        with torch.no_grad():
+            return [m.hidden(toks)]
+    _both(monkeypatch, run)
+    first = run()
+    for _ in range(10):
+        assert torch.equal(first[0], run()[0])
 
 
 def test_infinities_and_nan(monkeypatch):
