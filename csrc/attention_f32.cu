@@ -275,7 +275,7 @@ attn_f32_fwd(const AttnF32Params p) {
         Ms[kFBM + r] = sum;
       }
     }
-    cluster.sync();
+    cluster_sync_all();
     for (int i = rank * kFThreads + threadIdx.x; i < kFBM * HD; i += nc * kFThreads) {
       const int r = i / HD, d = i % HD, row = row0 + r;
       if (row >= p.Sq || d >= p.hd) continue;
@@ -290,7 +290,7 @@ attn_f32_fwd(const AttnF32Params p) {
       p.o.p[b * p.o.sb + row * p.o.ss + h * p.o.sh + d] = x * (1.f / sum);
       if (p.lse && d == 0) p.lse[((long long)b * p.Hq + h) * p.Sq + row] = mx + logf(sum);
     }
-    cluster.sync();                    // nobody leaves while its shared memory is being read
+    cluster_sync_all();                // nobody leaves while its shared memory is being read
     return;
   }
 #pragma unroll
@@ -455,7 +455,7 @@ attn_f32_decode(const AttnF32Params p) {
     }
     __syncthreads();
   }
-  cluster.sync();
+  cluster_sync_all();
   for (int i = rank * kFThreads + tid; i < rows * p.hd; i += nc * kFThreads) {
     const int r = i / p.hd, d = i % p.hd;
     float mx = -INFINITY;
@@ -471,7 +471,7 @@ attn_f32_decode(const AttnF32Params p) {
     p.o.p[b * p.o.sb + row * p.o.ss + h * p.o.sh + d] = x / sum;
     if (p.lse && d == 0) p.lse[((long long)b * p.Hq + h) * p.Sq + row] = sub + logf(sum);
   }
-  cluster.sync();          // nobody leaves while its shared memory is being read
+  cluster_sync_all();      // nobody leaves while its shared memory is being read
 }
 
 // -------------------------------------------------------------------------------------------------------------- backward

@@ -198,6 +198,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result) {
 }
 template <int kCols>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {
+  __syncwarp();      // .aligned: by the whole warp at once, wherever its lanes come from
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kCols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before_sync() {
@@ -275,8 +276,11 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// All threads of all CTAs of the cluster: arrive, then wait (orders shared-memory writes, e.g. barrier initialisation).
+// All threads of all CTAs of the cluster: arrive, then wait (orders shared-memory writes, e.g. barrier initialisation).  The
+// .aligned forms are undefined in a warp whose lanes arrive apart (after a role of one lane, after a loop that lanes leave in different
+// rounds): an arrival counted twice would let a CTA leave while others read its shared memory.  So the warp meets first.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -309,6 +313,7 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result) {
 }
 template <int kCols>
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kCols) : "memory");
 }
 // D[tmem of both CTAs] (+)= A * B with M = 256 (128 rows per CTA), issued by ONE thread of the leader CTA.

@@ -192,6 +192,7 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
         while (!mbar_try_wait(&done[(issued - 1) & 1], ((issued - 1) >> 1) & 1) && global_timer_ns() - t0 < kWaitLimitNs / 4) {}
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ fetch, split, add
     const uint32_t t_row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (warp >> 2) * COLS;

@@ -318,10 +318,7 @@ gemm_skinny_local_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
       }
     }
   }
-  if (p.splits > 1) {        // no CTA leaves while another reads its sums
-    __syncwarp();
-    cluster_sync_all();
-  }
+  if (p.splits > 1) cluster_sync_all();        // no CTA leaves while another reads its sums
 }
 
 template <int MP, int ST>
