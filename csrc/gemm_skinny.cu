@@ -7,7 +7,7 @@
 // useful bytes) and one slice of K; x is the narrow N = 32 / 64 side.  Work units = (N / 128) x (K splits) are chosen
 // to fill the SMs once, with TMA rings of 128 to 160 KB of W in flight per SM.  D[128 weight rows, M] lands
 // in 32 / 64 TMEM columns; a thread of the four epilogue warps owns one weight row = one output column.
-// The K splits of a tile (up to 8) are the CTAs of a cluster: each leaves its fp32 sums in its own shared memory and every one adds
+// The K splits of a tile (up to 16) are the CTAs of a cluster: each leaves its fp32 sums in its own shared memory and every one adds
 // an equal share of the outputs, in split order, and runs the epilogue on it.  Through a workspace in global memory, with the last
 // unit of a tile folding all of it, a split product took about 2 us more.
 // GLU: W holds F rows of gates and then F rows of values; a CTA's 128 rows are 64 gates and the 64 values that go with them.
@@ -104,7 +104,7 @@ __device__ __forceinline__ uint4 ld_relaxed_sys_v4(const uint2* p) {
   return v;
 }
 
-constexpr int kSkMaxSplits = 8;      // CTAs of a cluster
+constexpr int kSkMaxSplits = 16;     // CTAs of a cluster (above 8: allowed by attribute)
 struct SkinnyLocalParams {
   int M, N;                          // N: output columns (GLU: half the weight rows)
   __nv_bfloat16* C;
@@ -262,20 +262,23 @@ gemm_skinny_local_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] = 0.0f;
       if (p.splits > 1) {
-        float4 part[kSkMaxSplits][2];                      // all requested before the first is used
+#pragma unroll 1
+        for (int s0 = 0; s0 < p.splits; s0 += 8) {
+          float4 part[8][2];                               // eight splits requested before the first is used
 #pragma unroll
-        for (int s = 0; s < kSkMaxSplits; ++s)
-          if (s < p.splits) {
-            const uint32_t a = map_to_cta(at, s);
-            part[s][0] = ld_cluster_v4(a);
-            part[s][1] = ld_cluster_v4(a + 16);
-          }
+          for (int s = 0; s < 8; ++s)
+            if (s0 + s < p.splits) {
+              const uint32_t a = map_to_cta(at, s0 + s);
+              part[s][0] = ld_cluster_v4(a);
+              part[s][1] = ld_cluster_v4(a + 16);
+            }
 #pragma unroll
-        for (int s = 0; s < kSkMaxSplits; ++s)
-          if (s < p.splits) {
-            f[0] += part[s][0].x; f[1] += part[s][0].y; f[2] += part[s][0].z; f[3] += part[s][0].w;
-            f[4] += part[s][1].x; f[5] += part[s][1].y; f[6] += part[s][1].z; f[7] += part[s][1].w;
-          }
+          for (int s = 0; s < 8; ++s)
+            if (s0 + s < p.splits) {
+              f[0] += part[s][0].x; f[1] += part[s][0].y; f[2] += part[s][0].z; f[3] += part[s][0].w;
+              f[4] += part[s][1].x; f[5] += part[s][1].y; f[6] += part[s][1].z; f[7] += part[s][1].w;
+            }
+        }
       } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) f[e] += at[e];
@@ -714,6 +717,10 @@ static int launch_skinny_local(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   auto kern = gemm_skinny_local_kernel<MP, ST, GLU>;
   static SmemLimit limit;
   DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
+  if (p.splits > 8) {
+    static SmemLimit wide;
+    DPTB_CUDA_OK(wide.allow_wide_clusters(reinterpret_cast<const void*>(kern)));
+  }
   cudaLaunchAttribute at[2];
   int n = 0;
   if (p.splits > 1) {
@@ -788,6 +795,16 @@ extern "C" int dptb_gemm_skinny_swiglu(const DptbGemmArgs* a, void* stream_v) {
     return kErrUnsupported;
   return skinny_local(a, true, static_cast<cudaStream_t>(stream_v));
 }
+static int skinny_min_kb() {
+  static const int min_kb = [] {
+    const char* e = getenv("DPTB_SKINNY_MIN_KB");
+    const int v = e ? atoi(e) : 0;
+    return v > 0 ? v : 4;
+  }();
+  return min_kb;
+}
+// Splits of K that let the work units fill the SMs once, with at least `min_kb` k-blocks each.
+static int fill_splits(int tiles, int num_kb, int min_kb) { return std::max(1, std::min(sm_count() / tiles, num_kb / min_kb)); }
 static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTpOneShotArgs* os, void* stream_v) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   if (a->M <= 0 || a->N <= 0) return 0;
@@ -815,17 +832,7 @@ static int skinny_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const Dptb
   const int num_kb = (a->K + kSkBK - 1) / kSkBK;
   // Split K so that the work units fill the SMs once, with at least 4 k-blocks each.
   int splits = a->splits >= 1 ? a->splits : 1;
-  if (a->splits < 1) {
-    static const int min_kb = [] {
-      const char* e = getenv("DPTB_SKINNY_MIN_KB");
-      const int v = e ? atoi(e) : 0;
-      return v > 0 ? v : 4;
-    }();
-    const int by_sm = sm_count() / tiles;
-    const int by_k = num_kb / min_kb;
-    splits = by_sm < by_k ? by_sm : by_k;
-    if (splits < 1) splits = 1;
-  }
+  if (a->splits < 1) splits = fill_splits(tiles, num_kb, skinny_min_kb());
   if (splits > 1) {
     const bool have_ws = a->ws && a->counters && tiles <= a->num_counters &&
                          (long long)tiles * splits * mp * kSkBM * 4 <= a->ws_bytes;
@@ -882,17 +889,12 @@ static int skinny_local(const DptbGemmArgs* a, bool glu, cudaStream_t stream) {
   const int cols = glu ? kSkBM / 2 : kSkBM;
   const int tiles = (a->N + cols - 1) / cols;
   const int num_kb = (a->K + kSkBK - 1) / kSkBK;
-  // Splits of K: of 8 k-blocks and more as many as two CTAs an SM take (what counts is bytes in flight), shorter ones of 3 and more only
-  // while all CTAs stay within two thirds of the SMs (what counts is the chain; a meeting of many CTAs gets longer).  Measured (B200, 32
-  // rows, weights from HBM), splits: us: 768 x 768 1: 7.2, 2: 6.4, 4: 5.6, 8: 5.6; 2304 x 768 1: 7.7, 4: 6.4, 8: 6.7; 2048 x 2048 1:
-  // 13.6, 4: 8.1, 6: 8.2, 8: 9.2; 3072 x 2048 4: 8.6, 6: 10.1; 2048 x 5504 4: 12.7, 6: 11.4, 8: 12.2; 11008 x 2048 1: 15.4, 3: 13.9, 4: 19.2;
-  // 32768 x 2048 1: 27.9, 2: 33.8.  Partial tiles through global memory took 11.7 (2048 x 2048), 15.0 (2048 x 5504) and 15.3 us (11008 x 2048).
-  int splits = a->splits;
-  if (splits < 1) {
-    const int sms = sm_count();
-    const int loads = std::min(2 * sms / tiles, num_kb / 8), chain = std::min(2 * sms / (3 * tiles), num_kb / 3);
-    splits = std::max(loads, chain);
-  }
+  // Splits of K that fill the SMs once, of 8 k-blocks and more: where K is cut decides the bits of the result, and this is where it
+  // always was.  Shorter splits, or two CTAs an SM, are up to 1.5 us faster in places, with other bits.  Measured (B200, 32 rows, weights
+  // from HBM), splits: us: 768 x 768 1: 7.2, 2: 6.4, 4: 5.6, 8: 5.6; 2304 x 768 1: 7.7, 4: 6.4, 8: 6.7; 2048 x 2048 1: 13.6, 4: 8.1, 6:
+  // 8.2, 8: 9.2; 3072 x 2048 4: 8.6, 6: 10.1; 2048 x 5504 4: 12.7, 6: 11.4, 8: 12.2; 11008 x 2048 1: 15.4, 3: 13.9, 4: 19.2; 32768 x 2048
+  // 1: 27.9, 2: 33.8.  Partial tiles through global memory took 11.7 (2048 x 2048), 15.0 (2048 x 5504) and 15.3 us (11008 x 2048).
+  int splits = a->splits >= 1 ? a->splits : fill_splits(tiles, num_kb, std::max(8, skinny_min_kb()));
   splits = splits < 1 ? 1 : splits > kSkMaxSplits ? kSkMaxSplits : splits;
   SkinnyLocalParams p;
   p.M = a->M; p.N = a->N;
