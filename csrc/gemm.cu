@@ -66,6 +66,45 @@ gemm_simt_kernel(const TA* __restrict__ A, long long sam, long long sak, const T
     }
 }
 
+// The parts of K of a split product -> its epilogue: a warp adds 32 rows x 8 columns, a row a thread, in the order of the parts.  A
+// programmatic dependent of the product: its CTAs are there, and wait, when the last tile is done.  Bound by the parts' way through L2.
+// A sum inside the product needs CTAs that wait for one another, which is only safe when all of them are resident, or leaves it to the
+// last CTA of a tile.  B200, product and sum: 768 x 768 x 16384 26.1 us (last CTA of a tile: 34.7), 2304 x 768 x 16384 54.0 (58.7), 1024 x
+// 1024 x 6124 24.6 (30.0), 128 x 128 x 603 8.3 (9.1).
+constexpr int kFoldThreads = 128;
+__global__ void __launch_bounds__(kFoldThreads)
+gemm_fold_kernel(const GemmParams p, int bn) {
+  const int group = blockIdx.x * (kFoldThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int per_tile = 4 * (bn / 8), tile = group / per_tile, g = group - tile * per_tile;
+  const int ni = tile / p.tiles_m, mi = tile - ni * p.tiles_m;
+  const int c8 = (g >> 2) * 8;
+  const long long row = (long long)mi * kBM + (g & 3) * 32 + lane, col = (long long)ni * bn + c8;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (ni >= p.tiles_n || row >= p.M || col >= p.N) return;
+  const float* src = p.ws + (size_t)tile * p.splits * (bn * kBM) + (size_t)c8 * kBM + (g & 3) * 32 + lane;
+  float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+  for (int sp = 0; sp < p.splits; ++sp) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] += __ldcg(src + (size_t)sp * (bn * kBM) + i * kBM);
+  }
+  epilogue_row8(p, row, col, v);
+}
+static int launch_fold(const GemmParams& p, int bn, cudaStream_t stream) {
+  const long long groups = (long long)p.tiles_m * p.tiles_n * (bn / 2);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((groups + kFoldThreads / 32 - 1) / (kFoldThreads / 32)));
+  cfg.blockDim = dim3(kFoldThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return counted(1, (int)cudaLaunchKernelEx(&cfg, gemm_fold_kernel, p, bn));
+}
+
 }  // namespace dptb
 
 using namespace dptb;
@@ -133,7 +172,7 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
   if (!tc_ok) {
     p.tiles_m = p.tiles_n = p.num_kb = p.band = p.last_band = 0;
     p.by_tiles = p.by_band = p.by_rows = p.by_last_rows = make_fast_div(1);
-    p.splits = 1; p.kb_per_split = p.fold_all = 0; p.ws = nullptr; p.counters = nullptr;
+    p.splits = 1; p.kb_per_split = 0; p.ws = nullptr;
     dim3 grid((unsigned)((a->N + 63) / 64), (unsigned)((a->M + 63) / 64));
     const long long sam = a->trans_a ? 1 : a->lda, sak = a->trans_a ? a->lda : 1;
     const long long sbk = a->trans_b ? 1 : a->ldb, sbn = a->trans_b ? a->ldb : 1;
@@ -185,7 +224,7 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
         if ((ar || ag) && sp > 1) break;
         const long long units = (long long)sched_tiles * sp;
         if (sp > 1) {
-          if (!a->ws || !a->counters || tiles > a->num_counters) break;
+          if (!a->ws) break;
           if ((long long)tiles * sp * cand_bn * kBM * 4 > a->ws_bytes) break;
           if (num_kb / sp < 4) break;
         }
@@ -210,14 +249,12 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
   // (the order of the tensor-parallel forms is their own)
   order_tiles(p, tm_sched, (long long)(pair ? 2 : 1) * kBM * a->K * 2, (long long)a->N * a->K * 2, !ar && !ag);
   p.splits = splits;
-  p.fold_all = 0;
   p.kb_per_split = (num_kb + splits - 1) / splits;
   if ((long long)(splits - 1) * p.kb_per_split >= num_kb) {  // keep every split non-empty
     splits = (num_kb + p.kb_per_split - 1) / p.kb_per_split;
     p.splits = splits;
   }
   p.ws = static_cast<float*>(a->ws);
-  p.counters = a->counters;
   if (ar) {
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
     if (p.splits != 1 || tiles > ar->max_tiles || tiles * bn * kBM > ar->partial_elems) return kErrTooLarge;
@@ -305,7 +342,8 @@ static int gemm_impl(const DptbGemmArgs* a, const DptbTpArArgs* ar, const DptbTp
 
   const bool amn = a->trans_a != 0, bmn = a->trans_b == 0;
   const auto launch = amn ? (bmn ? &gemm_launch_tt : &gemm_launch_tn) : (bmn ? &gemm_launch_nn : &gemm_launch_nt);
-  return launch ? launch(pair, bn, tmA, tmB, em, p, stream) : kErrUnsupported;
+  rc = launch ? launch(pair, bn, tmA, tmB, em, p, stream) : kErrUnsupported;
+  return rc || p.splits == 1 ? rc : launch_fold(p, bn, stream);
 }
 
 extern "C" int dptb_gemm(const DptbGemmArgs* a, void* stream_v) { return gemm_impl(a, nullptr, nullptr, stream_v); }

@@ -114,13 +114,11 @@ struct GemmParams {
   // instruction caches, and a division of 20 instructions in each role cost a small product half a microsecond.
   int band, last_band;              // row tiles (pairs of them in a pair kernel) that are walked together; index of the last band
   FastDiv by_tiles, by_band, by_rows, by_last_rows;
-  // Split-K: each tile's K range is cut into `splits` work units of kb_per_split k-blocks; partial accumulators go
-  // through `ws` (fp32, [tile][split][BN][128]) and are folded in split order, so the result does not depend on arrival order:
-  // where every unit has a CTA of its own (fold_all) each of a tile's CTAs waits for the others (per-tile counter) and folds an equal
-  // share, else the last one to finish folds the tile.
-  int splits, kb_per_split, fold_all;
+  // Split-K: each tile's K range is cut into `splits` work units of kb_per_split k-blocks; partial accumulators go to `ws` (fp32,
+  // [column tile][row tile][split][BN][128]), and a kernel after this one adds them in split order and runs the epilogue (gemm.cu).  No
+  // CTA waits for another, whatever else is on the GPU.
+  int splits, kb_per_split;
   float* ws;
-  int* counters;
   TpAr ar;
   TpAg ag;
 };
@@ -906,7 +904,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_in_bar + 2 * kEpiWarps);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* epi_ctr = reinterpret_cast<int*>(tmem_slot + 2);       // arrival counter of the epilogue-warp barrier
-  volatile int* epi_last = reinterpret_cast<volatile int*>(tmem_slot + 3);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -929,7 +926,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (lane == 0) {
       *abort_flag = 0;
       *epi_ctr = 0;
-      *epi_last = 0;
     }
     // full / empty per stage, two accumulators full, two empty (the leader's is released by both CTAs), drain, epilogue inputs: a lane
     // each, and TMEM beside them (one thread after the other: 603 x 384 x 128 5.9 us, 5.7 so)
@@ -1221,7 +1217,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int smi, ni;
       tile_of_unit(p, stile, smi, ni);
       const int mi = PAIR ? smi * 2 + (int)cta_rank : (p.ar.world > 0 || p.ag.world > 0) ? tile_row_index(p, stile) : smi;
-      const int tile = PAIR ? ni * p.tiles_m + mi : stile;   // this CTA's own 128-row tile (workspace / counter index)
+      const int tile = PAIR ? ni * p.tiles_m + mi : stile;   // this CTA's own 128-row tile (index of the all-reduce protocol)
       const int m0 = mi * kBM;
       const int n0 = ni * BN;
       const uint32_t acc = local_tile & 1;
@@ -1474,8 +1470,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (lane == 0) release_acc(acc);
       } else {
         // Partial accumulator -> workspace, column-major inside the tile so that a warp writes 128 contiguous bytes.
-        float* wtile = p.ws + (size_t)tile * p.splits * (BN * kBM);
-        float* wmine = wtile + (size_t)split * (BN * kBM) + q * 32 + lane;
+        float* wmine = p.ws + ((size_t)(ni * p.tiles_m + mi) * p.splits + split) * (BN * kBM) + q * 32 + lane;
 #pragma unroll 1
         for (int c = half; c < BN / 64; c += 2) {
           if ((long long)n0 + c * 64 >= p.N) break;
@@ -1492,42 +1487,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) release_acc(acc);
-        __threadfence();
-        if (!epi_sync()) break;
-        if (ew == 0 && lane == 0) {
-          const int seen = atomicAdd(&p.counters[tile], 1) + 1;
-          int fold = seen == p.splits;
-          if (p.fold_all) {
-            fold = fold || wait_flag_ge(reinterpret_cast<const uint32_t*>(&p.counters[tile]), (uint32_t)p.splits);
-            if (!fold) *abort_flag = 1;
-          } else if (fold) {
-            p.counters[tile] = 0;  // ready for the next launch
-          }
-          *epi_last = fold;
-        }
-        if (!epi_sync()) break;
-        if (*epi_last != 0) {
-          __threadfence();
-          // Groups of 32 rows x 8 columns, a row a thread.
-          const int share = p.fold_all ? split : 0, shares = p.fold_all ? p.splits : 1;
-#pragma unroll 1
-          for (int g = share * kEpiWarps + ew; g < BN / 2; g += shares * kEpiWarps) {
-            const int rq = g & 3, c8 = (g >> 2) * 8;
-            const long long row = (long long)m0 + rq * 32 + lane, col = (long long)n0 + c8;
-            if (col >= p.N) break;
-            const float* src = wtile + (size_t)c8 * kBM + rq * 32 + lane;
-            float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 4      // (all 64 requested at once: 29.0 us instead of 26.1 at 768 x 768 x 16384)
-            for (int sp = 0; sp < p.splits; ++sp) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] += __ldcg(src + (size_t)sp * (BN * kBM) + i * kBM);
-            }
-            if (row < p.M) epilogue_row8(p, row, col, v);
-          }
-        }
-        if (!epi_sync()) break;  // epi_last may be rewritten only after every warp has read it
-        if (p.fold_all && ew == 0 && lane == 0 && atomicAdd(&p.counters[tile], 1) == 2 * p.splits - 1)
-          p.counters[tile] = 0;    // the last to leave: ready for the next launch
       }
     }
     if constexpr (!PAIR) {
@@ -1570,14 +1529,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 template <bool A_MN, bool B_MN, int BN, int STAGES>
-static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams p, cudaStream_t stream) {
+static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES>;
   auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES>;
   static SmemLimit limit;
   DPTB_CUDA_OK(limit.raise(reinterpret_cast<const void*>(kern), L::kTotal));
   const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int grid = tiles < sm_count() ? tiles : sm_count();
-  p.fold_all = p.splits > 1 && tiles <= grid;
   if (p.ar.world == 0)
     return counted(1, (int)launch_k(kern, dim3(grid), dim3(kGemmThreads), (size_t)L::kTotal, stream, tmA, tmB, NoPeerMaps{}, EpiMaps{}, p));
   kern<<<grid, kGemmThreads, L::kTotal, stream>>>(tmA, tmB, NoPeerMaps{}, EpiMaps{}, p);
@@ -1613,7 +1571,7 @@ static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
   return cached;
 }
 template <bool A_MN, bool B_MN, int BN, int STAGES, bool GLU = false>
-static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& em, GemmParams p,
+static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& em, const GemmParams& p,
                           cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES, BN / 2, 2>;
   auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true, GLU>;
@@ -1633,7 +1591,6 @@ static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   const int units = ((p.tiles_m + 1) / 2) * p.tiles_n * p.splits;
   const int clusters = units < max_clusters ? units : max_clusters;
   cfg.gridDim = dim3(2 * clusters);
-  p.fold_all = p.splits > 1 && units <= clusters;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   if (pdl_flag()) cfg.numAttrs = 2;
