@@ -14,9 +14,11 @@
 // memory and every CTA of the cluster adds an equal share of the rows, in the order of the parts, and runs the epilogue on it.
 // Deterministic, and no scratch in global memory.
 //
-// Bits below 2^-134 do not fit a bf16 part, and a value that is not finite, or rounds to infinity in bf16, makes NaN of its
-// parts.  An output that is not finite, or not zero and below 2^-100, is therefore computed once more as one run of fma over K: it
-// then is what multiply-adds make of it.
+// Not every value is the sum of three such parts: bits below 2^-133 have no bf16.  While it splits, a CTA marks the rows (of A and of
+// B) with elements that are not zero and below 2^-110.  Outputs of marked rows, outputs that are not finite (infinity, NaN and what rounds
+// to infinity in bf16 make NaN of their parts), and outputs that are not zero and below 2^-100, are computed again as multiply-adds:
+// the cluster does its tile once more with them, the outputs concerned take those sums, and all others keep the bits that they have
+// without such neighbours.
 //
 // Distance from fp64 (2-norm, relative; B200) against the multiply-add tiles: normal operands, 509 x 768 x 768 0.95e-7 (2.1e-7),
 // K = 3072 1.1e-7 (2.9e-7), 256 x 256 x 1024 1.0e-7 (1.6e-7); GELU outputs the same; operands that are all positive, where the
@@ -34,6 +36,7 @@ namespace dptb {
 constexpr int kTcBM = 128, kTcBK = kF32TcBK;
 constexpr int kTcMaxSplits = 8;                      // CTAs of a cluster
 constexpr int kTcThreads = 512;                      // 16 warps that fetch, split and add; one more issues the MMAs
+constexpr int kRedoBK = 16;
 
 template <int BN>
 struct TcF32Smem {
@@ -41,8 +44,11 @@ struct TcF32Smem {
   static constexpr int kStage = 3 * (kAPart + kBPart);
   static constexpr int kOutLd = BN + 4;                            // floats; 16-byte rows, quarter-warps on different banks
   static constexpr int kBarOff = 2 * kStage;
-  static constexpr int kTotal = kBarOff + 64 + 1024;
-  static_assert(kTcBM * kOutLd * 4 <= 2 * kStage, "the partial tile reuses the stages");
+  static constexpr int kAnyLostOff = kBarOff + 48, kRedoFlagOff = kBarOff + 52, kLostOff = kBarOff + 64;                    // a byte a row of A and of B: it has elements without three parts
+  static constexpr int kTotal = kLostOff + kTcBM + BN + 1024;
+  // The stages are used again: the partial tile, the same from multiply-adds, and their operands (kRedoBK terms, k-major).
+  static constexpr int kRedoOff = kTcBM * kOutLd * 4, kRedoAOff = 2 * kRedoOff, kRedoBOff = kRedoAOff + kRedoBK * (kTcBM + 4) * 4;
+  static_assert(kRedoBOff + kRedoBK * (BN + 4) * 4 <= 2 * kStage, "the partial tiles reuse the stages");
 };
 
 // Chunks of eight neighbouring elements of an operand's k-block, R rows (columns) of M (N) x 64 of K, one 16-byte piece of each part
@@ -76,17 +82,23 @@ struct SplitTile {
       }
     }
   }
-  __device__ __forceinline__ void split(uint8_t* parts) const {
+  // An element from 2^-110 on is the sum of its parts: its last bit is worth 2^-133 or more, the least that bf16 holds.  (The sign
+  // shifted out, less one, so that zero is the largest.)
+  static constexpr uint32_t kWhole = 2u * 0x08800000u - 1u;
+  static __device__ __forceinline__ uint32_t doubled(float x) { return 2u * __float_as_uint(x) - 1u; }
+  // `lost`: a byte for each of the R rows, set where an element is smaller and not zero.
+  __device__ __forceinline__ void split(uint8_t* parts, uint8_t* lost, int* any_lost) const {
 #pragma unroll
     for (int i = 0; i < kChunks; ++i) {
       int mn, k;
       place(i, mn, k);
       const int off = MN ? (mn >> 6) * (kTcBK * 128) + k * 128 + ((((mn >> 3) & 7) ^ (k & 7)) << 4)
                          : mn * 128 + (((k >> 3) ^ (mn & 7)) << 4);
-      uint32_t p[3][4];
+      uint32_t p[3][4], least = ~0u;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float a = v[i][2 * j], b = v[i][2 * j + 1];
+        least = __vimin3_u32(least, doubled(a), doubled(b));
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
           const uint32_t u = pack_bf16x2(a, b);
@@ -94,6 +106,16 @@ struct SplitTile {
           a -= __uint_as_float(u << 16);
           b -= __uint_as_float(u & 0xffff0000u);
         }
+      }
+      if (__builtin_expect(least < kWhole, 0)) {
+        if (MN) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (doubled(v[i][j]) < kWhole) lost[mn + j] = 1;
+        } else {
+          lost[mn] = 1;
+        }
+        *any_lost = 1;
       }
 #pragma unroll
       for (int s = 0; s < 3; ++s)
@@ -108,14 +130,92 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
   return v;
 }
 
-// One output as one run of multiply-adds over all of K.
-template <bool AMN, bool BMN>
-__device__ __noinline__ float run_of_fma(const float* A, const float* B, long long lda, long long ldb, int K, int row, int col) {
-  const float* a = A + (AMN ? row : row * lda);
-  const float* b = B + (BMN ? col : col * ldb);
-  float t = 0.0f;
-  for (int k = 0; k < K; ++k) t = fmaf(AMN ? a[k * lda] : a[k], BMN ? b[k * ldb] : b[k], t);
-  return t;
+// The tile's sums over this CTA's part of K as multiply-adds, into `out` [kTcBM][kOutLd]: by the 16 warps, kRedoBK terms at a time, the
+// next ones under way.  B200, a column of NaN in A: 509 x 768 x 768 57 us, 2048^3 883 us (14 and 156 without; multiply-add tiles alone 22 and 352).
+template <int BN, bool AMN, bool BMN>
+__device__ __noinline__ void multiply_add_tile(const GemmF32Params& p, uint8_t* smem, int m0, int n0, int k_begin, int k_end) {
+  using L = TcF32Smem<BN>;
+  constexpr int TX = BN / 4, ROWS = kTcBM * TX / kTcThreads;       // a thread: ROWS (8 or 4) rows of four columns
+  constexpr int EA = kTcBM * kRedoBK / kTcThreads, EB = BN * kRedoBK / kTcThreads;
+  float* out = reinterpret_cast<float*>(smem + L::kRedoOff);
+  float* as = reinterpret_cast<float*>(smem + L::kRedoAOff);       // [kRedoBK][kTcBM + 4]
+  float* bs = reinterpret_cast<float*>(smem + L::kRedoBOff);       // [kRedoBK][BN + 4]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;      // a warp: 4 x 8 threads
+  const int tx = warp % (TX / 8) * 8 + (lane & 7), ty = warp / (TX / 8) * 4 + (lane >> 3);
+  const float* const A = p.A;                                      // (read once: the barriers below make memory unknown)
+  const float* const B = p.B;
+  const long long lda = p.lda, ldb = p.ldb;
+  const int M = p.M, N = p.N;
+  float ra[EA], rb[EB];
+  auto at = [](int i, int rows, bool mn_major, int& mn, int& k) {
+    const int idx = threadIdx.x + i * kTcThreads;
+    mn = mn_major ? idx % rows : idx / kRedoBK;
+    k = mn_major ? idx / rows : idx % kRedoBK;
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < EA; ++i) {
+      int mn, k;
+      at(i, kTcBM, AMN, mn, k);
+      mn += m0; k += k0;
+      ra[i] = mn < M && k < k_end ? A[AMN ? (long long)k * lda + mn : (long long)mn * lda + k] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      int mn, k;
+      at(i, BN, BMN, mn, k);
+      mn += n0; k += k0;
+      rb[i] = mn < N && k < k_end ? B[BMN ? (long long)k * ldb + mn : (long long)mn * ldb + k] : 0.0f;
+    }
+  };
+  f32x2 acc[ROWS][2];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) acc[i][0] = acc[i][1] = 0ull;
+  fetch(k_begin);
+  for (int k0 = k_begin; k0 < k_end; k0 += kRedoBK) {
+    __syncwarp();
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < EA; ++i) {
+      int mn, k;
+      at(i, kTcBM, AMN, mn, k);
+      as[k * (kTcBM + 4) + mn] = ra[i];
+    }
+#pragma unroll
+    for (int i = 0; i < EB; ++i) {
+      int mn, k;
+      at(i, BN, BMN, mn, k);
+      bs[k * (BN + 4) + mn] = rb[i];
+    }
+    __syncwarp();
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+    if (k0 + kRedoBK < k_end) fetch(k0 + kRedoBK);
+    const int terms = min(kRedoBK, k_end - k0);                    // (no term beyond K: 0 times infinity)
+#pragma unroll 4
+    for (int k = 0; k < terms; ++k) {
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(bs + k * (BN + 4) + tx * 4);
+      float a[ROWS];
+#pragma unroll
+      for (int i = 0; i < ROWS; i += 4)
+        *reinterpret_cast<float4*>(&a[i]) = *reinterpret_cast<const float4*>(as + k * (kTcBM + 4) + ty * ROWS + i);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const f32x2 ai = f2_splat(a[i]);
+        acc[i][0] = f2_fma(ai, b.x, acc[i][0]);
+        acc[i][1] = f2_fma(ai, b.y, acc[i][1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    float4 v;
+    f2_unpack(acc[i][0], v.x, v.y);
+    f2_unpack(acc[i][1], v.z, v.w);
+    *reinterpret_cast<float4*>(out + (ty * ROWS + i) * L::kOutLd + tx * 4) = v;
+  }
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 // Whether a sum may stand: zero, or between 2^-100 and the largest finite value.
 __device__ __forceinline__ bool stands(float x) {
@@ -123,9 +223,57 @@ __device__ __forceinline__ bool stands(float x) {
   return u == 0 || u - 0x0d800000u < 0x7f800000u - 0x0d800000u;
 }
 
+// Sum of the parts of K of four neighbouring outputs, in the order of the parts.
+__device__ __forceinline__ float4 sum_of_parts(const float* at, int splits) {
+  if (splits == 1) return *reinterpret_cast<const float4*>(at);
+  float4 q[kTcMaxSplits];                        // all requested before the first is used
+#pragma unroll
+  for (int s = 0; s < kTcMaxSplits; ++s)
+    if (s < splits) q[s] = ld_cluster_v4(map_to_cta(at, s));
+  float4 v = q[0];
+#pragma unroll
+  for (int s = 1; s < kTcMaxSplits; ++s)
+    if (s < splits) { v.x += q[s].x; v.y += q[s].y; v.z += q[s].z; v.w += q[s].w; }
+  return v;
+}
+// This CTA's share of the tile's outputs; AGAIN: those that could not stand, as the sums of multiply-adds.
+template <int BN, bool AGAIN>
+__device__ __forceinline__ void finish_tile(const GemmF32Params& p, uint8_t* smem, int m0, int n0) {
+  using L = TcF32Smem<BN>;
+  constexpr int VECS = BN / 4;                       // 16-byte groups of a row
+  const float* out = reinterpret_cast<const float*>(smem);
+  const int rows = min(kTcBM, p.M - m0);
+  for (int e = blockIdx.z * kTcThreads + threadIdx.x; e < rows * VECS; e += p.splits * kTcThreads) {
+    const int r = e / VECS, c = e % VECS * 4;
+    const int row = m0 + r, col = n0 + c;
+    if (col >= p.N) continue;
+    float4 v = sum_of_parts(out + r * L::kOutLd + c, p.splits);
+    int todo = 15;
+    if (AGAIN || !(stands(v.x) & stands(v.y) & stands(v.z) & stands(v.w))) {
+      const int sick = (stands(v.x) ? 0 : 1) | (stands(v.y) ? 0 : 2) | (stands(v.z) ? 0 : 4) | (stands(v.w) ? 0 : 8);
+      todo = AGAIN ? sick : 15 & ~sick;
+      if (AGAIN) v = sum_of_parts(out + L::kRedoOff / 4 + r * L::kOutLd + c, p.splits);
+      else
+        for (int s = 0; s < p.splits; ++s) st_cluster_u32(map_to_cta(smem + L::kRedoFlagOff, s), 1);
+    }
+    if (!AGAIN && todo == 15 && p.vec_c && col + 3 < p.N) {
+      epilogue_f32x4(p, row, col, v);
+    } else {
+      const float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if ((todo >> j & 1) && col + j < p.N) epilogue_f32(p, row, col + j, o[j]);
+    }
+  }
+}
+template <int BN>
+__device__ __noinline__ void finish_again(const GemmF32Params& p, uint8_t* smem, int m0, int n0) {
+  finish_tile<BN, true>(p, smem, m0, n0);
+}
+
 template <int BN, bool AMN, bool BMN>
 __global__ void __launch_bounds__(kTcThreads + 32, 1)
-gemm_f32_tc_kernel(const GemmF32Params p) {
+gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
   using L = TcF32Smem<BN>;
   constexpr int COLS = BN / 4;                       // columns of a thread: four warps share a lane quarter of TMEM
   extern __shared__ uint8_t smem_raw[];
@@ -134,9 +282,13 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
   uint64_t* done = full + 2;                                           // [2]: its MMAs have completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* any_lost = reinterpret_cast<int*>(smem + L::kAnyLostOff);       // some element of this part has no three parts
+  volatile int* redo = reinterpret_cast<volatile int*>(smem + L::kRedoFlagOff);   // some output of the cluster's tile is computed again
+  uint8_t* lost = smem + L::kLostOff;                                  // [kTcBM] rows of A, [BN] of B
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < (kTcBM + BN) / 4) reinterpret_cast<uint32_t*>(lost)[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
-    *abort_flag = 0;
+    *abort_flag = *any_lost = *redo = 0;
     for (int s = 0; s < 2; ++s) {
       mbar_init(&full[s], kTcThreads / 32);
       mbar_init(&done[s], 1);
@@ -228,9 +380,9 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
       // (stage i & 1 is free: `collect` of block i - 2 has waited for the MMAs that read it)
       uint8_t* stage = smem + (i & 1) * L::kStage;
       const int k1 = k_begin + (i + 1) * kTcBK;
-      ta.split(stage);
+      ta.split(stage, lost, any_lost);
       if (i + 1 < blocks) ta.load(p.A, p.lda, m0, p.M, k1, k_end, p.vec_a);
-      tb.split(stage + 3 * L::kAPart);
+      tb.split(stage + 3 * L::kAPart, lost + kTcBM, any_lost);
       if (i + 1 < blocks) tb.load(p.B, p.ldb, n0, p.N, k1, k_end, p.vec_b);
       fence_proxy_async_smem();
       __syncwarp();
@@ -239,54 +391,38 @@ gemm_f32_tc_kernel(const GemmF32Params p) {
     }
     if (ok && blocks > 0) ok = collect(blocks - 1);
     // (every MMA has completed: the last block's are the last; in a CTA that gave up the sums are worthless anyhow)
-    float* row = out + ((warp & 3) * 32 + lane) * L::kOutLd + (warp >> 2) * COLS;
+    __syncwarp();
+    asm volatile("bar.sync 1, 512;" ::: "memory");   // (all marks are made)
+    const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * COLS;
+    if (__builtin_expect(*reinterpret_cast<volatile int*>(any_lost), 0)) {
+      // what cannot stand becomes NaN, in whatever part of K it was seen
+#pragma unroll
+      for (int j = 0; j < COLS; ++j)
+        if (lost[r] | lost[kTcBM + c0 + j]) acc[j] = __int_as_float(0x7fffffff);
+    }
+    float* row = out + r * L::kOutLd + c0;
 #pragma unroll
     for (int j = 0; j < COLS; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
   }
+  auto meet = [&] {
+    if (p.splits > 1) cluster_sync_all();
+    else __syncthreads();
+  };
   tc_fence_before_sync();
-  if (p.splits > 1) cluster_sync_all();
-  else __syncthreads();
+  meet();
   if (warp == kTcThreads / 32) {
     tc_fence_after_sync();
     tmem_dealloc<2 * BN>(tmem);
   }
 
-  constexpr int VECS = BN / 4;                       // 16-byte groups of a row
-  const int rows = min(kTcBM, p.M - m0);
-  for (int e = blockIdx.z * kTcThreads + threadIdx.x; e < rows * VECS && warp < kTcThreads / 32; e += p.splits * kTcThreads) {
-    const int r = e / VECS, c = e % VECS * 4;
-    const int row = m0 + r, col = n0 + c;
-    if (col >= p.N) continue;
-    const float* at = out + r * L::kOutLd + c;
-    float4 v;
-    if (p.splits > 1) {
-      float4 q[kTcMaxSplits];                        // all requested before the first is used
-#pragma unroll
-      for (int s = 0; s < kTcMaxSplits; ++s)
-        if (s < p.splits) q[s] = ld_cluster_v4(map_to_cta(at, s));
-      v = q[0];
-#pragma unroll
-      for (int s = 1; s < kTcMaxSplits; ++s)
-        if (s < p.splits) { v.x += q[s].x; v.y += q[s].y; v.z += q[s].z; v.w += q[s].w; }
-    } else {
-      v = *reinterpret_cast<const float4*>(at);
-    }
-    if (!(stands(v.x) & stands(v.y) & stands(v.z) & stands(v.w))) {
-      v.x = run_of_fma<AMN, BMN>(p.A, p.B, p.lda, p.ldb, p.K, row, col);
-      if (col + 1 < p.N) v.y = run_of_fma<AMN, BMN>(p.A, p.B, p.lda, p.ldb, p.K, row, col + 1);
-      if (col + 2 < p.N) v.z = run_of_fma<AMN, BMN>(p.A, p.B, p.lda, p.ldb, p.K, row, col + 2);
-      if (col + 3 < p.N) v.w = run_of_fma<AMN, BMN>(p.A, p.B, p.lda, p.ldb, p.K, row, col + 3);
-    }
-    if (p.vec_c && col + 3 < p.N) {
-      epilogue_f32x4(p, row, col, v);
-    } else {
-      const float o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (col + j < p.N) epilogue_f32(p, row, col + j, o[j]);
-    }
+  if (warp < kTcThreads / 32) finish_tile<BN, false>(p, smem, m0, n0);
+  meet();                                            // (no CTA leaves while another reads its partial tile)
+  if (*redo) {
+    if (warp < kTcThreads / 32) multiply_add_tile<BN, AMN, BMN>(p, smem, m0, n0, k_begin, k_end);
+    meet();
+    if (warp < kTcThreads / 32) finish_again<BN>(p, smem, m0, n0);
+    meet();
   }
-  if (p.splits > 1) cluster_sync_all();              // no CTA leaves while another reads its partial tile
 }
 
 template <int BN, bool AMN, bool BMN>
