@@ -408,9 +408,9 @@ static int product_f32(const DptbGemmArgs* a, cudaStream_t st) {
   }
   // Tensor cores where they are expected to be faster (1.8 us: what the model above leaves out, launch and first loads).  Not below
   // kOneRunK, and not for forced tiles.  The few rows of a short step run as programmatic dependents, where set-up and first weights stand
-  // beside the kernel ahead: 2 us less (an encoder of 6 layers, 23 rows of width 384: 285 us a pass with the multiply-add tiles, 290 with
-  // those requesting weights ahead, 270 so; alone 23 x 384 x 384 takes 7.0 us either way).  By rows and not by the launch, so that both
-  // give the same bits.
+  // beside the kernel ahead: 2 us less (an encoder of 6 layers, 23 rows of width 384: 314 us a pass with the multiply-add tiles, 296 so; 4
+  // layers of width 768, 40 rows: 387 and 293; alone 23 x 384 x 384 takes 7.0 and 7.5 us).  By rows and not by the launch, so that both give
+  // the same bits.
   if ((a->bn == 0 && a->splits < 1 && a->K >= kOneRunK) || a->bn == 1064 || a->bn == 1128) {
     int bn = a->bn - 1000, sp = a->splits < 1 ? 1 : a->splits;
     if (a->bn || f32_tc_plan(a->M, a->N, a->K, &bn, &sp) < best_cost / 1900.0 + (a->M <= 64 ? 3.8 : 1.8)) {

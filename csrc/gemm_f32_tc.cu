@@ -4,8 +4,10 @@
 // carry the other sign).  Of the nine products of two such values six are formed, h h, h m, m h, m m, h l, l h; what is left
 // out, m l + l m + l l, is below 2^-25 of the product, less than the rounding of one fp32 multiply.  Every bf16 product is exact; the
 // accumulator is not: tcgen05 truncates where an fma rounds, so a long chain drifts towards zero.  Therefore the small
-// products of a k-block go first (their truncations are 2^-8 of an ulp), h h last, and after 64 terms the block's sum leaves
-// TMEM and is added in fp32 registers, rounded to nearest: four truncated steps, not K / 16, ever meet in one accumulator.
+// products of a k-block go first (their truncations are 2^-8 of an ulp), h h last, in an accumulator for each half of the block, and after
+// 64 terms both leave TMEM and are added in fp32 registers, rounded to nearest: two truncated steps, not K / 16, ever meet in one
+// accumulator.  (With four, products of one sign, whose truncations add up, were further from fp64 than multiply-adds; 2048^3 took
+// 156 us with them, 167 so.)
 //
 // A CTA computes a 128 x BN tile over one part of K.  Its 16 warps do everything: fetch the next k-block from global memory
 // into registers, split the present one into shared memory (swizzled bf16 tiles in the operand's own orientation: K-major or
@@ -20,13 +22,13 @@
 // the cluster does its tile once more with them, the outputs concerned take those sums, and all others keep the bits that they have
 // without such neighbours.
 //
-// Distance from fp64 (2-norm, relative; B200) against the multiply-add tiles: normal operands, 509 x 768 x 768 0.95e-7 (2.1e-7),
-// K = 3072 1.1e-7 (2.9e-7), 256 x 256 x 1024 1.0e-7 (1.6e-7); GELU outputs the same; operands that are all positive, where the
-// truncations add up, 0.9e-7 (0.8e-7).
+// Distance from fp64 (2-norm, relative; B200) against the multiply-add tiles with their splits: normal operands, 509 x 768 x 768 0.81e-7
+// (2.1e-7), 509 x 768 x 3072 1.07e-7 (2.9e-7), 256 x 256 x 1024 0.85e-7 (1.6e-7); operands that are all positive, 509 x 768 x 768 0.60e-7
+// (0.81e-7), 23 x 384 x 384 0.63e-7 (0.65e-7).
 //
 // What bounds it: shared memory.  A k-block at BN = 128 writes 96 KB of parts and its MMAs read 192 KB, 2300 clocks at 128 bytes
-// each, against 1536 of the MMAs alone; fetching 64 KB ahead of the split only partly overlaps it (4000 clocks measured).  It is
-// still 2.4 times the rate of the packed multiply-adds (2048^3: 352 -> 144 us).
+// each, against 1536 of the MMAs alone; fetching 64 KB ahead of the split only partly overlaps it (4500 clocks measured).  It is
+// still 2.1 times the rate of the packed multiply-adds (2048^3: 352 -> 167 us).
 #include <atomic>
 
 #include "gemm_f32.cuh"
@@ -131,7 +133,7 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
 }
 
 // The tile's sums over this CTA's part of K as multiply-adds, into `out` [kTcBM][kOutLd]: by the 16 warps, kRedoBK terms at a time, the
-// next ones under way.  B200, a column of NaN in A: 509 x 768 x 768 57 us, 2048^3 883 us (14 and 156 without; multiply-add tiles alone 22 and 352).
+// next ones under way.  B200, a column of NaN in A: 509 x 768 x 768 57 us, 2048^3 901 us (15 and 167 without; multiply-add tiles alone 22 and 352).
 template <int BN, bool AMN, bool BMN>
 __device__ __noinline__ void multiply_add_tile(const GemmF32Params& p, uint8_t* smem, int m0, int n0, int k_begin, int k_end) {
   using L = TcF32Smem<BN>;
@@ -295,7 +297,7 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
     }
     mbar_fence_init();
   }
-  if (warp == kTcThreads / 32) tmem_alloc<2 * BN>(tmem_slot);
+  if (warp == kTcThreads / 32) tmem_alloc<4 * BN>(tmem_slot);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -332,9 +334,9 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
           for (int kk = 0; kk < kTcBK / 16; ++kk) {
             const uint32_t a = a0 + kA[c] * L::kAPart, b = b0 + kB[c] * L::kBPart;
             if (kk < steps)
-              umma_bf16(d, AMN ? make_smem_desc(a + kk * 2048, kTcBK * 128, 1024) : make_smem_desc(a + kk * 32, 16, 1024),
+              umma_bf16(c == 5 && kk >= 2 ? d + 2 * BN : d, AMN ? make_smem_desc(a + kk * 2048, kTcBK * 128, 1024) : make_smem_desc(a + kk * 32, 16, 1024),
                         BMN ? make_smem_desc(b + kk * 2048, kTcBK * 128, 1024) : make_smem_desc(b + kk * 32, 16, 1024), idesc,
-                        (c | kk) != 0);
+                        (c | kk) != 0 && !(c == 5 && kk == 2));
           }
         umma_commit(&done[i & 1]);
         issued = i + 1;
@@ -357,6 +359,7 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
     auto collect = [&](int i) -> bool {
       if (!__all_sync(0xffffffffu, mbar_wait(&done[i & 1], (i >> 1) & 1, abort_flag, kWaitTmemFullTimeout))) return false;
       tc_fence_after_sync();
+      const bool second = k_end - k_begin - i * kTcBK > 32;
 #pragma unroll
       for (int c = 0; c < COLS; c += 16) {
         uint32_t r[16];
@@ -364,6 +367,12 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
+        if (second) {
+          tmem_ld_32x16(t_row + (2 + (i & 1)) * BN + c, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
+        }
       }
       tc_fence_before_sync();
       return true;
@@ -412,7 +421,7 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32Params p) {
   meet();
   if (warp == kTcThreads / 32) {
     tc_fence_after_sync();
-    tmem_dealloc<2 * BN>(tmem);
+    tmem_dealloc<4 * BN>(tmem);
   }
 
   if (warp < kTcThreads / 32) finish_tile<BN, false>(p, smem, m0, n0);
@@ -485,10 +494,10 @@ static int resident_clusters(int splits) {
   return n;
 }
 
-// Microseconds that the best tile and split are expected to take: a wave of CTAs costs 6 us (launch, first loads, the last block's
-// sums, the parts' meeting) and each of its k-blocks 1.68 us at BN = 64, 2.03 us at BN = 128.  Measured (B200), x W^T, each with the
-// split this picks: 509 x 768 x 768 13.2 us (multiply-adds 21.9), 509 x 2304 x 768 20.1 (48.7), 509 x 3072 x 768 31.5 (60.0), 509 x 768
-// x 3072 31.7 (65.5), 1024 x 256 x 1024 13.3 (22.7), 1024 x 256 x 256 7.7 (10.4), 256 x 256 x 1024 9.8 (11.9), 2048^3 144 (352).
+// Microseconds that the best tile and split are expected to take: a wave of CTAs costs 5.5 us at BN = 64, 8.0 us at BN = 128 (launch, first
+// loads, the last block's sums, the parts' meeting) and each of its k-blocks 2.0 and 2.35 us.  Measured (B200), x W^T, each with the
+// split this picks: 509 x 768 x 768 14.8 us (multiply-adds 21.8), 509 x 2304 x 768 22.8 (48.7), 509 x 3072 x 768 36.3 (60.1), 509 x 768
+// x 3072 32.8 (65.8), 1024 x 256 x 1024 14.6 (22.7), 1024 x 256 x 256 8.3 (10.5), 256 x 256 x 1024 10.7 (11.9), 2048^3 167 (352).
 double f32_tc_plan(int M, int N, int K, int* bn, int* splits) {
   double best = 1e300;
   const int kb = (K + kTcBK - 1) / kTcBK;
@@ -499,7 +508,7 @@ double f32_tc_plan(int M, int N, int K, int* bn, int* splits) {
       if ((kb + per - 1) / per != s) continue;               // some part would be empty
       const int n = w == 64 ? resident_clusters<64>(s) : resident_clusters<128>(s);
       if (n <= 0) continue;
-      const double us = (double)((tiles + n - 1) / n) * (6.0 + per * (w == 64 ? 1.68 : 2.03));
+      const double us = (double)((tiles + n - 1) / n) * (w == 64 ? 5.5 + 2.0 * per : 8.0 + 2.35 * per);
       if (us < best) { best = us; *bn = w; *splits = s; }
     }
   }
