@@ -104,3 +104,18 @@ def test_no_further_from_fp64(Kd, kind):
     plain = error(64, 1)
     print(kind, Kd, {k: f"{v:.2e}" for k, v in got.items()}, f"{plain:.2e}")
     assert max(got.values()) <= plain
+
+
+# the tile and the parts of K that multiply-adds would take
+@pytest.mark.parametrize("M,N,Kd,bn,splits", [(509, 768, 768, 64, 6), (256, 256, 1024, 32, 16), (23, 384, 384, 32, 6),
+                                               (1024, 256, 1024, 64, 8), (200, 512, 640, 32, 10)])
+def test_one_sign_against_multiply_adds_in_parts(M, N, Kd, bn, splits):
+    def error(**kw):
+        total = 0.0
+        for seed in range(4):
+            a, w = _mk((M, Kd), 20 + seed).abs(), _mk((N, Kd), 30 + seed).abs()
+            out, ref = torch.empty(M, N, device="cuda"), a.double() @ w.double().t()
+            K.gemm(a, w, out, trans_b=True, **kw)
+            total += float((out.double() - ref).norm() / ref.norm())
+        return total
+    assert error() <= error(bn=bn, splits=splits)
