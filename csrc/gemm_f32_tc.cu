@@ -29,8 +29,7 @@
 // What bounds it: shared memory.  A k-block at BN = 128 writes 96 KB of parts and its MMAs read 192 KB, 2300 clocks at 128 bytes
 // each, against 1536 of the MMAs alone; fetching 64 KB ahead of the split only partly overlaps it (4500 clocks measured).  It is
 // still 2.1 times the rate of the packed multiply-adds (2048^3: 352 -> 167 us).
-#include <atomic>
-
+#include "common/cluster_limit.h"
 #include "gemm_f32.cuh"
 
 namespace dptb {
@@ -466,32 +465,20 @@ static cudaError_t launch_bn(const GemmF32Params& p, bool amn, bool bmn, cudaStr
 template <int BN>
 static int resident_clusters(int splits) {
   using L = TcF32Smem<BN>;
-  static std::atomic<int> known[16][kTcMaxSplits + 1];   // one more than the number; 0: not asked for yet
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16) return 0;
-  int n = known[dev][splits].load(std::memory_order_relaxed) - 1;
-  if (n < 0) {
-    auto kern = gemm_f32_tc_kernel<BN, false, false>;
-    static SmemLimit limit;
-    if (limit.raise(reinterpret_cast<const void*>(kern), L::kTotal) != cudaSuccess) return 0;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = splits;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(sm_count(), 1, splits);
-    cfg.blockDim = dim3(kTcThreads + 32);
-    cfg.dynamicSmemBytes = L::kTotal;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-    known[dev][splits].store(n + 1, std::memory_order_relaxed);
-  }
-  return n;
+  static ClusterLimit limits[kTcMaxSplits + 1];
+  static SmemLimit smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = splits;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count(), 1, splits);
+  cfg.blockDim = dim3(kTcThreads + 32);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return limits[splits].resident(reinterpret_cast<const void*>(gemm_f32_tc_kernel<BN, false, false>), smem, L::kTotal, cfg);
 }
 
 // Microseconds that the best tile and split are expected to take: a wave of CTAs costs 5.5 us at BN = 64, 8.0 us at BN = 128 (launch, first

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include "common/cluster_limit.h"
 #include "common/gemm_args.h"
 #include "common/host.h"
 #include "common/peer.cuh"
@@ -1545,31 +1546,6 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmP
 // CTA-pair variant: clusters of two CTAs, one 256-row tile per pair (see the kernel's PAIR parameter).
 constexpr int kPairStages256 = 5;   // 32 KB per stage and CTA, 64 KB of epilogue staging
 constexpr int kPairStages128 = 6;   // 24 KB per stage and CTA
-template <bool A_MN, bool B_MN, int BN, int STAGES, bool GLU>
-static int pair_clusters(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
-  // Clusters of this kernel that can be resident at once (a persistent grid must not exceed it), once per device.
-  using L = GemmSmem<BN, STAGES, BN / 2, 2>;
-  auto kern = gemm_tc_kernel<A_MN, B_MN, BN, STAGES, false, true, GLU>;
-  static SmemLimit limit;
-  static std::atomic<int> counts[64];      // one more than the number; 0: not asked for yet
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
-  int cached = counts[dev].load(std::memory_order_relaxed) - 1;
-  if (cached < 0) {
-    if (limit.raise(reinterpret_cast<const void*>(kern), L::kTotal) != cudaSuccess) return 0;
-    cfg->gridDim = dim3(2 * (sm_count() / 2));
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = 0;
-    }
-    cached = n;
-    counts[dev].store(n + 1, std::memory_order_relaxed);
-    if (getenv("DPTB_GEMM_VERBOSE")) fprintf(stderr, "gemm pair BN=%d: %d clusters of 2 CTAs can be resident\n", BN, n);
-  }
-  (void)attr;
-  return cached;
-}
 template <bool A_MN, bool B_MN, int BN, int STAGES, bool GLU = false>
 static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const EpiMaps& em, const GemmParams& p,
                           cudaStream_t stream) {
@@ -1586,7 +1562,11 @@ static int launch_tc_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int max_clusters = pair_clusters<A_MN, B_MN, BN, STAGES, GLU>(&cfg, attr);
+  // A persistent grid must not exceed what can be resident.
+  static ClusterLimit clusters_fit;
+  static SmemLimit smem;
+  cfg.gridDim = dim3(2 * (sm_count() / 2));
+  const int max_clusters = clusters_fit.resident(reinterpret_cast<const void*>(kern), smem, L::kTotal, cfg);
   if (max_clusters <= 0) return kErrUnsupported;
   const int units = ((p.tiles_m + 1) / 2) * p.tiles_n * p.splits;
   const int clusters = units < max_clusters ? units : max_clusters;
