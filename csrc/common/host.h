@@ -130,13 +130,18 @@ inline int& pdl_flag() {
 // dependent start early.  Both are no-ops in launches without the attribute / without such a dependent.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// Launches `kern`, as a programmatic dependent of the previous kernel on the stream when pdl_flag() is set.  Such a
-// kernel calls pdl_wait() before its first global access and pdl_launch_dependents() after it, never before: the kernel
-// after it must not start while the kernel two places back is still running.  Two exceptions.  The weight-streaming products
-// (gemm_skinny.cu, gemm_f32_tc.cu, the rows of gemm_f32.cu) request their second operand before the wait.  So no kernel of a chain may write what
-// a product in it takes as weight; a caller whose second operand is computed leaves the flag off around it.  And decoding attention
-// requests cache rows before this step's own (attention_decode.cu, the appending form of attention_f32.cu): they are written at least
-// two kernels before it.
+// Launches `kern`, as a programmatic dependent of the previous kernel on the stream when pdl_flag() is set.  Rules of such a chain:
+//   * Before pdl_wait() a kernel reads no global memory that a kernel of the chain writes, but for cache rows (below), and writes none.
+//     The weight-streaming products (gemm_skinny.cu, gemm_f32_tc.cu, the rows of gemm_f32.cu) request their second operand before the
+//     wait: no kernel of a chain may write what a product in it takes as weight, and a caller whose second operand is computed leaves
+//     the flag off around it.
+//   * A kernel completes only after its own wait, so that its completion means that of all kernels before it.
+//   * pdl_launch_dependents() comes after pdl_wait(): the kernel behind then starts when the one two places ahead of it is done.  The
+//     exception is the weight-streaming bf16 product, which calls it first: the kernel behind it may start while any of the last two
+//     run, which is safe for all that touch nothing but weights before their wait.
+//   * Decoding attention requests cache rows before this step's own (attention_decode.cu, the appending form of attention_f32.cu).  They
+//     are older than the step: every kernel that wrote them is at least two places ahead.  Directly behind a bf16 product it would need
+//     them older still; there the kernel that appends stands between.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   if (!pdl_flag()) {

@@ -151,7 +151,7 @@ gemm_skinny_local_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
   const int n0 = (int)(p.splits > 1 ? blockIdx.x / p.splits : blockIdx.x) * COLS;
   const int kb0 = split * p.kb_per_split;
   const int kb1 = min(p.num_kb, kb0 + p.kb_per_split);     // (never empty)
-  pdl_launch_dependents();   // the small kernel after this one waits for this grid's completion at its own top
+  pdl_launch_dependents();   // before the wait below: see launch_k (common/host.h) for what the kernel after this one may touch
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
@@ -208,6 +208,7 @@ gemm_skinny_local_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_c
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
+      pdl_wait();            // (the limit of the waits below does not count the kernels ahead)
       constexpr uint32_t idesc = make_idesc_bf16(kSkBM, MP, false, false);
       bool issued_any = false, ok = true;
       int consumed = 0;
@@ -416,6 +417,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
+      pdl_wait();            // (the limit of the waits below does not count the kernels ahead)
       constexpr uint32_t idesc = make_idesc_bf16(kSkBM, MP, false, false);
       bool issued_any = false, ok = true;
       int consumed = 0;
