@@ -273,11 +273,15 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
 //   fp32   (stacks of 4 layers) 1.05 to 1.37 times as fast at 1 to 64 rows of widths 128 to 1024, 1.18 to 1.28 at 72 to 128 rows of widths
 //          up to 768; sequences of up to 128: 1.15 at 8 x 119 rows of 384, 1.07 at 509 tokens, one each, of 768.  Longer sequences: 1.18
 //          at 256 rows of 384, but 0.91 at 509 of 768, where all rows have the same keys: CTAs that start where an SM is free crowd on the
-//          first ones.  Causal rows, the longest first, stand that better: 1.03.
-constexpr long long kChainedArea = 12 << 20, kChainedAreaF32 = 384 << 10, kChainedAreaF32Long = 128 << 10;
+//          first ones.  Causal rows, the longest first, stand that better: up to 640 rows 1.09 to 1.19 at widths 256 to 512, 1.04 at 509 and
+//          512 of 768, 1.00 at 640 of 512 and 768; from 768 rows on 1.07 to 1.10 at width 256, 0.92 to 1.06 at 384, 0.96 to 1.04 at 512, 0.88
+//          at 768.
+constexpr long long kChainedArea = 12 << 20, kChainedAreaF32 = 384 << 10, kChainedAreaF32Rows = 256 << 10, kChainedAreaF32Long = 128 << 10;
 static bool chained(const DptbStackArgs* a) {
   const long long area = (long long)a->B * a->S * a->D;
-  return area <= (a->bf16 ? kChainedArea : a->causal || a->S <= 128 ? kChainedAreaF32 : kChainedAreaF32Long);
+  if (a->bf16) return area <= kChainedArea;
+  if (a->S <= 128) return area <= kChainedAreaF32;
+  return area <= (!a->causal ? kChainedAreaF32Long : a->S <= 640 ? kChainedAreaF32 : kChainedAreaF32Rows);
 }
 extern "C" int dptb_stack_infer(const DptbStackArgs* a, const void* const* table, void* stream) {
   int& pdl = pdl_flag();
