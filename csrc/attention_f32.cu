@@ -15,7 +15,7 @@
 // Bound: shared-memory reads and fp32 issue (a thread does 4 x 4 outputs: 8 16-byte reads for 64 multiply-adds, as 32 packed
 // ones); at the sizes fp32 models run, the latency of a few tiles.  Measured as whole passes, chain per head -> these kernels:
 // training step of 6 layers x 8 sequences x 8 heads x 128 tokens x 32: 64.6 -> 8.7 ms; GPT-2 124M, prompt of 509 tokens:
-// 36.6 -> 12.4 ms, a token after it: 30.6 -> 11.9 ms (what is left there is the fp32 GEMM).
+// 36.6 -> 12.4 ms, a token after it: 30.6 -> 11.9 ms (what was left there was the fp32 GEMM and host work: 2.1 and 0.45 ms since).
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 

@@ -748,7 +748,9 @@ extern "C" int dptb_attn_fwd(const DptbAttnFwdArgs* a, void* stream) {
   // Sequences of one query tile: two heads a CTA once there are more heads than SMs; below, each has an SM to itself.  (There is no room
   // for a second V stage beside heads of 128.)  A unit is one chain of loads, scores, softmax and P V, of which the other warpgroup saw
   // nothing.  B200, one head a CTA (which then came and went) / two: 64 x 119 tokens, 12 heads of 32 31.1 / 16.6 us (26.5 with one
-  // head in the persistent form), of 64 33.6 / 19.9; 200 x 64, 8 heads of 64 58.6 / 28.2; 13 x 17, 12 heads of 32 10.3 / 7.2 us.
+  // head in the persistent form), of 64 33.6 / 19.9; 200 x 64, 8 heads of 64 58.6 / 28.2; 13 x 17, 12 heads of 32 10.3 / 7.2 us.  Longer
+  // keys as well, although a head's next tile then waits for its stage: 128 rows, 12 heads of 64, 16 x 1024 keys 31.2 / 22.7 (29.6 with one
+  // head in the persistent form), 16 x 4096 98.6 / 81.6 (90.1), 64 x 4096 288 / 239 us (258).
   const bool heads = a->Sq <= kAttnBM && (long long)a->Hq * a->B > sm_count();
   if (a->head_dim == 64 && heads) return attn_fwd_launch<64, 2, 2, 2, false, false, true>(a, st);
   if (a->head_dim == 64) return attn_fwd_launch<64, 2, 2, 2, false, false>(a, st);

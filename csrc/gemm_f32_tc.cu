@@ -125,12 +125,6 @@ struct SplitTile {
   }
 };
 
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
 // The tile's sums over this CTA's part of K as multiply-adds, into `out` [kTcBM][kOutLd]: by the 16 warps, kRedoBK terms at a time, the
 // next ones under way.  B200, a column of NaN in A: 509 x 768 x 768 57 us, 2048^3 901 us (15 and 167 without; multiply-add tiles alone 22 and 352).
 template <int BN, bool AMN, bool BMN>
@@ -214,9 +208,6 @@ __device__ __noinline__ void multiply_add_tile(const GemmF32Params& p, uint8_t* 
     f2_unpack(acc[i][1], v.z, v.w);
     *reinterpret_cast<float4*>(out + (ty * ROWS + i) * L::kOutLd + tx * 4) = v;
   }
-}
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 // Whether a sum may stand: zero, or between 2^-100 and the largest finite value.
 __device__ __forceinline__ bool stands(float x) {

@@ -114,11 +114,6 @@ struct SkinnyLocalParams {
   int num_kb, splits, kb_per_split;
   int vec_out;                       // 16-byte stores, and loads of the residual
 };
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
 
 template <int MP, int ST>
 struct SkinnySmem {
