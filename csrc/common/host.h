@@ -131,7 +131,8 @@ inline int& pdl_flag() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Launches `kern`, as a programmatic dependent of the previous kernel on the stream when pdl_flag() is set.  Rules of such a chain:
-//   * Before pdl_wait() a kernel reads no global memory that a kernel of the chain writes, but for cache rows (below), and writes none.
+//   * Before pdl_wait() a kernel reads no global memory that a kernel of the chain writes, but for cache rows (below) and the launch numbers
+//     of the collective products, whose last writer is at least two places ahead, and writes none.
 //     The weight-streaming products (gemm_skinny.cu, gemm_f32_tc.cu, the rows of gemm_f32.cu) request their second operand before the
 //     wait: no kernel of a chain may write what a product in it takes as weight, and a caller whose second operand is computed leaves
 //     the flag off around it.
