@@ -1,7 +1,8 @@
 // fp32 GEMM on the tensor cores: operands split into three bf16 parts, products summed as closely as multiply-adds sum them.
 //
 // An fp32 value is exactly h + m + l with three bf16 parts of 8 significant bits each (rounded to nearest, so m and l may
-// carry the other sign).  Of the nine products of two such values six are formed, h h, h m, m h, m m, h l, l h; what is left
+// carry the other sign; the splitting of Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For
+// Higher-Precision Computations", 2019).  Of the nine products of two such values six are formed, h h, h m, m h, m m, h l, l h; what is left
 // out, m l + l m + l l, is below 2^-25 of the product, less than the rounding of one fp32 multiply.  Every bf16 product is exact; the
 // accumulator is not: tcgen05 truncates where an fma rounds, so a long chain drifts towards zero.  Therefore the small
 // products of a k-block go first (their truncations are 2^-8 of an ulp), h h last, in an accumulator for each half of the block, and after
