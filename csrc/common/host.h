@@ -134,8 +134,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 //   * Before pdl_wait() a kernel reads no global memory that a kernel of the chain writes, but for cache rows (below) and the launch numbers
 //     of the collective products, whose last writer is at least two places ahead, and writes none.
 //     The weight-streaming products (gemm_skinny.cu, gemm_f32_tc.cu, the rows of gemm_f32.cu) request their second operand before the
-//     wait: no kernel of a chain may write what a product in it takes as weight, and a caller whose second operand is computed leaves
-//     the flag off around it.
+//     wait: no kernel of a chain, nor one right ahead of it, may write what a product in it takes as weight; a caller whose second
+//     operand is computed leaves the flag off around it.
 //   * A kernel completes only after its own wait, so that its completion means that of all kernels before it.
 //   * pdl_launch_dependents() comes after pdl_wait(): the kernel behind then starts when the one two places ahead of it is done.  The
 //     exception is the weight-streaming bf16 product, which calls it first: the kernel behind it may start while any of the last two

@@ -214,7 +214,15 @@ static int stack_launch(const DptbStackArgs* a, const void* const* table, void* 
       DPTB_STACK_OK(norm(cur, t[kN1G], t[kN1B], ws + l.norm, a->eps, a->rms));
       x = ws + l.norm;
     }
-    DPTB_STACK_OK(linear(x, D, t[kQkvW], t[kQkvB], ldqkv, qkv, 0, nullptr));
+    {
+      // A product that opens the chain is launched as usual: the kernel ahead of it is not of the chain and may have written its weight.
+      int& pdl = pdl_flag();
+      const int chain = pdl;
+      if (x == a->x) pdl = 0;
+      const int rc = linear(x, D, t[kQkvW], t[kQkvB], ldqkv, qkv, 0, nullptr);
+      pdl = chain;
+      if (rc) return rc;
+    }
     // Few fp32 rows that are not turned: the attention appends them to the caches itself.
     int attended = kErrUnsupported;
     if (a->cached && !a->bf16 && a->rotary_dim == 0 && a->past + a->S <= a->cap)
